@@ -6,6 +6,7 @@
 
 #define MDB_GEMM_MAX_SEG 3
 #define MDB_GEMM_MAX_PEERS 8
+#define MDB_GEMM_ROWS_MAX 8        // most rows of the few-row kernel (gemm_rows.cu)
 
 enum {
   MDB_ACT_NONE = 0,
@@ -83,6 +84,11 @@ typedef struct MdbGemmArgs {
 } MdbGemmArgs;
 
 int mdb_gemm_launch(const MdbGemmArgs* args, cudaStream_t stream);
+
+// few-row form (gemm_rows.cu): whether it computes what the arguments ask for, and its launch. mdb_gemm_launch takes it by
+// itself when the tile width is left to it (bn == 0).
+int mdb_gemm_rows_ok(const MdbGemmArgs* args);
+int mdb_gemm_rows(const MdbGemmArgs* args, cudaStream_t stream);
 
 // number of two-CTA clusters of the 256 x 256 GEMM kernel the current device can hold at once (74 on a B200 whose 148 SMs
 // all have their TPC partner, fewer otherwise)

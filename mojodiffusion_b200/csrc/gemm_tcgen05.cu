@@ -1131,6 +1131,8 @@ static int pair_mode() {
 extern "C" int mdb_gemm_launch(const MdbGemmArgs* a, cudaStream_t stream) {
   using namespace mdb;
   if (a->M <= 0 || a->N <= 0 || a->num_seg < 1 || a->num_seg > MDB_GEMM_MAX_SEG) return -2;
+  // up to eight rows the weights are streamed by all SMs instead of by the N / 128 CTAs that own a tile
+  if (a->M <= MDB_GEMM_ROWS_MAX && mdb_gemm_rows_ok(a)) return mdb_gemm_rows(a, stream);
   const int eb = a->kind == 1 ? 1 : 2;
   const int k_elems = BK_BYTES / eb;
   const bool paired = a->pair_offset > 0;

@@ -1,0 +1,46 @@
+"""Kernel variants chosen by size: each against the plain fp32 statement of the op at the sizes where it can go wrong."""
+import math
+
+import pytest
+import torch
+
+import mojodiffusion_b200.ops as O
+from mojodiffusion_b200.ops import native, reference as ref
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+if torch.cuda.is_available():
+    native.load(True)
+
+
+def _rand(*shape, scale=1.0, seed=0, dtype=torch.bfloat16):
+    g = torch.Generator(device="cpu").manual_seed(seed)
+    return (torch.randn(*shape, generator=g) * scale).to(dtype).to(DEV)
+
+
+def _close(out, want, name, rel=0.0):
+    """bf16 outputs of fp32 sums: half a bf16 ulp (2^-9) of the value, plus ``rel`` of the largest value for what the
+    inputs of the last rounding may differ by."""
+    native.check_status(out)
+    assert out.shape == want.shape and torch.isfinite(out.float()).all(), name
+    w = want.float()
+    err = (out.float() - w).abs()
+    bound = w.abs() * 2.0 ** -8 + (rel + 1e-5) * float(w.abs().max())
+    assert bool((err <= bound).all()), f"{name}: {float((err - bound).max())} over the bound, largest {float(w.abs().max())}"
+
+
+# rows 1 / 2 / 4 / 8 are the kernel's own sizes, 3 / 5 / 7 repeat a row, 9 is the first on the tiled kernel; K = 8 leaves 31 lanes
+# idle, 264 / 520 end in a partial step; N = 1000 ends inside a block, 9480 takes four columns per warp on 148 SMs
+@pytest.mark.parametrize("M", [1, 2, 3, 4, 5, 7, 8, 9])
+@pytest.mark.parametrize("N,K", [(56, 8), (1000, 264), (5000, 520), (9480, 3072)])
+def test_few_row_gemm(M, N, K):
+    x, w = _rand(M, K, seed=M), _rand(N, K, scale=1 / math.sqrt(K), seed=2)
+    bias, gate, res = _rand(N, seed=7), _rand(M, N, seed=8), _rand(M, N, seed=9)
+    _close(O.linear(x, w), x.float() @ w.float().t(), f"plain {M}x{N}x{K}")
+    for act in ("gelu_tanh", "silu", "gelu"):
+        out = O.linear(x, w, bias, act=act, residual=res, gate=gate, rows_per_group=1)
+        _close(out, ref.linear(x, w, bias, act, res, gate, 1, out_dtype=torch.float32), f"{act} {M}x{N}x{K}", rel=1e-4)
+    x2, w2 = _rand(M, 24, seed=3), _rand(N, 24, scale=0.1, seed=4)
+    _close(O.linear(x, w, extra=[(x2, w2)]), x.float() @ w.float().t() + x2.float() @ w2.float().t(), f"two segments {M}x{N}x{K}")
+    if N % 16 == 0:
+        _close(O.linear_glu(x, w, bias, "silu"), ref.linear_glu(x.float(), w.float(), bias.float(), "silu"), f"paired {M}x{N}x{K}", rel=1e-4)
