@@ -725,12 +725,13 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p) {
 // own 128 rows of A and its own 128 rows of B per K block (32 KB instead of the 48 KB a lone 128 x 256 CTA needs for
 // the same MMA time), so the shared-memory fill rate, which bounds the one-CTA kernel on DiT shapes, drops by a third
 // and the ring is 6 stages deep. The even CTA issues the MMAs for both; each CTA reads its own 128 x 256 fp32
-// accumulator from its own TMEM and runs the same fused epilogue. bf16 operands, any operand majors, paired (GLU)
-// mode, routed / staged-reduce epilogues; no fused gather, convolution or split-K (those stay on the one-CTA kernel).
+// accumulator from its own TMEM and runs the same fused epilogue. bf16 operands of any majors or K-major fp8 (KIND 1),
+// paired (GLU) mode, routed / staged-reduce epilogues; no fused gather, convolution or split-K (the gather and split-K stay
+// on the one-CTA kernel, 3 x 3 convolutions have a pair kernel of their own below).
 // ---------------------------------------------------------------------------------
 constexpr int PAIR_THREADS = 192;  // warps: 0 TMA, 1 UMMA issue (leader only), 2-5 epilogue
 
-template <int STAGES, bool A_MN, bool B_MN>
+template <int STAGES, bool A_MN, bool B_MN, int KIND>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
 gemm_tcgen05_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p) {
   constexpr int BN = 256;               // accumulator columns per CTA (the whole tile width)
@@ -740,7 +741,8 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmParams
   constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   constexpr int TMEM_COLS = 2 * BN;
   constexpr int KSTEPS = 4;
-  constexpr int K_ELEMS = 64;
+  constexpr int K_ELEMS = (KIND == 0) ? 64 : 128;
+  static_assert(!(KIND == 1 && (A_MN || B_MN)), "fp8 operands are K-major only");
 
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t full_bar[STAGES];    // used in the leader: both CTAs' loads of a stage have landed
@@ -863,7 +865,8 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmParams
   } else if (warp == 1) {
     // ------------------------------- UMMA issuer (leader CTA only) --------------
     if (leader) {
-      constexpr uint32_t idesc = make_idesc(1, UMMA_BF16, UMMA_BF16, A_MN ? 1u : 0u, B_MN ? 1u : 0u, 2 * BM, BN);
+      constexpr uint32_t idesc = (KIND == 0) ? make_idesc(1, UMMA_BF16, UMMA_BF16, A_MN ? 1u : 0u, B_MN ? 1u : 0u, 2 * BM, BN)
+                                             : make_idesc(1, UMMA_E4M3, UMMA_E4M3, 0u, 0u, 2 * BM, BN);
       int stage = 0;
       uint32_t phase = 0;
       int it = 0;
@@ -907,7 +910,10 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmParams
             for (int k = 0; k < KSTEPS; ++k) {
               const uint64_t a_k = da + static_cast<uint64_t>(A_MN ? (k * 2048) >> 4 : (k * 32) >> 4);
               const uint64_t b_k = db + static_cast<uint64_t>(B_MN ? (k * 2048) >> 4 : (k * 32) >> 4);
-              umma_f16_ss_pair(d_tmem, a_k, b_k, idesc, (kb | k) != 0 ? 1u : 0u);
+              if (KIND == 0)
+                umma_f16_ss_pair(d_tmem, a_k, b_k, idesc, (kb | k) != 0 ? 1u : 0u);
+              else
+                umma_f8_ss_pair(d_tmem, a_k, b_k, idesc, (kb | k) != 0 ? 1u : 0u);
             }
             umma_commit_pair(&empty_bar[stage], 3);   // the stage is free in both CTAs once these MMAs have read it
             if (kb == total_kb - 1) umma_commit_pair(&tfull_bar[acc], 3);
@@ -1063,14 +1069,11 @@ static int launch_variant(const GemmMaps& maps, const GemmParams& p, int num_sms
 // How many CTA pairs the device can hold at once: an SM whose partner in the same TPC is not available cannot host half
 // a pair, so the number differs from chip to chip. A persistent grid must not exceed it (surplus pairs would run their
 // whole tile list after the others finish) and the tile-shape choice uses it as the pair kernel's width.
-template <int STAGES, bool A_MN, bool B_MN>
-__global__ void gemm_tcgen05_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p);
-
 static int pair_capacity(int num_sms) {
   static int cached = 0;
   if (cached > 0) return cached;
   constexpr int SMEM = 6 * (BM * BK_BYTES + 128 * BK_BYTES) + 4 * 8192 + 1024;
-  auto kern = gemm_tcgen05_pair_kernel<6, false, false>;
+  auto kern = gemm_tcgen05_pair_kernel<6, false, false, 0>;
   int n = 0;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) == cudaSuccess) {
     cudaLaunchConfig_t cfg;
@@ -1093,11 +1096,11 @@ static int pair_capacity(int num_sms) {
   return cached;
 }
 
-template <int STAGES, bool A_MN, bool B_MN>
+template <int STAGES, bool A_MN, bool B_MN, int KIND>
 static int launch_pair_variant(const GemmMaps& maps, const GemmParams& p, int num_sms, cudaStream_t stream) {
   constexpr int SMEM = STAGES * (BM * BK_BYTES + 128 * BK_BYTES) + 4 * 8192 + 1024;   // ring + epilogue staging (4 warps x 8 KB)
   static_assert(SMEM <= 227 * 1024, "pipeline exceeds the shared memory of an SM");
-  auto kern = gemm_tcgen05_pair_kernel<STAGES, A_MN, B_MN>;
+  auto kern = gemm_tcgen05_pair_kernel<STAGES, A_MN, B_MN, KIND>;
   static bool attr_done = false;
   if (!attr_done) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
@@ -1139,7 +1142,7 @@ extern "C" int mdb_gemm_launch(const MdbGemmArgs* a, cudaStream_t stream) {
   const int sms = a->num_sms > 0 ? a->num_sms : device_sm_count();
   int bn = a->bn;
   // bn == 512 asks for the CTA-pair kernel (256 x 256 tile over two SMs); it shares the tensor maps of the 128 x 256 tile
-  const bool pair_ok = a->kind == 0 && a->conv_taps <= 0 && a->gather_world <= 1 && a->split_k <= 1;
+  const bool pair_ok = a->conv_taps <= 0 && a->gather_world <= 1 && a->split_k <= 1;
   bool use_pair = bn == 512 && pair_ok;
   if (bn == 512) bn = 256;
   const bool auto_tile = bn != 64 && bn != 128 && bn != 256;
@@ -1287,10 +1290,11 @@ extern "C" int mdb_gemm_launch(const MdbGemmArgs* a, cudaStream_t stream) {
 
 #define MDB_LAUNCH(BN_, ST_, AMN_, BMN_, KIND_) return launch_variant<BN_, ST_, AMN_, BMN_, KIND_>(maps, p, sms, stream)
   if (use_pair) {
-    if (!a->a_mn && !a->b_mn) return launch_pair_variant<6, false, false>(maps, p, sms, stream);
-    if (!a->a_mn && a->b_mn) return launch_pair_variant<6, false, true>(maps, p, sms, stream);
-    if (a->a_mn && a->b_mn) return launch_pair_variant<6, true, true>(maps, p, sms, stream);
-    return launch_pair_variant<6, true, false>(maps, p, sms, stream);
+    if (a->kind == 1) return a->a_mn || a->b_mn ? -4 : launch_pair_variant<6, false, false, 1>(maps, p, sms, stream);
+    if (!a->a_mn && !a->b_mn) return launch_pair_variant<6, false, false, 0>(maps, p, sms, stream);
+    if (!a->a_mn && a->b_mn) return launch_pair_variant<6, false, true, 0>(maps, p, sms, stream);
+    if (a->a_mn && a->b_mn) return launch_pair_variant<6, true, true, 0>(maps, p, sms, stream);
+    return launch_pair_variant<6, true, false, 0>(maps, p, sms, stream);
   }
   if (a->kind == 1) {
     if (a->a_mn || a->b_mn) return -4;

@@ -44,3 +44,15 @@ def test_few_row_gemm(M, N, K):
     _close(O.linear(x, w, extra=[(x2, w2)]), x.float() @ w.float().t() + x2.float() @ w2.float().t(), f"two segments {M}x{N}x{K}")
     if N % 16 == 0:
         _close(O.linear_glu(x, w, bias, "silu"), ref.linear_glu(x.float(), w.float(), bias.float(), "silu"), f"paired {M}x{N}x{K}", rel=1e-4)
+
+
+# fp8 on the CTA-pair kernel (M > 128 rows and enough tiles), with both scales in its epilogue; ragged in M, N and K
+@pytest.mark.parametrize("M,N,K", [(129, 256, 128), (300, 4096, 400), (2737, 1032, 4096)])
+def test_fp8_pair_gemm(M, N, K):
+    x, w = _rand(M, K, seed=1), _rand(N, K, scale=1 / math.sqrt(K), seed=2)
+    wq, ws = O.fp8_quant_rows(w)
+    xq, xs = O.fp8_quant_rows(x)
+    bias, res = _rand(N, seed=7), _rand(M, N, seed=9)
+    want = (xq.float() @ wq.float().t()) * xs[:, None] * ws[None] + bias.float()
+    _close(O.fp8_linear(x, wq, ws, bias), want, f"fp8 {M}x{N}x{K}", rel=1e-4)
+    _close(O.fp8_linear(x, wq, ws, bias, residual=res), want + res.float(), f"fp8 residual {M}x{N}x{K}", rel=1e-4)
