@@ -203,9 +203,10 @@ Tensor gemm(std::vector<Tensor> As, std::vector<Tensor> Bs, const optional<Tenso
   return out;
 }
 
-// x: NHWC bf16 [N, H, W, Cin]; w: [Cout, KH, KW, Cin] bf16; stride 1, "same"-style padding (pad_h, pad_w).
-Tensor conv2d_nhwc(const Tensor& x, const Tensor& w, const optional<Tensor>& bias, int64_t pad_h, int64_t pad_w,
-                   int64_t act, const optional<Tensor>& residual) {
+// x: NHWC bf16 [N, H, W, Cin]; w: [Cout, KH, KW, Cin] bf16; "same"-style padding (pad_h, pad_w). stride 2 (3 x 3 only) keeps
+// the output pixels offset, offset + 2, ... of the stride-1 result.
+Tensor conv2d_nhwc_strided(const Tensor& x, const Tensor& w, const optional<Tensor>& bias, int64_t pad_h, int64_t pad_w,
+                   int64_t act, const optional<Tensor>& residual, int64_t stride, int64_t offset) {
   TORCH_CHECK(x.is_cuda() && x.dim() == 4 && w.dim() == 4 && x.is_contiguous() && w.is_contiguous(), "conv2d_nhwc: NHWC");
   TORCH_CHECK(x.scalar_type() == at::kBFloat16 && w.scalar_type() == at::kBFloat16, "conv2d_nhwc: bf16");
   c10::cuda::CUDAGuard guard(x.device());
@@ -213,10 +214,14 @@ Tensor conv2d_nhwc(const Tensor& x, const Tensor& w, const optional<Tensor>& bia
   const int64_t Cout = w.size(0), KH = w.size(1), KW = w.size(2);
   TORCH_CHECK(w.size(3) == Cin && Cin % 64 == 0 && Cout % 8 == 0, "conv2d_nhwc: Cin multiple of 64, Cout multiple of 8");
   TORCH_CHECK(2 * pad_h == KH - 1 && 2 * pad_w == KW - 1, "conv2d_nhwc: output size must equal input size");
-  Tensor out = at::empty({N, H, W, Cout}, x.options());
+  TORCH_CHECK(stride == 1 || (stride == 2 && KH == 3 && KW == 3 && (offset == 0 || offset == 1)),
+              "conv2d_nhwc: stride 1, or 2 with a 3 x 3 filter and offset 0 / 1");
+  const int64_t Ho = stride == 2 ? (H - offset + 1) / 2 : H, Wo = stride == 2 ? (W - offset + 1) / 2 : W;
+  Tensor out = at::empty({N, Ho, Wo, Cout}, x.options());
+  if (stride == 2 && out.numel() == 0 && x.numel() > 0) return out;     // one row or column, sampled from the second on
   MdbGemmArgs g;
   memset(&g, 0, sizeof(g));
-  g.M = (int)(N * H * W); g.N = (int)Cout; g.num_seg = 1;
+  g.M = (int)(N * Ho * Wo); g.N = (int)Cout; g.num_seg = 1;
   g.K[0] = KH * KW * Cin;
   g.A[0] = x.data_ptr(); g.B[0] = w.data_ptr();
   g.lda[0] = Cin; g.ldb[0] = KH * KW * Cin;
@@ -230,11 +235,17 @@ Tensor conv2d_nhwc(const Tensor& x, const Tensor& w, const optional<Tensor>& bia
     g.ld_res = (int)Cout;
   }
   g.conv_taps = (int)(KH * KW); g.conv_kw = (int)KW; g.conv_pad_h = (int)pad_h; g.conv_pad_w = (int)pad_w;
-  g.conv_n = (int)N; g.conv_h = (int)H; g.conv_w = (int)W; g.conv_cin = (int)Cin;
+  g.conv_n = (int)N; g.conv_h = (int)Ho; g.conv_w = (int)Wo; g.conv_cin = (int)Cin;
+  g.conv_stride = (int)stride; g.conv_offset = (int)offset; g.conv_in_h = (int)H; g.conv_in_w = (int)W;
   g.num_sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
   g.status = status_ptr(x);
   check_rc(mdb_gemm_launch(&g, cur_stream()), "conv2d_nhwc");
   return out;
+}
+
+Tensor conv2d_nhwc(const Tensor& x, const Tensor& w, const optional<Tensor>& bias, int64_t pad_h, int64_t pad_w,
+                   int64_t act, const optional<Tensor>& residual) {
+  return conv2d_nhwc_strided(x, w, bias, pad_h, pad_w, act, residual, 1, 0);
 }
 
 Tensor group_norm_nhwc(const Tensor& x, const optional<Tensor>& w, const optional<Tensor>& b, int64_t groups, double eps,
@@ -977,6 +988,7 @@ TORCH_LIBRARY(mdb200, m) {
   m.def("gemm_pair_capacity", &gemm_pair_capacity);
   m.def("gemm", &gemm);
   m.def("conv2d_nhwc", &conv2d_nhwc);
+  m.def("conv2d_nhwc_strided", &conv2d_nhwc_strided);
   m.def("group_norm_nhwc", &group_norm_nhwc);
   m.def("group_norm_nhwc_bwd", &group_norm_nhwc_bwd);
   m.def("image_filter", &image_filter);

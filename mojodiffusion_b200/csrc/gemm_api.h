@@ -76,11 +76,14 @@ typedef struct MdbGemmArgs {
   // Split-K (split_k > 1): the K range is cut into split_k parts, each a separate work item of the persistent grid; the
   // parts are added (red.global.add) into the fp32 output, which the caller has zeroed. One K segment, no epilogue math.
   int split_k;
-  // Implicit-GEMM convolution, stride 1 (conv_taps = KH*KW > 0): A[0] is an NHWC bf16 image [conv_n, conv_h, conv_w,
+  // Implicit-GEMM convolution (conv_taps = KH*KW > 0): A[0] is an NHWC bf16 image [conv_n, conv_h, conv_w,
   // conv_cin] (conv_cin a multiple of 64), B[0] the filter [N, KH, KW, conv_cin] as a [N, KH*KW*conv_cin] matrix,
   // M = conv_n*conv_h*conv_w output pixels (output NHWC [.., N] with ld_out). Padding pad_h / pad_w is implicit:
   // taps that fall outside the image read zeros through the tensor map's out-of-range fill.
   int conv_taps, conv_kw, conv_pad_h, conv_pad_w, conv_n, conv_h, conv_w, conv_cin;
+  // conv_stride 2 (3 x 3 only): conv_h / conv_w are the OUTPUT size, the image is conv_in_h x conv_in_w, and output pixel i is
+  // centred on input pixel 2 i + conv_offset. 0 or 1: stride 1, image and output of one size.
+  int conv_stride, conv_offset, conv_in_h, conv_in_w;
 } MdbGemmArgs;
 
 int mdb_gemm_launch(const MdbGemmArgs* args, cudaStream_t stream);
@@ -97,6 +100,9 @@ int mdb_gemm_pair_capacity(int num_sms);
 // rank-N tiled tensor map (extents/strides innermost first; strides_bytes[0] ignored)
 int mdb_make_tmap(void* out_map, const void* ptr, int elem_bytes, int rank, const int64_t* extents,
                   const int64_t* strides_bytes, const int* box, int swizzle128);
+// the same with element strides (box extents count traversed elements: ceil(box / stride) of them land in shared memory)
+int mdb_make_tmap_strided(void* out_map, const void* ptr, int elem_bytes, int rank, const int64_t* extents,
+                          const int64_t* strides_bytes, const int* box, const int* elem_strides, int swizzle128);
 
 #ifdef __cplusplus
 }

@@ -32,6 +32,8 @@ constexpr int GATHER_STAGES = 2;          // shared-memory stages of the fused a
 constexpr int GATHER_PIECE = 16384;       // bytes per stage
 constexpr int NUM_THREADS = 224;  // warps: 0 TMA, 1 UMMA issue, 2-5 epilogue, 6 peer gather (all-gather fused GEMM)
 constexpr int CONV_TW = 16, CONV_TH = 8;  // conv mode: one M tile = 8 rows x 16 columns of output pixels
+// time of one 64-wide K step of a convolution's pair tile over that of a lone CTA's 128 x 256 tile (726 cycles)
+constexpr double CONV_PAIR_COST_256 = 0.72, CONV_PAIR_COST_128 = 0.42, CONV_PAIR_COST_64 = 0.26;
 
 struct alignas(64) GemmMaps {
   CUtensorMap a[MDB_GEMM_MAX_SEG];
@@ -82,6 +84,7 @@ struct GemmParams {
   // implicit-GEMM convolution (conv_taps > 0): A is an NHWC image read through a 4-D tensor map, one 16x8 pixel
   // patch per M tile, one shifted box per filter tap; rows outside the image are skipped by the epilogue
   int conv_taps, conv_kw, conv_pad_h, conv_pad_w, conv_h, conv_w, conv_tiles_h, conv_tiles_w, conv_cblocks, conv_tiles_m;
+  int conv_stride, conv_off_h, conv_off_w;   // pair kernel: input pixel of tap (kh, kw) = output pixel * stride + (kh, kw) + off
 };
 
 __device__ __forceinline__ float apply_act_rt(int act, float x) {
@@ -990,6 +993,215 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmParams
 }
 
 // ---------------------------------------------------------------------------------
+// 3 x 3 convolution on CTA pairs: each CTA owns one 8 x 16 patch of output pixels (128 rows of the implicit GEMM), the pair
+// shares a BN-channel tile of the filter (BN / 2 rows staged by each CTA, cta_group::2).
+// What bounds the convolution is how many bytes an SM takes in per multiply-add: about 64 bytes per clock, while a lone CTA
+// re-reads its 16 KB patch for every filter tap next to 32 KB of filter (726 cycles per 128 x 256 x 64 step where the tensor
+// core needs 512). Here the three vertical taps of a column kw share one staged box of 10 x 16 pixels: tap kh starts
+// kh * 16 rows (2048 bytes, a whole number of swizzle atoms) into it. Per three taps a CTA takes in 20 KB of pixels instead
+// of 48, and half of the filter tile. With HALO = false (stride 2, where neighbouring taps share no pixels) every tap
+// loads its own box through a tensor map with element strides.
+// Measured (B200): FLUX autoencoder decode to 1024 x 1024 23.3 -> 17.5 ms, encode of three 488 x 712 images 13.0 -> 8.8 ms.
+// Work order: channel tiles of one pair of patches are neighbours in the tile order, so the patch comes from L2 once.
+// ---------------------------------------------------------------------------------
+template <int BN, bool HALO>
+struct ConvPairShape {
+  static constexpr int BNH = BN / 2;                                   // filter rows staged by one CTA
+  static constexpr int TAPS = HALO ? 3 : 1;                            // taps served by one staged pixel box
+  static constexpr int A_BYTES = (HALO ? CONV_TH + 2 : CONV_TH) * CONV_TW * BK_BYTES;
+  static constexpr int B_BYTES = BNH * BK_BYTES;
+  static constexpr int A_STAGES = HALO ? (BN == 256 ? 3 : 5) : (BN == 256 ? 5 : 8);
+  static constexpr int B_STAGES = BN == 256 ? 7 : 8;
+  static constexpr int SMEM = A_STAGES * A_BYTES + B_STAGES * B_BYTES + 4 * 8192 + 1024;
+  static_assert(SMEM <= 227 * 1024, "pipeline exceeds the shared memory of an SM");
+  static_assert(B_BYTES % 1024 == 0 && A_BYTES % 1024 == 0, "stages start on swizzle atoms");
+};
+
+template <int BN, bool HALO>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
+conv_tcgen05_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p) {
+  using S = ConvPairShape<BN, HALO>;
+  constexpr int TMEM_COLS = 2 * BN;
+  constexpr int KSTEPS = 4, K_ELEMS = 64;
+
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ uint64_t a_full[S::A_STAGES], b_full[S::B_STAGES];      // used in the leader: both CTAs' loads have landed
+  __shared__ uint64_t a_empty[S::A_STAGES], b_empty[S::B_STAGES];    // in each CTA: the MMAs that read the stage are done
+  __shared__ uint64_t tfull_bar[2], tempty_bar[2];
+  __shared__ uint32_t tmem_base_s;
+  __shared__ int abort_s;
+
+  const uint32_t raw_addr = smem_u32(smem_raw);
+  uint8_t* smem_a = smem_raw + (((raw_addr + 1023u) & ~1023u) - raw_addr);
+  uint8_t* smem_b = smem_a + S::A_STAGES * S::A_BYTES;
+  uint8_t* smem_st = smem_b + S::B_STAGES * S::B_BYTES;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_ctarank();
+  const bool leader = rank == 0;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < S::A_STAGES; ++s) { mbar_init(&a_full[s], 1); mbar_init(&a_empty[s], 1); }
+    for (int s = 0; s < S::B_STAGES; ++s) { mbar_init(&b_full[s], 1); mbar_init(&b_empty[s], 1); }
+    for (int s = 0; s < 2; ++s) { mbar_init(&tfull_bar[s], 1); mbar_init(&tempty_bar[s], 8); }
+    abort_s = 0;
+    fence_mbar_init();
+  }
+  if (warp == 1) {
+    tmem_alloc_pair(&tmem_base_s, TMEM_COLS);
+    tmem_relinquish_pair();
+  }
+  if (warp == 0 && lane == 0) {
+    tma_prefetch_desc(&maps.a[0]);
+    tma_prefetch_desc(&maps.b[0]);
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_arrive();   // the peer's barriers exist before anything is sent to them
+  cluster_wait();
+  tc_fence_after();
+  const uint32_t tmem_base = tmem_base_s;
+  const uint32_t peer_abort = mapa_shared(smem_u32(&abort_s), rank ^ 1u);
+
+  const int tiles_n = (p.N + BN - 1) / BN;
+  const int num_tiles = ((p.conv_tiles_m + 1) / 2) * tiles_n;
+  const int cluster_id = blockIdx.x >> 1, num_clusters = gridDim.x >> 1;
+  const int groups = p.conv_cblocks * 3 * (3 / S::TAPS);              // pixel boxes per tile
+
+  if (warp == 0) {
+    // ------------------------------- TMA producer (both CTAs) -------------------
+    int as = 0, bs = 0;
+    uint32_t aph = 0, bph = 0;
+    bool ok = true, issued = false;
+    for (int tile = cluster_id; ok && tile < num_tiles; tile += num_clusters) {
+      const int n0 = (tile % tiles_n) * BN + static_cast<int>(rank) * S::BNH;
+      const int mt = (tile / tiles_n) * 2 + static_cast<int>(rank);   // past the last patch: image index past the batch, zeros
+      const int tw = mt % p.conv_tiles_w, th = (mt / p.conv_tiles_w) % p.conv_tiles_h;
+      const int img = mt / (p.conv_tiles_w * p.conv_tiles_h);
+      for (int g = 0; ok && g < groups; ++g) {
+        // pixel box g: (channel block, kw) with all kh, or (channel block, kw, kh)
+        const int cb = g / (groups / p.conv_cblocks), r = g - cb * (groups / p.conv_cblocks);
+        const int kw = HALO ? r : r / 3, kh0 = HALO ? 0 : r - (r / 3) * 3;
+        if (!__all_sync(0xffffffffu, mbar_wait(&a_empty[as], aph ^ 1u, &abort_s))) {
+          if (lane == 0) { report_status(p.status, STATUS_TIMEOUT, 31, as); st_shared_cluster_u32(peer_abort, 1u); }
+          ok = false;
+          break;
+        }
+        if (elect_one()) {
+          if (leader) mbar_expect_tx(&a_full[as], 2 * S::A_BYTES);
+          tma_load_4d_pair(smem_a + as * S::A_BYTES, &maps.a[0], mapa_shared(smem_u32(&a_full[as]), 0u), cb * K_ELEMS,
+                           tw * CONV_TW * p.conv_stride + kw + p.conv_off_w, th * CONV_TH * p.conv_stride + kh0 + p.conv_off_h, img);
+        }
+        __syncwarp();
+        issued = true;
+        if (++as == S::A_STAGES) { as = 0; aph ^= 1u; }
+        for (int t = 0; t < S::TAPS; ++t) {
+          const int k0 = (((kh0 + t) * 3 + kw) * p.conv_cblocks + cb) * K_ELEMS;
+          if (!__all_sync(0xffffffffu, mbar_wait(&b_empty[bs], bph ^ 1u, &abort_s))) {
+            if (lane == 0) { report_status(p.status, STATUS_TIMEOUT, 32, bs); st_shared_cluster_u32(peer_abort, 1u); }
+            ok = false;
+            break;
+          }
+          if (elect_one()) {
+            if (leader) mbar_expect_tx(&b_full[bs], 2 * S::B_BYTES);
+            tma_load_2d_pair(smem_b + bs * S::B_BYTES, &maps.b[0], mapa_shared(smem_u32(&b_full[bs]), 0u), k0, n0);
+          }
+          __syncwarp();
+          if (++bs == S::B_STAGES) { bs = 0; bph ^= 1u; }
+        }
+      }
+    }
+    if (!ok && issued) {
+      // abandoned: give the copies already in flight time to land before the CTA goes away (bounded)
+      const uint64_t t0 = globaltimer_ns();
+      while (globaltimer_ns() - t0 < 2000000ull) {
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    // ------------------------------- UMMA issuer (leader CTA only) --------------
+    if (leader) {
+      constexpr uint32_t idesc = make_idesc(1, UMMA_BF16, UMMA_BF16, 0u, 0u, 2 * BM, BN);
+      int as = 0, bs = 0, it = 0;
+      uint32_t aph = 0, bph = 0;
+      bool ok = true;
+      for (int tile = cluster_id; ok && tile < num_tiles; tile += num_clusters, ++it) {
+        const int acc = it & 1;
+        if (!__all_sync(0xffffffffu, mbar_wait(&tempty_bar[acc], ((it >> 1) & 1) ^ 1u, &abort_s))) {
+          if (lane == 0) { report_status(p.status, STATUS_TIMEOUT, 33, acc); st_shared_cluster_u32(peer_abort, 1u); }
+          break;
+        }
+        tc_fence_after();
+        const uint32_t d_tmem = tmem_base + acc * BN;
+        for (int g = 0; ok && g < groups; ++g) {
+          bool got = mbar_wait(&a_full[as], aph, &abort_s);
+          for (int t = 0; t < S::TAPS; ++t) {
+            if (!__all_sync(0xffffffffu, got && mbar_wait(&b_full[bs], bph, &abort_s))) {
+              if (lane == 0) { report_status(p.status, STATUS_TIMEOUT, 34, bs); st_shared_cluster_u32(peer_abort, 1u); }
+              ok = false;
+              break;
+            }
+            tc_fence_after();
+            const uint64_t da = make_desc_kmajor_sw128(smem_u32(smem_a + as * S::A_BYTES) + t * (CONV_TW * BK_BYTES));
+            const uint64_t db = make_desc_kmajor_sw128(smem_u32(smem_b + bs * S::B_BYTES));
+            if (elect_one()) {
+#pragma unroll
+              for (int k = 0; k < KSTEPS; ++k)
+                umma_f16_ss_pair(d_tmem, da + static_cast<uint64_t>((k * 32) >> 4), db + static_cast<uint64_t>((k * 32) >> 4), idesc,
+                                 (g | t | k) != 0 ? 1u : 0u);
+              umma_commit_pair(&b_empty[bs], 3);       // the stages are free in both CTAs once these MMAs have read them
+              if (t == S::TAPS - 1) {
+                umma_commit_pair(&a_empty[as], 3);
+                if (g == groups - 1) umma_commit_pair(&tfull_bar[acc], 3);
+              }
+            }
+            __syncwarp();
+            if (++bs == S::B_STAGES) { bs = 0; bph ^= 1u; }
+          }
+          if (++as == S::A_STAGES) { as = 0; aph ^= 1u; }
+        }
+      }
+    }
+    __syncwarp();
+  } else {
+    // ------------------------------- epilogue (4 warps per CTA) -----------------
+    const int quad = warp & 3;
+    bool aligned = ((reinterpret_cast<uintptr_t>(p.out) | static_cast<uintptr_t>(static_cast<size_t>(p.ld_out) * 2)) & 15) == 0;
+    if (p.bias) aligned = aligned && (reinterpret_cast<uintptr_t>(p.bias) & 15) == 0;
+    if (p.residual) aligned = aligned && ((reinterpret_cast<uintptr_t>(p.residual) | static_cast<uintptr_t>(static_cast<size_t>(p.ld_res) * 2)) & 15) == 0;
+    int it = 0;
+    for (int tile = cluster_id; tile < num_tiles; tile += num_clusters, ++it) {
+      const int acc = it & 1;
+      const bool got = __all_sync(0xffffffffu, mbar_wait(&tfull_bar[acc], (it >> 1) & 1, &abort_s));
+      if (!got) {
+        if (lane == 0) { report_status(p.status, STATUS_TIMEOUT, 35, acc); st_shared_cluster_u32(peer_abort, 1u); }
+        break;
+      }
+      tc_fence_after();
+      const int mt = (tile / tiles_n) * 2 + static_cast<int>(rank);
+      const int tw = mt % p.conv_tiles_w, th = (mt / p.conv_tiles_w) % p.conv_tiles_h;
+      const int img = mt / (p.conv_tiles_w * p.conv_tiles_h);
+      const int r = quad * 32 + lane;
+      const int oh = th * CONV_TH + r / CONV_TW, ow = tw * CONV_TW + r % CONV_TW;
+      const int row = (mt < p.conv_tiles_m && oh < p.conv_h && ow < p.conv_w) ? (img * p.conv_h + oh) * p.conv_w + ow : p.M;   // p.M = skipped
+      epilogue_tile(p, tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + acc * BN, 0, row, (tile % tiles_n) * BN, BN, false, aligned,
+                    smem_st + quad * 8192, lane);
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&tempty_bar[acc]), 0u));
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  cluster_arrive();   // neither CTA frees TMEM or leaves while its partner may still signal or read
+  cluster_wait();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc_pair(tmem_base, TMEM_COLS);
+  }
+}
+
+// ---------------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------------
 static PFN_cuTensorMapEncodeTiled_v12000 get_encode_fn() {
@@ -1009,6 +1221,10 @@ static PFN_cuTensorMapEncodeTiled_v12000 get_encode_fn() {
 
 extern "C" int mdb_make_tmap(void* out_map, const void* ptr, int elem_bytes, int rank, const int64_t* extents,
                              const int64_t* strides_bytes, const int* box, int swizzle128) {
+  return mdb_make_tmap_strided(out_map, ptr, elem_bytes, rank, extents, strides_bytes, box, nullptr, swizzle128);
+}
+extern "C" int mdb_make_tmap_strided(void* out_map, const void* ptr, int elem_bytes, int rank, const int64_t* extents,
+                                     const int64_t* strides_bytes, const int* box, const int* elem_strides, int swizzle128) {
   auto fn = mdb::get_encode_fn();
   if (!fn) return -1;
   // The encode call is a driver-API entry and needs a current context. A thread that has not made a runtime call yet
@@ -1025,7 +1241,7 @@ extern "C" int mdb_make_tmap(void* out_map, const void* ptr, int elem_bytes, int
   for (int i = 0; i < rank; ++i) {
     gdim[i] = static_cast<cuuint64_t>(extents[i]);
     bdim[i] = static_cast<cuuint32_t>(box[i]);
-    estr[i] = 1;
+    estr[i] = elem_strides ? static_cast<cuuint32_t>(elem_strides[i]) : 1;
     if (i > 0) gstr[i - 1] = static_cast<cuuint64_t>(strides_bytes[i]);
   }
   CUtensorMapDataType dt = elem_bytes == 1   ? CU_TENSOR_MAP_DATA_TYPE_UINT8
@@ -1117,6 +1333,19 @@ static int launch_pair_variant(const GemmMaps& maps, const GemmParams& p, int nu
   return static_cast<int>(cudaGetLastError());
 }
 
+template <int BN, bool HALO>
+static int launch_conv_pair(const GemmMaps& maps, const GemmParams& p, int num_sms, cudaStream_t stream) {
+  constexpr int SMEM = ConvPairShape<BN, HALO>::SMEM;
+  auto kern = conv_tcgen05_pair_kernel<BN, HALO>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+  if (e != cudaSuccess) return static_cast<int>(e);
+  const long long tiles = static_cast<long long>((p.conv_tiles_m + 1) / 2) * ((p.N + BN - 1) / BN);
+  const int max_pairs = pair_capacity(num_sms);
+  const int clusters = static_cast<int>(tiles < max_pairs ? tiles : max_pairs);
+  kern<<<2 * clusters, PAIR_THREADS, SMEM, stream>>>(maps, p);
+  return static_cast<int>(cudaGetLastError());
+}
+
 }  // namespace mdb
 
 extern "C" int mdb_gemm_pair_capacity(int num_sms) { return mdb::pair_capacity(num_sms > 0 ? num_sms : mdb::device_sm_count()); }
@@ -1134,6 +1363,13 @@ static int pair_mode() {
 extern "C" int mdb_gemm_launch(const MdbGemmArgs* a, cudaStream_t stream) {
   using namespace mdb;
   if (a->M <= 0 || a->N <= 0 || a->num_seg < 1 || a->num_seg > MDB_GEMM_MAX_SEG) return -2;
+  MdbGemmArgs flat;
+  if (a->conv_taps == 1 && a->conv_stride <= 1 && a->conv_pad_h == 0 && a->conv_pad_w == 0 && a->kind == 0) {
+    // a 1 x 1 convolution is a plain GEMM over the pixels: no patches that hang over the image's edge, all tilings open
+    flat = *a;
+    flat.conv_taps = 0;
+    a = &flat;
+  }
   // up to eight rows the weights are streamed by all SMs instead of by the N / 128 CTAs that own a tile
   if (a->M <= MDB_GEMM_ROWS_MAX && mdb_gemm_rows_ok(a)) return mdb_gemm_rows(a, stream);
   const int eb = a->kind == 1 ? 1 : 2;
@@ -1177,6 +1413,30 @@ extern "C" int mdb_gemm_launch(const MdbGemmArgs* a, cudaStream_t stream) {
       bn = 256;
     }
   }
+  // 3 x 3 convolutions: pair tiles of 2 patches x 256 / 128 / 64 channels or lone CTAs, by waves x time per 64-wide K step
+  int conv_pair = 0;
+  const int conv_stride = a->conv_taps > 0 && a->conv_stride > 1 ? a->conv_stride : 1;
+  if (a->conv_taps > 0) {
+    const int patches = a->conv_n * ((a->conv_h + CONV_TH - 1) / CONV_TH) * ((a->conv_w + CONV_TW - 1) / CONV_TW);
+    const bool ok3 = a->conv_taps == 9 && a->conv_kw == 3 && auto_tile && a->kind == 0 && !a->out_fp32 && pair_mode() != 0;
+    if (conv_stride > 1 && (conv_stride != 2 || a->conv_taps != 9 || a->conv_kw != 3)) return -11;
+    if (ok3 || conv_stride > 1) {
+      const int pairs = pair_capacity(sms);
+      const long long pt = (patches + 1) / 2;
+      const int w_of[3] = {256, 128, 64};
+      const double c_of[3] = {CONV_PAIR_COST_256, CONV_PAIR_COST_128, CONV_PAIR_COST_64};
+      double best = 1e30;
+      for (int i = 0; i < 3; ++i) {
+        const long long t = pt * ((a->N + w_of[i] - 1) / w_of[i]);
+        const double c = static_cast<double>((t + pairs - 1) / pairs) * c_of[i];
+        if (c < best) { best = c; conv_pair = w_of[i]; }
+      }
+      const long long t1 = static_cast<long long>(patches) * ((a->N + bn - 1) / bn);
+      const double lone = static_cast<double>((t1 + sms - 1) / sms) * (bn == 256 ? 1.0 : bn == 128 ? 0.55 : 0.32);
+      if (conv_stride == 1 && lone < best) conv_pair = 0;
+      if (conv_pair) bn = conv_pair;       // box of the filter's tensor map: bn / 2 rows
+    }
+  }
   GemmMaps maps;
   GemmParams p;
   memset(&p, 0, sizeof(p));
@@ -1195,10 +1455,13 @@ extern "C" int mdb_gemm_launch(const MdbGemmArgs* a, cudaStream_t stream) {
       if (a->conv_taps > 0) {
         if (s != 0 || a->a_mn || a->kind != 0) return -6;
         const int64_t cin = a->conv_cin;
-        int64_t e4[4] = {cin, a->conv_w, a->conv_h, a->conv_n};
-        int64_t s4[4] = {eb, cin * eb, a->conv_w * cin * eb, static_cast<int64_t>(a->conv_h) * a->conv_w * cin * eb};
-        int b4[4] = {k_elems, CONV_TW, CONV_TH, 1};
-        int r = mdb_make_tmap(&maps.a[s], a->A[s], eb, 4, e4, s4, b4, 1);
+        const int64_t in_h = conv_stride > 1 ? a->conv_in_h : a->conv_h, in_w = conv_stride > 1 ? a->conv_in_w : a->conv_w;
+        int64_t e4[4] = {cin, in_w, in_h, a->conv_n};
+        int64_t s4[4] = {eb, cin * eb, in_w * cin * eb, in_h * in_w * cin * eb};
+        // stride 1 on the pair kernel: two more rows of pixels serve all three vertical taps; stride 2: every second pixel
+        int b4[4] = {k_elems, CONV_TW * conv_stride, conv_pair && conv_stride == 1 ? CONV_TH + 2 : CONV_TH * conv_stride, 1};
+        int st4[4] = {1, conv_stride, conv_stride, 1};
+        int r = mdb_make_tmap_strided(&maps.a[s], a->A[s], eb, 4, e4, s4, b4, st4, 1);
         if (r) return 1000 + r;
         p.kblocks[s] = a->conv_taps * static_cast<int>((cin + k_elems - 1) / k_elems);
       } else
@@ -1274,6 +1537,9 @@ extern "C" int mdb_gemm_launch(const MdbGemmArgs* a, cudaStream_t stream) {
     if (a->conv_cin % k_elems) return -7;
     p.conv_kw = a->conv_kw; p.conv_pad_h = a->conv_pad_h; p.conv_pad_w = a->conv_pad_w;
     p.conv_h = a->conv_h; p.conv_w = a->conv_w;
+    p.conv_stride = conv_stride;
+    p.conv_off_h = (conv_stride > 1 ? a->conv_offset : 0) - a->conv_pad_h;
+    p.conv_off_w = (conv_stride > 1 ? a->conv_offset : 0) - a->conv_pad_w;
     p.conv_tiles_h = (a->conv_h + CONV_TH - 1) / CONV_TH;
     p.conv_tiles_w = (a->conv_w + CONV_TW - 1) / CONV_TW;
     p.conv_cblocks = a->conv_cin / k_elems;
@@ -1288,6 +1554,16 @@ extern "C" int mdb_gemm_launch(const MdbGemmArgs* a, cudaStream_t stream) {
   p.route_row_offset_b = a->route_row_offset_b;
   if (a->route_owner_cols > 0 && ((a->route_owner_cols % 32) || (p.route_part_cols % a->route_owner_cols))) return -5;
 
+  if (conv_pair && conv_stride == 1) {
+    if (conv_pair == 256) return launch_conv_pair<256, true>(maps, p, sms, stream);
+    if (conv_pair == 128) return launch_conv_pair<128, true>(maps, p, sms, stream);
+    return launch_conv_pair<64, true>(maps, p, sms, stream);
+  }
+  if (conv_pair) {
+    if (conv_pair == 256) return launch_conv_pair<256, false>(maps, p, sms, stream);
+    if (conv_pair == 128) return launch_conv_pair<128, false>(maps, p, sms, stream);
+    return launch_conv_pair<64, false>(maps, p, sms, stream);
+  }
 #define MDB_LAUNCH(BN_, ST_, AMN_, BMN_, KIND_) return launch_variant<BN_, ST_, AMN_, BMN_, KIND_>(maps, p, sms, stream)
   if (use_pair) {
     if (a->kind == 1) return a->a_mn || a->b_mn ? -4 : launch_pair_variant<6, false, false, 1>(maps, p, sms, stream);

@@ -1,8 +1,8 @@
 """Image ops in NHWC: convolution (implicit GEMM on tcgen05 through 4-D TMA boxes), GroupNorm+SiLU, nearest 2x
 upsample, 2x2 average pool, pixel (un)shuffle and latent patchify helpers.
 
-The native convolution covers stride 1 with "same" padding and Cin a multiple of 64 (the bulk of every VAE / UNet);
-other shapes (the 3- or 4-channel stem, strided down-sampling convs) use ``torch.nn.functional.conv2d``.
+The native convolution covers "same" padding at any channel count, with stride 1 or (3 x 3 filters) stride 2; other paddings
+use ``torch.nn.functional.conv2d``.
 Reference: serenitymojo/ops/conv.mojo:46-209 (im2col + GEMM), serenitymojo/models/vae/decoder2d.mojo:150-362,
 serenitymojo/ops/pixelshuffle.mojo:144-770, serenitymojo/ops/layout.mojo:44-383.
 """
@@ -43,18 +43,23 @@ def _pad_channels(t, mult: int, dim: int = -1):
     return torch.cat((t, t.new_zeros(shape)), dim=dim)
 
 
-def _conv_same_native(x, w_ohwi, bias, pad, act=None, residual=None):
-    """Stride-1 "same" convolution on the implicit-GEMM kernel for ANY channel counts: input channels are zero-padded to a
-    multiple of 64 (the 3- / 4-channel stems), output channels to a multiple of 8 (the 3- / 4-channel heads)."""
+def _conv_same_native(x, w_ohwi, bias, pad, act=None, residual=None, stride: int = 1, offset: int = 0):
+    """"Same" convolution on the implicit-GEMM kernel for ANY channel counts: input channels are zero-padded to a multiple of
+    64 (the 3- / 4-channel stems), output channels to a multiple of 8 (the 3- / 4-channel heads). A stride keeps the pixels
+    ``offset::stride`` of the result; stride 2 of a 3 x 3 filter computes only those, other strides sample."""
+    if stride > 1 and not (stride == 2 and tuple(w_ohwi.shape[1:3]) == (3, 3) and offset in (0, 1)):
+        return _conv_same_native(x, w_ohwi, bias, pad, act, residual)[:, offset::stride, offset::stride].contiguous()
     Cout, Cin = w_ohwi.shape[0], w_ohwi.shape[3]
     xp, wp = _pad_channels(x, 64), _pad_channels(w_ohwi, 64)
     if Cout % 8:
         wp = _pad_channels(wp, 8, 0)
         bias = _pad_channels(bias, 8, 0) if bias is not None else None
         residual = _pad_channels(residual, 8) if residual is not None else None
-    y = native.ops().conv2d_nhwc(xp.contiguous(), wp.contiguous(), bias, pad[0], pad[1], act_code(act),
-                                 residual.contiguous() if residual is not None else None)
-    return y[..., :Cout] if Cout % 8 else y
+    y = native.ops().conv2d_nhwc_strided(xp.contiguous(), wp.contiguous(), bias, pad[0], pad[1], act_code(act),
+                                         residual.contiguous() if residual is not None else None, stride, offset)
+    if Cout % 8:
+        y = y[..., :Cout] if stride == 1 else y[..., :Cout].contiguous()
+    return y
 
 
 def _rotated(w_ohwi):
@@ -95,9 +100,7 @@ class _Conv2dFn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, w, bias, stride, pad, offset):
-        y = _conv_same_native(x, w, bias, pad)
-        if stride > 1:
-            y = y[:, offset::stride, offset::stride].contiguous()
+        y = _conv_same_native(x, w, bias, pad, stride=stride, offset=offset)
         ctx.save_for_backward(x, w)
         ctx.meta = (stride, pad, offset, bias is not None)
         return y
@@ -139,7 +142,7 @@ def conv2d_nhwc(x, w_ohwi, bias=None, stride: int = 1, padding=1, act=None, resi
             return native.ops().conv2d_nhwc(x.contiguous(), w_ohwi.contiguous(), bias, pad[0], pad[1], act_code(act), res)
         return _conv_same_native(x, w_ohwi, bias, pad, act, residual)
     if ok and stride == 2:
-        y = _conv_same_native(x, w_ohwi, bias, pad, act)[:, offset::2, offset::2].contiguous()
+        y = _conv_same_native(x, w_ohwi, bias, pad, act, stride=2, offset=offset)
         return y + residual if residual is not None else y
     if offset:
         raise NotImplementedError("offset sampling is defined for the native path")

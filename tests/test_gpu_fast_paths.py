@@ -19,8 +19,8 @@ def _rand(*shape, scale=1.0, seed=0, dtype=torch.bfloat16):
 
 
 def _close(out, want, name, rel=0.0):
-    """bf16 outputs of fp32 sums: half a bf16 ulp (2^-9) of the value, plus ``rel`` of the largest value for what the
-    inputs of the last rounding may differ by."""
+    """bf16 outputs of fp32 sums: the rounding of the value (2^-9, doubled because two sums may round to neighbours), plus ``rel``
+    of the largest value for what the inputs of that rounding may differ by."""
     native.check_status(out)
     assert out.shape == want.shape and torch.isfinite(out.float()).all(), name
     w = want.float()
@@ -56,3 +56,33 @@ def test_fp8_pair_gemm(M, N, K):
     want = (xq.float() @ wq.float().t()) * xs[:, None] * ws[None] + bias.float()
     _close(O.fp8_linear(x, wq, ws, bias), want, f"fp8 {M}x{N}x{K}", rel=1e-4)
     _close(O.fp8_linear(x, wq, ws, bias, residual=res), want + res.float(), f"fp8 residual {M}x{N}x{K}", rel=1e-4)
+
+
+def _conv_ref(x, w, bias, stride=1, offset=0):
+    y = torch.nn.functional.conv2d(x.permute(0, 3, 1, 2).float(), w.permute(0, 3, 1, 2).float(), bias.float(), padding=1).permute(0, 2, 3, 1)
+    return y[:, offset::stride, offset::stride]
+
+
+def test_conv3x3_many_tiles_per_cluster():
+    from mojodiffusion_b200.ops import conv as C
+    for Cin, Cout in ((64, 128), (128, 256)):                  # several tiles per persistent cluster: every ring wraps
+        x, w = _rand(1, 200, 333, Cin, seed=1), _rand(Cout, 3, 3, Cin, scale=1 / math.sqrt(9 * Cin), seed=2)
+        with torch.no_grad():
+            _close(C.conv2d_nhwc(x, w, _rand(Cout, seed=3)), _conv_ref(x, w, _rand(Cout, seed=3)), f"{Cin} -> {Cout}")
+
+
+# one patch (its partner of the pair lies past the batch), images smaller than a patch, ragged edges both ways, an odd number of
+# patches; 8 / 64, 128 / 320 and 512 / 648 output channels take the 64-, 128- and 256-wide tiles on some of the sizes
+@pytest.mark.parametrize("N,H,W", [(1, 8, 16), (1, 5, 3), (2, 17, 33), (1, 9, 47), (3, 31, 50)])
+@pytest.mark.parametrize("Cin,Cout", [(64, 8), (128, 64), (64, 128), (192, 320), (128, 512), (64, 648)])
+def test_conv3x3_pair_tiles(N, H, W, Cin, Cout):
+    from mojodiffusion_b200.ops import conv as C
+    x, w = _rand(N, H, W, Cin, seed=1), _rand(Cout, 3, 3, Cin, scale=1 / math.sqrt(9 * Cin), seed=2)
+    bias, res = _rand(Cout, seed=3), _rand(N, H, W, Cout, seed=4)
+    with torch.no_grad():
+        _close(C.conv2d_nhwc(x, w, bias), _conv_ref(x, w, bias), "plain")
+        _close(C.conv2d_nhwc(x, w, bias, act="silu", residual=res), torch.nn.functional.silu(_conv_ref(x, w, bias)) + res.float(), "act + residual", rel=1e-4)
+        for off in (0, 1):
+            _close(C.conv2d_nhwc(x, w, bias, stride=2, offset=off), _conv_ref(x, w, bias, 2, off), f"stride 2 from {off}")
+        w1 = _rand(Cout, 1, 1, Cin, scale=1 / math.sqrt(Cin), seed=5)
+        _close(C.conv2d_nhwc(x, w1, bias, padding=0), x.float() @ w1[:, 0, 0].float().t() + bias.float(), "1 x 1")
