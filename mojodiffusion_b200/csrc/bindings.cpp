@@ -680,6 +680,115 @@ Tensor randn(std::vector<int64_t> shape, int64_t seed, int64_t offset, bool bf16
            "randn");
   return out;
 }
+// ------------------------------------------------------------------------------------------
+// decoder stack: one layer on R rows (R = batch while decoding, batch x prompt in the prefill)
+// ------------------------------------------------------------------------------------------
+const Tensor& llm_matrix(const Tensor& w, int64_t N, int64_t K, const Tensor& x, const char* what) {
+  TORCH_CHECK(w.device() == x.device() && w.scalar_type() == at::kBFloat16 && w.is_contiguous() && w.dim() == 2 && w.size(0) == N && w.size(1) == K,
+              "decoder layer: ", what, " must be a contiguous bf16 [", N, ", ", K, "]");
+  return w;
+}
+const void* llm_vector(const optional<Tensor>& v, int64_t n, const Tensor& x, const char* what) {
+  if (!v.has_value() || !v->defined()) return nullptr;
+  TORCH_CHECK(v->device() == x.device() && v->scalar_type() == at::kBFloat16 && v->is_contiguous() && v->numel() == n, "decoder layer: ", what);
+  return v->data_ptr();
+}
+// out = x w^T + bias in bf16 rows of ld_out elements
+void llm_project(const Tensor& x, const Tensor& w, const void* bias, void* out, int64_t ld_out) {
+  MdbGemmArgs g;
+  memset(&g, 0, sizeof(g));
+  g.M = (int)x.size(0); g.N = (int)w.size(0); g.num_seg = 1;
+  g.K[0] = x.size(1); g.A[0] = x.data_ptr(); g.B[0] = w.data_ptr(); g.lda[0] = x.size(1); g.ldb[0] = x.size(1);
+  g.alpha = 1.f; g.rows_per_group = 1; g.bias = bias;
+  g.out = out; g.ld_out = (int)ld_out;
+  g.num_sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
+  g.status = status_ptr(x);
+  check_rc(mdb_gemm_launch(&g, cur_stream()), "decoder projection");
+}
+void llm_check_rows(const Tensor& x) {
+  TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kBFloat16 && x.dim() == 2 && x.is_contiguous() && x.size(0) > 0 && x.size(1) % 8 == 0 &&
+                  x.size(1) <= 16384, "decoder layer: x [rows, hidden] contiguous bf16, hidden a multiple of 8 up to 16384");
+}
+// x += y (when given), returns RMSNorm(x) * w
+Tensor llm_add_rms(Tensor& x, const optional<Tensor>& y, const void* w, double eps) {
+  TORCH_CHECK(w != nullptr, "decoder layer: norm weight");
+  const void* py = nullptr;
+  if (y.has_value() && y->defined()) {
+    TORCH_CHECK(y->device() == x.device() && y->scalar_type() == at::kBFloat16 && y->is_contiguous() && y->sizes() == x.sizes(), "decoder layer: y");
+    py = y->data_ptr();
+  }
+  Tensor h = at::empty_like(x);
+  check_rc(mdb_add_rms_rows(x.data_ptr(), py, w, h.data_ptr(), x.size(0), (int)x.size(1), (float)eps, cur_stream()), "decoder norm");
+  return h;
+}
+// x: the residual stream, updated in place by y (the previous layer's MLP output, none for the first layer). RMSNorm, q | k | v
+// projections, per-head norm + rotation, cache append at positions pos .. pos + S - 1. Returns the packed rows
+// [B * S, (H + 2 Hkv) * Dh] (q final in place).
+Tensor llm_qkv(Tensor x, const optional<Tensor>& y, const Tensor& ln, const Tensor& wq, const Tensor& wk, const Tensor& wv, const optional<Tensor>& bq,
+               const optional<Tensor>& bk, const optional<Tensor>& bv, const optional<Tensor>& qn, const optional<Tensor>& kn, const Tensor& cosv,
+               const Tensor& sinv, Tensor k_cache, Tensor v_cache, int64_t S, int64_t pos, double eps) {
+  llm_check_rows(x);
+  c10::cuda::CUDAGuard guard(x.device());
+  TORCH_CHECK(k_cache.dim() == 4 && k_cache.is_contiguous() && v_cache.is_contiguous() && v_cache.sizes() == k_cache.sizes() &&
+                  k_cache.scalar_type() == at::kBFloat16 && v_cache.scalar_type() == at::kBFloat16 && k_cache.device() == x.device() &&
+                  v_cache.device() == x.device(), "decoder layer: caches [B, Hkv, T, Dh] bf16");
+  const int64_t R = x.size(0), D = x.size(1), Hkv = k_cache.size(1), T = k_cache.size(2), Dh = k_cache.size(3);
+  TORCH_CHECK(S > 0 && R % S == 0 && R / S == k_cache.size(0) && Dh > 0 && wq.size(0) % Dh == 0 && Dh % 8 == 0 && Dh <= 256 && pos >= 0 && pos + S <= T,
+              "decoder layer: rows / heads / positions do not match the cache");
+  const int64_t H = wq.size(0) / Dh, W = (H + 2 * Hkv) * Dh;
+  for (const Tensor* t : {&cosv, &sinv})
+    TORCH_CHECK(t->device() == x.device() && t->scalar_type() == at::kBFloat16 && t->is_contiguous() && t->dim() == 2 && t->size(1) == Dh &&
+                    t->size(0) >= pos + S, "decoder layer: rotary tables [positions, Dh] bf16");
+  Tensor h = llm_add_rms(x, y, llm_vector(ln, D, x, "norm weight"), eps);
+  Tensor qkv = at::empty({R, W}, x.options());
+  char* base = static_cast<char*>(qkv.data_ptr());
+  llm_project(h, llm_matrix(wq, H * Dh, D, x, "q weight"), llm_vector(bq, H * Dh, x, "q bias"), base, W);
+  llm_project(h, llm_matrix(wk, Hkv * Dh, D, x, "k weight"), llm_vector(bk, Hkv * Dh, x, "k bias"), base + 2 * H * Dh, W);
+  llm_project(h, llm_matrix(wv, Hkv * Dh, D, x, "v weight"), llm_vector(bv, Hkv * Dh, x, "v bias"), base + 2 * (H + Hkv) * Dh, W);
+  check_rc(mdb_qkv_rope_cache(base, llm_vector(qn, Dh, x, "q norm"), llm_vector(kn, Dh, x, "k norm"), cosv.data_ptr(), sinv.data_ptr(),
+                              k_cache.data_ptr(), v_cache.data_ptr(), R, (int)S, (int)H, (int)Hkv, (int)Dh, (int)T, (int)pos, (float)eps, cur_stream()),
+           "qkv_rope_cache");
+  return qkv;
+}
+// x += attention output projection (in place), returns the gated MLP of the new x (not yet added): attn [R, H * Dh]
+Tensor llm_out_mlp(Tensor x, const Tensor& attn, const Tensor& wo, const Tensor& ln, const Tensor& wg, const Tensor& wu, const Tensor& wd, double eps) {
+  llm_check_rows(x);
+  c10::cuda::CUDAGuard guard(x.device());
+  const int64_t R = x.size(0), D = x.size(1), F = wg.size(0), A = attn.size(-1);
+  TORCH_CHECK(attn.device() == x.device() && attn.scalar_type() == at::kBFloat16 && attn.is_contiguous() && attn.dim() == 2 && attn.size(0) == R &&
+                  A % 8 == 0 && F % 8 == 0, "decoder layer: attention rows");
+  Tensor y = at::empty_like(x);
+  llm_project(attn, llm_matrix(wo, D, A, x, "output weight"), nullptr, y.data_ptr(), D);
+  Tensor h = llm_add_rms(x, y, llm_vector(ln, D, x, "norm weight"), eps);
+  llm_matrix(wg, F, D, x, "gate weight");
+  llm_matrix(wu, F, D, x, "up weight");
+  Tensor m;
+  if (R <= MDB_GEMM_ROWS_MAX) {
+    m = at::empty({R, F}, x.options());
+    check_rc(mdb_glu_rows(h.data_ptr(), wg.data_ptr(), wu.data_ptr(), m.data_ptr(), (int)R, (int)F, (int)D, MDB_ACT_SILU, cur_stream()), "decoder mlp");
+  } else {
+    Tensor g = at::empty({R, F}, x.options()), u = at::empty({R, F}, x.options());
+    llm_project(h, wg, nullptr, g.data_ptr(), F);
+    llm_project(h, wu, nullptr, u.data_ptr(), F);
+    m = at::mul(at::silu(g), u);
+  }
+  Tensor out = at::empty_like(x);
+  llm_project(m, llm_matrix(wd, D, F, x, "down weight"), nullptr, out.data_ptr(), D);
+  return out;
+}
+// one query per sequence (the first H * Dh columns of qkv rows) over the first ``len`` rows of the caches -> [B, H * Dh]
+Tensor llm_decode_attention(const Tensor& qkv, const Tensor& k_cache, const Tensor& v_cache, int64_t H, int64_t len, double scale) {
+  TORCH_CHECK(qkv.is_cuda() && qkv.scalar_type() == at::kBFloat16 && qkv.dim() == 2 && qkv.stride(1) == 1 && k_cache.dim() == 4 &&
+                  k_cache.is_contiguous() && v_cache.is_contiguous() && v_cache.sizes() == k_cache.sizes() && k_cache.scalar_type() == at::kBFloat16 &&
+                  v_cache.scalar_type() == at::kBFloat16 && k_cache.device() == qkv.device() && v_cache.device() == qkv.device() &&
+                  qkv.size(0) == k_cache.size(0) && qkv.size(1) >= H * k_cache.size(3), "decode attention: qkv rows [B, ..], caches [B, Hkv, T, Dh] bf16");
+  c10::cuda::CUDAGuard guard(qkv.device());
+  const int64_t B = k_cache.size(0), Hkv = k_cache.size(1), T = k_cache.size(2), Dh = k_cache.size(3);
+  Tensor o = at::empty({B, H * Dh}, qkv.options());
+  check_rc(mdb_decode_attention(qkv.data_ptr(), qkv.stride(0), k_cache.data_ptr(), v_cache.data_ptr(), o.data_ptr(), (int)B, (int)H, (int)Hkv, (int)Dh,
+                                (int)T, (int)len, (float)scale, cur_stream()), "decode_attention");
+  return o;
+}
 std::tuple<Tensor, Tensor> fp8_quant_rows(const Tensor& x) {
   TORCH_CHECK(x.is_cuda() && x.dim() == 2 && x.stride(1) == 1 && x.scalar_type() == at::kBFloat16, "fp8_quant_rows");
   c10::cuda::CUDAGuard guard(x.device());
@@ -1013,6 +1122,9 @@ TORCH_LIBRARY(mdb200, m) {
   m.def("flow_match", &flow_match);
   m.def("mse_loss", &mse_loss);
   m.def("randn", &randn);
+  m.def("llm_qkv", &llm_qkv);
+  m.def("llm_out_mlp", &llm_out_mlp);
+  m.def("llm_decode_attention", &llm_decode_attention);
   m.def("fp8_quant_rows", &fp8_quant_rows);
   m.def("fp8_dequant", &fp8_dequant);
   m.def("mx_dequant", &mx_dequant);

@@ -3,9 +3,9 @@
 // What bounds it: the weights are read once and used for at most eight multiply-adds per element, so the time is that of
 // streaming B from HBM. The 128-row tensor-core tiles read the same bytes from only N / 128 CTAs, and one SM takes in about
 // 64 bytes per clock: a 1 x 3072 x 9216 projection kept 72 SMs waiting for 47 us where the weights need 9 us.
-// Here every warp owns C whole columns (rows of B): a lane reads 16 bytes of each of its columns per step, so a warp has
-// C x 512 contiguous bytes of B in flight per step and two steps are issued together; A (a few KB) comes from L1. C is
-// 4, 2 or 1, the widest that still gives every SM two blocks. No shared memory, no split of K: a column's sum is 32 lane
+// Here every warp owns C whole columns (rows of B): a lane reads 16 bytes of each of its columns per step and issues eight
+// such loads together (4 KB per warp in flight; with two, a 2560 x 9728 weight streamed at 2.3 TB/s); A (a few KB) comes from L1.
+// C is 4, 2 or 1, the widest that still gives every SM two blocks. No shared memory, no split of K: a column's sum is 32 lane
 // sums joined in a fixed order, so the result does not depend on scheduling.
 //
 // Role in the reference: the single-token and modulation-vector matrix-vector products, serenitymojo/ops/linear.mojo:40-180.
@@ -21,9 +21,10 @@ constexpr int ROWS_WARPS = 8;
 struct RowsParams {
   const __nv_bfloat16* A[MDB_GEMM_MAX_SEG];
   const __nv_bfloat16* B[MDB_GEMM_MAX_SEG];
+  const __nv_bfloat16* B2[MDB_GEMM_MAX_SEG];      // paired mode: row c of B2 is the second half of column c
   long long lda[MDB_GEMM_MAX_SEG], ldb[MDB_GEMM_MAX_SEG];
   int K[MDB_GEMM_MAX_SEG];
-  int num_seg, M, N, pair_offset, act, act_on_second, out_fp32, accumulate;
+  int num_seg, M, N, pair_offset, act, act_on_second, out_fp32, accumulate, round_halves;
   float alpha;
   const __nv_bfloat16 *bias, *residual, *gate;
   int ld_res, gate_stride, rows_per_group, ld_out;
@@ -49,12 +50,13 @@ __device__ __forceinline__ void dot8(float& acc, const float (&a)[8], const uint
   acc = fmaf(a[4], b2.x, acc); acc = fmaf(a[5], b2.y, acc); acc = fmaf(a[6], b3.x, acc); acc = fmaf(a[7], b3.y, acc);
 }
 
-// MR rows (M rounded up to 1, 2, 4, 8; the surplus repeats the last row), C columns per warp, PAIR: a column is rows c and
-// c + pair_offset of B (SwiGLU / GEGLU).
+// MR rows (M rounded up to 1, 2, 4, 8; the surplus repeats the last row), C columns per warp, PAIR: a column is row c of B and
+// row c of B2 (SwiGLU / GEGLU).
 template <int MR, int C, bool PAIR>
 __global__ void __launch_bounds__(ROWS_WARPS * 32)
-gemm_rows_kernel(const RowsParams p) {
+gemm_rows_kernel(const __grid_constant__ RowsParams p) {
   constexpr int W = PAIR ? 2 * C : C;             // rows of B a warp reads
+  constexpr int U = 8 / W;                        // steps of K issued together: eight 16-byte loads in flight per lane
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n0 = (blockIdx.x * ROWS_WARPS + warp) * C;
   if (n0 >= p.N) return;
@@ -68,39 +70,29 @@ gemm_rows_kernel(const RowsParams p) {
     const uint4* a[MR];
 #pragma unroll
     for (int c = 0; c < W; ++c) {
-      const int col = min(n0 + (PAIR ? c >> 1 : c), p.N - 1) + (PAIR && (c & 1) ? p.pair_offset : 0);
-      b[c] = reinterpret_cast<const uint4*>(p.B[s] + static_cast<size_t>(col) * p.ldb[s]);
+      const int col = min(n0 + (PAIR ? c >> 1 : c), p.N - 1);
+      b[c] = reinterpret_cast<const uint4*>((PAIR && (c & 1) ? p.B2[s] : p.B[s]) + static_cast<size_t>(col) * p.ldb[s]);
     }
 #pragma unroll
     for (int m = 0; m < MR; ++m) a[m] = reinterpret_cast<const uint4*>(p.A[s] + static_cast<size_t>(min(m, p.M - 1)) * p.lda[s]);
     const int kv = p.K[s] >> 3;                   // 16-byte vectors
-    int i = lane;
-    for (; i + 32 < kv; i += 64) {
-      uint4 v0[W], v1[W];
+    for (int i = lane; i < kv; i += 32 * U) {
+      uint4 v[U][W];
 #pragma unroll
-      for (int c = 0; c < W; ++c) { v0[c] = ldg_stream(b[c] + i); v1[c] = ldg_stream(b[c] + i + 32); }
+      for (int u = 0; u < U; ++u)
 #pragma unroll
-      for (int m = 0; m < MR; ++m) {
-        const uint4 u0 = __ldg(a[m] + i), u1 = __ldg(a[m] + i + 32);
-        const float2 x0 = unpack_bf16x2(u0.x), x1 = unpack_bf16x2(u0.y), x2 = unpack_bf16x2(u0.z), x3 = unpack_bf16x2(u0.w);
-        const float2 y0 = unpack_bf16x2(u1.x), y1 = unpack_bf16x2(u1.y), y2 = unpack_bf16x2(u1.z), y3 = unpack_bf16x2(u1.w);
-        const float f0[8] = {x0.x, x0.y, x1.x, x1.y, x2.x, x2.y, x3.x, x3.y};
-        const float f1[8] = {y0.x, y0.y, y1.x, y1.y, y2.x, y2.y, y3.x, y3.y};
+        for (int c = 0; c < W; ++c) v[u][c] = i + 32 * u < kv ? ldg_stream(b[c] + i + 32 * u) : make_uint4(0, 0, 0, 0);
 #pragma unroll
-        for (int c = 0; c < W; ++c) { dot8(acc[m][c], f0, v0[c]); dot8(acc[m][c], f1, v1[c]); }
-      }
-    }
-    if (i < kv) {
-      uint4 v0[W];
+      for (int u = 0; u < U; ++u) {
+        if (i + 32 * u >= kv) break;
 #pragma unroll
-      for (int c = 0; c < W; ++c) v0[c] = ldg_stream(b[c] + i);
+        for (int m = 0; m < MR; ++m) {
+          const uint4 t = __ldg(a[m] + i + 32 * u);
+          const float2 x0 = unpack_bf16x2(t.x), x1 = unpack_bf16x2(t.y), x2 = unpack_bf16x2(t.z), x3 = unpack_bf16x2(t.w);
+          const float f[8] = {x0.x, x0.y, x1.x, x1.y, x2.x, x2.y, x3.x, x3.y};
 #pragma unroll
-      for (int m = 0; m < MR; ++m) {
-        const uint4 u0 = __ldg(a[m] + i);
-        const float2 x0 = unpack_bf16x2(u0.x), x1 = unpack_bf16x2(u0.y), x2 = unpack_bf16x2(u0.z), x3 = unpack_bf16x2(u0.w);
-        const float f0[8] = {x0.x, x0.y, x1.x, x1.y, x2.x, x2.y, x3.x, x3.y};
-#pragma unroll
-        for (int c = 0; c < W; ++c) dot8(acc[m][c], f0, v0[c]);
+          for (int c = 0; c < W; ++c) dot8(acc[m][c], f, v[u][c]);
+        }
       }
     }
   }
@@ -122,7 +114,14 @@ gemm_rows_kernel(const RowsParams p) {
       if (PAIR) {
         float y = acc[m][PAIR ? 2 * c + 1 : c] * p.alpha;
         if (p.bias) y += __bfloat162float(p.bias[col + p.pair_offset]);
-        x = p.act_on_second ? x * rows_act(p.act, y) : rows_act(p.act, x) * y;
+        if (p.round_halves) {
+          // both projections and the activation rounded to bf16, as separate operations round them
+          x = __bfloat162float(__float2bfloat16_rn(x));
+          y = __bfloat162float(__float2bfloat16_rn(y));
+          x = __bfloat162float(__float2bfloat16_rn(rows_act(p.act, x))) * y;
+        } else {
+          x = p.act_on_second ? x * rows_act(p.act, y) : rows_act(p.act, x) * y;
+        }
       } else {
         x = rows_act(p.act, x);
       }
@@ -149,6 +148,13 @@ static int launch_rows(const RowsParams& p, int sms, cudaStream_t st) {
   return static_cast<int>(cudaGetLastError());
 }
 
+static int launch_rows_any(const RowsParams& p, int sms, bool pair, cudaStream_t st) {
+  if (p.M == 1) return pair ? launch_rows<1, true>(p, sms, st) : launch_rows<1, false>(p, sms, st);
+  if (p.M == 2) return pair ? launch_rows<2, true>(p, sms, st) : launch_rows<2, false>(p, sms, st);
+  if (p.M <= 4) return pair ? launch_rows<4, true>(p, sms, st) : launch_rows<4, false>(p, sms, st);
+  return pair ? launch_rows<8, true>(p, sms, st) : launch_rows<8, false>(p, sms, st);
+}
+
 }  // namespace mdb
 
 // True when the few-row kernel computes exactly what mdb_gemm_launch was asked for. It reads whole 16-byte vectors along K
@@ -172,6 +178,7 @@ extern "C" int mdb_gemm_rows(const MdbGemmArgs* a, cudaStream_t st) {
   for (int s = 0; s < a->num_seg; ++s) {
     p.A[s] = reinterpret_cast<const __nv_bfloat16*>(a->A[s]);
     p.B[s] = reinterpret_cast<const __nv_bfloat16*>(a->B[s]);
+    p.B2[s] = p.B[s] + static_cast<size_t>(a->pair_offset > 0 ? a->pair_offset : 0) * a->ldb[s];
     p.lda[s] = a->lda[s];
     p.ldb[s] = a->ldb[s];
     p.K[s] = static_cast<int>(a->K[s]);
@@ -183,10 +190,23 @@ extern "C" int mdb_gemm_rows(const MdbGemmArgs* a, cudaStream_t st) {
   p.gate = reinterpret_cast<const __nv_bfloat16*>(a->gate);
   p.ld_res = a->ld_res; p.gate_stride = a->gate_stride; p.rows_per_group = a->rows_per_group > 0 ? a->rows_per_group : 1;
   p.out = a->out; p.ld_out = a->ld_out; p.out_fp32 = a->out_fp32; p.accumulate = a->accumulate_out;
-  const int sms = a->num_sms > 0 ? a->num_sms : device_sm_count();
-  const bool pair = a->pair_offset > 0;
-  if (a->M == 1) return pair ? launch_rows<1, true>(p, sms, st) : launch_rows<1, false>(p, sms, st);
-  if (a->M == 2) return pair ? launch_rows<2, true>(p, sms, st) : launch_rows<2, false>(p, sms, st);
-  if (a->M <= 4) return pair ? launch_rows<4, true>(p, sms, st) : launch_rows<4, false>(p, sms, st);
-  return pair ? launch_rows<8, true>(p, sms, st) : launch_rows<8, false>(p, sms, st);
+  return launch_rows_any(p, a->num_sms > 0 ? a->num_sms : device_sm_count(), a->pair_offset > 0, st);
+}
+
+// act(x w1^T) * (x w2^T) with the two halves in weights of their own, each half and the activation rounded to bf16 before they
+// meet, M <= MDB_GEMM_ROWS_MAX rows; everything contiguous bf16
+extern "C" int mdb_glu_rows(const void* x, const void* w1, const void* w2, void* out, int M, int N, int K, int act, cudaStream_t st) {
+  using namespace mdb;
+  if (M <= 0 || M > MDB_GEMM_ROWS_MAX || N <= 0 || K <= 0 || K % 8 ||
+      ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w1) | reinterpret_cast<uintptr_t>(w2)) & 15))
+    return -1;
+  RowsParams p;
+  memset(&p, 0, sizeof(p));
+  p.A[0] = reinterpret_cast<const __nv_bfloat16*>(x);
+  p.B[0] = reinterpret_cast<const __nv_bfloat16*>(w1);
+  p.B2[0] = reinterpret_cast<const __nv_bfloat16*>(w2);
+  p.lda[0] = p.ldb[0] = p.K[0] = K;
+  p.num_seg = 1; p.M = M; p.N = N; p.act = act; p.alpha = 1.f; p.rows_per_group = 1; p.out = out; p.ld_out = N;
+  p.round_halves = 1;
+  return launch_rows_any(p, device_sm_count(), true, st);
 }

@@ -46,6 +46,26 @@ int mdb_qk_norm_rope_bwd(void* dbuf, const void* xbuf, const void* wq, const voi
 int mdb_rope_table(const float* pos, float* cosv, float* sinv, int tokens, int naxes, const int* axes_dim, float theta,
                    cudaStream_t st);
 
+// ---- llm_rows.cu
+// qkv rows (q | k | v heads of Dh): q normalised + rotated in place, k (normalised + rotated) and v appended to the caches
+// [B, Hkv, T, Dh] at positions pos0 .. pos0 + S - 1; qn / kn null: no norm
+int mdb_qkv_rope_cache(void* qkv, const void* qn, const void* kn, const void* cosv, const void* sinv, void* kc, void* vc, long long rows, int S,
+                       int H, int Hkv, int Dh, int T, int pos0, float eps, cudaStream_t st);
+// x += y (y null: nothing), h = RMSNorm(x) * w
+int mdb_add_rms_rows(void* x, const void* y, const void* w, void* h, long long rows, int D, float eps, cudaStream_t st);
+#define MDB_DECODE_ATTENTION_MAX 7936      // cache rows whose scores fit beside the partial sums in 48 KB of shared memory
+int mdb_decode_attention(const void* q, long long ldq, const void* kc, const void* vc, void* o, int B, int H, int Hkv, int Dh, int T, int len,
+                         float scale, cudaStream_t st);
+
+// ---- fused_rows.cu
+// P = softmax(S * scale) per row; leading dimensions multiples of 4 that cover the last partial group of four columns
+int mdb_softmax_rows(const float* s, void* p, long long rows, int cols, long long lds, long long ldp, float scale, cudaStream_t st);
+// in place on rows of a packed buffer: full-width RMSNorm (D columns from q_off and from k_off) + split-half rotation per head
+int mdb_rms_rope_rows(void* buf, const void* wq, const void* wk, const float* cosv, const float* sinv, long long rows, long long ld, int D,
+                      int Dh, int q_off, int k_off, int rows_per_batch, float eps, cudaStream_t st);
+// o[row, h, :] *= 2 * sigmoid(logit[row, h]) in place
+int mdb_head_gate(void* o, const void* logit, long long rows, int H, int Dh, long long ld_logit, cudaStream_t st);
+
 // ---- pointwise.cu
 int mdb_act_fwd(const void* x, void* y, const void* bias, long long n, int cols, int act, cudaStream_t st);
 int mdb_act_bwd(const void* x, const void* dy, void* dx, const void* bias, long long n, int cols, int act,

@@ -12,7 +12,9 @@ from typing import List, Optional, Sequence
 
 import torch
 
+from .. import ops
 from ..models.text.qwen3 import Qwen3Config, Qwen3Encoder, _rope
+from ..ops import native
 from .sampler import Rng, SamplerConfig, sample
 
 
@@ -39,6 +41,10 @@ class KVCache:
         self.v = torch.zeros(shape, dtype=dtype, device=device)
         self.length = 0
         self.max_len = max_len
+        self.rope = None                # (cos, sin) [max_len, head_dim] of every position, filled by the prefill on the GPU
+
+
+DECODE_ATTENTION_MAX = 7936             # cache rows the single-query attention kernel covers (scores in shared memory)
 
 
 class Qwen3Decoder:
@@ -56,6 +62,24 @@ class Qwen3Decoder:
         emb = torch.cat((ang, ang), dim=-1)
         return emb.cos().to(dtype), emb.sin().to(dtype)
 
+    def _native(self, x: torch.Tensor) -> bool:
+        """Whether the fused decode-step kernels cover this stack: bf16 on the GPU, 16-byte rows, heads of up to 256. They round
+        to bf16 where the separate operations do."""
+        c = self.cfg
+        return (native.use_native(x) and x.dtype == torch.bfloat16 and c.qk_norm and c.hidden_size % 8 == 0 and c.hidden_size <= 16384
+                and c.intermediate_size % 8 == 0 and c.head_dim % 8 == 0 and c.head_dim <= 256 and x.numel() > 0
+                and c.num_attention_heads % c.num_key_value_heads == 0)
+
+    def _qkv(self, l, x, y, cache, li, S, pos):
+        a, c = l.self_attn, self.cfg
+        return native.ops().llm_qkv(x, y, l.input_layernorm.weight, a.q_proj.weight, a.k_proj.weight, a.v_proj.weight, a.q_proj.bias, a.k_proj.bias,
+                                    a.v_proj.bias, a.q_norm.weight, a.k_norm.weight, cache.rope[0], cache.rope[1], cache.k[li], cache.v[li], S, pos, c.rms_norm_eps)
+
+    def _out_mlp(self, l, x, attn):
+        m = l.mlp
+        return native.ops().llm_out_mlp(x, attn, l.self_attn.o_proj.weight, l.post_attention_layernorm.weight, m.gate_proj.weight, m.up_proj.weight,
+                                        m.down_proj.weight, self.cfg.rms_norm_eps)
+
     @torch.no_grad()
     def prefill(self, ids: torch.Tensor, max_len: int) -> "tuple[torch.Tensor, KVCache]":
         """ids [B, S] -> (hidden of the last position [B, hidden], cache holding positions 0..S-1)."""
@@ -67,6 +91,8 @@ class Qwen3Decoder:
         cos, sin = cos[None, None], sin[None, None]
         mask = torch.full((S, S), float("-inf"), device=ids.device, dtype=x.dtype).triu(1)[None, None]
         rep = c.num_attention_heads // c.num_key_value_heads
+        if self._native(x):
+            cache.rope = self._angles(torch.arange(max_len, device=ids.device), x.dtype)      # for the decode steps
         for li, l in enumerate(m.layers):
             a = l.self_attn
             h = l.input_layernorm(x)
@@ -92,6 +118,13 @@ class Qwen3Decoder:
         if pos >= cache.max_len:
             raise RuntimeError("KV cache is full")
         x = m.embed_tokens(token)                                         # [B, hidden]
+        if cache.rope is not None and pos < DECODE_ATTENTION_MAX and self._native(x):
+            H, scale, y = c.num_attention_heads, c.head_dim ** -0.5, None
+            for li, l in enumerate(m.layers):
+                qkv = self._qkv(l, x, y, cache, li, 1, pos)
+                y = self._out_mlp(l, x, native.ops().llm_decode_attention(qkv, cache.k[li], cache.v[li], H, pos + 1, scale))
+            cache.length = pos + 1
+            return x + y if y is not None else x
         cos, sin = self._angles(torch.tensor([pos], device=token.device), x.dtype)
         for li, l in enumerate(m.layers):
             a = l.self_attn
@@ -110,6 +143,10 @@ class Qwen3Decoder:
     def logits(self, hidden: torch.Tensor) -> torch.Tensor:
         h = self.enc.model.norm(hidden)
         w = self.lm_head if self.lm_head is not None else self.enc.model.embed_tokens.weight
+        if (native.use_native(h) and h.dtype == w.dtype == torch.bfloat16 and h.dim() == 2 and 0 < h.shape[0] <= 8 and h.shape[1] % 8 == 0
+                and h.is_contiguous() and w.is_contiguous()):
+            # products of bf16 values are exact in fp32 and the few-row kernel sums in fp32: the table needs no fp32 copy
+            return ops.functional._gemm([h], [w], out_fp32=True)
         return h.float() @ w.float().t()
 
     @torch.no_grad()

@@ -86,3 +86,43 @@ def test_conv3x3_pair_tiles(N, H, W, Cin, Cout):
             _close(C.conv2d_nhwc(x, w, bias, stride=2, offset=off), _conv_ref(x, w, bias, 2, off), f"stride 2 from {off}")
         w1 = _rand(Cout, 1, 1, Cin, scale=1 / math.sqrt(Cin), seed=5)
         _close(C.conv2d_nhwc(x, w1, bias, padding=0), x.float() @ w1[:, 0, 0].float().t() + bias.float(), "1 x 1")
+
+
+# decoder layer kernels against the same stack in fp32 on the CPU: rows of one, eight and nine sequences (few-row / tiled
+# projections), head widths with one and with several rotary pairs per lane, with and without biases
+@pytest.mark.parametrize("B,S,H,Hkv,Dh,bias", [(1, 1, 4, 2, 64, False), (2, 11, 4, 1, 128, False), (8, 3, 6, 6, 40, True), (9, 65, 2, 2, 256, False)])
+def test_decoder_layers(B, S, H, Hkv, Dh, bias):
+    from mojodiffusion_b200.llm.decoder import Qwen3Decoder
+    from mojodiffusion_b200.models.text.qwen3 import Qwen3Config, Qwen3Encoder
+    cfg = Qwen3Config(vocab_size=200, hidden_size=264, intermediate_size=520, num_hidden_layers=3, num_attention_heads=H, num_key_value_heads=Hkv,
+                      head_dim=Dh, qkv_bias=bias)
+    enc = Qwen3Encoder(cfg, torch.bfloat16, DEV).eval()
+    g = torch.Generator(device=DEV).manual_seed(0)
+    with torch.no_grad():
+        for n, p in enc.named_parameters():
+            p.normal_(0.0, p.shape[-1] ** -0.5, generator=g) if p.dim() == 2 else p.normal_(0.0 if n.endswith("bias") else 1.0, 0.1, generator=g)
+    cpu = Qwen3Encoder(cfg, torch.float32).eval()
+    cpu.load_state_dict({k: v.float().cpu() for k, v in enc.state_dict().items()})
+    ids = torch.randint(0, 200, (B, S), generator=torch.Generator().manual_seed(1))
+    nxt = torch.randint(0, 200, (4, B), generator=torch.Generator().manual_seed(2))
+    outs = []
+    for dec, dev in ((Qwen3Decoder(enc), DEV), (Qwen3Decoder(cpu), "cpu")):
+        h, cache = dec.prefill(ids.to(dev), S + 4)
+        out = [dec.logits(h)]
+        for t in nxt:
+            out.append(dec.logits(dec.decode_step(t.to(dev), cache)))
+        outs.append(torch.stack(out).float().cpu())
+    native.check_status(torch.empty(0, device=DEV))
+    # about twenty bf16 roundings of 2^-9 / sqrt(3) each per layer, added in quadrature over three layers and the head, doubled
+    err = float((outs[0] - outs[1]).norm() / outs[1].norm())
+    assert err < 2 * 2.0 ** -9 / 3 ** 0.5 * 64 ** 0.5, err
+
+
+def test_few_row_gemm_accumulates_fp32():
+    from mojodiffusion_b200.ops.functional import _gemm
+    for M in (1, 3, 8, 40):
+        x, w, out = _rand(M, 264, seed=1), _rand(120, 264, seed=2, scale=0.1), _rand(M, 120, seed=3, dtype=torch.float32)
+        want = out + x.float() @ w.float().t()
+        _gemm([x], [w], out=out, out_fp32=True, accumulate=True)
+        native.check_status(out)
+        assert float((out - want).abs().max()) < 2e-5 * float(want.abs().max()), M
