@@ -20,6 +20,7 @@
 #include "gemm_api.h"
 
 #include <cudaTypedefs.h>
+#include <atomic>
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
@@ -1346,6 +1347,8 @@ static int launch_conv_pair(const GemmMaps& maps, const GemmParams& p, int num_s
   return static_cast<int>(cudaGetLastError());
 }
 
+#include "gemm_splitk.cuh"
+
 }  // namespace mdb
 
 extern "C" int mdb_gemm_pair_capacity(int num_sms) { return mdb::pair_capacity(num_sms > 0 ? num_sms : mdb::device_sm_count()); }
@@ -1412,6 +1415,34 @@ extern "C" int mdb_gemm_launch(const MdbGemmArgs* a, cudaStream_t stream) {
       use_pair = true;
       bn = 256;
     }
+  }
+  // Few tiles for the SMs there are: compare waves x K steps x time per step (cycles) of the tiling chosen above with narrower
+  // lone tiles and with clusters that share a tile's reduction. A step of a lone tile costs 726 / 400 / 232 cycles at 256 /
+  // 128 / 64 columns; filling the pipeline, meeting in shared memory and finishing the rows costs a split tile about 3000
+  // cycles more than it saves per step, which is why short reductions stay whole.
+  int splits = 0;
+  if (auto_tile && pair_mode() != 0 && a->kind == 0 && a->conv_taps <= 0 && a->gather_world <= 1 && a->split_k == 0 && !paired && !a->row_scale &&
+      !a->col_scale && a->route_owner_cols <= 0 && a->reduce_rows_per_owner <= 0 && !a->prof && !(a->a_mn && !a->b_mn)) {
+    int kb = 0;
+    for (int s = 0; s < a->num_seg; ++s) kb += static_cast<int>((a->K[s] + 63) / 64);
+    const long long tm = (a->M + BM - 1) / BM;
+    auto tiles_of = [&](int w) { return tm * ((a->N + w - 1) / w); };
+    auto step_of = [](int w) { return w == 256 ? 726.0 : w == 128 ? 400.0 : 232.0; };
+    const long long pt = static_cast<long long>((a->M + 2 * BM - 1) / (2 * BM)) * ((a->N + 255) / 256);
+    const int pairs = pair_capacity(sms);
+    double best = use_pair ? static_cast<double>((pt + pairs - 1) / pairs) * kb * 523.0
+                           : static_cast<double>((tiles_of(bn) + sms - 1) / sms) * kb * step_of(bn);
+    best *= 0.95;                                              // the whole-K tilings need no meeting: they win ties
+    if (use_pair || bn != 64) {
+      const double c = static_cast<double>((tiles_of(64) + sms - 1) / sms) * kb * step_of(64);
+      if (c < best) { best = c; bn = 64; use_pair = false; }
+    }
+    for (int w = 128; w >= 64; w -= 64)
+      for (int sp = 2; sp <= SPLIT_MAX && kb / sp >= 4; ++sp) {
+        const int cap = w == 128 ? split_capacity<128>(sp, sms) : split_capacity<64>(sp, sms);
+        const double c = static_cast<double>((tiles_of(w) + cap - 1) / cap) * (((kb + sp - 1) / sp) * step_of(w) + 3000.0);
+        if (c < best) { best = c; bn = w; splits = sp; use_pair = false; }
+      }
   }
   // 3 x 3 convolutions: pair tiles of 2 patches x 256 / 128 / 64 channels or lone CTAs, by waves x time per 64-wide K step
   int conv_pair = 0;
@@ -1563,6 +1594,11 @@ extern "C" int mdb_gemm_launch(const MdbGemmArgs* a, cudaStream_t stream) {
     if (conv_pair == 256) return launch_conv_pair<256, false>(maps, p, sms, stream);
     if (conv_pair == 128) return launch_conv_pair<128, false>(maps, p, sms, stream);
     return launch_conv_pair<64, false>(maps, p, sms, stream);
+  }
+  if (splits > 1) {
+    if (!a->a_mn && !a->b_mn) return bn == 128 ? launch_split<128, false, false>(maps, p, splits, stream) : launch_split<64, false, false>(maps, p, splits, stream);
+    if (!a->a_mn) return bn == 128 ? launch_split<128, false, true>(maps, p, splits, stream) : launch_split<64, false, true>(maps, p, splits, stream);
+    return bn == 128 ? launch_split<128, true, true>(maps, p, splits, stream) : launch_split<64, true, true>(maps, p, splits, stream);
   }
 #define MDB_LAUNCH(BN_, ST_, AMN_, BMN_, KIND_) return launch_variant<BN_, ST_, AMN_, BMN_, KIND_>(maps, p, sms, stream)
   if (use_pair) {

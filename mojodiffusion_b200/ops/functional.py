@@ -43,31 +43,10 @@ def _gemm(As, Bs, bias=None, residual=None, gate=None, rows_per_group=1, act=0, 
                        list(route_cfg), list(gather_ptrs), list(gather_cfg), gather_dst, gather_ready, split_k)
 
 
-_sm_count = {}
-
-
-def _num_sms(device) -> int:
-    idx = device.index if device.index is not None else torch.cuda.current_device()
-    n = _sm_count.get(idx)
-    if n is None:
-        n = _sm_count[idx] = torch.cuda.get_device_properties(idx).multi_processor_count
-    return n
-
-
 def _gemm_skinny(A, B, a_mn=False, b_mn=False, alpha=1.0):
-    """GEMM whose output has far fewer tiles than the GPU has SMs (LoRA down-projections and their gradients: N or M
-    of 16..64 against a long reduction): the reduction is split across the idle SMs and the parts are added in fp32."""
-    M = A.shape[1] if a_mn else A.shape[0]
-    N = B.shape[1] if b_mn else B.shape[0]
-    K = A.shape[0] if a_mn else A.shape[1]
-    tiles = ((M + 127) // 128) * ((N + 63) // 64)
-    kblocks = (K + 63) // 64
-    split = min(_num_sms(A.device) // max(tiles, 1), kblocks // 4, 16)
-    if split <= 1:
-        return _gemm([A], [B], a_mn=a_mn, b_mn=b_mn, alpha=alpha)
-    out = torch.zeros(M, N, dtype=torch.float32, device=A.device)
-    _gemm([A], [B], a_mn=a_mn, b_mn=b_mn, alpha=alpha, out=out, out_fp32=True, split_k=split, bn=64)
-    return out.to(A.dtype)
+    """GEMM whose output has far fewer tiles than the GPU has SMs (LoRA down-projections and their gradients: N or M of
+    16..64 against a long reduction). The launch splits the reduction over clusters of SMs and adds the parts on chip."""
+    return _gemm([A], [B], a_mn=a_mn, b_mn=b_mn, alpha=alpha)
 
 
 # --------------------------------------------------------------------------------------------
@@ -128,11 +107,13 @@ class _LoraLinearFn(torch.autograd.Function):
 
 def linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None, act=None,
            residual: Optional[torch.Tensor] = None, gate: Optional[torch.Tensor] = None, rows_per_group: int = 1,
-           extra: Sequence[tuple] = (), out: Optional[torch.Tensor] = None) -> torch.Tensor:
+           extra: Sequence[tuple] = (), out: Optional[torch.Tensor] = None, whole_k: bool = False) -> torch.Tensor:
     """``act(x @ w.T [+ a_i @ b_i.T ...] + bias)`` then ``residual + gate[row // rows_per_group] * value``.
 
     x: [..., K]; w: [N, K]; gate: [groups, N]; residual: [..., N]. On a GPU without autograd the whole
     expression is one tcgen05 GEMM launch; with autograd the epilogue pieces become separate differentiable ops.
+    ``whole_k``: every output keeps one accumulator over the whole reduction (no split over SMs), so that a row's result does
+    not depend on how many rows come with it.
     """
     lead = x.shape[:-1]
     if not native.use_native(x):
@@ -164,7 +145,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None
         r2 = _flat2d(residual) if residual is not None else None
         o2 = out.reshape(-1, out.shape[-1]) if out is not None else None
         y = _gemm([x2] + [_flat2d(a) for a, _ in extra], [w] + [b for _, b in extra], bias=bias, residual=r2,
-                  gate=gate, rows_per_group=rows_per_group, act=act_code(act), out=o2)
+                  gate=gate, rows_per_group=rows_per_group, act=act_code(act), out=o2, split_k=1 if whole_k else 0)
         return out if out is not None else y.reshape(*lead, w.shape[0])
     assert not extra, "extra K segments are an inference-path feature"
     y = _LinearFn.apply(x2, w, bias)
