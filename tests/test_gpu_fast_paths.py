@@ -146,3 +146,26 @@ def test_cluster_split_k(M, N, K):
     M8 = (M + 7) // 8 * 8
     xt = _rand(K, M8, seed=5)
     _close(_gemm([xt], [w.t().contiguous()], a_mn=True, b_mn=True, alpha=0.5), 0.5 * xt.float().t() @ w.float().t(), "both read transposed", rel=1e-4)
+
+
+# groups of 3 / 4 / 10 / 80 channels, slabs of whole groups beyond 2048 channels, one pixel, images that end inside a chunk
+@pytest.mark.parametrize("N,HW,C,G", [(1, 1, 64, 2), (2, 1000, 24, 8), (3, 4097, 128, 32), (2, 777, 320, 32), (2, 300, 2560, 32), (1, 50, 4096, 32),
+                                      (1, 300000, 8, 2)])
+def test_group_norm_forward_and_backward(N, HW, C, G):
+    from mojodiffusion_b200.ops import conv as K
+    x = _rand(N, 1, HW, C, seed=1) * 2 + 3                      # a mean of several standard deviations
+    w, b, dy = _rand(C, seed=2), _rand(C, seed=3), _rand(N, 1, HW, C, seed=4)
+    for act in (None, "silu"):
+        with torch.no_grad():
+            y = K.group_norm_nhwc(x, w, b, G, 1e-6, act)
+        leaf = [t.float().requires_grad_() for t in (x, w, b)]
+        want = torch.nn.functional.group_norm(leaf[0].permute(0, 3, 1, 2).double(), G, leaf[1].double(), leaf[2].double(), 1e-6).permute(0, 2, 3, 1)
+        want = torch.nn.functional.silu(want) if act else want
+        _close(y, want, f"forward {act}", rel=1e-5)
+        want.backward(dy.double())
+        p = [t.clone().requires_grad_() for t in (x, w, b)]
+        K.group_norm_nhwc(*p, G, 1e-6, act).backward(dy)
+        _close(p[0].grad, leaf[0].grad, f"dx {act}", rel=1e-4)
+        for i in (1, 2):                                        # fp32 sums over the pixels, then bf16: 2^-9 and the sum's own 1e-4
+            err = float((p[i].grad.float() - leaf[i].grad).norm() / leaf[i].grad.norm())
+            assert err < 2.0 ** -8 + 1e-3, (act, i, err)
