@@ -789,6 +789,13 @@ Tensor llm_decode_attention(const Tensor& qkv, const Tensor& k_cache, const Tens
                                 (int)T, (int)len, (float)scale, cur_stream()), "decode_attention");
   return o;
 }
+void softmax_rows(const Tensor& s, Tensor p, double scale) {
+  TORCH_CHECK(s.is_cuda() && s.dim() == 2 && s.stride(1) == 1 && s.scalar_type() == at::kFloat && p.device() == s.device() && p.dim() == 2 &&
+                  p.stride(1) == 1 && p.scalar_type() == at::kBFloat16 && p.sizes() == s.sizes(), "softmax_rows: fp32 scores, bf16 output of one shape");
+  c10::cuda::CUDAGuard guard(s.device());
+  check_rc(mdb_softmax_rows(s.data_ptr<float>(), p.data_ptr(), s.size(0), (int)s.size(1), s.stride(0), p.stride(0), (float)scale, cur_stream()),
+           "softmax_rows");
+}
 std::tuple<Tensor, Tensor> fp8_quant_rows(const Tensor& x) {
   TORCH_CHECK(x.is_cuda() && x.dim() == 2 && x.stride(1) == 1 && x.scalar_type() == at::kBFloat16, "fp8_quant_rows");
   c10::cuda::CUDAGuard guard(x.device());
@@ -1125,6 +1132,7 @@ TORCH_LIBRARY(mdb200, m) {
   m.def("llm_qkv", &llm_qkv);
   m.def("llm_out_mlp", &llm_out_mlp);
   m.def("llm_decode_attention", &llm_decode_attention);
+  m.def("softmax_rows", &softmax_rows);
   m.def("fp8_quant_rows", &fp8_quant_rows);
   m.def("fp8_dequant", &fp8_dequant);
   m.def("mx_dequant", &mx_dequant);

@@ -110,10 +110,7 @@ class AttnBlock(nn.Module):
         N, H, W, Cc = x.shape
         h = self.norm(x)
         q, k, v = [m(h).reshape(N, H * W, 1, Cc) for m in (self.q, self.k, self.v)]
-        if Cc in (64, 128):
-            o = ops.attention(q, k, v)
-        else:                                   # head dim 512 of the standard AE: plain attention math (one layer)
-            o = ops.reference.attention(q, k, v)
+        o = ops.attention(q, k, v)
         return self.proj_out(o.reshape(N, H, W, Cc), residual=x)
 
 

@@ -447,6 +447,27 @@ def split_cols(x: torch.Tensor, a: int):
     return x[..., :a], x[..., a:]
 
 
+def _wide_attention(q, k, v, scale: float):
+    """One head wider than the attention kernel's tiles (the 512-channel block of the image autoencoders): scores as one
+    tcgen05 GEMM into fp32, a softmax pass over their rows, the weighted sum as a second GEMM. At most 2^27 scores (fp32
+    scores and bf16 probabilities: 0.8 GB) are held at a time, so memory stays linear in the number of pixels."""
+    B, Sq, _, Dh = q.shape
+    Skv = k.shape[1]
+    ld = (Skv + 7) // 8 * 8                                  # 16-byte rows; the padding columns are never read
+    rows = min(Sq, max(256, (1 << 27) // ld // 256 * 256))
+    o = torch.empty(B, Sq, 1, Dh, dtype=q.dtype, device=q.device)
+    s = torch.empty(rows, ld, dtype=torch.float32, device=q.device)
+    p = torch.empty(rows, ld, dtype=q.dtype, device=q.device)
+    for b in range(B):
+        kb, vb, qb = _flat2d(k[b]), _flat2d(v[b]), _flat2d(q[b])
+        for r0 in range(0, Sq, rows):
+            n = min(rows, Sq - r0)
+            _gemm([qb[r0:r0 + n]], [kb], out=s[:n, :Skv], out_fp32=True)
+            _ops().softmax_rows(s[:n, :Skv], p[:n, :Skv], scale)
+            _gemm([p[:n, :Skv]], [vb], b_mn=True, out=o[b, r0:r0 + n, 0])
+    return o
+
+
 def attention(q, k, v, scale: Optional[float] = None, kv_len: Optional[torch.Tensor] = None,
               out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Scaled dot-product attention over [B, S, H, Dh] tensors (any strides with contiguous Dh).
@@ -455,6 +476,14 @@ def attention(q, k, v, scale: Optional[float] = None, kv_len: Optional[torch.Ten
     """
     Dh = q.shape[-1]
     scale = float(scale) if scale is not None else 1.0 / math.sqrt(Dh)
+    if (native.use_native(q) and q.dim() == 4 and q.shape[2] == 1 and Dh > 128 and Dh % 8 == 0 and kv_len is None
+            and q.dtype == k.dtype == v.dtype == torch.bfloat16 and q.shape[1] > 0 and k.shape[1] > 0
+            and not (torch.is_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad))):
+        o = _wide_attention(q, k, v, scale)
+        if out is not None:
+            out.copy_(o)
+            return out
+        return o
     if not native.use_native(q) or Dh not in (64, 128):     # other head widths (120, 256, ...): the torch statement / library kernel
         o = ref.attention(q, k, v, scale, kv_len)
         if out is not None:

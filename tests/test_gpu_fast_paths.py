@@ -169,3 +169,37 @@ def test_group_norm_forward_and_backward(N, HW, C, G):
         for i in (1, 2):                                        # fp32 sums over the pixels, then bf16: 2^-9 and the sum's own 1e-4
             err = float((p[i].grad.float() - leaf[i].grad).norm() / leaf[i].grad.norm())
             assert err < 2.0 ** -8 + 1e-3, (act, i, err)
+
+
+# one wide head: odd key counts (padded score rows), fewer rows than a tile, several chunks of rows when the scores pass the
+# bound, a width that is no multiple of 16
+@pytest.mark.parametrize("B,Sq,Skv,Dh", [(1, 5, 3, 512), (3, 333, 333, 512), (2, 300, 1001, 136), (1, 9000, 17001, 256)])
+def test_wide_single_head_attention(B, Sq, Skv, Dh):
+    q, k, v = (_rand(B, s, 1, Dh, seed=i) for i, s in ((1, Sq), (2, Skv), (3, Skv)))
+    with torch.no_grad():
+        out = O.attention(q, k, v)
+        pad = torch.empty(B, Sq, 2 * Dh, dtype=torch.bfloat16, device=DEV)
+        pad[..., :Dh] = q[:, :, 0]
+        strided = O.attention(pad[..., :Dh].unflatten(-1, (1, Dh)), k, v)
+    native.check_status(out)
+    want = torch.cat([torch.softmax(q[b, :, 0].float() @ k[b, :, 0].float().t() / math.sqrt(Dh), -1) @ v[b, :, 0].float() for b in range(B)]).view(B, Sq, 1, Dh)
+    # probabilities and the result are rounded to bf16 once each: 2^-9 / sqrt(3) of their size, in quadrature, doubled
+    assert float((out.float() - want).norm() / want.norm()) < 2 * 2.0 ** -9 * (2 / 3) ** 0.5
+    assert torch.equal(out, strided)
+
+
+@pytest.mark.parametrize("cols", [1, 3, 4, 1000, 16384, 16385, 40001])
+def test_softmax_rows(cols):
+    ld = (cols + 7) // 8 * 8
+    s = torch.full((7, ld), float("nan"), device=DEV)            # what the padding holds does not matter
+    s[:, :cols] = _rand(7, cols, scale=4, dtype=torch.float32)
+    s[1, :cols // 2] = float("-inf")
+    s[2, :cols] = 1e30
+    s[3, cols - 1] = float("nan")
+    p = torch.empty(7, ld, dtype=torch.bfloat16, device=DEV)
+    torch.ops.mdb200.softmax_rows(s[:, :cols], p[:, :cols], 0.7)
+    want = torch.softmax(s[:, :cols].double() * 0.7, -1)
+    assert torch.isnan(p[3, :cols]).all()
+    keep = [0, 1, 2, 4, 5, 6]
+    # bf16 rounding (2^-9) and the exponential's and sum's 1e-5, doubled
+    assert bool(((p[keep][:, :cols].double() - want[keep]).abs() <= want[keep] * 2 * (2.0 ** -9 + 1e-5) + 1e-38).all())
