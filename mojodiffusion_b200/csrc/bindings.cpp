@@ -796,6 +796,30 @@ void softmax_rows(const Tensor& s, Tensor p, double scale) {
   check_rc(mdb_softmax_rows(s.data_ptr<float>(), p.data_ptr(), s.size(0), (int)s.size(1), s.stride(0), p.stride(0), (float)scale, cur_stream()),
            "softmax_rows");
 }
+// buf [rows, W] bf16, rows of ``rows_per_batch`` tokens per sample; cos / sin [positions, Dh / 2] fp32
+void rms_rope_rows(Tensor buf, const Tensor& wq, const Tensor& wk, const Tensor& cosv, const Tensor& sinv, int64_t D, int64_t Dh, int64_t q_off,
+                   int64_t k_off, int64_t rows_per_batch, double eps) {
+  TORCH_CHECK(buf.is_cuda() && buf.scalar_type() == at::kBFloat16 && buf.dim() == 2 && buf.stride(1) == 1 && q_off >= 0 && k_off >= 0 &&
+                  q_off + D <= buf.size(1) && k_off + D <= buf.size(1), "rms_rope_rows: buf [rows, W] bf16 with both ranges inside");
+  for (const Tensor* w : {&wq, &wk})
+    TORCH_CHECK(w->is_cuda() && w->scalar_type() == at::kBFloat16 && w->is_contiguous() && w->numel() == D, "rms_rope_rows: weights [D] bf16");
+  for (const Tensor* t : {&cosv, &sinv})
+    TORCH_CHECK(t->is_cuda() && t->scalar_type() == at::kFloat && t->is_contiguous() && t->dim() == 2 && t->size(1) * 2 == Dh &&
+                    t->size(0) >= rows_per_batch, "rms_rope_rows: tables [positions, Dh / 2] fp32");
+  c10::cuda::CUDAGuard guard(buf.device());
+  check_rc(mdb_rms_rope_rows(buf.data_ptr(), wq.data_ptr(), wk.data_ptr(), cosv.data_ptr<float>(), sinv.data_ptr<float>(), buf.size(0), buf.stride(0),
+                             (int)D, (int)Dh, (int)q_off, (int)k_off, (int)rows_per_batch, (float)eps, cur_stream()),
+           "rms_rope_rows");
+}
+// o [..., H, Dh] contiguous bf16, logit [rows, H] bf16
+void head_gate(Tensor o, const Tensor& logit) {
+  TORCH_CHECK(o.is_cuda() && o.scalar_type() == at::kBFloat16 && o.is_contiguous() && o.dim() >= 2, "head_gate: o [..., H, Dh] bf16");
+  const int64_t H = o.size(-2), Dh = o.size(-1);
+  TORCH_CHECK(logit.is_cuda() && logit.scalar_type() == at::kBFloat16 && logit.dim() == 2 && logit.stride(1) == 1 && logit.size(1) == H &&
+                  logit.size(0) * H * Dh == o.numel(), "head_gate: logit [rows, H] bf16");
+  c10::cuda::CUDAGuard guard(o.device());
+  check_rc(mdb_head_gate(o.data_ptr(), logit.data_ptr(), logit.size(0), (int)H, (int)Dh, logit.stride(0), cur_stream()), "head_gate");
+}
 std::tuple<Tensor, Tensor> fp8_quant_rows(const Tensor& x) {
   TORCH_CHECK(x.is_cuda() && x.dim() == 2 && x.stride(1) == 1 && x.scalar_type() == at::kBFloat16, "fp8_quant_rows");
   c10::cuda::CUDAGuard guard(x.device());
@@ -1133,6 +1157,8 @@ TORCH_LIBRARY(mdb200, m) {
   m.def("llm_out_mlp", &llm_out_mlp);
   m.def("llm_decode_attention", &llm_decode_attention);
   m.def("softmax_rows", &softmax_rows);
+  m.def("rms_rope_rows", &rms_rope_rows);
+  m.def("head_gate", &head_gate);
   m.def("fp8_quant_rows", &fp8_quant_rows);
   m.def("fp8_dequant", &fp8_dequant);
   m.def("mx_dequant", &mx_dequant);

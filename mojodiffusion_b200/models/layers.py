@@ -179,8 +179,10 @@ def packed_projection(x: torch.Tensor, linears) -> torch.Tensor:
         lead = x.shape[:-1]
         out = torch.empty(*lead, sum(widths), dtype=x.dtype, device=x.device)
         c = 0
+        # fp8 projections of one input share its quantised rows
+        kw = dict(quantised=ops.fp8_quant_rows(x.reshape(-1, x.shape[-1]))) if all(getattr(l, "shares_quantised_rows", False) for l in linears) else {}
         for l, w in zip(linears, widths):
-            l(x, out=out[..., c:c + w])
+            l(x, out=out[..., c:c + w], **kw)
             c += w
         return out
     return torch.cat([l(x) for l in linears], dim=-1)

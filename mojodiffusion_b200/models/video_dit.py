@@ -46,6 +46,8 @@ class FP8Linear(nn.Module):
     """Linear whose weight is stored as float8_e4m3fn with one fp32 scale per output channel; activations are
     quantised per token on the fly and both scales are applied in the tcgen05 GEMM epilogue."""
 
+    shares_quantised_rows = True
+
     def __init__(self, lin: Linear):
         super().__init__()
         q, s = ops.fp8_quant_rows(lin.weight.detach())
@@ -55,12 +57,8 @@ class FP8Linear(nn.Module):
         self.bias = lin.bias
         self.slots = nn.ModuleList()
 
-    def forward(self, x, act=None, residual=None, gate=None, rows_per_group: int = 1, out=None):
-        y = ops.fp8_linear(x, self.weight, self.weight_scale, self.bias, act, residual, gate, rows_per_group)
-        if out is not None:
-            out.copy_(y)
-            return out
-        return y
+    def forward(self, x, act=None, residual=None, gate=None, rows_per_group: int = 1, out=None, quantised=None):
+        return ops.fp8_linear(x, self.weight, self.weight_scale, self.bias, act, residual, gate, rows_per_group, out=out, quantised=quantised)
 
 
 class MXFP8Linear(nn.Module):
@@ -92,6 +90,14 @@ class MXFP8Linear(nn.Module):
         return y
 
 
+def _fused_rows_ok(qkv: torch.Tensor, D: int, Dh: int, cos, sin) -> bool:
+    """Whether the one-pass q / k norm + rotation covers this projection: inference in bf16 on the GPU, rows of up to 16384
+    columns, heads of a multiple of 16, tables of one row per token."""
+    return (ops.native.use_native(qkv) and not torch.is_grad_enabled() and qkv.dtype == torch.bfloat16 and qkv.is_contiguous() and D <= 16384
+            and D % Dh == 0 and Dh % 16 == 0 and cos is not None and cos.dtype == torch.float32 and cos.dim() == 2 and cos.shape[1] * 2 == Dh
+            and cos.shape[0] >= qkv.shape[1] and cos.is_contiguous() and sin.is_contiguous() and sin.shape == cos.shape and sin.dtype == cos.dtype)
+
+
 class VideoAttention(nn.Module):
     def __init__(self, cfg: VideoDiTConfig, cross: bool, dtype, device):
         super().__init__()
@@ -112,6 +118,11 @@ class VideoAttention(nn.Module):
         H, Dh = cfg.heads, cfg.head_dim
         if not self.cross:
             qkv = packed_projection(x, (self.to_q, self.to_k, self.to_v))
+            if _fused_rows_ok(qkv, D, Dh, cos, sin):
+                # norm over the full width and rotation of q and k in one pass over the packed rows
+                ops.native.ops().rms_rope_rows(qkv.view(B * S, 3 * D), self.q_norm.weight, self.k_norm.weight, cos, sin, D, Dh, 0, D, S, self.q_norm.eps)
+                q, k, v = (qkv[..., i * D:(i + 1) * D].unflatten(-1, (H, Dh)) for i in range(3))
+                return self._gated(ops.attention(q, k, v, kv_len=kv_len), x).reshape(B, S, D)
             q = self.q_norm(qkv[..., 0:D])
             k = self.k_norm(qkv[..., D:2 * D])
             qk = torch.cat((q, k), dim=-1) if (torch.is_grad_enabled() or not x.is_cuda) else None
@@ -128,11 +139,19 @@ class VideoAttention(nn.Module):
             kv = packed_projection(context, (self.to_k, self.to_v))
             k = self.k_norm(kv[..., 0:D]).unflatten(-1, (H, Dh))
             v = kv[..., D:2 * D].unflatten(-1, (H, Dh))
-        o = ops.attention(q, k, v, kv_len=kv_len)
-        if hasattr(self, "to_gate_logits"):
-            g = 2.0 * torch.sigmoid(self.to_gate_logits(x).float())
-            o = (o.float() * g[..., None]).to(x.dtype)
-        return o.reshape(B, S, D)
+        return self._gated(ops.attention(q, k, v, kv_len=kv_len), x).reshape(B, S, D)
+
+    def _gated(self, o, x):
+        """Per-head output gates 2 * sigmoid(logit)."""
+        if not hasattr(self, "to_gate_logits"):
+            return o
+        logit = self.to_gate_logits(x)
+        if (ops.native.use_native(o) and not torch.is_grad_enabled() and o.dtype == logit.dtype == torch.bfloat16 and o.is_contiguous()
+                and self.cfg.head_dim % 8 == 0):
+            ops.native.ops().head_gate(o, logit.reshape(-1, logit.shape[-1]))
+            return o
+        g = 2.0 * torch.sigmoid(logit.float())
+        return (o.float() * g[..., None]).to(x.dtype)
 
 
 class VideoFF(nn.Module):

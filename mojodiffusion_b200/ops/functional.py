@@ -254,22 +254,43 @@ def linear_glu(x, w, bias=None, act="silu", act_on_second: bool = False):
     return y.reshape(*lead, F_)
 
 
-def fp8_linear(x, wq, w_scale, bias=None, act=None, residual=None, gate=None, rows_per_group: int = 1):
+def fp8_linear(x, wq, w_scale, bias=None, act=None, residual=None, gate=None, rows_per_group: int = 1, out=None, quantised=None):
     """fp8 (e4m3) weight and activation GEMM: x is quantised per token on the fly, wq [N, K] float8_e4m3fn with
-    per-output-channel scales w_scale [N]; both scales are applied in the epilogue."""
+    per-output-channel scales w_scale [N]; both scales are applied in the epilogue. ``out``: a buffer (or a column range of
+    one) to write into; ``quantised``: ``fp8_quant_rows`` of x, for several projections of the same rows."""
     lead = x.shape[:-1]
     if not native.use_native(x):
         w = wq.float() * w_scale.float()[:, None]
         xq, xs = ref.fp8_quant_rows(x.reshape(-1, x.shape[-1]))
         xd = xq.float() * xs[:, None]
         r2 = residual.reshape(-1, residual.shape[-1]) if residual is not None else None
-        return ref.linear(xd, w, bias, act, r2, gate, rows_per_group, out_dtype=x.dtype).reshape(*lead, wq.shape[0])
-    x2 = _flat2d(x)
-    xq, xs = _ops().fp8_quant_rows(x2)
+        y = ref.linear(xd, w, bias, act, r2, gate, rows_per_group, out_dtype=x.dtype).reshape(*lead, wq.shape[0])
+        if out is not None:
+            out.copy_(y)
+            return out
+        return y
+    xq, xs = quantised if quantised is not None else _ops().fp8_quant_rows(_flat2d(x))
     r2 = _flat2d(residual) if residual is not None else None
+    # a column range of a packed buffer is written in place when its rows are evenly spaced
+    o2 = _rows_view(out) if out is not None else None
     y = _gemm([xq], [wq], bias=bias, residual=r2, gate=gate, rows_per_group=rows_per_group, act=act_code(act),
-              row_scale=xs, col_scale=w_scale)
-    return y.reshape(*lead, wq.shape[0])
+              row_scale=xs, col_scale=w_scale, out=o2)
+    if out is None:
+        return y.reshape(*lead, wq.shape[0])
+    if o2 is None:
+        out.copy_(y.reshape(out.shape))
+    return out
+
+
+def _rows_view(t: torch.Tensor) -> Optional[torch.Tensor]:
+    """[..., N] as [rows, N] without a copy, or None when the leading dimensions have no common stride or the GEMM cannot
+    store there (bf16 rows with contiguous columns)."""
+    if t.dtype != torch.bfloat16 or t.stride(-1) != 1:
+        return None
+    try:
+        return t.view(-1, t.shape[-1])
+    except RuntimeError:
+        return None
 
 
 # --------------------------------------------------------------------------------------------

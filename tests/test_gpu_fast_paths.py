@@ -203,3 +203,39 @@ def test_softmax_rows(cols):
     keep = [0, 1, 2, 4, 5, 6]
     # bf16 rounding (2^-9) and the exponential's and sum's 1e-5, doubled
     assert bool(((p[keep][:, :cols].double() - want[keep]).abs() <= want[keep] * 2 * (2.0 ** -9 + 1e-5) + 1e-38).all())
+
+
+# one-pass q / k norm + rotation and the head gates against the fp32 module on the CPU: one and several heads per thread block
+# step, two samples (rotary rows repeat), a token count off every tile
+@pytest.mark.parametrize("hidden,heads,head_dim", [(256, 4, 64), (384, 3, 128), (4352, 34, 128)])
+def test_video_attention_rows(hidden, heads, head_dim):
+    from mojodiffusion_b200.models.video_dit import VideoAttention, VideoDiTConfig
+    axes = (head_dim // 2, head_dim // 4, head_dim // 4)
+    cfg = VideoDiTConfig(hidden=hidden, heads=heads, head_dim=head_dim, axes_dim=axes)
+    att = VideoAttention(cfg, False, torch.bfloat16, DEV)
+    with torch.no_grad():
+        for i, (n, p) in enumerate(att.named_parameters()):
+            p.copy_(_rand(*p.shape, seed=i, scale=p.shape[-1] ** -0.5) if p.dim() == 2 else _rand(*p.shape, seed=i, scale=0.1) + (1.0 if "norm" in n else 0.0))
+        ids = torch.stack(torch.meshgrid(torch.arange(3.), torch.arange(5.), torch.arange(7.), indexing="ij"), -1).reshape(-1, 3)
+        cos, sin = O.rope_table(ids.to(DEV), axes, 10000.0)
+        x = _rand(2, 105, hidden, seed=50)
+        out = att(x, None, cos, sin)
+        native.check_status(out)
+        cpu = VideoAttention(cfg, False, torch.float32, None)
+        cpu.load_state_dict({k: v.float().cpu() for k, v in att.state_dict().items()})
+        want = cpu(x.float().cpu(), None, cos.cpu(), sin.cpu())
+    # projections, q / k, probabilities, attention and gated output are rounded to bf16 once each: five in quadrature, doubled
+    assert float((out.float().cpu() - want).norm() / want.norm()) < 2 * 2.0 ** -9 * (5 / 3) ** 0.5
+
+
+def test_fp8_projections_share_quantised_rows():
+    from mojodiffusion_b200.models.layers import Linear, packed_projection
+    from mojodiffusion_b200.models.video_dit import FP8Linear
+    lins = [FP8Linear(Linear(384, n, True, torch.bfloat16, DEV)) for n in (256, 64, 128)]
+    for shape in ((2, 150, 384), (5, 384)):
+        x = _rand(*shape, seed=1)
+        with torch.no_grad():
+            got = packed_projection(x, lins)
+            want = torch.cat([l(x) for l in lins], -1)
+        native.check_status(got)
+        assert torch.equal(got, want)
