@@ -203,6 +203,29 @@ Tensor gemm(std::vector<Tensor> As, std::vector<Tensor> Bs, const optional<Tenso
   return out;
 }
 
+// The products of one adapted linear layer, y = x w^T + bias + (x A^T) B^T, issued from one call per direction: a training step
+// has hundreds of such layers of a few 10-microsecond launches each, and the call overhead of every product was longer than
+// the product. B carries the adapter's scale; alpha repeats it for dB.
+Tensor gemm_plain(std::vector<Tensor> As, std::vector<Tensor> Bs, const optional<Tensor>& bias, bool a_mn, bool b_mn, double alpha) {
+  return gemm(std::move(As), std::move(Bs), bias, c10::nullopt, c10::nullopt, 1, 0, 0, 0, c10::nullopt, false, a_mn, b_mn, c10::nullopt, c10::nullopt,
+              alpha, false, 0, c10::nullopt, {}, {}, {}, {}, c10::nullopt, c10::nullopt, 0);
+}
+std::tuple<Tensor, Tensor> lora_linear_fwd(const Tensor& x, const Tensor& w, const optional<Tensor>& bias, const Tensor& A, const Tensor& B) {
+  Tensor t = gemm_plain({x}, {A}, c10::nullopt, false, false, 1.0);
+  Tensor y = gemm_plain({x, t}, {w, B}, bias, false, false, 1.0);
+  return {y, t};
+}
+// -> (dx, dA, dB), those not asked for undefined
+std::tuple<Tensor, Tensor, Tensor> lora_linear_bwd(const Tensor& dy, const Tensor& x, const Tensor& w, const Tensor& A, const Tensor& B, const Tensor& t,
+                                                   double alpha, bool need_dx, bool need_dA, bool need_dB) {
+  Tensor dx, dA, dB, dt;
+  if (need_dx || need_dA) dt = gemm_plain({dy}, {B}, c10::nullopt, false, true, 1.0);
+  if (need_dx) dx = gemm_plain({dy, dt}, {w, A}, c10::nullopt, false, true, 1.0);
+  if (need_dA) dA = gemm_plain({dt}, {x}, c10::nullopt, true, true, 1.0);
+  if (need_dB) dB = gemm_plain({dy}, {t}, c10::nullopt, true, true, alpha);
+  return {dx, dA, dB};
+}
+
 // x: NHWC bf16 [N, H, W, Cin]; w: [Cout, KH, KW, Cin] bf16; "same"-style padding (pad_h, pad_w). stride 2 (3 x 3 only) keeps
 // the output pixels offset, offset + 2, ... of the stride-1 result.
 Tensor conv2d_nhwc_strided(const Tensor& x, const Tensor& w, const optional<Tensor>& bias, int64_t pad_h, int64_t pad_w,
@@ -1127,6 +1150,8 @@ TORCH_LIBRARY(mdb200, m) {
   m.def("launch_count", &launch_count);
   m.def("gemm_pair_capacity", &gemm_pair_capacity);
   m.def("gemm", &gemm);
+  m.def("lora_linear_fwd", &lora_linear_fwd);
+  m.def("lora_linear_bwd", &lora_linear_bwd);
   m.def("conv2d_nhwc", &conv2d_nhwc);
   m.def("conv2d_nhwc_strided", &conv2d_nhwc_strided);
   m.def("group_norm_nhwc", &group_norm_nhwc);

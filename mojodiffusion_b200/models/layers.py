@@ -89,7 +89,8 @@ class Linear(nn.Module):
         slots: List[LoRASlot] = list(self.slots)
         if len(slots) == 1 and slots[0].row0 == 0 and slots[0].row1 == self.out_features:
             s = slots[0]
-            return s.down, s.up * (s.scale * self.lora_multiplier)
+            scale = s.scale * self.lora_multiplier
+            return s.down, s.up if scale == 1.0 else s.up * scale
         down = torch.cat([s.down for s in slots], 0)
         R = down.shape[0]
         places, c0 = [], 0

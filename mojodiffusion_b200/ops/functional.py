@@ -78,9 +78,8 @@ class _LoraLinearFn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x2, w, bias, A, B, scale):
-        t = _gemm_skinny(x2, A)                    # [M, r]
         Bs = B if scale == 1.0 else (B.float() * scale).to(B.dtype)       # [N, r]
-        y = _gemm([x2, t], [w, Bs], bias=bias)
+        y, t = _ops().lora_linear_fwd(x2, w, bias, A, Bs)                 # t [M, r]
         ctx.save_for_backward(x2, w, A, B, t, Bs)
         ctx.scale = scale
         ctx.has_bias = bias is not None
@@ -90,18 +89,13 @@ class _LoraLinearFn(torch.autograd.Function):
     def backward(ctx, dy):
         x2, w, A, B, t, Bs = ctx.saved_tensors
         dy = _flat2d(dy)
-        dx = dw = db = dA = dB = None
-        dt = _gemm_skinny(dy, Bs, b_mn=True)       # [M, r] (already scaled)
-        if ctx.needs_input_grad[0]:
-            dx = _gemm([dy, dt], [w, A], b_mn=True)
+        dw = db = None
+        need = ctx.needs_input_grad
+        dx, dA, dB = _ops().lora_linear_bwd(dy, x2, w, A, Bs, t, ctx.scale, need[0], need[3], need[4])
         if ctx.needs_input_grad[1]:
             dw = _gemm([dy], [x2], a_mn=True, b_mn=True)
         if ctx.has_bias and ctx.needs_input_grad[2]:
             db = dy.float().sum(0).to(dy.dtype)
-        if ctx.needs_input_grad[3]:
-            dA = _gemm_skinny(dt, x2, a_mn=True, b_mn=True)           # [r, K]
-        if ctx.needs_input_grad[4]:
-            dB = _gemm_skinny(dy, t, a_mn=True, b_mn=True, alpha=ctx.scale)  # [N, r]
         return dx, dw, db, dA, dB, None
 
 
