@@ -1419,33 +1419,37 @@ extern "C" int mdb_gemm_launch(const MdbGemmArgs* a, cudaStream_t stream) {
       bn = 256;
     }
   }
-  // Few tiles for the SMs there are: compare waves x K steps x time per step (cycles) of the tiling chosen above with narrower
-  // lone tiles and with clusters that share a tile's reduction. A step of a lone tile costs 726 / 400 / 232 cycles at 256 /
-  // 128 / 64 columns; filling the pipeline, meeting in shared memory and finishing the rows costs a split tile about 3000
-  // cycles more than it saves per step, which is why short reductions stay whole.
+  // Few tiles for the SMs there are: compare the tiling chosen above with clusters that share a tile's reduction, in cycles. A 64-wide K step costs 533 cycles on a pair, 726 / 600 / 600 on a lone CTA of 256 / 128 / 64
+  // columns (measured; a 64-wide MMA issues no faster than a wider one). The epilogue of a whole-K tile takes about 5000 cycles per 128 columns of a CTA and hides behind the next
+  // tile's steps only, and rows whose length is no multiple of 32 columns leave its vector path (20000 cycles: adapters of rank
+  // 16). Starting a tile costs about 2500; meeting in shared memory and finishing the rows 5000, or 10000 for a pair's tile.
   int splits = 0;
+  bool pair_split = false;
   if (auto_tile && pair_mode() != 0 && a->kind == 0 && a->conv_taps <= 0 && a->gather_world <= 1 && a->split_k == 0 && !paired && !a->row_scale &&
       !a->col_scale && a->route_owner_cols <= 0 && a->reduce_rows_per_owner <= 0 && !a->prof && !(a->a_mn && !a->b_mn)) {
     int kb = 0;
     for (int s = 0; s < a->num_seg; ++s) kb += static_cast<int>((a->K[s] + 63) / 64);
     const long long tm = (a->M + BM - 1) / BM;
     auto tiles_of = [&](int w) { return tm * ((a->N + w - 1) / w); };
-    auto step_of = [](int w) { return w == 256 ? 726.0 : w == 128 ? 400.0 : 232.0; };
+    auto step_of = [](int w) { return w == 256 ? 726.0 : 600.0; };
+    auto whole = [&](long long tiles, int width, double step, double cols) {
+      const double epi = cols / 128 * 5000.0 + (a->N % 32 != 0 && a->N < 256 ? 20000.0 : 0.0), main = kb * step;
+      return static_cast<double>((tiles + width - 1) / width) * (main > epi ? main : epi) + epi + 2500.0;
+    };
     const long long pt = static_cast<long long>((a->M + 2 * BM - 1) / (2 * BM)) * ((a->N + 255) / 256);
-    const int pairs = pair_capacity(sms);
-    double best = use_pair ? static_cast<double>((pt + pairs - 1) / pairs) * kb * 523.0
-                           : static_cast<double>((tiles_of(bn) + sms - 1) / sms) * kb * step_of(bn);
+    double best = use_pair ? whole(pt, pair_capacity(sms), 533.0, 256) : whole(tiles_of(bn), sms, step_of(bn), bn);
     best *= 0.95;                                              // the whole-K tilings need no meeting: they win ties
-    if (use_pair || bn != 64) {
-      const double c = static_cast<double>((tiles_of(64) + sms - 1) / sms) * kb * step_of(64);
-      if (c < best) { best = c; bn = 64; use_pair = false; }
-    }
     for (int w = 128; w >= 64; w -= 64)
-      for (int sp = 2; sp <= SPLIT_MAX && kb / sp >= 4; ++sp) {
+      for (int sp = 1; sp <= SPLIT_MAX && (sp == 1 || kb / sp >= 4); ++sp) {
         const int cap = w == 128 ? split_capacity<128>(sp, sms) : split_capacity<64>(sp, sms);
-        const double c = static_cast<double>((tiles_of(w) + cap - 1) / cap) * (((kb + sp - 1) / sp) * step_of(w) + 3000.0);
+        const double c = static_cast<double>((tiles_of(w) + cap - 1) / cap) * (((kb + sp - 1) / sp) * step_of(w) + 7500.0);
         if (c < best) { best = c; bn = w; splits = sp; use_pair = false; }
       }
+    for (int sp = 2; sp <= PSPLIT_MAX && kb / sp >= 4 && !a->a_mn && a->M > BM; ++sp) {
+      const int cap = pair_split_capacity(sp, sms);
+      const double c = static_cast<double>((pt + cap - 1) / cap) * (((kb + sp - 1) / sp) * 533.0 + 12500.0);
+      if (c < best) { best = c; bn = 256; splits = sp; use_pair = false; pair_split = true; }
+    }
   }
   // 3 x 3 convolutions: pair tiles of 2 patches x 256 / 128 / 64 channels or lone CTAs, by waves x time per 64-wide K step
   int conv_pair = 0;
@@ -1598,7 +1602,8 @@ extern "C" int mdb_gemm_launch(const MdbGemmArgs* a, cudaStream_t stream) {
     if (conv_pair == 128) return launch_conv_pair<128, false>(maps, p, sms, stream);
     return launch_conv_pair<64, false>(maps, p, sms, stream);
   }
-  if (splits > 1) {
+  if (pair_split) return a->b_mn ? launch_pair_split<true>(maps, p, splits, stream) : launch_pair_split<false>(maps, p, splits, stream);
+  if (splits > 0) {
     if (!a->a_mn && !a->b_mn) return bn == 128 ? launch_split<128, false, false>(maps, p, splits, stream) : launch_split<64, false, false>(maps, p, splits, stream);
     if (!a->a_mn) return bn == 128 ? launch_split<128, false, true>(maps, p, splits, stream) : launch_split<64, false, true>(maps, p, splits, stream);
     return bn == 128 ? launch_split<128, true, true>(maps, p, splits, stream) : launch_split<64, true, true>(maps, p, splits, stream);

@@ -130,7 +130,8 @@ def test_few_row_gemm_accumulates_fp32():
 
 # few tiles against a long reduction: the launch shares each tile's K range over a cluster. Rows and columns off the tile, K off
 # the 64-wide step, a second segment that starts inside a share, N below one 8-column group of the finish
-@pytest.mark.parametrize("M,N,K", [(9, 64, 4096), (45, 2560, 9728), (256, 3072, 12288), (200, 40, 3080), (512, 1000, 2056), (130, 20, 8200)])
+@pytest.mark.parametrize("M,N,K", [(9, 64, 4096), (45, 2560, 9728), (256, 3072, 12288), (200, 40, 3080), (512, 1000, 2056), (130, 20, 8200), (512, 3072, 15360),
+                                   (300, 3000, 6200)])
 def test_cluster_split_k(M, N, K):
     from mojodiffusion_b200.ops.functional import _gemm
     N8 = (N + 7) // 8 * 8
@@ -239,3 +240,26 @@ def test_fp8_projections_share_quantised_rows():
             want = torch.cat([l(x) for l in lins], -1)
         native.check_status(got)
         assert torch.equal(got, want)
+
+
+# every combination of epilogue terms on whole and ragged tiles of the lone and the pair kernel (N = 1160 leaves 8 columns of a
+# 128-wide group, M = 300 rows beyond a tile; bn 512 is the pair kernel)
+@pytest.mark.parametrize("bn", [128, 256, 512])
+@pytest.mark.parametrize("N", [1152, 1160])
+def test_epilogue_terms(bn, N):
+    from mojodiffusion_b200.ops.functional import _gemm
+    from mojodiffusion_b200.ops.reference import act_code
+    M, K = 300, 200
+    x, w = _rand(M, K, seed=1), _rand(N, K, scale=1 / math.sqrt(K), seed=2)
+    bias, gate, res = _rand(N, seed=7), _rand(2, N, seed=8), _rand(M, N, seed=9)
+    for act in (None, "silu", "gelu_tanh", "gelu"):
+        for b in (None, bias):
+            for g, r in ((None, None), (None, res), (gate, res), (gate, None)):
+                out = _gemm([x], [w], bias=b, residual=r, gate=g, rows_per_group=150, act=act_code(act), bn=bn)
+                want = ref.linear(x, w, b, act, r, g, 150, out_dtype=torch.float32) if g is None or r is not None else \
+                    ref.linear(x, w, b, act, out_dtype=torch.float32) * gate.float().repeat_interleave(150, 0)
+                _close(out, want, f"{bn} {N} {act} bias {b is not None} gate {g is not None} residual {r is not None}", rel=1e-4)
+    for act in ("silu", "gelu_tanh", "gelu"):
+        for second in (0, 1):
+            out = _gemm([x], [w], bias=bias, act=act_code(act), pair_offset=N // 2, act_on_second=second, bn=bn)
+            _close(out, ref.linear_glu(x.float(), w.float(), bias.float(), act, bool(second)), f"paired {bn} {N} {act} {second}", rel=1e-4)
