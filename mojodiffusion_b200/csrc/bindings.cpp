@@ -1153,6 +1153,9 @@ TORCH_LIBRARY(mdb200, m) {
   m.def("lora_linear_fwd", &lora_linear_fwd);
   m.def("lora_linear_bwd", &lora_linear_bwd);
   m.def("conv2d_nhwc", &conv2d_nhwc);
+  m.def("softmax_rows", &softmax_rows);
+  m.def("rms_rope_rows", &rms_rope_rows);
+  m.def("head_gate", &head_gate);
   m.def("conv2d_nhwc_strided", &conv2d_nhwc_strided);
   m.def("group_norm_nhwc", &group_norm_nhwc);
   m.def("group_norm_nhwc_bwd", &group_norm_nhwc_bwd);
@@ -1181,9 +1184,6 @@ TORCH_LIBRARY(mdb200, m) {
   m.def("llm_qkv", &llm_qkv);
   m.def("llm_out_mlp", &llm_out_mlp);
   m.def("llm_decode_attention", &llm_decode_attention);
-  m.def("softmax_rows", &softmax_rows);
-  m.def("rms_rope_rows", &rms_rope_rows);
-  m.def("head_gate", &head_gate);
   m.def("fp8_quant_rows", &fp8_quant_rows);
   m.def("fp8_dequant", &fp8_dequant);
   m.def("mx_dequant", &mx_dequant);

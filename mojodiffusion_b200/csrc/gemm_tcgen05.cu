@@ -33,8 +33,6 @@ constexpr int GATHER_STAGES = 2;          // shared-memory stages of the fused a
 constexpr int GATHER_PIECE = 16384;       // bytes per stage
 constexpr int NUM_THREADS = 224;  // warps: 0 TMA, 1 UMMA issue, 2-5 epilogue, 6 peer gather (all-gather fused GEMM)
 constexpr int CONV_TW = 16, CONV_TH = 8;  // conv mode: one M tile = 8 rows x 16 columns of output pixels
-// time of one 64-wide K step of a convolution's pair tile over that of a lone CTA's 128 x 256 tile (726 cycles)
-constexpr double CONV_PAIR_COST_256 = 0.72, CONV_PAIR_COST_128 = 0.42, CONV_PAIR_COST_64 = 0.26;
 
 struct alignas(64) GemmMaps {
   CUtensorMap a[MDB_GEMM_MAX_SEG];
@@ -998,14 +996,14 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_con
 
 // ---------------------------------------------------------------------------------
 // 3 x 3 convolution on CTA pairs: each CTA owns one 8 x 16 patch of output pixels (128 rows of the implicit GEMM), the pair
-// shares a BN-channel tile of the filter (BN / 2 rows staged by each CTA, cta_group::2).
+// shares a 256- or 128-channel tile of the filter (half of its rows staged by each CTA, cta_group::2).
 // What bounds the convolution is how many bytes an SM takes in per multiply-add: about 64 bytes per clock, while a lone CTA
 // re-reads its 16 KB patch for every filter tap next to 32 KB of filter (726 cycles per 128 x 256 x 64 step where the tensor
 // core needs 512). Here the three vertical taps of a column kw share one staged box of 10 x 16 pixels: tap kh starts
 // kh * 16 rows (2048 bytes, a whole number of swizzle atoms) into it. Per three taps a CTA takes in 20 KB of pixels instead
 // of 48, and half of the filter tile. With HALO = false (stride 2, where neighbouring taps share no pixels) every tap
 // loads its own box through a tensor map with element strides.
-// Measured (B200): FLUX autoencoder decode to 1024 x 1024 23.3 -> 17.5 ms, encode of three 488 x 712 images 13.0 -> 8.8 ms.
+// Measured (B200), convolutions alone: 1024 x 1024 decode 13.4 -> 7.2 ms (1.42 PFLOP/s), encode of three 488 x 712 images 8.4 -> 3.8 ms.
 // Work order: channel tiles of one pair of patches are neighbours in the tile order, so the patch comes from L2 once.
 // ---------------------------------------------------------------------------------
 template <int BN, bool HALO>
@@ -1014,8 +1012,8 @@ struct ConvPairShape {
   static constexpr int TAPS = HALO ? 3 : 1;                            // taps served by one staged pixel box
   static constexpr int A_BYTES = (HALO ? CONV_TH + 2 : CONV_TH) * CONV_TW * BK_BYTES;
   static constexpr int B_BYTES = BNH * BK_BYTES;
-  static constexpr int A_STAGES = HALO ? (BN == 256 ? 3 : 5) : (BN == 256 ? 5 : 8);
-  static constexpr int B_STAGES = BN == 256 ? 7 : 8;
+  static constexpr int A_STAGES = HALO ? (BN == 256 ? 3 : 5) : 5;
+  static constexpr int B_STAGES = HALO ? (BN == 256 ? 7 : 8) : 6;
   static constexpr int SMEM = A_STAGES * A_BYTES + B_STAGES * B_BYTES + 4 * 8192 + 1024;
   static_assert(SMEM <= 227 * 1024, "pipeline exceeds the shared memory of an SM");
   static_assert(B_BYTES % 1024 == 0 && A_BYTES % 1024 == 0, "stages start on swizzle atoms");
@@ -1451,29 +1449,22 @@ extern "C" int mdb_gemm_launch(const MdbGemmArgs* a, cudaStream_t stream) {
       if (c < best) { best = c; bn = 256; splits = sp; use_pair = false; pair_split = true; }
     }
   }
-  // 3 x 3 convolutions: pair tiles of 2 patches x 256 / 128 / 64 channels or lone CTAs, by waves x time per 64-wide K step
-  int conv_pair = 0;
+  // 3 x 3 convolutions: waves x time of one 64-wide K step (726 cycles of a lone CTA's 128 x 256 tile = 1; a pair's tile of two
+  // patches x 256 channels takes 533). The 128-wide pair tile serves layers of up to 128 channels only: it saves a sixth (383 us
+  // against 440 for 128 -> 128 at 1024 x 1024), because a narrower MMA issues no faster; small images stay on lone CTAs.
+  bool conv_pair = false;
   const int conv_stride = a->conv_taps > 0 && a->conv_stride > 1 ? a->conv_stride : 1;
   if (a->conv_taps > 0) {
-    const int patches = a->conv_n * ((a->conv_h + CONV_TH - 1) / CONV_TH) * ((a->conv_w + CONV_TW - 1) / CONV_TW);
-    const bool ok3 = a->conv_taps == 9 && a->conv_kw == 3 && auto_tile && a->kind == 0 && !a->out_fp32 && pair_mode() != 0;
     if (conv_stride > 1 && (conv_stride != 2 || a->conv_taps != 9 || a->conv_kw != 3)) return -11;
-    if (ok3 || conv_stride > 1) {
-      const int pairs = pair_capacity(sms);
-      const long long pt = (patches + 1) / 2;
-      const int w_of[3] = {256, 128, 64};
-      const double c_of[3] = {CONV_PAIR_COST_256, CONV_PAIR_COST_128, CONV_PAIR_COST_64};
-      double best = 1e30;
-      for (int i = 0; i < 3; ++i) {
-        const long long t = pt * ((a->N + w_of[i] - 1) / w_of[i]);
-        const double c = static_cast<double>((t + pairs - 1) / pairs) * c_of[i];
-        if (c < best) { best = c; conv_pair = w_of[i]; }
-      }
-      const long long t1 = static_cast<long long>(patches) * ((a->N + bn - 1) / bn);
-      const double lone = static_cast<double>((t1 + sms - 1) / sms) * (bn == 256 ? 1.0 : bn == 128 ? 0.55 : 0.32);
-      if (conv_stride == 1 && lone < best) conv_pair = 0;
-      if (conv_pair) bn = conv_pair;       // box of the filter's tensor map: bn / 2 rows
-    }
+    const long long patches = static_cast<long long>(a->conv_n) * ((a->conv_h + CONV_TH - 1) / CONV_TH) * ((a->conv_w + CONV_TW - 1) / CONV_TW);
+    const int pairs = pair_capacity(sms);
+    const int wide = a->N > 128 || conv_stride > 1 ? 256 : 128;
+    const long long t_pair = (patches + 1) / 2 * ((a->N + wide - 1) / wide), t_lone = patches * ((a->N + bn - 1) / bn);
+    const double pair = static_cast<double>((t_pair + pairs - 1) / pairs) * (wide == 256 ? 0.73 : 0.62);
+    const double lone = static_cast<double>((t_lone + sms - 1) / sms) * (bn == 256 ? 1.0 : bn == 128 ? 0.83 : 0.62);
+    conv_pair = conv_stride > 1 ||
+                (a->conv_taps == 9 && a->conv_kw == 3 && auto_tile && a->kind == 0 && !a->out_fp32 && pair_mode() != 0 && pair <= lone);
+    if (conv_pair) bn = wide;    // filter box: half of the tile's rows
   }
   GemmMaps maps;
   GemmParams p;
@@ -1592,15 +1583,9 @@ extern "C" int mdb_gemm_launch(const MdbGemmArgs* a, cudaStream_t stream) {
   p.route_row_offset_b = a->route_row_offset_b;
   if (a->route_owner_cols > 0 && ((a->route_owner_cols % 32) || (p.route_part_cols % a->route_owner_cols))) return -5;
 
-  if (conv_pair && conv_stride == 1) {
-    if (conv_pair == 256) return launch_conv_pair<256, true>(maps, p, sms, stream);
-    if (conv_pair == 128) return launch_conv_pair<128, true>(maps, p, sms, stream);
-    return launch_conv_pair<64, true>(maps, p, sms, stream);
-  }
   if (conv_pair) {
-    if (conv_pair == 256) return launch_conv_pair<256, false>(maps, p, sms, stream);
-    if (conv_pair == 128) return launch_conv_pair<128, false>(maps, p, sms, stream);
-    return launch_conv_pair<64, false>(maps, p, sms, stream);
+    if (conv_stride > 1) return launch_conv_pair<256, false>(maps, p, sms, stream);
+    return bn == 256 ? launch_conv_pair<256, true>(maps, p, sms, stream) : launch_conv_pair<128, true>(maps, p, sms, stream);
   }
   if (pair_split) return a->b_mn ? launch_pair_split<true>(maps, p, splits, stream) : launch_pair_split<false>(maps, p, splits, stream);
   if (splits > 0) {

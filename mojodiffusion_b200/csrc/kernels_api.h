@@ -66,15 +66,6 @@ int mdb_rms_rope_rows(void* buf, const void* wq, const void* wk, const float* co
 // o[row, h, :] *= 2 * sigmoid(logit[row, h]) in place
 int mdb_head_gate(void* o, const void* logit, long long rows, int H, int Dh, long long ld_logit, cudaStream_t st);
 
-// ---- fused_rows.cu
-// P = softmax(S * scale) per row; leading dimensions multiples of 4 that cover the last partial group of four columns
-int mdb_softmax_rows(const float* s, void* p, long long rows, int cols, long long lds, long long ldp, float scale, cudaStream_t st);
-// in place on rows of a packed buffer: full-width RMSNorm (D columns from q_off and from k_off) + split-half rotation per head
-int mdb_rms_rope_rows(void* buf, const void* wq, const void* wk, const float* cosv, const float* sinv, long long rows, long long ld, int D,
-                      int Dh, int q_off, int k_off, int rows_per_batch, float eps, cudaStream_t st);
-// o[row, h, :] *= 2 * sigmoid(logit[row, h]) in place
-int mdb_head_gate(void* o, const void* logit, long long rows, int H, int Dh, long long ld_logit, cudaStream_t st);
-
 // ---- pointwise.cu
 int mdb_act_fwd(const void* x, void* y, const void* bias, long long n, int cols, int act, cudaStream_t st);
 int mdb_act_bwd(const void* x, const void* dy, void* dx, const void* bias, long long n, int cols, int act,

@@ -72,7 +72,7 @@ def test_conv3x3_many_tiles_per_cluster():
 
 
 # one patch (its partner of the pair lies past the batch), images smaller than a patch, ragged edges both ways, an odd number of
-# patches; 8 / 64, 128 / 320 and 512 / 648 output channels take the 64-, 128- and 256-wide tiles on some of the sizes
+# patches; output channels below, at and beyond one 256-wide tile
 @pytest.mark.parametrize("N,H,W", [(1, 8, 16), (1, 5, 3), (2, 17, 33), (1, 9, 47), (3, 31, 50)])
 @pytest.mark.parametrize("Cin,Cout", [(64, 8), (128, 64), (64, 128), (192, 320), (128, 512), (64, 648)])
 def test_conv3x3_pair_tiles(N, H, W, Cin, Cout):
@@ -126,27 +126,6 @@ def test_few_row_gemm_accumulates_fp32():
         _gemm([x], [w], out=out, out_fp32=True, accumulate=True)
         native.check_status(out)
         assert float((out - want).abs().max()) < 2e-5 * float(want.abs().max()), M
-
-
-# few tiles against a long reduction: the launch shares each tile's K range over a cluster. Rows and columns off the tile, K off
-# the 64-wide step, a second segment that starts inside a share, N below one 8-column group of the finish
-@pytest.mark.parametrize("M,N,K", [(9, 64, 4096), (45, 2560, 9728), (256, 3072, 12288), (200, 40, 3080), (512, 1000, 2056), (130, 20, 8200), (512, 3072, 15360),
-                                   (300, 3000, 6200)])
-def test_cluster_split_k(M, N, K):
-    from mojodiffusion_b200.ops.functional import _gemm
-    N8 = (N + 7) // 8 * 8
-    x, w = _rand(M, K, seed=1), _rand(N8, K, scale=1 / math.sqrt(K), seed=2)
-    bias, gate, res = _rand(N, seed=7), _rand(2, N8, seed=8)[:, :N], _rand(M, N8, seed=9)[:, :N]
-    want = x.float() @ w[:N].float().t()
-    _close(_gemm([x], [w[:N]]), want, "plain")
-    _close(_gemm([x], [w[:N]], out_fp32=True), want, "fp32 out")
-    x2, w2 = _rand(M, 16, seed=3), _rand(N, 16, scale=0.1, seed=4)
-    full = ref.linear(x, w[:N], bias, "gelu_tanh", res, gate, (M + 1) // 2, [(x2, w2)], out_dtype=torch.float32)
-    _close(_gemm([x, x2], [w[:N], w2], bias=bias, residual=res, gate=gate, rows_per_group=(M + 1) // 2, act=1), full, "epilogue", rel=1e-4)
-    _close(_gemm([x], [w.t().contiguous()], b_mn=True), x.float() @ w.float().t(), "B read transposed")
-    M8 = (M + 7) // 8 * 8
-    xt = _rand(K, M8, seed=5)
-    _close(_gemm([xt], [w.t().contiguous()], a_mn=True, b_mn=True, alpha=0.5), 0.5 * xt.float().t() @ w.float().t(), "both read transposed", rel=1e-4)
 
 
 # groups of 3 / 4 / 10 / 80 channels, slabs of whole groups beyond 2048 channels, one pixel, images that end inside a chunk
@@ -240,6 +219,27 @@ def test_fp8_projections_share_quantised_rows():
             want = torch.cat([l(x) for l in lins], -1)
         native.check_status(got)
         assert torch.equal(got, want)
+
+
+# few tiles against a long reduction: the launch shares each tile's K range over a cluster. Rows and columns off the tile, K off
+# the 64-wide step, a second segment that starts inside a share, N below one 8-column group of the finish
+@pytest.mark.parametrize("M,N,K", [(9, 64, 4096), (45, 2560, 9728), (256, 3072, 12288), (200, 40, 3080), (512, 1000, 2056), (130, 20, 8200), (512, 3072, 15360),
+                                   (300, 3000, 6200)])
+def test_cluster_split_k(M, N, K):
+    from mojodiffusion_b200.ops.functional import _gemm
+    N8 = (N + 7) // 8 * 8
+    x, w = _rand(M, K, seed=1), _rand(N8, K, scale=1 / math.sqrt(K), seed=2)
+    bias, gate, res = _rand(N, seed=7), _rand(2, N8, seed=8)[:, :N], _rand(M, N8, seed=9)[:, :N]
+    want = x.float() @ w[:N].float().t()
+    _close(_gemm([x], [w[:N]]), want, "plain")
+    _close(_gemm([x], [w[:N]], out_fp32=True), want, "fp32 out")
+    x2, w2 = _rand(M, 16, seed=3), _rand(N, 16, scale=0.1, seed=4)
+    full = ref.linear(x, w[:N], bias, "gelu_tanh", res, gate, (M + 1) // 2, [(x2, w2)], out_dtype=torch.float32)
+    _close(_gemm([x, x2], [w[:N], w2], bias=bias, residual=res, gate=gate, rows_per_group=(M + 1) // 2, act=1), full, "epilogue", rel=1e-4)
+    _close(_gemm([x], [w.t().contiguous()], b_mn=True), x.float() @ w.float().t(), "B read transposed")
+    M8 = (M + 7) // 8 * 8
+    xt = _rand(K, M8, seed=5)
+    _close(_gemm([xt], [w.t().contiguous()], a_mn=True, b_mn=True, alpha=0.5), 0.5 * xt.float().t() @ w.float().t(), "both read transposed", rel=1e-4)
 
 
 # every combination of epilogue terms on whole and ragged tiles of the lone and the pair kernel (N = 1160 leaves 8 columns of a
