@@ -289,14 +289,16 @@ __device__ __forceinline__ void epilogue_row32(const GemmParams& p, int row, int
 }
 
 // Epilogue of one accumulator tile for one warp (its 32 TMEM lanes = 32 output rows). bf16 outputs whose tile lies fully
-// inside the matrix go through an 8 KB per-warp staging buffer in shared memory, 128 columns at a time: every lane packs
-// its row's slabs into the buffer, then the warp stores whole 256-byte row segments (16 lanes x 16 bytes per row, two
-// rows per instruction). Local stores become full cache lines and peer-routed stores (sequence-parallel scatter, staged
-// reduce-scatter) cross NVLink as 256-byte writes instead of 64-byte fragments of 32 different rows. Everything else
-// (fp32 outputs, ragged edges, unaligned pointers) keeps the direct per-lane stores.
+// inside the matrix go through a per-warp staging buffer in shared memory (32 rows of GW columns), GW columns at a time: every
+// lane packs its row's slabs into the buffer, then the warp stores whole row segments of 2 * GW bytes (GW / 8 lanes x 16 bytes
+// per row). Local stores become full cache lines and peer-routed stores (sequence-parallel scatter, staged reduce-scatter) cross
+// NVLink as 128- or 256-byte writes instead of 64-byte fragments of 32 different rows. Everything else (fp32 outputs, ragged
+// edges, unaligned pointers) keeps the direct per-lane stores.
+template <int GW>
 __device__ __forceinline__ void epilogue_tile(const GemmParams& p, uint32_t taddr, int pair_col_off, int row, int n0,
                                               int out_cols, bool paired, bool aligned, uint8_t* stage_warp, int lane) {
-  const bool staged = stage_warp != nullptr && aligned && !p.out_fp32 && (out_cols & 127) == 0 && n0 + out_cols <= p.N;
+  constexpr int CH = GW / 8;                                    // 16-byte chunks of a staged row
+  const bool staged = stage_warp != nullptr && aligned && !p.out_fp32 && out_cols % GW == 0 && n0 + out_cols <= p.N;
   if (!staged) {
 #pragma unroll 1
     for (int c = 0; c < out_cols / 32; ++c) {
@@ -308,26 +310,26 @@ __device__ __forceinline__ void epilogue_tile(const GemmParams& p, uint32_t tadd
     }
     return;
   }
-  uint4* my_row = reinterpret_cast<uint4*>(stage_warp + lane * 256);
-  const int swz = lane & 15;
+  uint4* my_row = reinterpret_cast<uint4*>(stage_warp + lane * (2 * GW));
+  const int swz = lane & (CH - 1);
 #pragma unroll 1
-  for (int g = 0; g < out_cols / 128; ++g) {
+  for (int g = 0; g < out_cols / GW; ++g) {
 #pragma unroll 1
-    for (int c = 0; c < 4; ++c) {
+    for (int c = 0; c < GW / 32; ++c) {
       uint32_t r0[32], r1[32];
-      tmem_ld_32x32b_x32(taddr + g * 128 + c * 32, r0);
-      if (paired) tmem_ld_32x32b_x32(taddr + pair_col_off + g * 128 + c * 32, r1);
+      tmem_ld_32x32b_x32(taddr + g * GW + c * 32, r0);
+      if (paired) tmem_ld_32x32b_x32(taddr + pair_col_off + g * GW + c * 32, r1);
       tmem_wait_ld();
-      epilogue_row32(p, row, n0 + g * 128 + c * 32, r0, r1, paired, true, my_row, c * 4, swz);
+      epilogue_row32(p, row, n0 + g * GW + c * 32, r0, r1, paired, true, my_row, c * 4, swz);
     }
     __syncwarp();
-    const int chunk = lane & 15;
+    const int chunk = lane & (CH - 1);
 #pragma unroll 4
-    for (int i = 0; i < 16; ++i) {
-      const int rl = 2 * i + (lane >> 4);                       // row of the warp this lane copies in this pass
+    for (int i = 0; i < CH; ++i) {
+      const int rl = (32 / CH) * i + lane / CH;                 // row of the warp this lane copies in this pass
       const int rr = __shfl_sync(0xffffffffu, row, rl);         // its global output row (p.M or more: not stored)
-      const uint4 v = reinterpret_cast<const uint4*>(stage_warp + rl * 256)[chunk ^ (rl & 15)];
-      if (rr < p.M) *reinterpret_cast<uint4*>(out_slab_ptr(p, rr, n0 + g * 128 + chunk * 8, 2)) = v;
+      const uint4 v = reinterpret_cast<const uint4*>(stage_warp + rl * (2 * GW))[chunk ^ (rl & (CH - 1))];
+      if (rr < p.M) *reinterpret_cast<uint4*>(out_slab_ptr(p, rr, n0 + g * GW + chunk * 8, 2)) = v;
     }
     __syncwarp();
   }
@@ -704,7 +706,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant
       const int out_cols = paired ? BN / 2 : BN;
       // the staging buffers share their 32 KB with the stages of the fused all-gather, which therefore stores directly
       uint8_t* stage_warp = p.gather_world > 1 ? nullptr : smem + STAGES * STAGE_BYTES + quad * 8192;
-      epilogue_tile(p, taddr, BN / 2, row, n0, out_cols, paired, aligned, stage_warp, lane);
+      epilogue_tile<128>(p, taddr, BN / 2, row, n0, out_cols, paired, aligned, stage_warp, lane);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tempty_bar[acc]);
@@ -971,7 +973,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_con
       const int row = m0 + quad * 32 + lane;
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + acc * BN;
       const int out_cols = paired ? BNH : BN;
-      epilogue_tile(p, taddr, BNH, row, n0, out_cols, paired, aligned, smem + STAGES * STAGE_BYTES + quad * 8192, lane);
+      epilogue_tile<128>(p, taddr, BNH, row, n0, out_cols, paired, aligned, smem + STAGES * STAGE_BYTES + quad * 8192, lane);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&tempty_bar[acc]), 0u));
@@ -1004,25 +1006,30 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_con
 // of 48, and half of the filter tile. With HALO = false (stride 2, where neighbouring taps share no pixels) every tap
 // loads its own box through a tensor map with element strides.
 // Measured (B200), convolutions alone: 1024 x 1024 decode 13.4 -> 7.2 ms (1.42 PFLOP/s), encode of three 488 x 712 images 8.4 -> 3.8 ms.
+// RESIDENT (up to 128 input and output channels): all nine taps of the filter fit beside the pixel ring (147 KB per CTA) and are
+// loaded once per CTA instead of once per tile; with them the tile took in 408 KB for 256 pixels and the L2 was the bound
+// (128 -> 128 at 1024 x 1024: 440 -> 355 us).
 // Work order: channel tiles of one pair of patches are neighbours in the tile order, so the patch comes from L2 once.
 // ---------------------------------------------------------------------------------
-template <int BN, bool HALO>
+template <int BN, bool HALO, bool RESIDENT>
 struct ConvPairShape {
+  static_assert(!RESIDENT || (HALO && BN == 128), "the resident filter is that of one 128-channel tile");
   static constexpr int BNH = BN / 2;                                   // filter rows staged by one CTA
   static constexpr int TAPS = HALO ? 3 : 1;                            // taps served by one staged pixel box
   static constexpr int A_BYTES = (HALO ? CONV_TH + 2 : CONV_TH) * CONV_TW * BK_BYTES;
   static constexpr int B_BYTES = BNH * BK_BYTES;
-  static constexpr int A_STAGES = HALO ? (BN == 256 ? 3 : 5) : 5;
-  static constexpr int B_STAGES = HALO ? (BN == 256 ? 7 : 8) : 6;
-  static constexpr int SMEM = A_STAGES * A_BYTES + B_STAGES * B_BYTES + 4 * 8192 + 1024;
+  static constexpr int A_STAGES = RESIDENT ? 3 : HALO ? (BN == 256 ? 3 : 5) : 5;
+  static constexpr int B_STAGES = RESIDENT ? 18 : HALO ? (BN == 256 ? 7 : 8) : 6;
+  static constexpr int STAGE_COLS = RESIDENT ? 64 : 128;               // columns staged at a time by an epilogue warp
+  static constexpr int SMEM = A_STAGES * A_BYTES + B_STAGES * B_BYTES + 4 * 64 * STAGE_COLS + 1024;
   static_assert(SMEM <= 227 * 1024, "pipeline exceeds the shared memory of an SM");
   static_assert(B_BYTES % 1024 == 0 && A_BYTES % 1024 == 0, "stages start on swizzle atoms");
 };
 
-template <int BN, bool HALO>
+template <int BN, bool HALO, bool RESIDENT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
 conv_tcgen05_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ GemmParams p) {
-  using S = ConvPairShape<BN, HALO>;
+  using S = ConvPairShape<BN, HALO, RESIDENT>;
   constexpr int TMEM_COLS = 2 * BN;
   constexpr int KSTEPS = 4, K_ELEMS = 64;
 
@@ -1096,9 +1103,10 @@ conv_tcgen05_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_con
         __syncwarp();
         issued = true;
         if (++as == S::A_STAGES) { as = 0; aph ^= 1u; }
+        if (RESIDENT && tile != cluster_id) continue;                // the filter is there since the first tile
         for (int t = 0; t < S::TAPS; ++t) {
           const int k0 = (((kh0 + t) * 3 + kw) * p.conv_cblocks + cb) * K_ELEMS;
-          if (!__all_sync(0xffffffffu, mbar_wait(&b_empty[bs], bph ^ 1u, &abort_s))) {
+          if (!RESIDENT && !__all_sync(0xffffffffu, mbar_wait(&b_empty[bs], bph ^ 1u, &abort_s))) {
             if (lane == 0) { report_status(p.status, STATUS_TIMEOUT, 32, bs); st_shared_cluster_u32(peer_abort, 1u); }
             ok = false;
             break;
@@ -1136,6 +1144,7 @@ conv_tcgen05_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_con
         const uint32_t d_tmem = tmem_base + acc * BN;
         for (int g = 0; ok && g < groups; ++g) {
           bool got = mbar_wait(&a_full[as], aph, &abort_s);
+          if (RESIDENT) { bs = g * S::TAPS; bph = 0; }               // stage = position in the tile, filled once
           for (int t = 0; t < S::TAPS; ++t) {
             if (!__all_sync(0xffffffffu, got && mbar_wait(&b_full[bs], bph, &abort_s))) {
               if (lane == 0) { report_status(p.status, STATUS_TIMEOUT, 34, bs); st_shared_cluster_u32(peer_abort, 1u); }
@@ -1150,7 +1159,7 @@ conv_tcgen05_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_con
               for (int k = 0; k < KSTEPS; ++k)
                 umma_f16_ss_pair(d_tmem, da + static_cast<uint64_t>((k * 32) >> 4), db + static_cast<uint64_t>((k * 32) >> 4), idesc,
                                  (g | t | k) != 0 ? 1u : 0u);
-              umma_commit_pair(&b_empty[bs], 3);       // the stages are free in both CTAs once these MMAs have read them
+              if (!RESIDENT) umma_commit_pair(&b_empty[bs], 3);   // the stages are free in both CTAs once these MMAs have read them
               if (t == S::TAPS - 1) {
                 umma_commit_pair(&a_empty[as], 3);
                 if (g == groups - 1) umma_commit_pair(&tfull_bar[acc], 3);
@@ -1185,8 +1194,8 @@ conv_tcgen05_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_con
       const int r = quad * 32 + lane;
       const int oh = th * CONV_TH + r / CONV_TW, ow = tw * CONV_TW + r % CONV_TW;
       const int row = (mt < p.conv_tiles_m && oh < p.conv_h && ow < p.conv_w) ? (img * p.conv_h + oh) * p.conv_w + ow : p.M;   // p.M = skipped
-      epilogue_tile(p, tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + acc * BN, 0, row, (tile % tiles_n) * BN, BN, false, aligned,
-                    smem_st + quad * 8192, lane);
+      epilogue_tile<S::STAGE_COLS>(p, tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + acc * BN, 0, row, (tile % tiles_n) * BN, BN, false, aligned,
+                    smem_st + quad * (64 * S::STAGE_COLS), lane);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&tempty_bar[acc]), 0u));
@@ -1335,10 +1344,10 @@ static int launch_pair_variant(const GemmMaps& maps, const GemmParams& p, int nu
   return static_cast<int>(cudaGetLastError());
 }
 
-template <int BN, bool HALO>
+template <int BN, bool HALO, bool RESIDENT>
 static int launch_conv_pair(const GemmMaps& maps, const GemmParams& p, int num_sms, cudaStream_t stream) {
-  constexpr int SMEM = ConvPairShape<BN, HALO>::SMEM;
-  auto kern = conv_tcgen05_pair_kernel<BN, HALO>;
+  constexpr int SMEM = ConvPairShape<BN, HALO, RESIDENT>::SMEM;
+  auto kern = conv_tcgen05_pair_kernel<BN, HALO, RESIDENT>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
   if (e != cudaSuccess) return static_cast<int>(e);
   const long long tiles = static_cast<long long>((p.conv_tiles_m + 1) / 2) * ((p.N + BN - 1) / BN);
@@ -1584,8 +1593,9 @@ extern "C" int mdb_gemm_launch(const MdbGemmArgs* a, cudaStream_t stream) {
   if (a->route_owner_cols > 0 && ((a->route_owner_cols % 32) || (p.route_part_cols % a->route_owner_cols))) return -5;
 
   if (conv_pair) {
-    if (conv_stride > 1) return launch_conv_pair<256, false>(maps, p, sms, stream);
-    return bn == 256 ? launch_conv_pair<256, true>(maps, p, sms, stream) : launch_conv_pair<128, true>(maps, p, sms, stream);
+    if (conv_stride > 1) return launch_conv_pair<256, false, false>(maps, p, sms, stream);
+    if (bn == 256) return launch_conv_pair<256, true, false>(maps, p, sms, stream);
+    return p.conv_cblocks <= 2 ? launch_conv_pair<128, true, true>(maps, p, sms, stream) : launch_conv_pair<128, true, false>(maps, p, sms, stream);
   }
   if (pair_split) return a->b_mn ? launch_pair_split<true>(maps, p, splits, stream) : launch_pair_split<false>(maps, p, splits, stream);
   if (splits > 0) {

@@ -65,7 +65,7 @@ def _conv_ref(x, w, bias, stride=1, offset=0):
 
 def test_conv3x3_many_tiles_per_cluster():
     from mojodiffusion_b200.ops import conv as C
-    for Cin, Cout in ((64, 128), (128, 256)):                  # several tiles per persistent cluster: every ring wraps
+    for Cin, Cout in ((64, 128), (128, 128), (192, 96), (128, 256)):   # several tiles per persistent cluster: every ring wraps
         x, w = _rand(1, 200, 333, Cin, seed=1), _rand(Cout, 3, 3, Cin, scale=1 / math.sqrt(9 * Cin), seed=2)
         with torch.no_grad():
             _close(C.conv2d_nhwc(x, w, _rand(Cout, seed=3)), _conv_ref(x, w, _rand(Cout, seed=3)), f"{Cin} -> {Cout}")
