@@ -263,3 +263,19 @@ def test_epilogue_terms(bn, N):
         for second in (0, 1):
             out = _gemm([x], [w], bias=bias, act=act_code(act), pair_offset=N // 2, act_on_second=second, bn=bn)
             _close(out, ref.linear_glu(x.float(), w.float(), bias.float(), act, bool(second)), f"paired {bn} {N} {act} {second}", rel=1e-4)
+
+
+# rows on the block kernel (2048 .. 16384) give the bytes and scales of the one-warp kernel, which takes the same rows padded with
+# zeros beyond 16384; a zero row, a row with an infinity, strided rows
+@pytest.mark.parametrize("D", [2048, 2056, 4096, 5000, 16384])
+def test_fp8_quant_rows_block(D):
+    x = _rand(37, D, seed=1)
+    x[3] = 0
+    x[4, D - 1] = float("inf")
+    x[5] *= 1e-30
+    pad = torch.zeros(37, 16392, dtype=torch.bfloat16, device=DEV)
+    pad[:, :D] = x
+    wq, ws = torch.ops.mdb200.fp8_quant_rows(pad)
+    for src in (x, pad[:, :D]):
+        q, s = torch.ops.mdb200.fp8_quant_rows(src)
+        assert torch.equal(s, ws) and torch.equal(q.view(torch.uint8), wq[:, :D].contiguous().view(torch.uint8))
