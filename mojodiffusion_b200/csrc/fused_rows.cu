@@ -138,19 +138,19 @@ rms_rope_rows_kernel(__nv_bfloat16* __restrict__ buf, const __nv_bfloat16* __res
     const int i = threadIdx.x + k * NR_THREADS;
     if (i < items) {
       const int h0 = (i % per_head) * 8, c = (i / per_head) * Dh + h0;
+      const uint4 wa = *reinterpret_cast<const uint4*>(w + c), wb = *reinterpret_cast<const uint4*>(w + c + half);
+      const float4 c0 = *reinterpret_cast<const float4*>(cosv + tok + h0), c1 = *reinterpret_cast<const float4*>(cosv + tok + h0 + 4);
+      const float4 s0 = *reinterpret_cast<const float4*>(sinv + tok + h0), s1 = *reinterpret_cast<const float4*>(sinv + tok + h0 + 4);
+      const float cs[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w}, sn[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
+      const uint32_t wa4[4] = {wa.x, wa.y, wa.z, wa.w}, wb4[4] = {wb.x, wb.y, wb.z, wb.w};
       uint32_t u4[4], t4[4];
 #pragma unroll
-      for (int j = 0; j < 8; j += 2) {
-        float ra[2], rb[2];
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const float va = a[k][j + e] * rstd * __bfloat162float(w[c + j + e]), vb = b[k][j + e] * rstd * __bfloat162float(w[c + half + j + e]);
-          const float cs = cosv[tok + h0 + j + e], sn = sinv[tok + h0 + j + e];
-          ra[e] = va * cs - vb * sn;
-          rb[e] = vb * cs + va * sn;
-        }
-        u4[j >> 1] = pack_bf16x2(ra[0], ra[1]);
-        t4[j >> 1] = pack_bf16x2(rb[0], rb[1]);
+      for (int j = 0; j < 4; ++j) {
+        const float2 fa = unpack_bf16x2(wa4[j]), fb = unpack_bf16x2(wb4[j]);
+        const float a0 = a[k][2 * j] * rstd * fa.x, a1 = a[k][2 * j + 1] * rstd * fa.y;
+        const float b0 = b[k][2 * j] * rstd * fb.x, b1 = b[k][2 * j + 1] * rstd * fb.y;
+        u4[j] = pack_bf16x2(a0 * cs[2 * j] - b0 * sn[2 * j], a1 * cs[2 * j + 1] - b1 * sn[2 * j + 1]);
+        t4[j] = pack_bf16x2(b0 * cs[2 * j] + a0 * sn[2 * j], b1 * cs[2 * j + 1] + a1 * sn[2 * j + 1]);
       }
       *reinterpret_cast<uint4*>(x + c) = make_uint4(u4[0], u4[1], u4[2], u4[3]);
       *reinterpret_cast<uint4*>(x + c + half) = make_uint4(t4[0], t4[1], t4[2], t4[3]);
@@ -196,6 +196,7 @@ extern "C" int mdb_softmax_rows(const float* s, void* p, long long rows, int col
 extern "C" int mdb_rms_rope_rows(void* buf, const void* wq, const void* wk, const float* cosv, const float* sinv, long long rows, long long ld, int D,
                                  int Dh, int q_off, int k_off, int rows_per_batch, float eps, cudaStream_t st) {
   if (D % Dh || Dh % 16 || (D >> 4) > NR_THREADS * NR_ITEMS || ld % 8 || q_off % 8 || k_off % 8 || (reinterpret_cast<uintptr_t>(buf) & 15) ||
+      ((reinterpret_cast<uintptr_t>(wq) | reinterpret_cast<uintptr_t>(wk) | reinterpret_cast<uintptr_t>(cosv) | reinterpret_cast<uintptr_t>(sinv)) & 15) ||
       rows_per_batch <= 0 || rows > 2147483647ll)
     return -1;
   if (rows <= 0) return 0;

@@ -90,12 +90,13 @@ class MXFP8Linear(nn.Module):
         return y
 
 
-def _fused_rows_ok(qkv: torch.Tensor, D: int, Dh: int, cos, sin) -> bool:
+def _fused_rows_ok(qkv: torch.Tensor, D: int, Dh: int, cos, sin, wq, wk) -> bool:
     """Whether the one-pass q / k norm + rotation covers this projection: inference in bf16 on the GPU, rows of up to 16384
-    columns, heads of a multiple of 16, tables of one row per token."""
+    columns, heads of a multiple of 16, tables of one row per token, 16-byte aligned operands."""
     return (ops.native.use_native(qkv) and not torch.is_grad_enabled() and qkv.dtype == torch.bfloat16 and qkv.is_contiguous() and D <= 16384
             and D % Dh == 0 and Dh % 16 == 0 and cos is not None and cos.dtype == torch.float32 and cos.dim() == 2 and cos.shape[1] * 2 == Dh
-            and cos.shape[0] >= qkv.shape[1] and cos.is_contiguous() and sin.is_contiguous() and sin.shape == cos.shape and sin.dtype == cos.dtype)
+            and cos.shape[0] >= qkv.shape[1] and cos.is_contiguous() and sin.is_contiguous() and sin.shape == cos.shape and sin.dtype == cos.dtype
+            and all(t.data_ptr() % 16 == 0 for t in (qkv, cos, sin, wq, wk)))
 
 
 class VideoAttention(nn.Module):
@@ -118,7 +119,7 @@ class VideoAttention(nn.Module):
         H, Dh = cfg.heads, cfg.head_dim
         if not self.cross:
             qkv = packed_projection(x, (self.to_q, self.to_k, self.to_v))
-            if _fused_rows_ok(qkv, D, Dh, cos, sin):
+            if _fused_rows_ok(qkv, D, Dh, cos, sin, self.q_norm.weight, self.k_norm.weight):
                 # norm over the full width and rotation of q and k in one pass over the packed rows
                 ops.native.ops().rms_rope_rows(qkv.view(B * S, 3 * D), self.q_norm.weight, self.k_norm.weight, cos, sin, D, Dh, 0, D, S, self.q_norm.eps)
                 q, k, v = (qkv[..., i * D:(i + 1) * D].unflatten(-1, (H, Dh)) for i in range(3))
