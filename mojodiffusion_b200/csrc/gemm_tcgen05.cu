@@ -1459,8 +1459,8 @@ extern "C" int mdb_gemm_launch(const MdbGemmArgs* a, cudaStream_t stream) {
     }
   }
   // 3 x 3 convolutions: waves x time of one 64-wide K step (726 cycles of a lone CTA's 128 x 256 tile = 1; a pair's tile of two
-  // patches x 256 channels takes 533). The 128-wide pair tile serves layers of up to 128 channels only: it saves a sixth (383 us
-  // against 440 for 128 -> 128 at 1024 x 1024), because a narrower MMA issues no faster; small images stay on lone CTAs.
+  // patches x 256 channels takes 533). The 128-wide pair tile serves layers of up to 128 channels only: with its filter
+  // resident it takes 355 us against 440 for 128 -> 128 at 1024 x 1024, no more because a narrower MMA issues no faster; small images stay on lone CTAs.
   bool conv_pair = false;
   const int conv_stride = a->conv_taps > 0 && a->conv_stride > 1 ? a->conv_stride : 1;
   if (a->conv_taps > 0) {
