@@ -75,7 +75,8 @@ typedef struct MdbGemmArgs {
   int reduce_src_rank;
   // Split-K (split_k > 1): the K range is cut into split_k parts, each a separate work item of the persistent grid; the
   // parts are added (red.global.add) into the fp32 output, which the caller has zeroed. One K segment, no epilogue math.
-  // 0: the launch may share a tile's reduction over a cluster (gemm_splitk.cuh) where tiles are few; 1: it may not.
+  // 0: any form, also those that cut K (the few-row kernel, clusters that share a tile's reduction); 1: every output keeps one
+  // accumulator over the whole K range, so that a row does not depend on the number of rows.
   int split_k;
   // Implicit-GEMM convolution (conv_taps = KH*KW > 0): A[0] is an NHWC bf16 image [conv_n, conv_h, conv_w,
   // conv_cin] (conv_cin a multiple of 64), B[0] the filter [N, KH, KW, conv_cin] as a [N, KH*KW*conv_cin] matrix,

@@ -159,9 +159,10 @@ static int launch_rows_any(const RowsParams& p, int sms, bool pair, cudaStream_t
 
 // True when the few-row kernel computes exactly what mdb_gemm_launch was asked for. It reads whole 16-byte vectors along K
 // and rows of 16-byte alignment (what the tensor maps of the tiled kernel also ask for); everything with a scale, a routed /
-// gathered / reduced operand, an MN-major operand or a caller-chosen tile stays on the tiled kernels.
+// gathered / reduced operand, an MN-major operand, a caller-chosen tile or split_k != 0 (1: one accumulator per output, as a
+// longer input has it, while the sums here are joined from 32 lanes) stays on the tiled kernels.
 extern "C" int mdb_gemm_rows_ok(const MdbGemmArgs* a) {
-  if (a->M > MDB_GEMM_ROWS_MAX || a->kind != 0 || a->a_mn || a->b_mn || a->bn != 0 || a->conv_taps > 0 || a->split_k > 1 ||
+  if (a->M > MDB_GEMM_ROWS_MAX || a->kind != 0 || a->a_mn || a->b_mn || a->bn != 0 || a->conv_taps > 0 || a->split_k != 0 ||
       a->gather_world > 1 || a->route_owner_cols > 0 || a->reduce_rows_per_owner > 0 || a->row_scale || a->col_scale || a->prof)
     return 0;
   for (int s = 0; s < a->num_seg; ++s) {

@@ -54,10 +54,11 @@ def _gemm_skinny(A, B, a_mn=False, b_mn=False, alpha=1.0):
 # --------------------------------------------------------------------------------------------
 class _LinearFn(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, x2, w, bias):
+    def forward(ctx, x2, w, bias, whole_k):
         ctx.save_for_backward(x2, w)
         ctx.has_bias = bias is not None
-        return _gemm([x2], [w], bias=bias)
+        ctx.split_k = 1 if whole_k else 0
+        return _gemm([x2], [w], bias=bias, split_k=ctx.split_k)
 
     @staticmethod
     def backward(ctx, dy):
@@ -65,12 +66,12 @@ class _LinearFn(torch.autograd.Function):
         dy = _flat2d(dy)
         dx = dw = db = None
         if ctx.needs_input_grad[0]:
-            dx = _gemm([dy], [w], b_mn=True)
+            dx = _gemm([dy], [w], b_mn=True, split_k=ctx.split_k)
         if ctx.needs_input_grad[1]:
             dw = _gemm([dy], [x2], a_mn=True, b_mn=True)
         if ctx.has_bias and ctx.needs_input_grad[2]:
             db = dy.float().sum(0).to(dy.dtype)
-        return dx, dw, db
+        return dx, dw, db, None
 
 
 class _LoraLinearFn(torch.autograd.Function):
@@ -106,8 +107,9 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None
 
     x: [..., K]; w: [N, K]; gate: [groups, N]; residual: [..., N]. On a GPU without autograd the whole
     expression is one tcgen05 GEMM launch; with autograd the epilogue pieces become separate differentiable ops.
-    ``whole_k``: every output keeps one accumulator over the whole reduction (no split over SMs), so that a row's result does
-    not depend on how many rows come with it.
+    ``whole_k``: every output keeps one accumulator over the whole reduction (no split over SMs or lanes), so that a row's
+    result, and the gradient of a row of x, does not depend on how many rows come with it. Without it the number of rows may
+    choose the order of the sums.
     """
     lead = x.shape[:-1]
     if not native.use_native(x):
@@ -126,7 +128,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None
         pad = torch.nn.functional.pad
         y = linear(pad(x, (0, kp)), pad(w, (0, kp, 0, npad)), pad(bias, (0, npad)) if bias is not None else None, act,
                    pad(residual, (0, npad)) if residual is not None else None,
-                   pad(gate, (0, npad)) if gate is not None else None, rows_per_group)
+                   pad(gate, (0, npad)) if gate is not None else None, rows_per_group, whole_k=whole_k)
         y = y[..., :w.shape[0]]
         if out is not None:
             out.copy_(y)
@@ -142,7 +144,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None
                   gate=gate, rows_per_group=rows_per_group, act=act_code(act), out=o2, split_k=1 if whole_k else 0)
         return out if out is not None else y.reshape(*lead, w.shape[0])
     assert not extra, "extra K segments are an inference-path feature"
-    y = _LinearFn.apply(x2, w, bias)
+    y = _LinearFn.apply(x2, w, bias, whole_k)
     y = activation(y, act)
     if gate is not None or residual is not None:
         r2 = residual.reshape(-1, residual.shape[-1]) if residual is not None else torch.zeros_like(y)

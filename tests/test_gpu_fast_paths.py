@@ -279,3 +279,21 @@ def test_fp8_quant_rows_block(D):
     for src in (x, pad[:, :D]):
         q, s = torch.ops.mdb200.fp8_quant_rows(src)
         assert torch.equal(s, ws) and torch.equal(q.view(torch.uint8), wq[:, :D].contiguous().view(torch.uint8))
+
+
+# a row of linear(whole_k=True) has the same bits whatever rows come with it: few rows, rows that the launch would share over a
+# cluster, and whole tiles; a K and an N that are padded to the 16-byte rule; the autograd route and its input gradient
+@pytest.mark.parametrize("N,K", [(2560, 9728), (512, 8192), (64, 4096), (60, 4100)])
+def test_whole_k_rows_do_not_depend_on_their_number(N, K):
+    x, w, bias, dy = _rand(300, K, seed=1), _rand(N, K, scale=1 / math.sqrt(K), seed=2), _rand(N, seed=3), _rand(300, N, seed=4)
+    full, full_dx = O.linear(x, w, bias, whole_k=True), None
+    _close(full, x.float() @ w.float().t() + bias.float(), f"{N}x{K}", rel=1e-4)
+    for m in (300, 1, 7, 8, 9, 45, 129, 256):
+        assert torch.equal(O.linear(x[:m], w, bias, whole_k=True), full[:m]), m
+        leaf = x[:m].clone().requires_grad_()
+        y = O.linear(leaf, w, bias, whole_k=True)
+        assert torch.equal(y, full[:m]), m
+        y.backward(dy[:m])
+        full_dx = leaf.grad if full_dx is None else full_dx
+        assert torch.equal(leaf.grad, full_dx[:m]), m
+    native.check_status(full)
