@@ -39,7 +39,8 @@ class _Lin(nn.Module):
         self.bias = nn.Parameter(torch.zeros(o, dtype=dtype, device=device)) if bias else None
 
     def forward(self, x):
-        return ops.linear(x, self.weight, self.bias)
+        # one accumulator per output: a token's features do not change with the length of the prompt around it
+        return ops.linear(x, self.weight, self.bias, whole_k=True)
 
 
 class _Attn(nn.Module):

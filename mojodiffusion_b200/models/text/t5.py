@@ -36,7 +36,8 @@ class _W(nn.Module):
         self.weight = nn.Parameter(torch.empty(o, i, dtype=dtype, device=device).normal_(0, 0.02))
 
     def forward(self, x):
-        return ops.linear(x, self.weight)
+        # one accumulator per output: a token's features do not change with the length of the prompt around it
+        return ops.linear(x, self.weight, whole_k=True)
 
 
 class _Norm(nn.Module):

@@ -297,3 +297,15 @@ def test_whole_k_rows_do_not_depend_on_their_number(N, K):
         full_dx = leaf.grad if full_dx is None else full_dx
         assert torch.equal(leaf.grad, full_dx[:m]), m
     native.check_status(full)
+
+
+# projections of the text encoders at long reductions: a token's row does not depend on the length of the prompt
+def test_text_encoder_projections_do_not_depend_on_prompt_length():
+    from mojodiffusion_b200.models.text import clip, gpt_oss, qwen3, t5
+    for lin in (clip._Lin(5120, 1280, torch.bfloat16, DEV), t5._W(10240, 4096, torch.bfloat16, DEV), gpt_oss._Lin(4096, 2880, torch.bfloat16, DEV),
+                qwen3._W(9728, 2560, torch.bfloat16, DEV, True)):
+        x = _rand(1, 300, lin.weight.shape[1], seed=1)
+        with torch.no_grad():
+            full = lin(x)
+            for n in (1, 8, 9, 45, 129):
+                assert torch.equal(lin(x[:, :n]), full[:, :n]), (type(lin).__module__, n)
