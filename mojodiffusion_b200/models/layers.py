@@ -171,6 +171,23 @@ class LayerNorm(nn.Module):
                                  rows_per_group=rows_per_group, eps=self.eps, rms=False)
 
 
+def globally_hooked() -> bool:
+    """Whether a forward hook or pre-hook is registered for all modules."""
+    return bool(torch.nn.modules.module._global_forward_hooks or torch.nn.modules.module._global_forward_pre_hooks)
+
+
+def own_parameters(module, cls):
+    """The parameter dict of a module whose call runs the forward of ``cls`` and nothing else (exactly that class, so no
+    subclass, parametrisation or replacement; no hook of its own; no forward set on the instance), otherwise None."""
+    d = module.__dict__
+    return d["_parameters"] if type(module) is cls and not (d["_forward_hooks"] or d["_forward_pre_hooks"] or "forward" in d) else None
+
+
+def runs_as_defined(module, cls) -> bool:
+    """Whether a fused kernel may read the weights of ``module`` and do its work instead of calling it."""
+    return own_parameters(module, cls) is not None and not globally_hooked()
+
+
 def packed_projection(x: torch.Tensor, linears) -> torch.Tensor:
     """Run several Linear modules on the same input and return their outputs side by side in ONE buffer
     ([..., sum(out_features)]): on the GPU inference path each GEMM stores straight into its column slice, so

@@ -15,7 +15,7 @@ import torch
 import torch.nn as nn
 
 from .. import ops
-from .layers import Linear, RMSNorm, init_module_weights, packed_projection, timestep_embedding
+from .layers import Linear, RMSNorm, init_module_weights, packed_projection, runs_as_defined, timestep_embedding
 
 
 @dataclass
@@ -90,13 +90,16 @@ class MXFP8Linear(nn.Module):
         return y
 
 
-def _fused_rows_ok(qkv: torch.Tensor, D: int, Dh: int, cos, sin, wq, wk) -> bool:
+def _fused_rows_ok(qkv: torch.Tensor, D: int, Dh: int, cos, sin, q_norm, k_norm) -> bool:
     """Whether the one-pass q / k norm + rotation covers this projection: inference in bf16 on the GPU, rows of up to 16384
-    columns, heads of a multiple of 16, tables of one row per token, 16-byte aligned operands."""
+    columns, heads of a multiple of 16, tables of one row per token, two plain RMSNorm modules of one epsilon, 16-byte aligned
+    operands."""
     return (ops.native.use_native(qkv) and not torch.is_grad_enabled() and qkv.dtype == torch.bfloat16 and qkv.is_contiguous() and D <= 16384
             and D % Dh == 0 and Dh % 16 == 0 and cos is not None and cos.dtype == torch.float32 and cos.dim() == 2 and cos.shape[1] * 2 == Dh
             and cos.shape[0] >= qkv.shape[1] and cos.is_contiguous() and sin.is_contiguous() and sin.shape == cos.shape and sin.dtype == cos.dtype
-            and all(t.data_ptr() % 16 == 0 for t in (qkv, cos, sin, wq, wk)))
+            and runs_as_defined(q_norm, RMSNorm) and runs_as_defined(k_norm, RMSNorm) and q_norm.eps == k_norm.eps
+            and all(w.dtype == torch.bfloat16 and w.is_contiguous() and w.numel() == D for w in (q_norm.weight, k_norm.weight))
+            and all(t.device == qkv.device and t.data_ptr() % 16 == 0 for t in (qkv, cos, sin, q_norm.weight, k_norm.weight)))
 
 
 class VideoAttention(nn.Module):
@@ -119,7 +122,7 @@ class VideoAttention(nn.Module):
         H, Dh = cfg.heads, cfg.head_dim
         if not self.cross:
             qkv = packed_projection(x, (self.to_q, self.to_k, self.to_v))
-            if _fused_rows_ok(qkv, D, Dh, cos, sin, self.q_norm.weight, self.k_norm.weight):
+            if _fused_rows_ok(qkv, D, Dh, cos, sin, self.q_norm, self.k_norm):
                 # norm over the full width and rotation of q and k in one pass over the packed rows
                 ops.native.ops().rms_rope_rows(qkv.view(B * S, 3 * D), self.q_norm.weight, self.k_norm.weight, cos, sin, D, Dh, 0, D, S, self.q_norm.eps)
                 q, k, v = (qkv[..., i * D:(i + 1) * D].unflatten(-1, (H, Dh)) for i in range(3))

@@ -309,3 +309,46 @@ def test_text_encoder_projections_do_not_depend_on_prompt_length():
             full = lin(x)
             for n in (1, 8, 9, 45, 129):
                 assert torch.equal(lin(x[:, :n]), full[:, :n]), (type(lin).__module__, n)
+
+
+# what a program does to the q / k norms of a video attention takes effect: a hook on either side, an epsilon of one of them, another
+# module in its place (its hook-free twin on the fp32 CPU path is the oracle)
+@pytest.mark.parametrize("change", ["pre-hook", "hook", "global hook", "eps", "module", "forward"])
+def test_video_attention_keeps_to_its_norm_modules(change):
+    from mojodiffusion_b200.models.video_dit import VideoAttention, VideoDiTConfig
+    cfg = VideoDiTConfig(hidden=256, heads=4, head_dim=64, axes_dim=(32, 16, 16))
+    ids = torch.stack(torch.meshgrid(torch.arange(3.), torch.arange(5.), torch.arange(7.), indexing="ij"), -1).reshape(-1, 3)
+    cos, sin = O.rope_table(ids.to(DEV), cfg.axes_dim, 10000.0)
+    x, handles = _rand(2, 105, 256, seed=50), []
+    att = VideoAttention(cfg, False, torch.bfloat16, DEV)
+    cpu = VideoAttention(cfg, False, torch.float32, None)
+    with torch.no_grad():
+        for i, (n, p) in enumerate(att.named_parameters()):
+            p.copy_(_rand(*p.shape, seed=i, scale=p.shape[-1] ** -0.5) if p.dim() == 2 else _rand(*p.shape, seed=i, scale=0.1) + (1.0 if "norm" in n else 0.0))
+        cpu.load_state_dict({k: v.float().cpu() for k, v in att.state_dict().items()})
+        plain = att(x, None, cos, sin)
+        for m in (att, cpu):
+            if change == "pre-hook":
+                m.q_norm.register_forward_pre_hook(lambda mod, args: (args[0].roll(1, -1),))
+            elif change == "hook":
+                m.k_norm.register_forward_hook(lambda mod, args, out: out.roll(1, -1))
+            elif change == "global hook":
+                norms = (m.q_norm, m.k_norm)
+                handles.append(torch.nn.modules.module.register_module_forward_hook(lambda mod, args, out, norms=norms: out.roll(1, -1) if mod is norms[1] else None))
+            elif change == "eps":
+                m.k_norm.eps = 1.0
+            elif change == "module":
+                m.k_norm = torch.nn.Identity()
+            else:
+                m.q_norm.forward = lambda t: t * 0.5
+        try:
+            with torch.no_grad():
+                out, want = att(x, None, cos, sin), cpu(x.float().cpu(), None, cos.cpu(), sin.cpu())
+        finally:
+            for h in handles:
+                h.remove()
+    native.check_status(out)
+    # as above, and one rounding more where the norm stands apart from the rotation
+    bound = 2 * 2.0 ** -9 * (6 / 3) ** 0.5
+    assert float((out.float().cpu() - want).norm() / want.norm()) < bound
+    assert float((plain.float().cpu() - want).norm() / want.norm()) > 4 * bound         # the change does show
