@@ -197,8 +197,9 @@ def packed_projection(x: torch.Tensor, linears) -> torch.Tensor:
         lead = x.shape[:-1]
         out = torch.empty(*lead, sum(widths), dtype=x.dtype, device=x.device)
         c = 0
-        # fp8 projections of one input share its quantised rows
-        kw = dict(quantised=ops.fp8_quant_rows(x.reshape(-1, x.shape[-1]))) if all(getattr(l, "shares_quantised_rows", False) for l in linears) else {}
+        # fp8 projections of one input share its quantised rows; a hook or another forward may give one of them another input
+        share = all("shares_quantised_rows" in vars(type(l)) and runs_as_defined(l, type(l)) for l in linears)
+        kw = dict(quantised=ops.fp8_quant_rows(x.reshape(-1, x.shape[-1]))) if share else {}
         for l, w in zip(linears, widths):
             l(x, out=out[..., c:c + w], **kw)
             c += w

@@ -352,3 +352,27 @@ def test_video_attention_keeps_to_its_norm_modules(change):
     bound = 2 * 2.0 ** -9 * (6 / 3) ** 0.5
     assert float((out.float().cpu() - want).norm() / want.norm()) < bound
     assert float((plain.float().cpu() - want).norm() / want.norm()) > 4 * bound         # the change does show
+
+
+# fp8 projections that a program has changed get their own input, not the shared quantised rows
+@pytest.mark.parametrize("change", ["pre-hook", "subclass", "forward"])
+def test_changed_fp8_projections_quantise_their_own_rows(change):
+    from mojodiffusion_b200.models.layers import Linear, packed_projection
+    from mojodiffusion_b200.models.video_dit import FP8Linear
+
+    class Halved(FP8Linear):
+        def forward(self, x, act=None, residual=None, gate=None, rows_per_group=1, out=None):
+            return super().forward(x * 0.5, act, residual, gate, rows_per_group, out)
+
+    lins = [(Halved if change == "subclass" and i == 1 else FP8Linear)(Linear(384, n, True, torch.bfloat16, DEV)) for i, n in enumerate((256, 64, 128))]
+    if change == "pre-hook":
+        lins[1].register_forward_pre_hook(lambda mod, args: (args[0] * 0.5,))
+    elif change == "forward":
+        plain = lins[1].forward
+        lins[1].forward = lambda x, out=None: plain(x * 0.5, out=out)
+    x = _rand(2, 150, 384, seed=1)
+    with torch.no_grad():
+        got = packed_projection(x, lins)
+        want = torch.cat([O.fp8_linear(x * 0.5 if i == 1 else x, l.weight, l.weight_scale, l.bias) for i, l in enumerate(lins)], -1)
+    native.check_status(got)
+    assert torch.equal(got, want)
