@@ -38,12 +38,19 @@ template <bool CACHED>
 __global__ void __launch_bounds__(SM_THREADS)
 softmax_rows_kernel(const float* __restrict__ s, __nv_bfloat16* __restrict__ p, int cols, long long lds, long long ldp, float scale_log2) {
   __shared__ float red[32];
-  const float4* sr = reinterpret_cast<const float4*>(s + static_cast<size_t>(blockIdx.x) * lds);
-  uint2* pr = reinterpret_cast<uint2*>(p + static_cast<size_t>(blockIdx.x) * ldp);
+  const float* sr = s + static_cast<size_t>(blockIdx.x) * lds;
+  __nv_bfloat16* pr = p + static_cast<size_t>(blockIdx.x) * ldp;
   const int nv = (cols + 3) >> 2;
-  auto load = [&](int i) {                       // scaled scores, columns past the end are -inf
-    float4 v = sr[i];
+  auto load = [&](int i) {                       // scaled scores; columns past the end are not touched and count as -inf
     const int c = i * 4;
+    float4 v;
+    if (c + 3 < cols) {
+      v = *reinterpret_cast<const float4*>(sr + c);
+    } else {
+      v = make_float4(sr[c], -INFINITY, -INFINITY, -INFINITY);
+      if (c + 1 < cols) v.y = sr[c + 1];
+      if (c + 2 < cols) v.z = sr[c + 2];
+    }
     // __fmul_rn: a product fused with the subtraction of the (rounded) maximum would be off by the maximum's rounding
     v.x = __fmul_rn(v.x, scale_log2);
     v.y = c + 1 < cols ? __fmul_rn(v.y, scale_log2) : -INFINITY;
@@ -85,7 +92,16 @@ softmax_rows_kernel(const float* __restrict__ s, __nv_bfloat16* __restrict__ p, 
   }
   sum = fr_block<SM_THREADS, false>(sum, red);
   const float inv = 1.f / sum;
-  auto put = [&](int i, float4 t) { pr[i] = make_uint2(pack_bf16x2(t.x * inv, t.y * inv), pack_bf16x2(t.z * inv, t.w * inv)); };
+  auto put = [&](int i, float4 t) {
+    const int c = i * 4;
+    if (c + 3 < cols) {
+      *reinterpret_cast<uint2*>(pr + c) = make_uint2(pack_bf16x2(t.x * inv, t.y * inv), pack_bf16x2(t.z * inv, t.w * inv));
+    } else {
+      pr[c] = __float2bfloat16_rn(t.x * inv);
+      if (c + 1 < cols) pr[c + 1] = __float2bfloat16_rn(t.y * inv);
+      if (c + 2 < cols) pr[c + 2] = __float2bfloat16_rn(t.z * inv);
+    }
+  };
   if (CACHED) {
 #pragma unroll
     for (int k = 0; k < SM_VEC; ++k) {
@@ -184,7 +200,7 @@ using namespace mdb;
 typedef __nv_bfloat16 bf16;
 
 extern "C" int mdb_softmax_rows(const float* s, void* p, long long rows, int cols, long long lds, long long ldp, float scale, cudaStream_t st) {
-  if (cols <= 0 || lds % 4 || ldp % 4 || lds < (cols + 3) / 4 * 4 || ldp < (cols + 3) / 4 * 4 || rows > 2147483647ll) return -1;
+  if (cols <= 0 || lds % 4 || ldp % 4 || lds < cols || ldp < cols || rows > 2147483647ll) return -1;
   if ((reinterpret_cast<uintptr_t>(s) & 15) || (reinterpret_cast<uintptr_t>(p) & 7)) return -1;
   if (rows <= 0) return 0;
   const float k = scale * 1.4426950408889634f;

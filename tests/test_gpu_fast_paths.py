@@ -376,3 +376,15 @@ def test_changed_fp8_projections_quantise_their_own_rows(change):
         want = torch.cat([O.fp8_linear(x * 0.5 if i == 1 else x, l.weight, l.weight_scale, l.bias) for i, l in enumerate(lins)], -1)
     native.check_status(got)
     assert torch.equal(got, want)
+
+
+# a block of columns inside a wider buffer: the columns beside it keep what they held
+@pytest.mark.parametrize("cols", [1, 2, 3, 5, 1001, 16385, 16391])
+def test_softmax_rows_writes_its_columns_only(cols):
+    ld = (cols + 7) // 8 * 8 + 8
+    s, p = _rand(5, ld, seed=1, dtype=torch.float32), _rand(5, ld, seed=2)
+    beside = p[:, cols:].clone()
+    torch.ops.mdb200.softmax_rows(s[:, :cols], p[:, :cols], 1.0)
+    assert torch.equal(p[:, cols:], beside)
+    want = torch.softmax(s[:, :cols].double(), -1)
+    assert bool(((p[:, :cols].double() - want).abs() <= want * 2 * (2.0 ** -9 + 1e-5)).all())
