@@ -146,9 +146,9 @@ group_norm_finalize_kernel(const float* __restrict__ part, float* __restrict__ s
   }
 }
 
-// y = act((x - mean) * rstd * w[c] + b[c]); act 0 none, 2 SiLU. A thread keeps one 8-channel vector (its mean, rstd * w and b
-// in registers) and walks the pixels, four loads in flight, so the loop is one 16-byte load, two operations per channel, the
-// activation and one store. (The earlier form re-derived channel, group and sample by division for every element: 99 us per
+// y = act((x - mean) * rstd * w[c] + b[c]); act 0 none, 2 SiLU. A thread keeps one 8-channel vector (its mean, rstd, w and b
+// in registers) and walks the pixels, four loads in flight, so the loop is one 16-byte load, three operations per channel, the
+// activation and one store. rstd and w are not multiplied beforehand: their product can overflow where no result does. (The earlier form re-derived channel, group and sample by division for every element: 99 us per
 // call on the 1024 x 1024 decoder where the bytes need about 45.)
 __global__ void __launch_bounds__(256)
 group_norm_apply_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y,
@@ -158,12 +158,13 @@ group_norm_apply_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __re
   const int cv = min(sv, (C >> 3) - v0), lanes = blockDim.x / cv;
   if (static_cast<int>(threadIdx.x) >= lanes * cv) return;
   const int v = v0 + threadIdx.x % cv, pl = threadIdx.x / cv;
-  float mean[8], mul[8], add[8];
+  float mean[8], rstd[8], mul[8], add[8];
 #pragma unroll
   for (int k = 0; k < 8; ++k) {
     const int c = v * 8 + k, g = c / cpg;
     mean[k] = stats[2 * (n * G + g)];
-    mul[k] = stats[2 * (n * G + g) + 1] * (w ? __bfloat162float(w[c]) : 1.f);
+    rstd[k] = stats[2 * (n * G + g) + 1];
+    mul[k] = w ? __bfloat162float(w[c]) : 1.f;
     add[k] = w && b ? __bfloat162float(b[c]) : 0.f;
   }
   const int p0 = blockIdx.x * ppb, p1 = min(p0 + ppb, HW);
@@ -176,7 +177,8 @@ group_norm_apply_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __re
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const float2 f = unpack_bf16x2(w4[k]);
-      float t0 = (f.x - mean[2 * k]) * mul[2 * k] + add[2 * k], t1 = (f.y - mean[2 * k + 1]) * mul[2 * k + 1] + add[2 * k + 1];
+      float t0 = (f.x - mean[2 * k]) * rstd[2 * k] * mul[2 * k] + add[2 * k];
+      float t1 = (f.y - mean[2 * k + 1]) * rstd[2 * k + 1] * mul[2 * k + 1] + add[2 * k + 1];
       if (act == 2) { t0 = silu_f(t0); t1 = silu_f(t1); }
       o4[k] = pack_bf16x2(t0, t1);
     }

@@ -388,3 +388,11 @@ def test_softmax_rows_writes_its_columns_only(cols):
     assert torch.equal(p[:, cols:], beside)
     want = torch.softmax(s[:, :cols].double(), -1)
     assert bool(((p[:, :cols].double() - want).abs() <= want * 2 * (2.0 ** -9 + 1e-5)).all())
+
+
+# a constant group is normalised to zero, so only the bias is left whatever the weight; 1 / sqrt(eps) times the weight overflows
+def test_group_norm_large_weight_on_a_constant_group():
+    from mojodiffusion_b200.ops import conv as K
+    x, w, b = torch.full((1, 4, 4, 64), 3.0, dtype=torch.bfloat16, device=DEV), torch.full((64,), 3e38, dtype=torch.bfloat16, device=DEV), _rand(64, seed=1)
+    with torch.no_grad():
+        assert torch.equal(K.group_norm_nhwc(x, w, b, 8, 1e-6), b.expand(1, 4, 4, 64))
