@@ -788,7 +788,7 @@ Tensor llm_out_mlp(Tensor x, const Tensor& attn, const Tensor& wo, const Tensor&
   Tensor m;
   if (R <= MDB_GEMM_ROWS_MAX) {
     m = at::empty({R, F}, x.options());
-    check_rc(mdb_glu_rows(h.data_ptr(), wg.data_ptr(), wu.data_ptr(), m.data_ptr(), (int)R, (int)F, (int)D, MDB_ACT_SILU, cur_stream()), "decoder mlp");
+    check_rc(mdb_glu_rows(h.data_ptr(), wg.data_ptr(), wu.data_ptr(), m.data_ptr(), (int)R, (int)F, (int)D, cur_stream()), "decoder mlp");
   } else {
     Tensor g = at::empty({R, F}, x.options()), u = at::empty({R, F}, x.options());
     llm_project(h, wg, nullptr, g.data_ptr(), F);

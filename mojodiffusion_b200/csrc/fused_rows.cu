@@ -1,6 +1,8 @@
+// build: precise-math
 // Row kernels that replace chains of elementwise passes around attention: scaled softmax of a score matrix, full-width
 // RMSNorm + rotary embedding of packed q and k in place, per-head output gates. bf16 tensors, fp32 arithmetic, 16-byte
-// accesses; each element crosses memory once per direction.
+// accesses; each element crosses memory once per direction. Built without fast math: the torch operations that these kernels
+// replace use the precise exponential and division.
 //
 // Reference behaviour: serenitymojo/ops/attention.mojo:18-180 (math-mode softmax), serenitymojo/models/dit/ltx2_dit.mojo:518-652
 // (norm over the inner dimension, split rotation, 2 * sigmoid head gates).
@@ -181,7 +183,7 @@ head_gate_kernel(__nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict_
   for (long long i = blockIdx.x * 256ll + threadIdx.x; i < vecs; i += gridDim.x * 256ll) {
     const long long row = i / rv;
     const int h = static_cast<int>(i - row * rv) / hv;
-    const float g = 2.f * sigmoid_f(__bfloat162float(logit[row * ld_logit + h]));
+    const float g = 2.f * (1.f / (1.f + expf(-__bfloat162float(logit[row * ld_logit + h]))));
     uint4* q = reinterpret_cast<uint4*>(o) + i;
     const uint4 u = *q;
     uint32_t w[4] = {u.x, u.y, u.z, u.w};

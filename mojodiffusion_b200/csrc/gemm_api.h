@@ -94,8 +94,8 @@ int mdb_gemm_launch(const MdbGemmArgs* args, cudaStream_t stream);
 // itself when the tile width is left to it (bn == 0).
 int mdb_gemm_rows_ok(const MdbGemmArgs* args);
 int mdb_gemm_rows(const MdbGemmArgs* args, cudaStream_t stream);
-// act(x w1^T) * (x w2^T), halves and activation rounded to bf16, M <= MDB_GEMM_ROWS_MAX contiguous rows of K, weights [N, K]
-int mdb_glu_rows(const void* x, const void* w1, const void* w2, void* out, int M, int N, int K, int act, cudaStream_t st);
+// silu(x w1^T) * (x w2^T), halves and activation rounded to bf16, M <= MDB_GEMM_ROWS_MAX contiguous rows of K, weights [N, K]
+int mdb_glu_rows(const void* x, const void* w1, const void* w2, void* out, int M, int N, int K, cudaStream_t st);
 
 // number of two-CTA clusters of the 256 x 256 GEMM kernel the current device can hold at once (74 on a B200 whose 148 SMs
 // all have their TPC partner, fewer otherwise)

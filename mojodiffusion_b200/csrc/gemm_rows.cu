@@ -39,6 +39,12 @@ __device__ __forceinline__ float rows_act(int act, float x) {
     default: return x;
   }
 }
+// SiLU for results that are rounded to bf16 and used again: this file is built with fast math, whose exponential is off by up to
+// 2^-17 at |x| of 60 and flips that rounding where the torch operation does not. One lane evaluates it per result, so double
+// precision costs nothing that shows.
+__device__ __forceinline__ float rows_silu_exact(float x) {
+  return static_cast<float>(static_cast<double>(x) / (1.0 + exp(-static_cast<double>(x))));
+}
 __device__ __forceinline__ uint4 ldg_stream(const uint4* p) {   // weights: read once, not kept in L1
   uint4 v;
   asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
@@ -115,10 +121,10 @@ gemm_rows_kernel(const __grid_constant__ RowsParams p) {
         float y = acc[m][PAIR ? 2 * c + 1 : c] * p.alpha;
         if (p.bias) y += __bfloat162float(p.bias[col + p.pair_offset]);
         if (p.round_halves) {
-          // both projections and the activation rounded to bf16, as separate operations round them
+          // both projections and the SiLU rounded to bf16, as separate operations round them
           x = __bfloat162float(__float2bfloat16_rn(x));
           y = __bfloat162float(__float2bfloat16_rn(y));
-          x = __bfloat162float(__float2bfloat16_rn(rows_act(p.act, x))) * y;
+          x = __bfloat162float(__float2bfloat16_rn(rows_silu_exact(x))) * y;
         } else {
           x = p.act_on_second ? x * rows_act(p.act, y) : rows_act(p.act, x) * y;
         }
@@ -194,9 +200,9 @@ extern "C" int mdb_gemm_rows(const MdbGemmArgs* a, cudaStream_t st) {
   return launch_rows_any(p, a->num_sms > 0 ? a->num_sms : device_sm_count(), a->pair_offset > 0, st);
 }
 
-// act(x w1^T) * (x w2^T) with the two halves in weights of their own, each half and the activation rounded to bf16 before they
+// silu(x w1^T) * (x w2^T) with the two halves in weights of their own, each half and the activation rounded to bf16 before they
 // meet, M <= MDB_GEMM_ROWS_MAX rows; everything contiguous bf16
-extern "C" int mdb_glu_rows(const void* x, const void* w1, const void* w2, void* out, int M, int N, int K, int act, cudaStream_t st) {
+extern "C" int mdb_glu_rows(const void* x, const void* w1, const void* w2, void* out, int M, int N, int K, cudaStream_t st) {
   using namespace mdb;
   if (M <= 0 || M > MDB_GEMM_ROWS_MAX || N <= 0 || K <= 0 || K % 8 ||
       ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w1) | reinterpret_cast<uintptr_t>(w2)) & 15))
@@ -207,7 +213,7 @@ extern "C" int mdb_glu_rows(const void* x, const void* w1, const void* w2, void*
   p.B[0] = reinterpret_cast<const __nv_bfloat16*>(w1);
   p.B2[0] = reinterpret_cast<const __nv_bfloat16*>(w2);
   p.lda[0] = p.ldb[0] = p.K[0] = K;
-  p.num_seg = 1; p.M = M; p.N = N; p.act = act; p.alpha = 1.f; p.rows_per_group = 1; p.out = out; p.ld_out = N;
+  p.num_seg = 1; p.M = M; p.N = N; p.act = MDB_ACT_SILU; p.alpha = 1.f; p.rows_per_group = 1; p.out = out; p.ld_out = N;
   p.round_halves = 1;
   return launch_rows_any(p, device_sm_count(), true, st);
 }

@@ -1,8 +1,10 @@
+// build: precise-math
 // Row kernels of the decoder stack around its projections: per-head RMSNorm + rotary embedding of q and k with the cache append,
 // and attention of one query per sequence over that cache. bf16 storage, fp32 arithmetic.
 //
 // Both work on a few rows, so they are bound by latency: what they save is launches (the same steps as elementwise torch
-// operations were 67 launches a layer, and the host could not issue them as fast as the GPU ran them).
+// operations were 67 launches a layer, and the host could not issue them as fast as the GPU ran them). Exponentials, divisions and
+// roundings are the precise ones that those operations use; sums of products are written as fmaf where it matters for time.
 //
 // Reference behaviour: serenitymojo/llm/decoder.mojo:1-150, serenitymojo/llm/sqa.mojo:1-116.
 #include "common.cuh"
@@ -182,7 +184,7 @@ decode_attention_kernel(const __nv_bfloat16* __restrict__ q, long long ldq, cons
   __syncthreads();
   float sum = 0.f;
   for (int t = threadIdx.x; t < len; t += DA_THREADS) {
-    const float e = __expf(da_sm[t] - m);
+    const float e = expf(da_sm[t] - m);
     da_sm[t] = e;
     sum += e;
   }

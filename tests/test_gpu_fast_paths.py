@@ -396,3 +396,38 @@ def test_group_norm_large_weight_on_a_constant_group():
     x, w, b = torch.full((1, 4, 4, 64), 3.0, dtype=torch.bfloat16, device=DEV), torch.full((64,), 3e38, dtype=torch.bfloat16, device=DEV), _rand(64, seed=1)
     with torch.no_grad():
         assert torch.equal(K.group_norm_nhwc(x, w, b, 8, 1e-6), b.expand(1, 4, 4, 64))
+
+
+def test_head_gate_rounds_as_the_torch_statement():
+    o, logit = _rand(2000, 32, 128, seed=1), _rand(2000, 32, seed=2, scale=20.0)
+    want = (o.float() * (2.0 * torch.sigmoid(logit.float()))[..., None]).to(torch.bfloat16)
+    torch.ops.mdb200.head_gate(o, logit)
+    assert torch.equal(o, want)
+
+
+# identity weights make the gated MLP of a decoder step silu(h) * h of its normalised input, and rows of +-1 normalise to +-1 exactly:
+# the result is known to the bit, here for every bf16 value from 2^-7 to 87
+def test_decoder_mlp_rounds_a_precise_silu():
+    bits = torch.arange(0x3c00, 0x42b0, dtype=torch.int32).to(torch.int16)
+    ln = bits.view(torch.bfloat16).to(DEV)
+    D = ln.numel()
+    eye = torch.eye(D, dtype=torch.bfloat16, device=DEV)
+    x = torch.ones(2, D, dtype=torch.bfloat16, device=DEV)
+    x[1] = -1
+    h = x * ln
+    out = torch.ops.mdb200.llm_out_mlp(x, torch.zeros(2, D, dtype=torch.bfloat16, device=DEV), eye, ln, eye, eye, eye, 1e-6)
+    native.check_status(out)
+    assert torch.equal(out, torch.nn.functional.silu(h.double()).float().to(torch.bfloat16) * h)
+
+
+# one-hot keys and values: the outputs are the probabilities. Errors beyond the bf16 rounding (2^-8) are those of the fp32
+# exponential, sum and quotient, a few 2^-24
+def test_decode_attention_probabilities():
+    B, H, Dh, T = 8, 32, 128, 128
+    q = torch.zeros(B, H * Dh, dtype=torch.bfloat16, device=DEV)
+    q.copy_(-torch.rand(B, H * Dh, generator=torch.Generator().manual_seed(1)) * 60)
+    eye = torch.eye(T, Dh, dtype=torch.bfloat16, device=DEV).expand(B, H, T, Dh).contiguous()
+    out = torch.ops.mdb200.llm_decode_attention(q, eye, eye, H, T, 1.0).view(B, H, T).double()
+    want = torch.softmax(q.view(B, H, Dh).double(), -1)
+    worst = float(((out - want).abs() / want - 2.0 ** -8).max())
+    assert worst < 16 * 2.0 ** -24, worst
