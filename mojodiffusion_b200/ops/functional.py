@@ -485,6 +485,15 @@ def _wide_attention(q, k, v, scale: float):
     return o
 
 
+def _wide_ok(q, k, v) -> bool:
+    """Whether ``_wide_attention`` covers these operands: one bf16 head of the same width on all sides, no broadcasting between
+    them, no gradient and no transform that has to see the torch operations."""
+    return (q.dim() == k.dim() == 4 and q.shape[2] == 1 and q.shape[3] > 128 and q.shape[3] % 8 == 0 and q.shape[1] > 0 and k.shape[1] > 0
+            and q.shape[0] == k.shape[0] and q.shape[2:] == k.shape[2:] and k.shape == v.shape and q.device == k.device == v.device
+            and q.dtype == k.dtype == v.dtype == torch.bfloat16
+            and not (torch.is_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad)) and native.direct(q, k, v))
+
+
 def attention(q, k, v, scale: Optional[float] = None, kv_len: Optional[torch.Tensor] = None,
               out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Scaled dot-product attention over [B, S, H, Dh] tensors (any strides with contiguous Dh).
@@ -493,9 +502,7 @@ def attention(q, k, v, scale: Optional[float] = None, kv_len: Optional[torch.Ten
     """
     Dh = q.shape[-1]
     scale = float(scale) if scale is not None else 1.0 / math.sqrt(Dh)
-    if (native.use_native(q) and q.dim() == 4 and q.shape[2] == 1 and Dh > 128 and Dh % 8 == 0 and kv_len is None
-            and q.dtype == k.dtype == v.dtype == torch.bfloat16 and q.shape[1] > 0 and k.shape[1] > 0
-            and not (torch.is_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad))):
+    if native.use_native(q) and kv_len is None and _wide_ok(q, k, v):
         o = _wide_attention(q, k, v, scale)
         if out is not None:
             out.copy_(o)

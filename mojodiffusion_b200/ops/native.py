@@ -12,6 +12,7 @@ import threading
 from pathlib import Path
 
 import torch
+from torch.autograd import forward_ad
 
 _LIB = Path(__file__).resolve().parent.parent / "_C.so"
 _lock = threading.Lock()
@@ -63,6 +64,15 @@ def use_native(t: torch.Tensor) -> bool:
         return False
     load(True)
     return True
+
+
+def direct(*tensors: torch.Tensor) -> bool:
+    """Whether nothing but the kernels looks at an operation on these tensors: plain tensors outside every functorch transform
+    (vmap, grad, jvp), forward-mode AD level, dispatch mode and trace. Ops that also have a form in torch operations keep to it
+    otherwise."""
+    return (all(type(t) is torch.Tensor or type(t) is torch.nn.Parameter for t in tensors)
+            and torch._C._functorch.peek_interpreter_stack() is None and forward_ad._current_level < 0
+            and torch._C._len_torch_dispatch_stack() == 0 and not torch.jit.is_tracing() and not torch.compiler.is_compiling())
 
 
 def check_status(like: torch.Tensor | None = None, reset: bool = True) -> None:

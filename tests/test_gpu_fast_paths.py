@@ -431,3 +431,41 @@ def test_decode_attention_probabilities():
     want = torch.softmax(q.view(B, H, Dh).double(), -1)
     worst = float(((out - want).abs() / want - 2.0 ** -8).max())
     assert worst < 16 * 2.0 ** -24, worst
+
+
+# one wide head in the forms that only the torch operations have: batch or value width that differ, vmap, forward-mode AD, a
+# dispatch mode; the plain call is the oracle of each
+@pytest.mark.parametrize("form", ["one key batch", "value width", "many key heads", "vmap", "forward AD", "dispatch mode"])
+def test_wide_single_head_attention_other_forms(form):
+    from torch.autograd import forward_ad
+    from torch.utils._python_dispatch import TorchDispatchMode
+    B, Sq, Skv, Dh = 3, 33, 40, 256
+    q, k, v = (_rand(B, s, 1, Dh, seed=i) for i, s in ((1, Sq), (2, Skv), (3, Skv)))
+    with torch.no_grad():
+        plain = O.attention(q, k, v)
+        if form == "one key batch":
+            got, want = O.attention(q, k[:1], v[:1]), O.attention(q, k[:1].repeat(B, 1, 1, 1), v[:1].repeat(B, 1, 1, 1))
+        elif form == "value width":
+            got, want = O.attention(q, k, v[..., :136]), plain[..., :136]
+        elif form == "many key heads":
+            got = O.attention(q, torch.cat((k, k), 2), torch.cat((v, v), 2))
+            want = torch.cat((plain, plain), 2)
+        elif form == "vmap":
+            got, want = torch.func.vmap(O.attention)(q[:, None], k[:, None], v[:, None])[:, 0], plain
+        elif form == "forward AD":
+            # the library kernel has none: it says so and does not drop the tangent
+            with forward_ad.dual_level(), pytest.raises(NotImplementedError):
+                O.attention(q, k, forward_ad.make_dual(v, _rand(B, Skv, 1, Dh, seed=9)))
+            got = want = plain
+        else:
+            seen = []
+
+            class Log(TorchDispatchMode):
+                def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+                    seen.append(str(func))
+                    return func(*args, **(kwargs or {}))
+            with Log():
+                got = O.attention(q, k, v)
+            want = plain
+            assert any("attention" in s or "softmax" in s for s in seen), seen
+    assert got.shape == want.shape and float((got.float() - want.float()).norm() / want.float().norm()) < 2.0 ** -7
