@@ -706,6 +706,21 @@ Tensor randn(std::vector<int64_t> shape, int64_t seed, int64_t offset, bool bf16
 // ------------------------------------------------------------------------------------------
 // decoder stack: one layer on R rows (R = batch while decoding, batch x prompt in the prefill)
 // ------------------------------------------------------------------------------------------
+// Contiguous, 16-byte aligned bf16 memory of one GPU, all of them, with the shapes given: two numbers per tensor, rows and columns,
+// columns 0 for a vector, rows -1 for any shape.
+bool bf16_operands_ok(const std::vector<Tensor>& ts, const std::vector<int64_t>& shapes) {
+  TORCH_CHECK(shapes.size() == 2 * ts.size(), "bf16_operands_ok: two numbers per tensor");
+  for (size_t i = 0; i < ts.size(); ++i) {
+    const Tensor& t = ts[i];
+    const int64_t rows = shapes[2 * i], cols = shapes[2 * i + 1];
+    if (!t.is_cuda() || t.device() != ts[0].device() || t.scalar_type() != at::kBFloat16 || t.layout() != at::kStrided || !t.is_contiguous() ||
+        t.unsafeGetTensorImpl()->is_python_dispatch() || reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 != 0)
+      return false;
+    if (rows >= 0 && !(t.dim() == (cols ? 2 : 1) && t.size(0) == rows && (!cols || t.size(1) == cols))) return false;
+  }
+  return true;
+}
+int64_t llm_decode_attention_max() { return MDB_DECODE_ATTENTION_MAX; }
 const Tensor& llm_matrix(const Tensor& w, int64_t N, int64_t K, const Tensor& x, const char* what) {
   TORCH_CHECK(w.device() == x.device() && w.scalar_type() == at::kBFloat16 && w.is_contiguous() && w.dim() == 2 && w.size(0) == N && w.size(1) == K,
               "decoder layer: ", what, " must be a contiguous bf16 [", N, ", ", K, "]");
@@ -1181,6 +1196,8 @@ TORCH_LIBRARY(mdb200, m) {
   m.def("flow_match", &flow_match);
   m.def("mse_loss", &mse_loss);
   m.def("randn", &randn);
+  m.def("bf16_operands_ok", &bf16_operands_ok);
+  m.def("llm_decode_attention_max", &llm_decode_attention_max);
   m.def("llm_qkv", &llm_qkv);
   m.def("llm_out_mlp", &llm_out_mlp);
   m.def("llm_decode_attention", &llm_decode_attention);

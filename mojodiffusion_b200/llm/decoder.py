@@ -13,7 +13,8 @@ from typing import List, Optional, Sequence
 import torch
 
 from .. import ops
-from ..models.text.qwen3 import Qwen3Config, Qwen3Encoder, _rope
+from ..models.layers import globally_hooked, own_parameters
+from ..models.text.qwen3 import _MLP, _Norm, _W, Qwen3Config, Qwen3Encoder, _rope
 from ..ops import native
 from .sampler import Rng, SamplerConfig, sample
 
@@ -41,10 +42,7 @@ class KVCache:
         self.v = torch.zeros(shape, dtype=dtype, device=device)
         self.length = 0
         self.max_len = max_len
-        self.rope = None                # (cos, sin) [max_len, head_dim] of every position, filled by the prefill on the GPU
-
-
-DECODE_ATTENTION_MAX = 7936             # cache rows the single-query attention kernel covers (scores in shared memory)
+        self.rope = None                # (cos, sin) [positions, head_dim] for the fused decode step, filled by the prefill on the GPU
 
 
 class Qwen3Decoder:
@@ -63,22 +61,51 @@ class Qwen3Decoder:
         return emb.cos().to(dtype), emb.sin().to(dtype)
 
     def _native(self, x: torch.Tensor) -> bool:
-        """Whether the fused decode-step kernels cover this stack: bf16 on the GPU, 16-byte rows, heads of up to 256. They round
-        to bf16 where the separate operations do."""
+        """Whether the fused decode-step kernels cover this configuration: bf16 on the GPU, 16-byte rows, heads of up to 256. They
+        round to bf16 where the separate operations do."""
         c = self.cfg
         return (native.use_native(x) and x.dtype == torch.bfloat16 and c.qk_norm and c.hidden_size % 8 == 0 and c.hidden_size <= 16384
                 and c.intermediate_size % 8 == 0 and c.head_dim % 8 == 0 and c.head_dim <= 256 and x.numel() > 0
                 and c.num_attention_heads % c.num_key_value_heads == 0)
 
-    def _qkv(self, l, x, y, cache, li, S, pos):
-        a, c = l.self_attn, self.cfg
-        return native.ops().llm_qkv(x, y, l.input_layernorm.weight, a.q_proj.weight, a.k_proj.weight, a.v_proj.weight, a.q_proj.bias, a.k_proj.bias,
-                                    a.v_proj.bias, a.q_norm.weight, a.k_norm.weight, cache.rope[0], cache.rope[1], cache.k[li], cache.v[li], S, pos, c.rms_norm_eps)
-
-    def _out_mlp(self, l, x, attn):
-        m = l.mlp
-        return native.ops().llm_out_mlp(x, attn, l.self_attn.o_proj.weight, l.post_attention_layernorm.weight, m.gate_proj.weight, m.up_proj.weight,
-                                        m.down_proj.weight, self.cfg.rms_norm_eps)
+    def _fused_layers(self, x: torch.Tensor, cache: KVCache, pos: int):
+        """Per layer ((norm, q, k, v, biases, q norm, k norm), (o, norm, gate, up, down)) for the fused kernels, or None when the
+        separate operations have to run: a module that a program hooked, replaced or gave another epsilon or bias, weights or
+        caches of another type, shape or layout. Looked at anew on every step."""
+        c, rope = self.cfg, getattr(cache, "rope", None)
+        if rope is None or not self._native(x) or pos >= native.ops().llm_decode_attention_max() or x.dim() != 2 or globally_hooked():
+            return None
+        D, Dh, F, eps = c.hidden_size, c.head_dim, c.intermediate_size, c.rms_norm_eps
+        Q, KV = c.num_attention_heads * Dh, c.num_key_value_heads * Dh
+        layers, flat = [], []
+        for l in self.enc.model.layers:
+            a, m = l._modules["self_attn"], l._modules["mlp"]
+            if own_parameters(m, _MLP) is None:
+                return None
+            a, m, ps = a._modules, m._modules, []
+            for mod, cls in ((l._modules["input_layernorm"], _Norm), (a["q_proj"], _W), (a["k_proj"], _W), (a["v_proj"], _W), (a["q_norm"], _Norm), (a["k_norm"], _Norm),
+                             (a["o_proj"], _W), (l._modules["post_attention_layernorm"], _Norm), (m["gate_proj"], _W), (m["up_proj"], _W), (m["down_proj"], _W)):
+                p = own_parameters(mod, cls)
+                if p is None or (cls is _Norm and mod.eps != eps) or mod.__dict__.get("bias") is not None:
+                    return None
+                ps.append(p)
+            n1, wq, wk, wv, nq, nk, wo, n2, wg, wu, wd = ws = [p.get("weight") for p in ps]
+            if any(ps[i].get("bias") is not None for i in (6, 8, 9, 10)) or any(w is None for w in ws):
+                return None
+            bias = [ps[i].get("bias") for i in (1, 2, 3)]
+            layers.append(((n1, wq, wk, wv, *bias, nq, nk), (wo, n2, wg, wu, wd)))
+            flat += ws
+            flat += [b for b in bias if b is not None]
+        has = [b is not None for b in layers[0][0][4:7]] if layers else []
+        if any([b is not None for b in qkv[4:7]] != has for qkv, _ in layers):
+            return None
+        # one call looks at type, device, layout, alignment and shape of all of them: the launches refuse what the separate
+        # operations broadcast or copy
+        shapes = [D, 0, Q, D, KV, D, KV, D, Dh, 0, Dh, 0, D, Q, D, 0, F, D, F, D, D, F] + [v for n, h in zip((Q, KV, KV), has) if h for v in (n, 0)]
+        kv = (len(layers), x.shape[0], c.num_key_value_heads, cache.k.shape[3] if cache.k.dim() == 5 else 0, Dh)
+        if kv[3] <= pos or cache.k.shape != kv or cache.v.shape != kv or any(t.dim() != 2 or t.shape[0] <= pos or t.shape[1] != Dh for t in rope):
+            return None
+        return layers if native.ops().bf16_operands_ok([x, cache.k, cache.v, *rope, *flat], [-1, 0] * 5 + shapes * len(layers)) else None
 
     @torch.no_grad()
     def prefill(self, ids: torch.Tensor, max_len: int) -> "tuple[torch.Tensor, KVCache]":
@@ -92,7 +119,8 @@ class Qwen3Decoder:
         mask = torch.full((S, S), float("-inf"), device=ids.device, dtype=x.dtype).triu(1)[None, None]
         rep = c.num_attention_heads // c.num_key_value_heads
         if self._native(x):
-            cache.rope = self._angles(torch.arange(max_len, device=ids.device), x.dtype)      # for the decode steps
+            reach = min(max_len, native.ops().llm_decode_attention_max())
+            cache.rope = self._angles(torch.arange(reach, device=ids.device), x.dtype)        # for the decode steps
         for li, l in enumerate(m.layers):
             a = l.self_attn
             h = l.input_layernorm(x)
@@ -118,11 +146,12 @@ class Qwen3Decoder:
         if pos >= cache.max_len:
             raise RuntimeError("KV cache is full")
         x = m.embed_tokens(token)                                         # [B, hidden]
-        if cache.rope is not None and pos < DECODE_ATTENTION_MAX and self._native(x):
-            H, scale, y = c.num_attention_heads, c.head_dim ** -0.5, None
-            for li, l in enumerate(m.layers):
-                qkv = self._qkv(l, x, y, cache, li, 1, pos)
-                y = self._out_mlp(l, x, native.ops().llm_decode_attention(qkv, cache.k[li], cache.v[li], H, pos + 1, scale))
+        layers = self._fused_layers(x, cache, pos)
+        if layers is not None:
+            o, H, eps, scale, y = native.ops(), c.num_attention_heads, c.rms_norm_eps, c.head_dim ** -0.5, None
+            for li, (qkv, out_mlp) in enumerate(layers):
+                q = o.llm_qkv(x, y, *qkv, *cache.rope, cache.k[li], cache.v[li], 1, pos, eps)
+                y = o.llm_out_mlp(x, o.llm_decode_attention(q, cache.k[li], cache.v[li], H, pos + 1, scale), *out_mlp, eps)
             cache.length = pos + 1
             return x + y if y is not None else x
         cos, sin = self._angles(torch.tensor([pos], device=token.device), x.dtype)
@@ -143,8 +172,8 @@ class Qwen3Decoder:
     def logits(self, hidden: torch.Tensor) -> torch.Tensor:
         h = self.enc.model.norm(hidden)
         w = self.lm_head if self.lm_head is not None else self.enc.model.embed_tokens.weight
-        if (native.use_native(h) and h.dtype == w.dtype == torch.bfloat16 and h.dim() == 2 and 0 < h.shape[0] <= 8 and h.shape[1] % 8 == 0
-                and h.is_contiguous() and w.is_contiguous()):
+        if (native.use_native(h) and native.direct(h, w) and h.dtype == w.dtype == torch.bfloat16 and h.dim() == w.dim() == 2 and 0 < h.shape[0] <= 8
+                and h.shape[1] == w.shape[1] and h.shape[1] % 8 == 0 and native.ops().bf16_operands_ok([h, w], [-1, 0, -1, 0])):
             # products of bf16 values are exact in fp32 and the few-row kernel sums in fp32: the table needs no fp32 copy
             return ops.functional._gemm([h], [w], out_fp32=True)
         return h.float() @ w.float().t()

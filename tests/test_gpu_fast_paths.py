@@ -469,3 +469,74 @@ def test_wide_single_head_attention_other_forms(form):
             want = plain
             assert any("attention" in s or "softmax" in s for s in seen), seen
     assert got.shape == want.shape and float((got.float() - want.float()).norm() / want.float().norm()) < 2.0 ** -7
+
+
+# what a program does to the modules, weights or cache of a decoder takes effect in the decode step and nothing that the separate
+# operations take is refused: the same change on the fp32 CPU stack is the oracle
+@pytest.mark.parametrize("change", ["none", "norm hook", "projection hook", "global pre-hook", "epsilon", "bias", "plain bias", "module", "forward", "weight offset",
+                                    "beams", "strided cache", "no tables", "token column", "table offset", "vmap logits"])
+def test_decode_step_keeps_to_its_modules(change):
+    from mojodiffusion_b200.llm.decoder import Qwen3Decoder
+    from mojodiffusion_b200.models.text.qwen3 import Qwen3Config, Qwen3Encoder
+    cfg = Qwen3Config(vocab_size=200, hidden_size=264, intermediate_size=520, num_hidden_layers=2, num_attention_heads=4, num_key_value_heads=2, head_dim=64)
+    enc, cpu = Qwen3Encoder(cfg, torch.bfloat16, DEV).eval(), Qwen3Encoder(cfg, torch.float32).eval()
+    g = torch.Generator(device=DEV).manual_seed(0)
+    with torch.no_grad():
+        for n, p in enc.named_parameters():
+            p.normal_(0.0, p.shape[-1] ** -0.5, generator=g) if p.dim() == 2 else p.normal_(1.0, 0.1, generator=g)
+    cpu.load_state_dict({k: v.float().cpu() for k, v in enc.state_dict().items()})
+    B = 1 if change == "token column" else 3
+    ids, tok = torch.randint(0, 200, (B, 7), generator=torch.Generator().manual_seed(1)), torch.randint(0, 200, (B,), generator=torch.Generator().manual_seed(2))
+    handles, outs = [], []
+    for e, dev in ((enc, DEV), (cpu, "cpu")):
+        dec, l = Qwen3Decoder(e), e.model.layers[1]
+        hidden, cache = dec.prefill(ids.to(dev), 12)
+        t = tok.to(dev)
+        if change == "norm hook":
+            l.input_layernorm.register_forward_hook(lambda mod, args, out: out * 2)
+        elif change == "projection hook":
+            l.mlp.down_proj.register_forward_pre_hook(lambda mod, args: (args[0] * 2,))
+        elif change == "global pre-hook":
+            k_norm = l.self_attn.k_norm
+            handles.append(torch.nn.modules.module.register_module_forward_pre_hook(lambda mod, args, k_norm=k_norm: (args[0].roll(1, -1),) if mod is k_norm else None))
+        elif change == "epsilon":
+            l.self_attn.q_norm.eps = 4.0
+        elif change == "bias":
+            l.self_attn.o_proj.bias = torch.nn.Parameter(_rand(264, seed=5).to(dev, l.self_attn.o_proj.weight.dtype))
+        elif change == "plain bias":
+            l.mlp.up_proj.bias = _rand(520, seed=5).to(dev, l.mlp.up_proj.weight.dtype)
+        elif change == "module":
+            l.mlp = torch.nn.Identity()
+        elif change == "forward":
+            l.mlp.forward = lambda h: h * 0.5
+        elif change == "weight offset":
+            w = e.model.norm.weight.data
+            for n in (l.self_attn.k_norm, l.input_layernorm):
+                buf = torch.empty(n.weight.numel() + 1, dtype=w.dtype, device=dev)
+                buf[1:] = n.weight.data * 2
+                n.weight.data = buf[1:]
+        elif change == "beams":
+            cache.k, cache.v = cache.k[:, :1].expand(-1, B, -1, -1, -1).clone(), cache.v[:, :1].expand(-1, B, -1, -1, -1).clone()
+        elif change == "strided cache":
+            cache.k, cache.v = (c.transpose(2, 3).contiguous().transpose(2, 3) for c in (cache.k, cache.v))
+        elif change == "no tables":
+            del cache.rope
+        elif change == "token column":
+            t = t[:, None]
+        elif change == "table offset":
+            table = torch.empty(200 * 264 + 4, dtype=e.model.embed_tokens.weight.dtype, device=dev)
+            table[4:] = e.model.embed_tokens.weight.data.flatten()
+            dec.lm_head = table[4:].view(200, 264)
+        try:
+            h = dec.decode_step(t, cache)
+            h = dec.decode_step(t, cache) if change != "token column" else h[:, 0]
+            if change == "vmap logits":
+                outs.append(torch.func.vmap(lambda r: dec.logits(r[None])[0])(h).float().cpu())
+            else:
+                outs.append(dec.logits(h).float().cpu())
+        finally:
+            while handles:
+                handles.pop().remove()
+    native.check_status(torch.empty(0, device=DEV))
+    # as for the layers above, with two layers
+    assert float((outs[0] - outs[1]).norm() / outs[1].norm()) < 2 * 2.0 ** -9 / 3 ** 0.5 * 44 ** 0.5
