@@ -704,7 +704,7 @@ Tensor randn(std::vector<int64_t> shape, int64_t seed, int64_t offset, bool bf16
   return out;
 }
 // ------------------------------------------------------------------------------------------
-// decoder stack: one layer on R rows (R = batch while decoding, batch x prompt in the prefill)
+// decoder stack: one layer of a decode step, one row per sequence
 // ------------------------------------------------------------------------------------------
 // Contiguous, 16-byte aligned bf16 memory of one GPU, all of them, with the shapes given: two numbers per tensor, rows and columns,
 // columns 0 for a vector, rows -1 for any shape.
@@ -760,23 +760,23 @@ Tensor llm_add_rms(Tensor& x, const optional<Tensor>& y, const void* w, double e
   return h;
 }
 // x: the residual stream, updated in place by y (the previous layer's MLP output, none for the first layer). RMSNorm, q | k | v
-// projections, per-head norm + rotation, cache append at positions pos .. pos + S - 1. Returns the packed rows
-// [B * S, (H + 2 Hkv) * Dh] (q final in place).
+// projections, per-head norm + rotation, cache append at position pos. Returns the packed rows [B, (H + 2 Hkv) * Dh] (q final
+// in place).
 Tensor llm_qkv(Tensor x, const optional<Tensor>& y, const Tensor& ln, const Tensor& wq, const Tensor& wk, const Tensor& wv, const optional<Tensor>& bq,
-               const optional<Tensor>& bk, const optional<Tensor>& bv, const optional<Tensor>& qn, const optional<Tensor>& kn, const Tensor& cosv,
-               const Tensor& sinv, Tensor k_cache, Tensor v_cache, int64_t S, int64_t pos, double eps) {
+               const optional<Tensor>& bk, const optional<Tensor>& bv, const Tensor& qn, const Tensor& kn, const Tensor& cosv, const Tensor& sinv,
+               Tensor k_cache, Tensor v_cache, int64_t pos, double eps) {
   llm_check_rows(x);
   c10::cuda::CUDAGuard guard(x.device());
   TORCH_CHECK(k_cache.dim() == 4 && k_cache.is_contiguous() && v_cache.is_contiguous() && v_cache.sizes() == k_cache.sizes() &&
                   k_cache.scalar_type() == at::kBFloat16 && v_cache.scalar_type() == at::kBFloat16 && k_cache.device() == x.device() &&
                   v_cache.device() == x.device(), "decoder layer: caches [B, Hkv, T, Dh] bf16");
   const int64_t R = x.size(0), D = x.size(1), Hkv = k_cache.size(1), T = k_cache.size(2), Dh = k_cache.size(3);
-  TORCH_CHECK(S > 0 && R % S == 0 && R / S == k_cache.size(0) && Dh > 0 && wq.size(0) % Dh == 0 && Dh % 8 == 0 && Dh <= 256 && pos >= 0 && pos + S <= T,
+  TORCH_CHECK(R == k_cache.size(0) && Dh > 0 && wq.size(0) % Dh == 0 && Dh % 8 == 0 && Dh <= 256 && pos >= 0 && pos < T,
               "decoder layer: rows / heads / positions do not match the cache");
   const int64_t H = wq.size(0) / Dh, W = (H + 2 * Hkv) * Dh;
   for (const Tensor* t : {&cosv, &sinv})
     TORCH_CHECK(t->device() == x.device() && t->scalar_type() == at::kBFloat16 && t->is_contiguous() && t->dim() == 2 && t->size(1) == Dh &&
-                    t->size(0) >= pos + S, "decoder layer: rotary tables [positions, Dh] bf16");
+                    t->size(0) > pos, "decoder layer: rotary tables [positions, Dh] bf16");
   Tensor h = llm_add_rms(x, y, llm_vector(ln, D, x, "norm weight"), eps);
   Tensor qkv = at::empty({R, W}, x.options());
   char* base = static_cast<char*>(qkv.data_ptr());
@@ -784,7 +784,7 @@ Tensor llm_qkv(Tensor x, const optional<Tensor>& y, const Tensor& ln, const Tens
   llm_project(h, llm_matrix(wk, Hkv * Dh, D, x, "k weight"), llm_vector(bk, Hkv * Dh, x, "k bias"), base + 2 * H * Dh, W);
   llm_project(h, llm_matrix(wv, Hkv * Dh, D, x, "v weight"), llm_vector(bv, Hkv * Dh, x, "v bias"), base + 2 * (H + Hkv) * Dh, W);
   check_rc(mdb_qkv_rope_cache(base, llm_vector(qn, Dh, x, "q norm"), llm_vector(kn, Dh, x, "k norm"), cosv.data_ptr(), sinv.data_ptr(),
-                              k_cache.data_ptr(), v_cache.data_ptr(), R, (int)S, (int)H, (int)Hkv, (int)Dh, (int)T, (int)pos, (float)eps, cur_stream()),
+                              k_cache.data_ptr(), v_cache.data_ptr(), R, (int)H, (int)Hkv, (int)Dh, (int)T, (int)pos, (float)eps, cur_stream()),
            "qkv_rope_cache");
   return qkv;
 }

@@ -47,10 +47,10 @@ int mdb_rope_table(const float* pos, float* cosv, float* sinv, int tokens, int n
                    cudaStream_t st);
 
 // ---- llm_rows.cu
-// qkv rows (q | k | v heads of Dh): q normalised + rotated in place, k (normalised + rotated) and v appended to the caches
-// [B, Hkv, T, Dh] at positions pos0 .. pos0 + S - 1; qn / kn null: no norm
-int mdb_qkv_rope_cache(void* qkv, const void* qn, const void* kn, const void* cosv, const void* sinv, void* kc, void* vc, long long rows, int S,
-                       int H, int Hkv, int Dh, int T, int pos0, float eps, cudaStream_t st);
+// qkv rows (q | k | v heads of Dh), one per sequence: q normalised + rotated in place, k (normalised + rotated) and v appended to
+// the caches [rows, Hkv, T, Dh] at position pos
+int mdb_qkv_rope_cache(void* qkv, const void* qn, const void* kn, const void* cosv, const void* sinv, void* kc, void* vc, long long rows, int H,
+                       int Hkv, int Dh, int T, int pos, float eps, cudaStream_t st);
 // x += y (y null: nothing), h = RMSNorm(x) * w
 int mdb_add_rms_rows(void* x, const void* y, const void* w, void* h, long long rows, int D, float eps, cudaStream_t st);
 #define MDB_DECODE_ATTENTION_MAX 7936      // cache rows whose scores fit beside the partial sums in 48 KB of shared memory

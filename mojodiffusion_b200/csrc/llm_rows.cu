@@ -78,23 +78,22 @@ add_rms_rows_kernel(__nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restri
   }
 }
 
-// qkv [B * S rows, (H + 2 Hkv) * Dh] (q | k | v). One warp per (row, head): q heads are normalised and rotated in place, k heads
-// go normalised and rotated to k_cache[b, h, pos0 + s], v heads as they are to v_cache. Rotation pairs element i with
-// i + Dh / 2; table rows are positions pos0 + s ([positions, Dh], bf16).
+// qkv [rows, (H + 2 Hkv) * Dh] (q | k | v), one row per sequence. One warp per (row, head): q heads are normalised and rotated in
+// place, k heads go normalised and rotated to k_cache[row, h, pos], v heads as they are to v_cache. Rotation pairs element i with
+// i + Dh / 2; table rows are positions ([positions, Dh], bf16).
 __global__ void __launch_bounds__(128)
 qkv_rope_cache_kernel(__nv_bfloat16* __restrict__ qkv, const __nv_bfloat16* __restrict__ qn, const __nv_bfloat16* __restrict__ kn,
                       const __nv_bfloat16* __restrict__ cosv, const __nv_bfloat16* __restrict__ sinv, __nv_bfloat16* __restrict__ kc,
-                      __nv_bfloat16* __restrict__ vc, long long rows, int S, int H, int Hkv, int Dh, int T, int pos0, float eps) {
+                      __nv_bfloat16* __restrict__ vc, long long rows, int H, int Hkv, int Dh, int T, int pos, float eps) {
   const int heads = H + 2 * Hkv, lane = threadIdx.x & 31;
   const long long item = blockIdx.x * 4ll + (threadIdx.x >> 5);
   if (item >= rows * heads) return;
   const long long row = item / heads;
-  const int h = static_cast<int>(item - row * heads), s = static_cast<int>(row % S);
-  const long long b = row / S;
+  const int h = static_cast<int>(item - row * heads);
   __nv_bfloat16* x = qkv + row * heads * Dh + static_cast<long long>(h) * Dh;
   const int half = Dh >> 1;
   if (h >= H + Hkv) {
-    __nv_bfloat16* o = vc + ((b * Hkv + (h - H - Hkv)) * T + pos0 + s) * Dh;
+    __nv_bfloat16* o = vc + ((row * Hkv + (h - H - Hkv)) * T + pos) * Dh;
     for (int i = lane; i < Dh; i += 32) o[i] = x[i];
     return;
   }
@@ -107,16 +106,16 @@ qkv_rope_cache_kernel(__nv_bfloat16* __restrict__ qkv, const __nv_bfloat16* __re
     c[k] = i < half ? __bfloat162float(x[i + half]) : 0.f;
     ss += a[k] * a[k] + c[k] * c[k];
   }
-  const float rstd = w ? rsqrtf(lr_sum(ss) / Dh + eps) : 1.f;
-  __nv_bfloat16* o = h < H ? x : kc + ((b * Hkv + (h - H)) * T + pos0 + s) * Dh;
-  const __nv_bfloat16 *ct = cosv + static_cast<long long>(pos0 + s) * Dh, *st = sinv + static_cast<long long>(pos0 + s) * Dh;
+  const float rstd = rsqrtf(lr_sum(ss) / Dh + eps);
+  __nv_bfloat16* o = h < H ? x : kc + ((row * Hkv + (h - H)) * T + pos) * Dh;
+  const __nv_bfloat16 *ct = cosv + static_cast<long long>(pos) * Dh, *st = sinv + static_cast<long long>(pos) * Dh;
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     const int i = lane + 32 * k;
     if (i < half) {
       // rounded to bf16 after each product, as the separate multiplications round
-      const float u = w ? lr_round(lr_round(a[k] * rstd) * __bfloat162float(w[i])) : a[k];
-      const float v = w ? lr_round(lr_round(c[k] * rstd) * __bfloat162float(w[i + half])) : c[k];
+      const float u = lr_round(lr_round(a[k] * rstd) * __bfloat162float(w[i]));
+      const float v = lr_round(lr_round(c[k] * rstd) * __bfloat162float(w[i + half]));
       o[i] = __float2bfloat16_rn(lr_round(u * __bfloat162float(ct[i])) - lr_round(v * __bfloat162float(st[i])));
       o[i + half] = __float2bfloat16_rn(lr_round(v * __bfloat162float(ct[i + half])) + lr_round(u * __bfloat162float(st[i + half])));
     }
@@ -232,14 +231,14 @@ extern "C" int mdb_add_rms_rows(void* x, const void* y, const void* w, void* h, 
   return (int)cudaGetLastError();
 }
 
-extern "C" int mdb_qkv_rope_cache(void* qkv, const void* qn, const void* kn, const void* cosv, const void* sinv, void* kc, void* vc, long long rows, int S,
-                                  int H, int Hkv, int Dh, int T, int pos0, float eps, cudaStream_t st) {
-  if (Dh % 2 || Dh > 256 || Dh <= 0 || Hkv <= 0 || S <= 0 || pos0 < 0 || pos0 + S > T) return -1;
+extern "C" int mdb_qkv_rope_cache(void* qkv, const void* qn, const void* kn, const void* cosv, const void* sinv, void* kc, void* vc, long long rows, int H,
+                                  int Hkv, int Dh, int T, int pos, float eps, cudaStream_t st) {
+  if (Dh % 2 || Dh > 256 || Dh <= 0 || Hkv <= 0 || pos < 0 || pos >= T || !qn || !kn) return -1;
   const long long blocks = (rows * (H + 2 * Hkv) + 3) / 4;
   if (blocks <= 0) return 0;
   if (blocks > 2147483647ll) return -1;
   qkv_rope_cache_kernel<<<(unsigned)blocks, 128, 0, st>>>((bf16*)qkv, (const bf16*)qn, (const bf16*)kn, (const bf16*)cosv, (const bf16*)sinv, (bf16*)kc,
-                                                          (bf16*)vc, rows, S, H, Hkv, Dh, T, pos0, eps);
+                                                          (bf16*)vc, rows, H, Hkv, Dh, T, pos, eps);
   return (int)cudaGetLastError();
 }
 

@@ -150,7 +150,7 @@ class Qwen3Decoder:
         if layers is not None:
             o, H, eps, scale, y = native.ops(), c.num_attention_heads, c.rms_norm_eps, c.head_dim ** -0.5, None
             for li, (qkv, out_mlp) in enumerate(layers):
-                q = o.llm_qkv(x, y, *qkv, *cache.rope, cache.k[li], cache.v[li], 1, pos, eps)
+                q = o.llm_qkv(x, y, *qkv, *cache.rope, cache.k[li], cache.v[li], pos, eps)
                 y = o.llm_out_mlp(x, o.llm_decode_attention(q, cache.k[li], cache.v[li], H, pos + 1, scale), *out_mlp, eps)
             cache.length = pos + 1
             return x + y if y is not None else x
