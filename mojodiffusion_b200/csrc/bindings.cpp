@@ -110,7 +110,7 @@ Tensor gemm(std::vector<Tensor> As, std::vector<Tensor> Bs, const optional<Tenso
   g.accumulate_out = accumulate;
   g.bn = static_cast<int>(bn);
   g.split_k = static_cast<int>(split_k);
-  TORCH_CHECK(split_k <= 1 || (out_fp32 && out_opt.has_value()), "gemm: split-K adds into a caller-zeroed fp32 out");
+  TORCH_CHECK(split_k <= 1, "gemm: split_k is 0 (any form) or 1 (whole reductions)");
   g.pair_offset = static_cast<int>(pair_offset > 0 ? pair_offset : 0);
   g.act = static_cast<int>(act);
   g.act_on_second = static_cast<int>(act_on_second);

@@ -73,8 +73,6 @@ typedef struct MdbGemmArgs {
   // With a bf16 output (out_fp32 == 0) the reduce-scatter is STAGED instead: the row is stored (plain vector stores) into
   // slot reduce_src_rank of the owner's bf16 [world, rows_per_owner, ld_out] staging buffer; the owner sums the slots.
   int reduce_src_rank;
-  // Split-K (split_k > 1): the K range is cut into split_k parts, each a separate work item of the persistent grid; the
-  // parts are added (red.global.add) into the fp32 output, which the caller has zeroed. One K segment, no epilogue math.
   // 0: any form, also those that cut K (the few-row kernel, clusters that share a tile's reduction); 1: every output keeps one
   // accumulator over the whole K range, so that a row does not depend on the number of rows.
   int split_k;
