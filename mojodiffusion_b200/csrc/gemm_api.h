@@ -89,7 +89,7 @@ typedef struct MdbGemmArgs {
 int mdb_gemm_launch(const MdbGemmArgs* args, cudaStream_t stream);
 
 // few-row form (gemm_rows.cu): whether it computes what the arguments ask for, and its launch. mdb_gemm_launch takes it by
-// itself when the tile width is left to it (bn == 0).
+// itself when the tile width is left to it (bn == 0) and it is the fastest form.
 int mdb_gemm_rows_ok(const MdbGemmArgs* args);
 int mdb_gemm_rows(const MdbGemmArgs* args, cudaStream_t stream);
 // silu(x w1^T) * (x w2^T), halves and activation rounded to bf16, M <= MDB_GEMM_ROWS_MAX contiguous rows of K, weights [N, K]

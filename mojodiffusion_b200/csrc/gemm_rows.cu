@@ -1,5 +1,6 @@
 // Few-row GEMM: out[M, N] = epi(sum_seg A_seg[M, K_seg] * B_seg[N, K_seg]^T) for M <= 8, bf16 operands, fp32 sums.
 //
+// For few rows and for small weights (choose_form in gemm_tcgen05.cu has the measured line).
 // What bounds it: the weights are read once and used for at most eight multiply-adds per element, so the time is that of
 // streaming B from HBM. The 128-row tensor-core tiles read the same bytes from only N / 128 CTAs, and one SM takes in about
 // 64 bytes per clock: a 1 x 3072 x 9216 projection kept 72 SMs waiting for 47 us where the weights need 9 us.

@@ -2,13 +2,13 @@
 // belongs to a cluster of S CTAs; each runs a contiguous share of the K blocks (over all segments) into its own TMEM
 // accumulator, the parts meet in distributed shared memory and every CTA finishes 128 / S rows of the tile.
 //
-// Two forms: single CTAs with 128 x 128 / 128 x 64 tiles, and CTA pairs (cta_group::2) with 256 x 256 tiles, which take in a third
-// of the bytes per multiply-add and serve the larger outputs (512 x 3072 x 15360: 84 us on single CTAs, see the measured figure
-// at the pair kernel).
+// Two forms: single CTAs with 128 x 128 / 128 x 64 tiles, and CTA pairs (cta_group::2) with 256 x 256 tiles, which take in half
+// the bytes per multiply-add and serve the larger outputs (512 x 3072 x 15360: 84 us on clusters of four single CTAs, 56 on clusters
+// of two pairs, 80 on pairs that keep whole reductions).
 //
 // What it is for: outputs with fewer tiles than the GPU has SMs (a few hundred token rows, LoRA down-projections and their
-// gradients). There one SM takes in about 64 bytes per clock, so a tile of a long reduction takes kblocks x 400 cycles
-// (128 x 128) whatever the other SMs do; S CTAs cut that by S. The parts are added in CTA order in fp32, once, before the
+// gradients). There one SM takes in about 64 bytes per clock, so a tile of a long reduction takes kblocks x 600 cycles
+// (128 x 128, 32 KB a block) whatever the other SMs do; S CTAs cut that by S. The parts are added in CTA order in fp32, once, before the
 // epilogue and the only rounding: no zero-filled fp32 output, no atomics, no cast pass, and a result that does not depend on
 // scheduling.
 

@@ -21,6 +21,7 @@
 
 #include <cudaTypedefs.h>
 #include <atomic>
+#include <cmath>
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
@@ -996,7 +997,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_con
 // loads its own box through a tensor map with element strides.
 // Measured (B200), convolutions alone: 1024 x 1024 decode 13.4 -> 7.2 ms (1.42 PFLOP/s), encode of three 488 x 712 images 8.4 -> 3.8 ms.
 // RESIDENT (up to 128 input and output channels): all nine taps of the filter fit beside the pixel ring (147 KB per CTA) and are
-// loaded once per CTA instead of once per tile; with them the tile took in 408 KB for 256 pixels and the L2 was the bound
+// loaded once per CTA instead of once per tile; with them a pair took in 528 KB per tile of 256 pixels and the L2 was the bound
 // (128 -> 128 at 1024 x 1024: 440 -> 355 us).
 // Work order: channel tiles of one pair of patches are neighbours in the tile order, so the patch comes from L2 once.
 // ---------------------------------------------------------------------------------
@@ -1361,6 +1362,75 @@ static int pair_mode() {
   return mode;
 }
 
+namespace mdb {
+// The form of a bf16 GEMM that is left to the launch: few-row kernel, one CTA or CTA pair per tile, or clusters that share a tile's
+// reduction. Every form is estimated in microseconds and the lowest one taken.
+//
+// The terms are fitted to measured times of all forms over 1457 calls (M 1 to 65536, N and K 16 to 21504, the three operand
+// layouts, with and without epilogue terms; B200, weights from HBM). Over them the choice is 1.4 % above the best form of each
+// (geometric mean; 18 of them more than 20 %). What they say:
+//  - a 64-wide K step takes 0.32 / 0.34 / 0.46 us of a lone CTA with 64 / 128 / 256 columns (a narrow MMA issues hardly faster) and
+//    0.34 of a pair;
+//  - a tile's epilogue takes 1.6 to 3 us, three times that with activation, gate or residual, and hides behind the next tile's
+//    steps only; rows that end off 32 columns leave its vector path (N = 16: 8 us more);
+//  - a cluster's tile starts, meets in shared memory and ends in 6 to 9 us, and finishing its rows costs a CTA 2.2 to 7.2 us / splits
+//    (six times that with epilogue terms): it pays for long reductions only, and never for tiles that come in many waves
+//    (65536 x 128 x 128: 65 us in clusters of one, 17 on the persistent tiles). 15 % are added for it, so that it wins clear cases;
+//  - the few-row kernel streams weights at 5 to 6 TB/s for one row, but unpacks A once per column and row: at eight rows it is at
+//    1.7 (8 x 18432 x 3072: 65 us, tiles 33), and each column costs a warp its reduction over the lanes.
+struct GemmForm {
+  int bn, splits;          // splits 0: whole reductions; otherwise CTAs (or pairs) per cluster
+  bool pair, rows;
+};
+static GemmForm choose_form(const MdbGemmArgs* a, int sms, bool pairs, bool rows_ok) {
+  const bool paired = a->pair_offset > 0, whole_only = a->split_k != 0 || paired || (a->a_mn && !a->b_mn) || !pairs;
+  double kb = 0, k_all = 0;
+  for (int s = 0; s < a->num_seg; ++s) { kb += static_cast<double>((a->K[s] + 63) / 64); k_all += static_cast<double>(a->K[s]); }
+  const double n_all = paired ? 2.0 * a->N : a->N;                           // rows of B
+  const double memory = 2.0 * (a->M * k_all + n_all * k_all + static_cast<double>(a->M) * a->N) / 3.6e6;
+  const bool heavy = a->act != 0 || a->gate || a->residual || paired;
+  const double whole_terms = heavy ? 3.0 : a->bias ? 1.4 : 1.0, split_terms = heavy ? 6.2 : a->bias ? 2.1 : 1.0;
+  auto ceil_div = [](double x, double y) { return std::ceil(x / y); };
+  auto with_memory = [&](double t) { return std::sqrt(std::sqrt(t * t * t * t + memory * memory * memory * memory)); };   // neither hides wholly behind the other
+  auto tiles = [&](double tm, double tn) { return ceil_div(a->M, tm) * ceil_div(a->N, tn); };
+  auto step = [](int w) { return w == 64 ? 0.32 : w == 128 ? 0.34 : 0.46; };
+  GemmForm best = {256, 0, false, false};
+  double best_us = 1e30;
+  auto offer = [&](double us, GemmForm f) { if (us < best_us) { best_us = us; best = f; } };
+
+  auto whole = [&](double n_tiles, int width, double step_us, double epilogue) {
+    const double e = epilogue * whole_terms + (a->N % 32 != 0 && a->N < 256 ? 8.0 : 0.0), main = kb * step_us;
+    return with_memory(5.0 + ceil_div(n_tiles, width) * (main > e ? main : e) + e);
+  };
+  offer(whole(tiles(BM, paired ? 128 : 256), sms, step(256), 3.0), {256, 0, false, false});
+  if (!paired) {
+    offer(whole(tiles(BM, 128), sms, step(128), 2.1), {128, 0, false, false});
+    offer(whole(tiles(BM, 64), sms, step(64), 1.6), {64, 0, false, false});
+  }
+  if (pairs && a->M > BM) offer(whole(tiles(2 * BM, paired ? 128 : 256), pair_capacity(sms), 0.34, 2.9), {256, 0, true, false});
+  if (!whole_only) {
+    for (int w = 128; w >= 64; w -= 64)
+      for (int sp = 1; sp <= SPLIT_MAX && (sp == 1 || kb / sp >= 4); ++sp) {
+        const int cap = w == 128 ? split_capacity<128>(sp, sms) : split_capacity<64>(sp, sms);
+        const double fixed = w == 128 ? 7.0 + 3.55 * split_terms / sp : 5.9 + 2.2 * split_terms / sp;
+        offer(with_memory(1.15 * ceil_div(tiles(BM, w), cap) * (ceil_div(kb, sp) * step(w) + fixed)), {w, sp, false, false});
+      }
+    for (int sp = 2; sp <= PSPLIT_MAX && kb / sp >= 4 && !a->a_mn && a->M > BM; ++sp)
+      offer(with_memory(1.15 * ceil_div(tiles(2 * BM, 256), pair_split_capacity(sp, sms)) * (ceil_div(kb, sp) * 0.34 + 9.0 + 7.2 * split_terms / sp)), {256, sp, true, false});
+  }
+  if (rows_ok) {
+    const int r = a->M == 1 ? 0 : a->M == 2 ? 1 : a->M <= 4 ? 2 : 3;          // rows rounded up to 1, 2, 4, 8
+    static const double base[4] = {2.5, 2.7, 3.3, 4.0}, per_k[4] = {0.83e-3, 1.0e-3, 1.3e-3, 1.8e-3}, per_column[4] = {0.16e-3, 0.27e-3, 0.95e-3, 1.75e-3};
+    static const double per_mb_one[4] = {0.2, 0.28, 0.38, 0.7}, per_mb[4] = {0.165, 0.2, 0.32, 0.46};     // one column per warp, several
+    const bool one = n_all < 32.0 * sms || (paired && r == 3);
+    const double stream = n_all * k_all * 2e-6 * (one ? per_mb_one[r] : per_mb[r]), lane = k_all * per_k[r];
+    const double columns = a->N * per_column[r] * (heavy && !paired ? 2.0 : 1.0), both = std::sqrt(stream * stream + columns * columns);
+    offer(base[r] + (lane > both ? lane : both), {0, 0, false, true});
+  }
+  return best;
+}
+}  // namespace mdb
+
 extern "C" int mdb_gemm_launch(const MdbGemmArgs* a, cudaStream_t stream) {
   using namespace mdb;
   if (a->M <= 0 || a->N <= 0 || a->num_seg < 1 || a->num_seg > MDB_GEMM_MAX_SEG || a->split_k > 1) return -2;
@@ -1371,8 +1441,6 @@ extern "C" int mdb_gemm_launch(const MdbGemmArgs* a, cudaStream_t stream) {
     flat.conv_taps = 0;
     a = &flat;
   }
-  // up to eight rows the weights are streamed by all SMs instead of by the N / 128 CTAs that own a tile
-  if (a->M <= MDB_GEMM_ROWS_MAX && mdb_gemm_rows_ok(a)) return mdb_gemm_rows(a, stream);
   const int eb = a->kind == 1 ? 1 : 2;
   const int k_elems = BK_BYTES / eb;
   const bool paired = a->pair_offset > 0;
@@ -1383,7 +1451,18 @@ extern "C" int mdb_gemm_launch(const MdbGemmArgs* a, cudaStream_t stream) {
   bool use_pair = bn == 512 && pair_ok;
   if (bn == 512) bn = 256;
   const bool auto_tile = bn != 64 && bn != 128 && bn != 256;
-  if (bn != 64 && bn != 128 && bn != 256) {
+  int splits = 0;
+  bool pair_split = false;
+  const bool plain = a->kind == 0 && a->conv_taps <= 0 && a->gather_world <= 1 && !a->row_scale && !a->col_scale && a->route_owner_cols <= 0 &&
+                     a->reduce_rows_per_owner <= 0 && !a->prof;
+  if (auto_tile && plain) {
+    const GemmForm f = choose_form(a, sms, pair_mode() != 0, mdb_gemm_rows_ok(a) != 0);
+    if (f.rows) return mdb_gemm_rows(a, stream);
+    bn = f.bn;
+    splits = f.splits;
+    use_pair = f.pair && f.splits == 0;
+    pair_split = f.pair && f.splits > 0;
+  } else if (auto_tile) {
     // default tile choice: 128x256 unless the narrower 128x128 tile fills the machine noticeably better
     // (fewer idle SMs in the last wave); 128x64 only for very skinny outputs
     const int tm = (a->M + BM - 1) / BM;
@@ -1397,7 +1476,7 @@ extern "C" int mdb_gemm_launch(const MdbGemmArgs* a, cudaStream_t stream) {
     if (!paired && a->N <= 64) bn = 64;
   }
   if (paired && bn != 256) bn = 256;
-  if (auto_tile && pair_ok && a->M > BM && pair_mode() != 0) {
+  if (auto_tile && !plain && pair_ok && a->M > BM && pair_mode() != 0) {
     // CTA pair (256 x 256 tile on two SMs) or lone CTAs? Compare waves x time per tile. A lone CTA's 128 x 256 tile moves
     // 96 KB through shared memory per K block (48 KB written by TMA, 48 KB read by the tensor core): 726 cycles measured,
     // bound by the 128 B/clk of shared memory. A pair tile moves 64 KB per SM and runs at the tensor rate: 523 cycles.
@@ -1412,38 +1491,6 @@ extern "C" int mdb_gemm_launch(const MdbGemmArgs* a, cudaStream_t stream) {
     if (cost2 <= cost1) {
       use_pair = true;
       bn = 256;
-    }
-  }
-  // Few tiles for the SMs there are: compare the tiling chosen above with clusters that share a tile's reduction, in cycles. A 64-wide K step costs 533 cycles on a pair, 726 / 600 / 600 on a lone CTA of 256 / 128 / 64
-  // columns (measured; a 64-wide MMA issues no faster than a wider one). The epilogue of a whole-K tile takes about 5000 cycles per 128 columns of a CTA and hides behind the next
-  // tile's steps only, and rows whose length is no multiple of 32 columns leave its vector path (20000 cycles: adapters of rank
-  // 16). Starting a tile costs about 2500; meeting in shared memory and finishing the rows 5000, or 10000 for a pair's tile.
-  int splits = 0;
-  bool pair_split = false;
-  if (auto_tile && pair_mode() != 0 && a->kind == 0 && a->conv_taps <= 0 && a->gather_world <= 1 && a->split_k == 0 && !paired && !a->row_scale &&
-      !a->col_scale && a->route_owner_cols <= 0 && a->reduce_rows_per_owner <= 0 && !a->prof && !(a->a_mn && !a->b_mn)) {
-    int kb = 0;
-    for (int s = 0; s < a->num_seg; ++s) kb += static_cast<int>((a->K[s] + 63) / 64);
-    const long long tm = (a->M + BM - 1) / BM;
-    auto tiles_of = [&](int w) { return tm * ((a->N + w - 1) / w); };
-    auto step_of = [](int w) { return w == 256 ? 726.0 : 600.0; };
-    auto whole = [&](long long tiles, int width, double step, double cols) {
-      const double epi = cols / 128 * 5000.0 + (a->N % 32 != 0 && a->N < 256 ? 20000.0 : 0.0), main = kb * step;
-      return static_cast<double>((tiles + width - 1) / width) * (main > epi ? main : epi) + epi + 2500.0;
-    };
-    const long long pt = static_cast<long long>((a->M + 2 * BM - 1) / (2 * BM)) * ((a->N + 255) / 256);
-    double best = use_pair ? whole(pt, pair_capacity(sms), 533.0, 256) : whole(tiles_of(bn), sms, step_of(bn), bn);
-    best *= 0.95;                                              // the whole-K tilings need no meeting: they win ties
-    for (int w = 128; w >= 64; w -= 64)
-      for (int sp = 1; sp <= SPLIT_MAX && (sp == 1 || kb / sp >= 4); ++sp) {
-        const int cap = w == 128 ? split_capacity<128>(sp, sms) : split_capacity<64>(sp, sms);
-        const double c = static_cast<double>((tiles_of(w) + cap - 1) / cap) * (((kb + sp - 1) / sp) * step_of(w) + 7500.0);
-        if (c < best) { best = c; bn = w; splits = sp; use_pair = false; }
-      }
-    for (int sp = 2; sp <= PSPLIT_MAX && kb / sp >= 4 && !a->a_mn && a->M > BM; ++sp) {
-      const int cap = pair_split_capacity(sp, sms);
-      const double c = static_cast<double>((pt + cap - 1) / cap) * (((kb + sp - 1) / sp) * 533.0 + 12500.0);
-      if (c < best) { best = c; bn = 256; splits = sp; use_pair = false; pair_split = true; }
     }
   }
   // 3 x 3 convolutions: waves x time of one 64-wide K step (726 cycles of a lone CTA's 128 x 256 tile = 1; a pair's tile of two

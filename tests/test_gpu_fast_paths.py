@@ -439,14 +439,15 @@ def test_decode_attention_probabilities():
 def test_wide_single_head_attention_other_forms(form):
     from torch.autograd import forward_ad
     from torch.utils._python_dispatch import TorchDispatchMode
-    B, Sq, Skv, Dh = 3, 33, 40, 256
+    B, Sq, Skv, Dh = 3, 33, 2000, 512
     q, k, v = (_rand(B, s, 1, Dh, seed=i) for i, s in ((1, Sq), (2, Skv), (3, Skv)))
+    assert O.functional._wide_ok(q, k, v)                       # the plain call is on the GEMMs
     with torch.no_grad():
         plain = O.attention(q, k, v)
         if form == "one key batch":
             got, want = O.attention(q, k[:1], v[:1]), O.attention(q, k[:1].repeat(B, 1, 1, 1), v[:1].repeat(B, 1, 1, 1))
         elif form == "value width":
-            got, want = O.attention(q, k, v[..., :136]), plain[..., :136]
+            got, want = O.attention(q, k, v[..., :256]), plain[..., :256]
         elif form == "many key heads":
             got = O.attention(q, torch.cat((k, k), 2), torch.cat((v, v), 2))
             want = torch.cat((plain, plain), 2)
@@ -540,3 +541,27 @@ def test_decode_step_keeps_to_its_modules(change):
     native.check_status(torch.empty(0, device=DEV))
     # as for the layers above, with two layers
     assert float((outs[0] - outs[1]).norm() / outs[1].norm()) < 2 * 2.0 ** -9 / 3 ** 0.5 * 44 ** 0.5
+
+
+def test_epilogue_terms_of_narrow_tiles():
+    for N in (640, 1160):
+        test_epilogue_terms(64, N)
+
+
+# sizes drawn over the range that the launch chooses its form for, in the three operand layouts, against the fp32 product
+@pytest.mark.parametrize("seed", range(8))
+def test_gemm_forms_left_to_the_launch(seed):
+    import random
+    from mojodiffusion_b200.ops.functional import _gemm
+    r = random.Random(seed)
+    for _ in range(12):
+        M, N, K = (int(round(math.exp(r.uniform(math.log(lo), math.log(hi))))) for lo, hi in ((1, 5000), (8, 6000), (8, 6000)))
+        N8, K8, M8 = ((t + 7) // 8 * 8 for t in (N, K, M))
+        x, w, bias, res = _rand(M, K8, seed=1)[:, :K], _rand(N, K8, scale=1 / math.sqrt(K), seed=2)[:, :K], _rand(N, seed=3), _rand(M, N, seed=4)
+        want = x.float() @ w.float().t()
+        _close(_gemm([x], [w]), want, f"NT {M}x{N}x{K}")
+        _close(_gemm([x], [w], bias=bias, residual=res, act=2), ref.linear(x, w, bias, "silu", res, None, 1, out_dtype=torch.float32), f"terms {M}x{N}x{K}", rel=1e-4)
+        wt, xt = torch.zeros(K, N8, dtype=torch.bfloat16, device=DEV), torch.zeros(K, M8, dtype=torch.bfloat16, device=DEV)
+        wt[:, :N], xt[:, :M] = w.t(), x.t()
+        _close(_gemm([x], [wt[:, :N]], b_mn=True), want, f"NN {M}x{N}x{K}")
+        _close(_gemm([xt[:, :M]], [wt[:, :N]], a_mn=True, b_mn=True), want, f"TN {M}x{N}x{K}")
