@@ -120,8 +120,11 @@ softmax_rows_kernel(const float* __restrict__ s, __nv_bfloat16* __restrict__ p, 
 // further, so both halves of a rotation are in one thread; a row of 4096 columns is one item per thread. Replaces two norms
 // into fresh buffers, two copies back into the packed rows and a rotation pass (six passes over q and k: 232 us per layer at
 // 6144 x 4096) by one (119 us).
+// A block has as many threads as the row has items, up to 256 (rows of 256 columns: 16 items; a block of 256 threads for them made
+// the pass slower than the separate operations, 238 against 206 us for an attention of 6144 tokens).
 constexpr int NR_THREADS = 256, NR_ITEMS = 4;
-__global__ void __launch_bounds__(NR_THREADS)
+template <int THREADS, int ITEMS>
+__global__ void __launch_bounds__(THREADS)
 rms_rope_rows_kernel(__nv_bfloat16* __restrict__ buf, const __nv_bfloat16* __restrict__ wq, const __nv_bfloat16* __restrict__ wk,
                      const float* __restrict__ cosv, const float* __restrict__ sinv, long long ld, int D, int Dh, int q_off, int k_off,
                      int rows_per_batch, float eps) {
@@ -130,11 +133,11 @@ rms_rope_rows_kernel(__nv_bfloat16* __restrict__ buf, const __nv_bfloat16* __res
   const __nv_bfloat16* w = blockIdx.y ? wk : wq;
   __nv_bfloat16* x = buf + row * ld + (blockIdx.y ? k_off : q_off);
   const int half = Dh >> 1, per_head = half >> 3, items = D >> 4;
-  float a[NR_ITEMS][8], b[NR_ITEMS][8];
+  float a[ITEMS][8], b[ITEMS][8];
   float ss = 0.f;
 #pragma unroll
-  for (int k = 0; k < NR_ITEMS; ++k) {
-    const int i = threadIdx.x + k * NR_THREADS;
+  for (int k = 0; k < ITEMS; ++k) {
+    const int i = threadIdx.x + k * THREADS;
     if (i < items) {
       const int c = (i / per_head) * Dh + (i % per_head) * 8;
       const uint4 u = *reinterpret_cast<const uint4*>(x + c), t = *reinterpret_cast<const uint4*>(x + c + half);
@@ -148,12 +151,12 @@ rms_rope_rows_kernel(__nv_bfloat16* __restrict__ buf, const __nv_bfloat16* __res
       }
     }
   }
-  ss = fr_block<NR_THREADS, false>(ss, red);
+  ss = fr_block<THREADS, false>(ss, red);
   const float rstd = rsqrtf(ss / D + eps);
   const size_t tok = static_cast<size_t>(row % rows_per_batch) * half;
 #pragma unroll
-  for (int k = 0; k < NR_ITEMS; ++k) {
-    const int i = threadIdx.x + k * NR_THREADS;
+  for (int k = 0; k < ITEMS; ++k) {
+    const int i = threadIdx.x + k * THREADS;
     if (i < items) {
       const int h0 = (i % per_head) * 8, c = (i / per_head) * Dh + h0;
       const uint4 wa = *reinterpret_cast<const uint4*>(w + c), wb = *reinterpret_cast<const uint4*>(w + c + half);
@@ -218,8 +221,14 @@ extern "C" int mdb_rms_rope_rows(void* buf, const void* wq, const void* wk, cons
       rows_per_batch <= 0 || rows > 2147483647ll)
     return -1;
   if (rows <= 0) return 0;
-  rms_rope_rows_kernel<<<dim3((unsigned)rows, 2), NR_THREADS, 0, st>>>((bf16*)buf, (const bf16*)wq, (const bf16*)wk, cosv, sinv, ld, D, Dh, q_off, k_off,
-                                                                     rows_per_batch, eps);
+  const int items = D >> 4;
+  auto kern = items <= 32    ? rms_rope_rows_kernel<32, 1>
+              : items <= 64  ? rms_rope_rows_kernel<64, 1>
+              : items <= 128 ? rms_rope_rows_kernel<128, 1>
+              : items <= 256 ? rms_rope_rows_kernel<NR_THREADS, 1>
+                             : rms_rope_rows_kernel<NR_THREADS, NR_ITEMS>;
+  const int threads = items <= 32 ? 32 : items <= 64 ? 64 : items <= 128 ? 128 : NR_THREADS;
+  kern<<<dim3((unsigned)rows, 2), threads, 0, st>>>((bf16*)buf, (const bf16*)wq, (const bf16*)wk, cosv, sinv, ld, D, Dh, q_off, k_off, rows_per_batch, eps);
   return (int)cudaGetLastError();
 }
 

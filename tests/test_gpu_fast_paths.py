@@ -548,6 +548,12 @@ def test_epilogue_terms_of_narrow_tiles():
         test_epilogue_terms(64, N)
 
 
+# rows of 64, 128 and 256 items: the widths at which the one-pass q / k kernel changes its block
+@pytest.mark.parametrize("hidden,heads,head_dim", [(512, 8, 64), (528, 33, 16), (1024, 16, 64), (2048, 16, 128), (4096, 32, 128)])
+def test_video_attention_row_blocks(hidden, heads, head_dim):
+    test_video_attention_rows(hidden, heads, head_dim)
+
+
 # sizes drawn over the range that the launch chooses its form for, in the three operand layouts, against the fp32 product
 @pytest.mark.parametrize("seed", range(8))
 def test_gemm_forms_left_to_the_launch(seed):
