@@ -827,11 +827,17 @@ Tensor llm_decode_attention(const Tensor& qkv, const Tensor& k_cache, const Tens
                                 (int)T, (int)len, (float)scale, cur_stream()), "decode_attention");
   return o;
 }
-void softmax_rows(const Tensor& s, Tensor p, double scale) {
+void softmax_rows(const Tensor& s, Tensor p, double scale, const optional<Tensor>& low) {
   TORCH_CHECK(s.is_cuda() && s.dim() == 2 && s.stride(1) == 1 && s.scalar_type() == at::kFloat && p.device() == s.device() && p.dim() == 2 &&
                   p.stride(1) == 1 && p.scalar_type() == at::kBFloat16 && p.sizes() == s.sizes(), "softmax_rows: fp32 scores, bf16 output of one shape");
   c10::cuda::CUDAGuard guard(s.device());
-  check_rc(mdb_softmax_rows(s.data_ptr<float>(), p.data_ptr(), s.size(0), (int)s.size(1), s.stride(0), p.stride(0), (float)scale, cur_stream()),
+  void* pl = nullptr;
+  if (low.has_value() && low->defined()) {
+    TORCH_CHECK(low->device() == s.device() && low->scalar_type() == at::kBFloat16 && low->sizes() == p.sizes() && low->strides() == p.strides(),
+                "softmax_rows: the low part is laid out as the output");
+    pl = low->data_ptr();
+  }
+  check_rc(mdb_softmax_rows(s.data_ptr<float>(), p.data_ptr(), pl, s.size(0), (int)s.size(1), s.stride(0), p.stride(0), (float)scale, cur_stream()),
            "softmax_rows");
 }
 // buf [rows, W] bf16, rows of ``rows_per_batch`` tokens per sample; cos / sin [positions, Dh / 2] fp32
@@ -1168,7 +1174,7 @@ TORCH_LIBRARY(mdb200, m) {
   m.def("lora_linear_fwd", &lora_linear_fwd);
   m.def("lora_linear_bwd", &lora_linear_bwd);
   m.def("conv2d_nhwc", &conv2d_nhwc);
-  m.def("softmax_rows", &softmax_rows);
+  m.def("softmax_rows(Tensor s, Tensor(a!) p, float scale, Tensor(b!)? low=None) -> ()", &softmax_rows);
   m.def("rms_rope_rows", &rms_rope_rows);
   m.def("head_gate", &head_gate);
   m.def("conv2d_nhwc_strided", &conv2d_nhwc_strided);

@@ -32,16 +32,19 @@ __device__ __forceinline__ float fr_block(float v, float* red) {
   return MAX ? fr_warp_max(t) : fr_warp_sum(t);
 }
 
-// P[r, :] = softmax(S[r, :] * scale) (fp32 scores, bf16 probabilities). One block per row; up to 16384 columns stay in registers
+// P[r, :] = softmax(S[r, :] * scale) (fp32 scores, bf16 probabilities and, when asked for, what their rounding left as a second bf16
+// row: two terms hold a probability to 2^-17). One block per row; up to 16384 columns stay in registers
 // (CACHED), so the scores are read once; longer rows are read three times, from L2 after the first. Bound by HBM: 6 bytes per
 // score. The row maximum ignores NaN scores, their exponentials carry the NaN into the sum and so into the whole row.
 constexpr int SM_THREADS = 512, SM_VEC = 8;
 template <bool CACHED>
 __global__ void __launch_bounds__(SM_THREADS)
-softmax_rows_kernel(const float* __restrict__ s, __nv_bfloat16* __restrict__ p, int cols, long long lds, long long ldp, float scale_log2) {
+softmax_rows_kernel(const float* __restrict__ s, __nv_bfloat16* __restrict__ p, __nv_bfloat16* __restrict__ low, int cols, long long lds, long long ldp,
+                    float scale_log2) {
   __shared__ float red[32];
   const float* sr = s + static_cast<size_t>(blockIdx.x) * lds;
   __nv_bfloat16* pr = p + static_cast<size_t>(blockIdx.x) * ldp;
+  __nv_bfloat16* lr = low ? low + static_cast<size_t>(blockIdx.x) * ldp : nullptr;
   const int nv = (cols + 3) >> 2;
   auto load = [&](int i) {                       // scaled scores; columns past the end are not touched and count as -inf
     const int c = i * 4;
@@ -94,14 +97,23 @@ softmax_rows_kernel(const float* __restrict__ s, __nv_bfloat16* __restrict__ p, 
   }
   sum = fr_block<SM_THREADS, false>(sum, red);
   const float inv = 1.f / sum;
-  auto put = [&](int i, float4 t) {
-    const int c = i * 4;
+  auto store = [&](__nv_bfloat16* row, int c, uint2 q) {
     if (c + 3 < cols) {
-      *reinterpret_cast<uint2*>(pr + c) = make_uint2(pack_bf16x2(t.x * inv, t.y * inv), pack_bf16x2(t.z * inv, t.w * inv));
+      *reinterpret_cast<uint2*>(row + c) = q;
     } else {
-      pr[c] = __float2bfloat16_rn(t.x * inv);
-      if (c + 1 < cols) pr[c + 1] = __float2bfloat16_rn(t.y * inv);
-      if (c + 2 < cols) pr[c + 2] = __float2bfloat16_rn(t.z * inv);
+      const __nv_bfloat162 *h0 = reinterpret_cast<const __nv_bfloat162*>(&q.x), *h1 = reinterpret_cast<const __nv_bfloat162*>(&q.y);
+      row[c] = h0->x;
+      if (c + 1 < cols) row[c + 1] = h0->y;
+      if (c + 2 < cols) row[c + 2] = h1->x;
+    }
+  };
+  auto put = [&](int i, float4 t) {
+    t = make_float4(t.x * inv, t.y * inv, t.z * inv, t.w * inv);
+    const uint2 q = make_uint2(pack_bf16x2(t.x, t.y), pack_bf16x2(t.z, t.w));
+    store(pr, i * 4, q);
+    if (lr) {
+      const float2 a = unpack_bf16x2(q.x), b = unpack_bf16x2(q.y);
+      store(lr, i * 4, make_uint2(pack_bf16x2(t.x - a.x, t.y - a.y), pack_bf16x2(t.z - b.x, t.w - b.y)));
     }
   };
   if (CACHED) {
@@ -204,13 +216,13 @@ head_gate_kernel(__nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict_
 using namespace mdb;
 typedef __nv_bfloat16 bf16;
 
-extern "C" int mdb_softmax_rows(const float* s, void* p, long long rows, int cols, long long lds, long long ldp, float scale, cudaStream_t st) {
+extern "C" int mdb_softmax_rows(const float* s, void* p, void* low, long long rows, int cols, long long lds, long long ldp, float scale, cudaStream_t st) {
   if (cols <= 0 || lds % 4 || ldp % 4 || lds < cols || ldp < cols || rows > 2147483647ll) return -1;
-  if ((reinterpret_cast<uintptr_t>(s) & 15) || (reinterpret_cast<uintptr_t>(p) & 7)) return -1;
+  if ((reinterpret_cast<uintptr_t>(s) & 15) || ((reinterpret_cast<uintptr_t>(p) | reinterpret_cast<uintptr_t>(low)) & 7)) return -1;
   if (rows <= 0) return 0;
   const float k = scale * 1.4426950408889634f;
-  if (cols <= 4 * SM_THREADS * SM_VEC) softmax_rows_kernel<true><<<(unsigned)rows, SM_THREADS, 0, st>>>(s, (bf16*)p, cols, lds, ldp, k);
-  else softmax_rows_kernel<false><<<(unsigned)rows, SM_THREADS, 0, st>>>(s, (bf16*)p, cols, lds, ldp, k);
+  if (cols <= 4 * SM_THREADS * SM_VEC) softmax_rows_kernel<true><<<(unsigned)rows, SM_THREADS, 0, st>>>(s, (bf16*)p, (bf16*)low, cols, lds, ldp, k);
+  else softmax_rows_kernel<false><<<(unsigned)rows, SM_THREADS, 0, st>>>(s, (bf16*)p, (bf16*)low, cols, lds, ldp, k);
   return (int)cudaGetLastError();
 }
 

@@ -58,8 +58,8 @@ int mdb_decode_attention(const void* q, long long ldq, const void* kc, const voi
                          float scale, cudaStream_t st);
 
 // ---- fused_rows.cu
-// P = softmax(S * scale) per row; leading dimensions multiples of 4; nothing beside the columns is read or written
-int mdb_softmax_rows(const float* s, void* p, long long rows, int cols, long long lds, long long ldp, float scale, cudaStream_t st);
+// P = softmax(S * scale) per row, low (or null, same leading dimension) = what the rounding of P left; leading dimensions multiples of 4; nothing beside the columns is read or written
+int mdb_softmax_rows(const float* s, void* p, void* low, long long rows, int cols, long long lds, long long ldp, float scale, cudaStream_t st);
 // in place on rows of a packed buffer: full-width RMSNorm (D columns from q_off and from k_off) + split-half rotation per head
 int mdb_rms_rope_rows(void* buf, const void* wq, const void* wk, const float* cosv, const float* sinv, long long rows, long long ld, int D,
                       int Dh, int q_off, int k_off, int rows_per_batch, float eps, cudaStream_t st);

@@ -464,34 +464,49 @@ def split_cols(x: torch.Tensor, a: int):
     return x[..., :a], x[..., a:]
 
 
+#: scores that ``_wide_attention`` holds at a time (fp32, and two bf16 terms per probability: 0.5 GB)
+WIDE_SCORES = 1 << 26
+
+
 def _wide_attention(q, k, v, scale: float):
-    """One head wider than the attention kernel's tiles (the 512-channel block of the image autoencoders): scores as one
-    tcgen05 GEMM into fp32, a softmax pass over their rows, the weighted sum as a second GEMM. At most 2^27 scores (fp32
-    scores and bf16 probabilities: 0.8 GB) are held at a time, so memory stays linear in the number of pixels."""
+    """One head wider than the attention kernels' tiles (the 512-channel block of the image autoencoders): scores as one
+    tcgen05 GEMM into fp32, a softmax pass over their rows, the weighted sum as a second GEMM. A probability goes in as two bf16
+    terms, so the result carries no rounding but its own (relative error 0.0017 on normal inputs; 0.0022 for the library kernel
+    and 0.0024 with one term, which round the probabilities). Memory stays linear in the number of pixels."""
     B, Sq, _, Dh = q.shape
     Skv = k.shape[1]
     ld = (Skv + 7) // 8 * 8                                  # 16-byte rows; the padding columns are never read
-    rows = min(Sq, max(256, (1 << 27) // ld // 256 * 256))
+    rows = min(Sq, max(256, WIDE_SCORES // ld // 256 * 256))
     o = torch.empty(B, Sq, 1, Dh, dtype=q.dtype, device=q.device)
     s = torch.empty(rows, ld, dtype=torch.float32, device=q.device)
-    p = torch.empty(rows, ld, dtype=q.dtype, device=q.device)
+    p = torch.empty(2, rows, ld, dtype=q.dtype, device=q.device)
     for b in range(B):
         kb, vb, qb = _flat2d(k[b]), _flat2d(v[b]), _flat2d(q[b])
         for r0 in range(0, Sq, rows):
             n = min(rows, Sq - r0)
             _gemm([qb[r0:r0 + n]], [kb], out=s[:n, :Skv], out_fp32=True)
-            _ops().softmax_rows(s[:n, :Skv], p[:n, :Skv], scale)
-            _gemm([p[:n, :Skv]], [vb], b_mn=True, out=o[b, r0:r0 + n, 0])
+            _ops().softmax_rows(s[:n, :Skv], p[0, :n, :Skv], scale, p[1, :n, :Skv])
+            _gemm([p[0, :n, :Skv], p[1, :n, :Skv]], [vb, vb], b_mn=True, out=o[b, r0:r0 + n, 0])
     return o
 
 
+def _wide_pays(B: int, Sq: int, Skv: int, Dh: int) -> bool:
+    """Whether ``_wide_attention`` is the faster form. Up to a width of 256 the library has its tiled kernel, which is faster at every
+    size. Beyond, it walks the keys one by one, 64 queries to a block (16384 pixels of width 512: 3590 us against 1500), while the
+    GEMMs take three launches per sample. Microseconds, fitted to 90 sizes of width 264 to 1024; the wrong side is taken within
+    a third of either time."""
+    library = 6 + (0.03 + 1.2e-4 * Dh) * Skv * max(1.0, B * Sq / 6080)
+    return Dh > 256 and B * (26 + 4.5e-3 * Sq + 5.3e-6 * Sq * Skv * max(1.0, Dh / 800)) < library
+
+
 def _wide_ok(q, k, v) -> bool:
-    """Whether ``_wide_attention`` covers these operands: one bf16 head of the same width on all sides, no broadcasting between
-    them, no gradient and no transform that has to see the torch operations."""
+    """Whether ``_wide_attention`` covers these operands and pays: one bf16 head of the same width on all sides, no broadcasting
+    between them, no gradient and no transform that has to see the torch operations."""
     return (q.dim() == k.dim() == 4 and q.shape[2] == 1 and q.shape[3] > 128 and q.shape[3] % 8 == 0 and q.shape[1] > 0 and k.shape[1] > 0
             and q.shape[0] == k.shape[0] and q.shape[2:] == k.shape[2:] and k.shape == v.shape and q.device == k.device == v.device
             and q.dtype == k.dtype == v.dtype == torch.bfloat16
-            and not (torch.is_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad)) and native.direct(q, k, v))
+            and not (torch.is_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad))
+            and _wide_pays(q.shape[0], q.shape[1], k.shape[1], q.shape[3]) and native.direct(q, k, v))
 
 
 def attention(q, k, v, scale: Optional[float] = None, kv_len: Optional[torch.Tensor] = None,

@@ -543,6 +543,17 @@ def test_decode_step_keeps_to_its_modules(change):
     assert float((outs[0] - outs[1]).norm() / outs[1].norm()) < 2 * 2.0 ** -9 / 3 ** 0.5 * 44 ** 0.5
 
 
+# the GEMM form of one wide head rounds its result only: 2^-9 / sqrt(3) of its size, doubled for the spread of that estimate (one bf16 term per
+# probability adds as much again). Odd key counts, one key, several chunks of rows, a width off 16
+@pytest.mark.parametrize("B,Sq,Skv,Dh", [(1, 5, 3, 512), (2, 7, 1, 512), (3, 333, 333, 512), (2, 300, 1001, 136), (1, 5000, 17001, 256)])
+def test_wide_attention_on_gemms_rounds_once(B, Sq, Skv, Dh):
+    q, k, v = (_rand(B, s, 1, Dh, seed=i) for i, s in ((1, Sq), (2, Skv), (3, Skv)))
+    out = O.functional._wide_attention(q, k, v, 1 / math.sqrt(Dh))
+    native.check_status(out)
+    want = torch.cat([torch.softmax(q[b, :, 0].double() @ k[b, :, 0].double().t() / math.sqrt(Dh), -1) @ v[b, :, 0].double() for b in range(B)]).view(B, Sq, 1, Dh)
+    assert float((out.double() - want).norm() / want.norm()) < 2 * 2.0 ** -9 / 3 ** 0.5
+
+
 def test_epilogue_terms_of_narrow_tiles():
     for N in (640, 1160):
         test_epilogue_terms(64, N)
