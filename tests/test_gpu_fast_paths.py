@@ -582,3 +582,9 @@ def test_gemm_forms_left_to_the_launch(seed):
         wt[:, :N], xt[:, :M] = w.t(), x.t()
         _close(_gemm([x], [wt[:, :N]], b_mn=True), want, f"NN {M}x{N}x{K}")
         _close(_gemm([xt[:, :M]], [wt[:, :N]], a_mn=True, b_mn=True), want, f"TN {M}x{N}x{K}")
+
+
+# beyond 2048 channels: pixels on either side of the lines between one block per group and chunks of pixels (forward 512, backward 160)
+@pytest.mark.parametrize("N,HW", [(1, 8), (2, 159), (1, 160), (1, 511), (2, 512)])
+def test_group_norm_wide_tensors_of_few_pixels(N, HW):
+    test_group_norm_forward_and_backward(N, HW, 2560, 32)
