@@ -371,7 +371,8 @@ __global__ void fp8_quant_rows_kernel(const __nv_bfloat16* __restrict__ x, __nv_
 }
 // The same for rows of 2048 to 16384 elements: a block of 256 threads per row that keeps the row in registers, so it is read once
 // and eight warps share it. (One warp walked a row of 4096 in 16 dependent steps, twice: 2737 rows of 4096 12.4 -> 5.4 us; their 34 MB take 5.)
-// Shorter rows would leave most of the block idle and stay on one warp each; the bytes are the same either way.
+// Shorter rows would leave most of the block idle and stay on one warp each, and so do rows of less than 3072 when there are enough of
+// them to keep every SM reading (6144 x 2048: 7.0 us a warp per row, 8.0 a block; 512 x 2048: 3.0 and 2.4).
 template <int VPT>
 __global__ void __launch_bounds__(256)
 fp8_quant_rows_block_kernel(const __nv_bfloat16* __restrict__ x, __nv_fp8_storage_t* __restrict__ q, float* __restrict__ scale, int D, int ldx, int ldq) {
@@ -654,7 +655,7 @@ extern "C" int mdb_fp8_quant_rows(const void* x, void* q, float* scale, long lon
                                   cudaStream_t st) {
   if (D % 8 || ldx % 8 || ldq % 8) return -1;
   if (rows == 0) return 0;
-  if (D >= 2048 && D <= 16384 && rows <= 2147483647ll) {
+  if (D >= 2048 && D <= 16384 && (D >= 3072 || rows < 4096) && rows <= 2147483647ll) {
     const int vpt = (D / 8 + 255) / 256;
     const bf16* xp = (const bf16*)x;
     __nv_fp8_storage_t* qp = (__nv_fp8_storage_t*)q;
