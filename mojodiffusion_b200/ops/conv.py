@@ -94,8 +94,8 @@ def conv2d_weight_grad(x, dy, KH: int, KW: int, pad):
 
 
 class _Conv2dFn(torch.autograd.Function):
-    """Convolution with native forward and native input gradient (the same kernel on the rotated weights; a stride-2
-    layer is the stride-1 result sampled at every second position, its gradient scattered back before the rotation).
+    """Convolution with native forward and native input gradient (the same kernel on the rotated weights; the gradient of
+    a stride-2 layer is scattered back to every second position first).
     Weight and bias gradients are computed only when asked for."""
 
     @staticmethod
@@ -125,7 +125,7 @@ class _Conv2dFn(torch.autograd.Function):
 
 
 def conv2d_nhwc(x, w_ohwi, bias=None, stride: int = 1, padding=1, act=None, residual=None, offset: int = 0):
-    """``stride`` 2 samples the stride-1 "same" result at ``offset::2`` (offset 0: symmetric padding as in the UNet
+    """``stride`` 2 computes the pixels ``offset::2`` of the stride-1 "same" result (offset 0: symmetric padding as in the UNet
     down-samplers; offset 1: the right / bottom padded stride-2 convolution of the LDM encoders)."""
     pad = (padding, padding) if isinstance(padding, int) else tuple(padding)
     KH, KW, Cin = w_ohwi.shape[1], w_ohwi.shape[2], w_ohwi.shape[3]
