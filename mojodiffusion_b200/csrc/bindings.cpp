@@ -706,13 +706,14 @@ Tensor randn(std::vector<int64_t> shape, int64_t seed, int64_t offset, bool bf16
 // ------------------------------------------------------------------------------------------
 // decoder stack: one layer of a decode step, one row per sequence
 // ------------------------------------------------------------------------------------------
-// Contiguous, 16-byte aligned bf16 memory of one GPU, all of them, with the shapes given: two numbers per tensor, rows and columns,
-// columns 0 for a vector, rows -1 for any shape.
+// Contiguous, 16-byte aligned bf16 memory of one GPU, all of them. Tensor i has the shape shapes[i % count]: two numbers, rows and
+// columns, columns 0 for a vector, rows -1 for any shape.
 bool bf16_operands_ok(const std::vector<Tensor>& ts, const std::vector<int64_t>& shapes) {
-  TORCH_CHECK(shapes.size() == 2 * ts.size(), "bf16_operands_ok: two numbers per tensor");
+  TORCH_CHECK(!shapes.empty() && shapes.size() % 2 == 0, "bf16_operands_ok: two numbers per shape");
+  const size_t count = shapes.size() / 2;
   for (size_t i = 0; i < ts.size(); ++i) {
     const Tensor& t = ts[i];
-    const int64_t rows = shapes[2 * i], cols = shapes[2 * i + 1];
+    const int64_t rows = shapes[i % count * 2], cols = shapes[i % count * 2 + 1];
     if (!t.is_cuda() || t.device() != ts[0].device() || t.scalar_type() != at::kBFloat16 || t.layout() != at::kStrided || !t.is_contiguous() ||
         t.unsafeGetTensorImpl()->is_python_dispatch() || reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 != 0)
       return false;

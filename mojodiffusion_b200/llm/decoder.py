@@ -77,35 +77,46 @@ class Qwen3Decoder:
             return None
         D, Dh, F, eps = c.hidden_size, c.head_dim, c.intermediate_size, c.rms_norm_eps
         Q, KV = c.num_attention_heads * Dh, c.num_key_value_heads * Dh
-        layers, flat = [], []
+        layers, flat, has = [], [], None
         for l in self.enc.model.layers:
-            a, m = l._modules["self_attn"], l._modules["mlp"]
-            if own_parameters(m, _MLP) is None:
+            l = l._modules
+            a, mlp, norm = l["self_attn"]._modules, l["mlp"], own_parameters(l["input_layernorm"], _Norm)
+            post, q_norm, k_norm = own_parameters(l["post_attention_layernorm"], _Norm), own_parameters(a["q_norm"], _Norm), own_parameters(a["k_norm"], _Norm)
+            if own_parameters(mlp, _MLP) is None or norm is None or post is None or q_norm is None or k_norm is None:
                 return None
-            a, m, ps = a._modules, m._modules, []
-            for mod, cls in ((l._modules["input_layernorm"], _Norm), (a["q_proj"], _W), (a["k_proj"], _W), (a["v_proj"], _W), (a["q_norm"], _Norm), (a["k_norm"], _Norm),
-                             (a["o_proj"], _W), (l._modules["post_attention_layernorm"], _Norm), (m["gate_proj"], _W), (m["up_proj"], _W), (m["down_proj"], _W)):
-                p = own_parameters(mod, cls)
-                if p is None or (cls is _Norm and mod.eps != eps) or mod.__dict__.get("bias") is not None:
+            if not l["input_layernorm"].eps == l["post_attention_layernorm"].eps == a["q_norm"].eps == a["k_norm"].eps == eps:
+                return None
+            m, ps = mlp._modules, []
+            for mod in (a["q_proj"], a["k_proj"], a["v_proj"], a["o_proj"], m["gate_proj"], m["up_proj"], m["down_proj"]):
+                p = own_parameters(mod, _W)
+                if p is None or mod.__dict__.get("bias") is not None:      # a plain tensor in the place of the parameter
                     return None
                 ps.append(p)
-            n1, wq, wk, wv, nq, nk, wo, n2, wg, wu, wd = ws = [p.get("weight") for p in ps]
-            if any(ps[i].get("bias") is not None for i in (6, 8, 9, 10)) or any(w is None for w in ws):
+            q, k, v, o, gate, up, down = ps
+            if "bias" in o or "bias" in gate or "bias" in up or "bias" in down:
                 return None
-            bias = [ps[i].get("bias") for i in (1, 2, 3)]
-            layers.append(((n1, wq, wk, wv, *bias, nq, nk), (wo, n2, wg, wu, wd)))
-            flat += ws
-            flat += [b for b in bias if b is not None]
-        has = [b is not None for b in layers[0][0][4:7]] if layers else []
-        if any([b is not None for b in qkv[4:7]] != has for qkv, _ in layers):
-            return None
-        # one call looks at type, device, layout, alignment and shape of all of them: the launches refuse what the separate
+            bias = [p.get("bias") for p in (q, k, v)]
+            some = [t for t in bias if t is not None]
+            if has is None:
+                has = len(some)
+            try:
+                qkv = (norm["weight"], q["weight"], k["weight"], v["weight"], *bias, q_norm["weight"], k_norm["weight"])
+                rest = (o["weight"], post["weight"], gate["weight"], up["weight"], down["weight"])
+            except KeyError:                                               # a weight that is no parameter any more
+                return None
+            if len(some) != has or has not in (0, 3):
+                return None
+            layers.append((qkv, rest))
+            flat += [t for t in qkv if t is not None] if has == 0 else qkv
+            flat += rest
+        # one call looks at type, device, layout, alignment and shape of all weights: the launches refuse what the separate
         # operations broadcast or copy
-        shapes = [D, 0, Q, D, KV, D, KV, D, Dh, 0, Dh, 0, D, Q, D, 0, F, D, F, D, D, F] + [v for n, h in zip((Q, KV, KV), has) if h for v in (n, 0)]
+        shapes = [D, 0, Q, D, KV, D, KV, D, *([Q, 0, KV, 0, KV, 0] if has else []), Dh, 0, Dh, 0, D, Q, D, 0, F, D, F, D, D, F]
         kv = (len(layers), x.shape[0], c.num_key_value_heads, cache.k.shape[3] if cache.k.dim() == 5 else 0, Dh)
         if kv[3] <= pos or cache.k.shape != kv or cache.v.shape != kv or any(t.dim() != 2 or t.shape[0] <= pos or t.shape[1] != Dh for t in rope):
             return None
-        return layers if native.ops().bf16_operands_ok([x, cache.k, cache.v, *rope, *flat], [-1, 0] * 5 + shapes * len(layers)) else None
+        ok = native.ops().bf16_operands_ok
+        return layers if ok([x, cache.k, cache.v, *rope], [-1, 0]) and (not layers or flat[0].device == x.device and ok(flat, shapes)) else None
 
     @torch.no_grad()
     def prefill(self, ids: torch.Tensor, max_len: int) -> "tuple[torch.Tensor, KVCache]":
@@ -173,7 +184,7 @@ class Qwen3Decoder:
         h = self.enc.model.norm(hidden)
         w = self.lm_head if self.lm_head is not None else self.enc.model.embed_tokens.weight
         if (native.use_native(h) and native.direct(h, w) and h.dtype == w.dtype == torch.bfloat16 and h.dim() == w.dim() == 2 and 0 < h.shape[0] <= 8
-                and h.shape[1] == w.shape[1] and h.shape[1] % 8 == 0 and native.ops().bf16_operands_ok([h, w], [-1, 0, -1, 0])):
+                and h.shape[1] == w.shape[1] and h.shape[1] % 8 == 0 and native.ops().bf16_operands_ok([h, w], [-1, 0])):
             # products of bf16 values are exact in fp32 and the few-row kernel sums in fp32: the table needs no fp32 copy
             return ops.functional._gemm([h], [w], out_fp32=True)
         return h.float() @ w.float().t()
