@@ -131,7 +131,8 @@ softmax_rows_kernel(const float* __restrict__ s, __nv_bfloat16* __restrict__ p, 
 // split-half rotation inside each head of Dh columns. A work item is 8 columns of a head's first half with the 8 columns Dh / 2
 // further, so both halves of a rotation are in one thread; a row of 4096 columns is one item per thread. Replaces two norms
 // into fresh buffers, two copies back into the packed rows and a rotation pass (six passes over q and k: 232 us per layer at
-// 6144 x 4096) by one (119 us).
+// 6144 x 4096) by one: 119 us with room for four items per thread, 61 where one is enough (201 MB: 3.3 TB/s, bound by the chain of
+// load, two barriers and store of a row; 52 us under ncu from cold caches).
 // A block has as many threads as the row has items, up to 256 (rows of 256 columns: 16 items; a block of 256 threads for them made
 // the pass slower than the separate operations, 238 against 206 us for an attention of 6144 tokens).
 constexpr int NR_THREADS = 256, NR_ITEMS = 4;
