@@ -38,6 +38,7 @@ constexpr int CONV_TW = 16, CONV_TH = 8;  // conv mode: one M tile = 8 rows x 16
 struct alignas(64) GemmMaps {
   CUtensorMap a[MDB_GEMM_MAX_SEG];
   CUtensorMap b[MDB_GEMM_MAX_SEG];
+  CUtensorMap out;   // GemmParams::bulk_out only
 };
 
 // Kernel parameters are __grid_constant__: the run-time index into route_out otherwise makes the compiler copy all 416 bytes of them
@@ -61,6 +62,7 @@ struct GemmParams {
   int ld_out;
   int out_fp32;
   int accumulate_out;  // out += result (fp32 out only)
+  int bulk_out;        // the output is a local, 16-byte aligned bf16 matrix (or image): rows leave through maps.out, see BulkEpilogue
   int* status;
   long long* prof;  // optional [grid, 8] cycle counters (profiling builds of the caller)
   long long* trace;  // optional per-K-block time line of CTAs 0 and 1: [2 CTAs][3 roles][trace_len] clock64 values
@@ -287,7 +289,20 @@ __device__ __forceinline__ void epilogue_row32(const GemmParams& p, int row, int
   }
 }
 
-// Epilogue of one accumulator tile for one warp (its 32 TMEM lanes = 32 output rows). bf16 outputs whose tile lies fully
+// Epilogue of one accumulator tile for one warp (its 32 TMEM lanes = 32 output rows), each lane storing its own row.
+__device__ __forceinline__ void epilogue_direct(const GemmParams& p, uint32_t taddr, int pair_col_off, int row, int n0, int out_cols,
+                                                bool paired, bool aligned) {
+#pragma unroll 1
+  for (int c = 0; c < out_cols / 32; ++c) {
+    uint32_t r0[32], r1[32];
+    tmem_ld_32x32b_x32(taddr + c * 32, r0);
+    if (paired) tmem_ld_32x32b_x32(taddr + pair_col_off + c * 32, r1);
+    tmem_wait_ld();
+    epilogue_row32(p, row, n0 + c * 32, r0, r1, paired, aligned);
+  }
+}
+
+// The same with row segments staged for peers. bf16 outputs whose tile lies fully
 // inside the matrix go through a per-warp staging buffer in shared memory (32 rows of GW columns), GW columns at a time: every
 // lane packs its row's slabs into the buffer, then the warp stores whole row segments of 2 * GW bytes (GW / 8 lanes x 16 bytes
 // per row). Local stores become full cache lines and peer-routed stores (sequence-parallel scatter, staged reduce-scatter) cross
@@ -299,14 +314,7 @@ __device__ __forceinline__ void epilogue_tile(const GemmParams& p, uint32_t tadd
   constexpr int CH = GW / 8;                                    // 16-byte chunks of a staged row
   const bool staged = stage_warp != nullptr && aligned && !p.out_fp32 && out_cols % GW == 0 && n0 + out_cols <= p.N;
   if (!staged) {
-#pragma unroll 1
-    for (int c = 0; c < out_cols / 32; ++c) {
-      uint32_t r0[32], r1[32];
-      tmem_ld_32x32b_x32(taddr + c * 32, r0);
-      if (paired) tmem_ld_32x32b_x32(taddr + pair_col_off + c * 32, r1);
-      tmem_wait_ld();
-      epilogue_row32(p, row, n0 + c * 32, r0, r1, paired, aligned);
-    }
+    epilogue_direct(p, taddr, pair_col_off, row, n0, out_cols, paired, aligned);
     return;
   }
   uint4* my_row = reinterpret_cast<uint4*>(stage_warp + lane * (2 * GW));
@@ -333,6 +341,208 @@ __device__ __forceinline__ void epilogue_tile(const GemmParams& p, uint32_t tadd
     __syncwarp();
   }
 }
+
+// eight bf16 terms of the epilogue, kept packed until they are used; n of them exist, the rest reads as `fill`
+__device__ __noinline__ uint4 load_terms_tail(const __nv_bfloat16* p, int n, uint32_t fill) {
+  uint32_t w[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const uint32_t lo = 2 * i < n ? reinterpret_cast<const uint16_t*>(p)[2 * i] : fill & 0xffffu;
+    const uint32_t hi = 2 * i + 1 < n ? reinterpret_cast<const uint16_t*>(p)[2 * i + 1] : fill >> 16;
+    w[i] = lo | hi << 16;
+  }
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
+__device__ __forceinline__ uint4 load_terms(const __nv_bfloat16* p, int n, uint32_t fill) {
+  return n >= 8 ? *reinterpret_cast<const uint4*>(p) : load_terms_tail(p, n, fill);
+}
+// wait for the TMEM loads of this thread; r is tied to it, so that nothing computed from r moves above
+__device__ __forceinline__ void tmem_wait_ld(uint32_t (&r)[32]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]), "+r"(r[9]),
+                 "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]), "+r"(r[16]), "+r"(r[17]), "+r"(r[18]),
+                 "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]), "+r"(r[23]), "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]),
+                 "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31])
+               :
+               : "memory");
+}
+
+// Epilogue of one accumulator tile for one warp when the output is a local bf16 matrix (GemmParams::bulk_out). What bounds it is
+// latency: a warp is alone on its scheduler and next to 227 KB of shared memory there is no L1 to speak of, so every global load
+// in the loop over the columns costs 350 to 700 cycles, every run-time flag 40. A tile of 256 columns took 10 000 cycles (15 000
+// with a bias, 21 000 with GELU, 29 000 with gate and residual): bias and residual were loaded per 32-column slab, and the staged
+// rows were copied out with a division-laden address per 16 bytes. Here it takes 5 000, 5 000, 9 400 and 13 000: 8192 x 5120 x 640
+// with bias 84 -> 46 us, with GELU 115 -> 62, with gate and residual 152 -> 92 (B200). Eight warps instead of four take no less
+// (TMEM reads and shuffles are shared) and spill.
+//  - load() runs before the accumulator is complete: each lane holds eight of the tile's columns of bias, gate and scales, which a
+//    slab gets by warp shuffles, and the first 64 columns of its row's residual (the next 64 are always on their way);
+//  - a missing term is replaced by its neutral value (-0 added, 1 multiplied: exact) instead of a branch; run() is compiled with and
+//    without gate and residual (TERMS), and in the pair kernel for each activation;
+//  - the next slab's TMEM load is in flight while one is computed;
+//  - 64 columns of the warp's 32 rows leave as one tiled bulk store from a swizzled 4 KB buffer (two per warp), which also clips
+//    ragged rows, columns and image edges.
+// The arithmetic per element is that of epilogue_row32.
+constexpr uint32_t TERM_ZERO = 0x80008000u, TERM_ONE = 0x3f803f80u;     // bf16 pairs: -0 and 1
+template <int KIND>
+struct BulkEpilogue {
+  const GemmParams& p;
+  int row, n0, out_cols, lane;      // row: this lane's output row (for residual, gate and row scale); p.M or more is not stored
+  bool paired;
+  uint4 bias, bias2, gate;
+  uint4 res[8];
+  float scale[KIND == 1 ? 8 : 1], scale2[KIND == 1 ? 8 : 1];
+  bool gate_shared;                 // the warp's rows have one gate
+
+  __device__ __forceinline__ BulkEpilogue(const GemmParams& p_, int row_, int n0_, int out_cols_, int lane_, bool paired_)
+      : p(p_), row(row_), n0(n0_), out_cols(out_cols_), lane(lane_), paired(paired_), gate_shared(true) {}
+  __device__ __forceinline__ int term_row() const { return row < p.M ? row : p.M - 1; }
+  __device__ __forceinline__ const __nv_bfloat16* gate_row() const { return p.gate + static_cast<size_t>(term_row() / p.rows_per_group) * p.gate_stride; }
+  __device__ __forceinline__ void load_residual(int col, uint4 (&d)[8]) const {
+    const __nv_bfloat16* r = p.residual + static_cast<size_t>(term_row()) * p.ld_res + col;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) d[i] = load_terms(r + 8 * i, p.N - col - 8 * i, TERM_ZERO);
+  }
+  __device__ __forceinline__ void load() {
+    const int c = n0 + lane * 8, n = lane * 8 < out_cols ? p.N - c : 0;
+    bias = bias2 = make_uint4(TERM_ZERO, TERM_ZERO, TERM_ZERO, TERM_ZERO);
+    gate = make_uint4(TERM_ONE, TERM_ONE, TERM_ONE, TERM_ONE);
+    if (p.bias) {
+      bias = load_terms(p.bias + c, n, TERM_ZERO);
+      if (paired) bias2 = load_terms(p.bias + c + p.pair_offset, n, TERM_ZERO);
+    }
+    if (p.gate) {
+      const int g = term_row() / p.rows_per_group;
+      gate_shared = __all_sync(0xffffffffu, g == __shfl_sync(0xffffffffu, g, 0));
+      if (gate_shared) gate = load_terms(gate_row() + c, n, TERM_ONE);
+    }
+    if (KIND == 1) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        scale[j] = p.col_scale && j < n ? p.col_scale[c + j] : 1.f;
+        scale2[j] = p.col_scale && paired && j < n ? p.col_scale[c + p.pair_offset + j] : 1.f;
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) res[i] = make_uint4(TERM_ZERO, TERM_ZERO, TERM_ZERO, TERM_ZERO);
+    if (p.residual) load_residual(n0, res);
+  }
+  // v op= the terms of slab s, eight columns per lane from lanes 4 s .. 4 s + 3
+  template <bool MUL>
+  __device__ __forceinline__ void columns(const uint4& u, int s, float (&v)[32]) const {
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+      const uint32_t mine = (k & 3) == 0 ? u.x : (k & 3) == 1 ? u.y : (k & 3) == 2 ? u.z : u.w;
+      const float2 f = unpack_bf16x2(__shfl_sync(0xffffffffu, mine, 4 * s + (k >> 2)));
+      v[2 * k] = MUL ? v[2 * k] * f.x : v[2 * k] + f.x;
+      v[2 * k + 1] = MUL ? v[2 * k + 1] * f.y : v[2 * k + 1] + f.y;
+    }
+  }
+  __device__ __forceinline__ void scales(const float* sc, int s, float (&v)[32]) const {
+#pragma unroll
+    for (int j = 0; j < 32; ++j) v[j] *= __shfl_sync(0xffffffffu, sc[j & 7], 4 * s + (j >> 3));
+  }
+  // turn: bulk stores this warp has issued, which take the staging buffers in turn; release(): called once the accumulator has been
+  // read; store(buffer, column): issues the bulk store of 64 columns
+  template <bool PAIRED, int ACT, bool TERMS, int BUFFERS, typename Release, typename Store>
+  __device__ __forceinline__ void run_mode(uint32_t taddr, int pair_col_off, uint8_t* stage, int& turn, Release release, Store store) {
+    const float rs = (KIND == 1 && p.row_scale ? p.row_scale[term_row()] : 1.f) * p.alpha;
+    uint32_t r[32], r2[32];
+    tmem_ld_32x32b_x32(taddr, r);
+    if (PAIRED) tmem_ld_32x32b_x32(taddr + pair_col_off, r2);
+    const int groups = min(out_cols, p.N - n0 + 63) / 64;            // those with a column of the matrix: every group is stored
+#pragma unroll 1
+    for (int g = 0; g < groups; ++g) {
+      uint4 now[8];
+      if (TERMS) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) now[i] = res[i];
+        if (p.residual && g + 1 < groups) load_residual(n0 + g * 64 + 64, res);
+      }
+      uint8_t* buf = stage + (turn++ % BUFFERS) * 4096;
+      uint4* my_row = reinterpret_cast<uint4*>(buf + lane * 128);
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        const int s = 2 * g + half;
+        float v[32], w[32];
+        tmem_wait_ld(r);
+        if (PAIRED) tmem_wait_ld(r2);
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+          v[j] = __uint_as_float(r[j]) * rs;
+          if (PAIRED) w[j] = __uint_as_float(r2[j]) * rs;
+        }
+        if (half == 0 || g + 1 < groups) {
+          tmem_ld_32x32b_x32(taddr + (s + 1) * 32, r);
+          if (PAIRED) tmem_ld_32x32b_x32(taddr + pair_col_off + (s + 1) * 32, r2);
+        } else {
+          release();
+        }
+        if (KIND == 1) scales(scale, s, v);
+        columns<false>(bias, s, v);
+        if (PAIRED) {
+          if (KIND == 1) scales(scale2, s, w);
+          columns<false>(bias2, s, w);
+          if (p.act_on_second) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) { const float x = v[j]; v[j] = w[j]; w[j] = x; }
+          }
+        }
+        if (ACT < 0) act32_rt(p.act, v);
+        else act32<ACT>(v);
+        if (PAIRED) {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) v[j] *= w[j];
+        }
+        if (TERMS) {
+          if (gate_shared) {
+            columns<true>(gate, s, v);
+          } else {
+            const int col = n0 + s * 32;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const uint4 u = load_terms(gate_row() + col + 8 * i, p.N - col - 8 * i, TERM_ONE);
+              const uint32_t x[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+              for (int k = 0; k < 4; ++k) { const float2 f = unpack_bf16x2(x[k]); v[8 * i + 2 * k] *= f.x; v[8 * i + 2 * k + 1] *= f.y; }
+            }
+          }
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const uint32_t x[4] = {now[4 * half + i].x, now[4 * half + i].y, now[4 * half + i].z, now[4 * half + i].w};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) { const float2 f = unpack_bf16x2(x[k]); v[8 * i + 2 * k] += f.x; v[8 * i + 2 * k + 1] += f.y; }
+          }
+        }
+        if (half == 0) {
+          if (lane == 0) tma_store_wait_read<BUFFERS - 1>();      // the store that used this buffer last has read it
+          __syncwarp();
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          my_row[(half * 4 + j) ^ (lane & 7)] = make_uint4(pack_bf16x2(v[8 * j], v[8 * j + 1]), pack_bf16x2(v[8 * j + 2], v[8 * j + 3]),
+                                                           pack_bf16x2(v[8 * j + 4], v[8 * j + 5]), pack_bf16x2(v[8 * j + 6], v[8 * j + 7]));
+      }
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) {
+        store(buf, n0 + g * 64);
+        tma_store_commit();
+      }
+    }
+  }
+  template <bool PAIRED, bool FIXED, int BUFFERS, typename Release, typename Store>
+  __device__ __forceinline__ void run(uint32_t taddr, int pair_col_off, uint8_t* stage, int& turn, Release release, Store store) {
+    const bool terms = !PAIRED && (p.gate || p.residual);
+#define MDB_RUN(ACT_, TERMS_) run_mode<PAIRED, ACT_, TERMS_, BUFFERS>(taddr, pair_col_off, stage, turn, release, store)
+    if (!PAIRED && terms && p.act == MDB_ACT_NONE) MDB_RUN(MDB_ACT_NONE, !PAIRED);
+    else if (!PAIRED && terms) MDB_RUN(-1, !PAIRED);
+    else if (!PAIRED && p.act == MDB_ACT_NONE) MDB_RUN(MDB_ACT_NONE, false);
+    else if (FIXED && p.act == MDB_ACT_GELU_TANH) MDB_RUN(FIXED ? MDB_ACT_GELU_TANH : -1, false);
+    else if (FIXED && p.act == MDB_ACT_GELU_ERF) MDB_RUN(FIXED ? MDB_ACT_GELU_ERF : -1, false);
+    else MDB_RUN(-1, false);
+#undef MDB_RUN
+  }
+};
 
 __device__ __forceinline__ int ld_acquire_gpu(const int* p) {
   int v;
@@ -362,7 +572,8 @@ __device__ __forceinline__ int tile_n_index(const GemmParams& p, int tile, int t
 }
 
 // KIND: 0 = bf16 operands (kind::f16), 1 = fp8 e4m3 operands (kind::f8f6f4)
-template <int BN, int STAGES, bool A_MN, bool B_MN, int KIND>
+// BULK: GemmParams::bulk_out
+template <int BN, int STAGES, bool A_MN, bool B_MN, int KIND, bool BULK>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_tcgen05_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ GemmParams p) {
   constexpr int A_BYTES = BM * BK_BYTES;
@@ -664,7 +875,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant
     if (p.col_scale) aligned = aligned && ((reinterpret_cast<uintptr_t>(p.col_scale) | static_cast<uintptr_t>(p.pair_offset * 4)) & 15) == 0;
     if (p.gate) aligned = aligned && ((reinterpret_cast<uintptr_t>(p.gate) | static_cast<uintptr_t>(p.gate_stride * 2)) & 15) == 0;
     if (p.residual) aligned = aligned && ((reinterpret_cast<uintptr_t>(p.residual) | static_cast<uintptr_t>(static_cast<size_t>(p.ld_res) * 2)) & 15) == 0;
-    int it = 0;
+    int it = 0, turn = 0;
     long long t_twait = 0, t_work = 0;
     for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, ++it) {
       const int acc = it & 1;
@@ -672,6 +883,19 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant
       const int m0 = tile_m_index(p, tile, tiles_m, tiles_n) * BM;
       const int nblk = tile_n_index(p, tile, tiles_m, tiles_n);
       const int n0 = paired ? nblk * (BN / 2) : nblk * BN;
+      const int out_cols = paired ? BN / 2 : BN;
+      int row = m0 + quad * 32 + lane, img = 0, ow0 = 0, oh0 = 0;
+      if (p.conv_taps > 0) {
+        const int mt = tile % tiles_m;
+        const int tw = mt % p.conv_tiles_w, th = (mt / p.conv_tiles_w) % p.conv_tiles_h;
+        img = mt / (p.conv_tiles_w * p.conv_tiles_h);
+        ow0 = tw * CONV_TW;
+        oh0 = th * CONV_TH + quad * (32 / CONV_TW);
+        const int oh = oh0 + lane / CONV_TW, ow = ow0 + lane % CONV_TW;
+        row = (oh < p.conv_h && ow < p.conv_w) ? (img * p.conv_h + oh) * p.conv_w + ow : p.M;  // p.M = skipped
+      }
+      BulkEpilogue<KIND> bulk(p, row, n0, out_cols, lane, paired);
+      if (BULK) bulk.load();
       const long long tq0 = p.prof ? clock64() : 0;
       // warp-uniform decision: the TMEM loads below are warp-collective
       const bool got = __all_sync(0xffffffffu, mbar_wait(&tfull_bar[acc], acc_phase, &abort_s));
@@ -683,26 +907,32 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant
       const long long tq1 = p.prof ? clock64() : 0;
       t_twait += tq1 - tq0;
       if (p.trace && blockIdx.x < 2 && warp == 2 && lane == 0 && 2 * it + 1 < p.trace_len) p.trace[(blockIdx.x * 3 + 2) * p.trace_len + 2 * it] = clock64();
-      int row = m0 + quad * 32 + lane;
-      if (p.conv_taps > 0) {
-        const int mt = tile % tiles_m;
-        const int tw = mt % p.conv_tiles_w, th = (mt / p.conv_tiles_w) % p.conv_tiles_h;
-        const int img = mt / (p.conv_tiles_w * p.conv_tiles_h);
-        const int r = quad * 32 + lane;
-        const int oh = th * CONV_TH + r / CONV_TW, ow = tw * CONV_TW + r % CONV_TW;
-        row = (oh < p.conv_h && ow < p.conv_w) ? (img * p.conv_h + oh) * p.conv_w + ow : p.M;  // p.M = skipped
-      }
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + acc * BN;
-      const int out_cols = paired ? BN / 2 : BN;
-      // the staging buffers share their 32 KB with the stages of the fused all-gather, which therefore stores directly
-      uint8_t* stage_warp = p.gather_world > 1 ? nullptr : smem + STAGES * STAGE_BYTES + quad * 8192;
-      epilogue_tile<128>(p, taddr, BN / 2, row, n0, out_cols, paired, aligned, stage_warp, lane);
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&tempty_bar[acc]);
+      uint8_t* stages = smem + STAGES * STAGE_BYTES;
+      auto release = [&] {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&tempty_bar[acc]);
+      };
+      if constexpr (BULK) {
+        auto store = [&](const uint8_t* buf, int col) {
+          if (p.conv_taps > 0) {
+            if (oh0 < p.conv_h) tma_store_4d(&maps.out, buf, col, ow0, oh0, img);
+          } else if (m0 + quad * 32 < p.M) {
+            tma_store_2d(&maps.out, buf, col, m0 + quad * 32);
+          }
+        };
+        if (BN == 256 && paired) bulk.template run<BN == 256, false, 2>(taddr, BN / 2, stages + quad * 8192, turn, release, store);
+        else bulk.template run<false, false, 2>(taddr, 0, stages + quad * 8192, turn, release, store);
+      } else {
+        // the staging buffers share their 32 KB with the stages of the fused all-gather, which therefore stores directly
+        epilogue_tile<128>(p, taddr, BN / 2, row, n0, out_cols, paired, aligned, p.gather_world > 1 ? nullptr : stages + quad * 8192, lane);
+        release();
+      }
       if (p.prof) t_work += clock64() - tq1;
       if (p.trace && blockIdx.x < 2 && warp == 2 && lane == 0 && 2 * it + 1 < p.trace_len) p.trace[(blockIdx.x * 3 + 2) * p.trace_len + 2 * it + 1] = clock64();
     }
+    if (BULK && lane == 0) tma_store_wait<0>();   // the rows are out before the staging buffers go away
     if (p.prof && warp == 2 && lane == 0) {
       p.prof[blockIdx.x * 8 + 4] = t_twait;
       p.prof[blockIdx.x * 8 + 5] = t_work;
@@ -728,7 +958,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant
 // ---------------------------------------------------------------------------------
 constexpr int PAIR_THREADS = 192;  // warps: 0 TMA, 1 UMMA issue (leader only), 2-5 epilogue
 
-template <int STAGES, bool A_MN, bool B_MN, int KIND>
+template <int STAGES, bool A_MN, bool B_MN, int KIND, bool BULK>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
 gemm_tcgen05_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ GemmParams p) {
   constexpr int BN = 256;               // accumulator columns per CTA (the whole tile width)
@@ -939,7 +1169,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_con
     if (p.col_scale) aligned = aligned && ((reinterpret_cast<uintptr_t>(p.col_scale) | static_cast<uintptr_t>(p.pair_offset * 4)) & 15) == 0;
     if (p.gate) aligned = aligned && ((reinterpret_cast<uintptr_t>(p.gate) | static_cast<uintptr_t>(p.gate_stride * 2)) & 15) == 0;
     if (p.residual) aligned = aligned && ((reinterpret_cast<uintptr_t>(p.residual) | static_cast<uintptr_t>(static_cast<size_t>(p.ld_res) * 2)) & 15) == 0;
-    int it = 0;
+    int it = 0, turn = 0;
     long long t_twait = 0, t_work = 0;
     for (int tile = cluster_id; tile < num_tiles; tile += num_clusters, ++it) {
       const int acc = it & 1;
@@ -947,6 +1177,10 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_con
       const int m0 = (tile % tiles_m) * (2 * BM) + static_cast<int>(rank) * BM;
       const int nblk = tile / tiles_m;
       const int n0 = paired ? nblk * BNH : nblk * BN;
+      const int out_cols = paired ? BNH : BN;
+      const int row = m0 + quad * 32 + lane;
+      BulkEpilogue<KIND> bulk(p, row, n0, out_cols, lane, paired);
+      if (BULK) bulk.load();
       const long long tq0 = p.prof ? clock64() : 0;
       const bool got = __all_sync(0xffffffffu, mbar_wait(&tfull_bar[acc], acc_phase, &abort_s));
       if (!got) {
@@ -960,16 +1194,27 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_con
       const long long tq1 = p.prof ? clock64() : 0;
       t_twait += tq1 - tq0;
       if (p.trace && blockIdx.x < 2 && warp == 2 && lane == 0 && 2 * it + 1 < p.trace_len) p.trace[(blockIdx.x * 3 + 2) * p.trace_len + 2 * it] = clock64();
-      const int row = m0 + quad * 32 + lane;
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + acc * BN;
-      const int out_cols = paired ? BNH : BN;
-      epilogue_tile<128>(p, taddr, BNH, row, n0, out_cols, paired, aligned, smem + STAGES * STAGE_BYTES + quad * 8192, lane);
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&tempty_bar[acc]), 0u));
+      uint8_t* stages = smem + STAGES * STAGE_BYTES;
+      auto release = [&] {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&tempty_bar[acc]), 0u));
+      };
+      if constexpr (BULK) {
+        auto store = [&](const uint8_t* buf, int col) {
+          if (m0 + quad * 32 < p.M) tma_store_2d(&maps.out, buf, col, m0 + quad * 32);
+        };
+        if (paired) bulk.template run<true, true, 2>(taddr, BNH, stages + quad * 8192, turn, release, store);
+        else bulk.template run<false, true, 2>(taddr, 0, stages + quad * 8192, turn, release, store);
+      } else {
+        epilogue_tile<128>(p, taddr, BNH, row, n0, out_cols, paired, aligned, stages + quad * 8192, lane);
+        release();
+      }
       if (p.prof) t_work += clock64() - tq1;
       if (p.trace && blockIdx.x < 2 && warp == 2 && lane == 0 && 2 * it + 1 < p.trace_len) p.trace[(blockIdx.x * 3 + 2) * p.trace_len + 2 * it + 1] = clock64();
     }
+    if (BULK && lane == 0) tma_store_wait<0>();   // the rows are out before the staging buffers go away
     if (p.prof && warp == 2 && lane == 0) {
       p.prof[blockIdx.x * 8 + 4] = t_twait;
       p.prof[blockIdx.x * 8 + 5] = t_work;
@@ -1010,13 +1255,13 @@ struct ConvPairShape {
   static constexpr int B_BYTES = BNH * BK_BYTES;
   static constexpr int A_STAGES = RESIDENT ? 3 : HALO ? (BN == 256 ? 3 : 5) : 5;
   static constexpr int B_STAGES = RESIDENT ? 18 : HALO ? (BN == 256 ? 7 : 8) : 6;
-  static constexpr int STAGE_COLS = RESIDENT ? 64 : 128;               // columns staged at a time by an epilogue warp
-  static constexpr int SMEM = A_STAGES * A_BYTES + B_STAGES * B_BYTES + 4 * 64 * STAGE_COLS + 1024;
+  static constexpr int BUFFERS = RESIDENT ? 1 : 2;                     // 4 KB staging buffers of an epilogue warp
+  static constexpr int SMEM = A_STAGES * A_BYTES + B_STAGES * B_BYTES + 4 * BUFFERS * 4096 + 1024;
   static_assert(SMEM <= 227 * 1024, "pipeline exceeds the shared memory of an SM");
   static_assert(B_BYTES % 1024 == 0 && A_BYTES % 1024 == 0, "stages start on swizzle atoms");
 };
 
-template <int BN, bool HALO, bool RESIDENT>
+template <int BN, bool HALO, bool RESIDENT, bool BULK>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
 conv_tcgen05_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ GemmParams p) {
   using S = ConvPairShape<BN, HALO, RESIDENT>;
@@ -1169,27 +1414,41 @@ conv_tcgen05_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_con
     bool aligned = ((reinterpret_cast<uintptr_t>(p.out) | static_cast<uintptr_t>(static_cast<size_t>(p.ld_out) * 2)) & 15) == 0;
     if (p.bias) aligned = aligned && (reinterpret_cast<uintptr_t>(p.bias) & 15) == 0;
     if (p.residual) aligned = aligned && ((reinterpret_cast<uintptr_t>(p.residual) | static_cast<uintptr_t>(static_cast<size_t>(p.ld_res) * 2)) & 15) == 0;
-    int it = 0;
+    int it = 0, turn = 0;
     for (int tile = cluster_id; tile < num_tiles; tile += num_clusters, ++it) {
       const int acc = it & 1;
+      const int n0 = (tile % tiles_n) * BN;
+      const int mt = (tile / tiles_n) * 2 + static_cast<int>(rank);
+      const int tw = mt % p.conv_tiles_w, th = (mt / p.conv_tiles_w) % p.conv_tiles_h;
+      const int img = mt / (p.conv_tiles_w * p.conv_tiles_h);
+      const int ow0 = tw * CONV_TW, oh0 = th * CONV_TH + quad * (32 / CONV_TW);
+      const int oh = oh0 + lane / CONV_TW, ow = ow0 + lane % CONV_TW;
+      const int row = (mt < p.conv_tiles_m && oh < p.conv_h && ow < p.conv_w) ? (img * p.conv_h + oh) * p.conv_w + ow : p.M;   // p.M = skipped
+      BulkEpilogue<0> bulk(p, row, n0, BN, lane, false);
+      if (BULK) bulk.load();
       const bool got = __all_sync(0xffffffffu, mbar_wait(&tfull_bar[acc], (it >> 1) & 1, &abort_s));
       if (!got) {
         if (lane == 0) { report_status(p.status, STATUS_TIMEOUT, 35, acc); st_shared_cluster_u32(peer_abort, 1u); }
         break;
       }
       tc_fence_after();
-      const int mt = (tile / tiles_n) * 2 + static_cast<int>(rank);
-      const int tw = mt % p.conv_tiles_w, th = (mt / p.conv_tiles_w) % p.conv_tiles_h;
-      const int img = mt / (p.conv_tiles_w * p.conv_tiles_h);
-      const int r = quad * 32 + lane;
-      const int oh = th * CONV_TH + r / CONV_TW, ow = tw * CONV_TW + r % CONV_TW;
-      const int row = (mt < p.conv_tiles_m && oh < p.conv_h && ow < p.conv_w) ? (img * p.conv_h + oh) * p.conv_w + ow : p.M;   // p.M = skipped
-      epilogue_tile<S::STAGE_COLS>(p, tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + acc * BN, 0, row, (tile % tiles_n) * BN, BN, false, aligned,
-                    smem_st + quad * (64 * S::STAGE_COLS), lane);
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&tempty_bar[acc]), 0u));
+      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + acc * BN;
+      auto release = [&] {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&tempty_bar[acc]), 0u));
+      };
+      if constexpr (BULK) {
+        auto store = [&](const uint8_t* buf, int col) {
+          if (mt < p.conv_tiles_m && oh0 < p.conv_h) tma_store_4d(&maps.out, buf, col, ow0, oh0, img);
+        };
+        bulk.template run<false, false, S::BUFFERS>(taddr, 0, smem_st + quad * (S::BUFFERS * 4096), turn, release, store);
+      } else {
+        epilogue_direct(p, taddr, 0, row, n0, BN, false, aligned);
+        release();
+      }
     }
+    if (BULK && lane == 0) tma_store_wait<0>();   // the rows are out before the staging buffers go away
   }
 
   tc_fence_before();
@@ -1256,7 +1515,7 @@ extern "C" int mdb_make_tmap_strided(void* out_map, const void* ptr, int elem_by
 
 namespace mdb {
 
-template <int BN, int STAGES, bool A_MN, bool B_MN, int KIND>
+template <int BN, int STAGES, bool A_MN, bool B_MN, int KIND, bool BULK>
 static int launch_variant(const GemmMaps& maps, const GemmParams& p, int num_sms, cudaStream_t stream) {
   constexpr int STAGE_BYTES = BM * BK_BYTES + BN * BK_BYTES;
   // operand ring + 32 KB that serve as the epilogue's staging buffers (4 warps x 8 KB) or, with a fused all-gather, as its
@@ -1265,7 +1524,7 @@ static int launch_variant(const GemmMaps& maps, const GemmParams& p, int num_sms
   static_assert(GATHER_STAGES * GATHER_PIECE == 4 * 8192, "staging buffers and gather stages share one region");
   static_assert(SMEM_GATHER <= 227 * 1024, "pipeline + staging exceed the shared memory of an SM");
   const int SMEM = SMEM_GATHER;
-  auto kern = gemm_tcgen05_kernel<BN, STAGES, A_MN, B_MN, KIND>;
+  auto kern = gemm_tcgen05_kernel<BN, STAGES, A_MN, B_MN, KIND, BULK>;
   static bool attr_done = false;
   if (!attr_done) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_GATHER);
@@ -1289,7 +1548,7 @@ static int pair_capacity(int num_sms) {
   static int cached = 0;
   if (cached > 0) return cached;
   constexpr int SMEM = 6 * (BM * BK_BYTES + 128 * BK_BYTES) + 4 * 8192 + 1024;
-  auto kern = gemm_tcgen05_pair_kernel<6, false, false, 0>;
+  auto kern = gemm_tcgen05_pair_kernel<6, false, false, 0, true>;
   int n = 0;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) == cudaSuccess) {
     cudaLaunchConfig_t cfg;
@@ -1312,11 +1571,11 @@ static int pair_capacity(int num_sms) {
   return cached;
 }
 
-template <int STAGES, bool A_MN, bool B_MN, int KIND>
+template <int STAGES, bool A_MN, bool B_MN, int KIND, bool BULK>
 static int launch_pair_variant(const GemmMaps& maps, const GemmParams& p, int num_sms, cudaStream_t stream) {
   constexpr int SMEM = STAGES * (BM * BK_BYTES + 128 * BK_BYTES) + 4 * 8192 + 1024;   // ring + epilogue staging (4 warps x 8 KB)
   static_assert(SMEM <= 227 * 1024, "pipeline exceeds the shared memory of an SM");
-  auto kern = gemm_tcgen05_pair_kernel<STAGES, A_MN, B_MN, KIND>;
+  auto kern = gemm_tcgen05_pair_kernel<STAGES, A_MN, B_MN, KIND, BULK>;
   static bool attr_done = false;
   if (!attr_done) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
@@ -1336,7 +1595,7 @@ static int launch_pair_variant(const GemmMaps& maps, const GemmParams& p, int nu
 template <int BN, bool HALO, bool RESIDENT>
 static int launch_conv_pair(const GemmMaps& maps, const GemmParams& p, int num_sms, cudaStream_t stream) {
   constexpr int SMEM = ConvPairShape<BN, HALO, RESIDENT>::SMEM;
-  auto kern = conv_tcgen05_pair_kernel<BN, HALO, RESIDENT>;
+  auto kern = p.bulk_out ? conv_tcgen05_pair_kernel<BN, HALO, RESIDENT, true> : conv_tcgen05_pair_kernel<BN, HALO, RESIDENT, false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
   if (e != cudaSuccess) return static_cast<int>(e);
   const long long tiles = static_cast<long long>((p.conv_tiles_m + 1) / 2) * ((p.N + BN - 1) / BN);
@@ -1367,12 +1626,12 @@ namespace mdb {
 // reduction. Every form is estimated in microseconds and the lowest one taken.
 //
 // The terms are fitted to measured times of all forms over 1457 calls (M 1 to 65536, N and K 16 to 21504, the three operand
-// layouts, with and without epilogue terms; B200, weights from HBM). Over them the choice is 1.4 % above the best form of each
-// (geometric mean; 18 of them more than 20 %). What they say:
-//  - a 64-wide K step takes 0.32 / 0.34 / 0.46 us of a lone CTA with 64 / 128 / 256 columns (a narrow MMA issues hardly faster) and
-//    0.34 of a pair;
-//  - a tile's epilogue takes 1.6 to 3 us, three times that with activation, gate or residual, and hides behind the next tile's
-//    steps only; rows that end off 32 columns leave its vector path (N = 16: 8 us more);
+// layouts, with and without epilogue terms; B200, weights from HBM). Over them the choice is 1.6 % above the best form of each
+// (geometric mean; 39 of them more than 20 %). What they say:
+//  - a 64-wide K step takes 0.37 / 0.39 / 0.44 us of a lone CTA with 64 / 128 / 256 columns (it is bound by what the SM takes in) and
+//    0.335 of a pair;
+//  - a tile's epilogue takes 1 to 2.1 us, twice that with an activation or with gate and residual, three times with both, and hides
+//    behind the next tile's steps only; where the lanes store the rows themselves (fp32, odd strides) half as much again;
 //  - a cluster's tile starts, meets in shared memory and ends in 6 to 9 us, and finishing its rows costs a CTA 2.2 to 7.2 us / splits
 //    (six times that with epilogue terms): it pays for long reductions only, and never for tiles that come in many waves
 //    (65536 x 128 x 128: 65 us in clusters of one, 17 on the persistent tiles). 15 % are added for it, so that it wins clear cases;
@@ -1389,31 +1648,34 @@ static GemmForm choose_form(const MdbGemmArgs* a, int sms, bool pairs, bool rows
   const double n_all = paired ? 2.0 * a->N : a->N;                           // rows of B
   const double memory = 2.0 * (a->M * k_all + n_all * k_all + static_cast<double>(a->M) * a->N) / 3.6e6;
   const bool heavy = a->act != 0 || a->gate || a->residual || paired;
-  const double whole_terms = heavy ? 3.0 : a->bias ? 1.4 : 1.0, split_terms = heavy ? 6.2 : a->bias ? 2.1 : 1.0;
+  const bool bulk = !a->out_fp32 && ((reinterpret_cast<uintptr_t>(a->out) | static_cast<uintptr_t>(static_cast<size_t>(a->ld_out) * 2)) & 15) == 0;
+  const double whole_terms = (heavy ? ((a->act || paired) && (a->gate || a->residual) ? 3.1 : 2.2) : 1.0) * (bulk ? 1.0 : 1.5);
+  const double split_terms = heavy ? 6.2 : a->bias ? 2.1 : 1.0;
   auto ceil_div = [](double x, double y) { return std::ceil(x / y); };
   auto with_memory = [&](double t) { return std::sqrt(std::sqrt(t * t * t * t + memory * memory * memory * memory)); };   // neither hides wholly behind the other
   auto tiles = [&](double tm, double tn) { return ceil_div(a->M, tm) * ceil_div(a->N, tn); };
-  auto step = [](int w) { return w == 64 ? 0.32 : w == 128 ? 0.34 : 0.46; };
+  auto step = [](int w) { return w == 64 ? 0.37 : w == 128 ? 0.39 : 0.44; };
+  auto split_step = [](int w) { return w == 64 ? 0.32 : 0.34; };
   GemmForm best = {256, 0, false, false};
   double best_us = 1e30;
   auto offer = [&](double us, GemmForm f) { if (us < best_us) { best_us = us; best = f; } };
 
   auto whole = [&](double n_tiles, int width, double step_us, double epilogue) {
-    const double e = epilogue * whole_terms + (a->N % 32 != 0 && a->N < 256 ? 8.0 : 0.0), main = kb * step_us;
-    return with_memory(5.0 + ceil_div(n_tiles, width) * (main > e ? main : e) + e);
+    const double e = epilogue * whole_terms, main = kb * step_us;
+    return with_memory(4.3 + ceil_div(n_tiles, width) * (main > e ? main : e) + e);
   };
-  offer(whole(tiles(BM, paired ? 128 : 256), sms, step(256), 3.0), {256, 0, false, false});
+  offer(whole(tiles(BM, paired ? 128 : 256), sms, step(256), 2.0), {256, 0, false, false});
   if (!paired) {
-    offer(whole(tiles(BM, 128), sms, step(128), 2.1), {128, 0, false, false});
-    offer(whole(tiles(BM, 64), sms, step(64), 1.6), {64, 0, false, false});
+    offer(whole(tiles(BM, 128), sms, step(128), 1.35), {128, 0, false, false});
+    offer(whole(tiles(BM, 64), sms, step(64), 1.0), {64, 0, false, false});
   }
-  if (pairs && a->M > BM) offer(whole(tiles(2 * BM, paired ? 128 : 256), pair_capacity(sms), 0.34, 2.9), {256, 0, true, false});
+  if (pairs && a->M > BM) offer(whole(tiles(2 * BM, paired ? 128 : 256), pair_capacity(sms), 0.335, 2.1), {256, 0, true, false});
   if (!whole_only) {
     for (int w = 128; w >= 64; w -= 64)
       for (int sp = 1; sp <= SPLIT_MAX && (sp == 1 || kb / sp >= 4); ++sp) {
         const int cap = w == 128 ? split_capacity<128>(sp, sms) : split_capacity<64>(sp, sms);
         const double fixed = w == 128 ? 7.0 + 3.55 * split_terms / sp : 5.9 + 2.2 * split_terms / sp;
-        offer(with_memory(1.15 * ceil_div(tiles(BM, w), cap) * (ceil_div(kb, sp) * step(w) + fixed)), {w, sp, false, false});
+        offer(with_memory(1.15 * ceil_div(tiles(BM, w), cap) * (ceil_div(kb, sp) * split_step(w) + fixed)), {w, sp, false, false});
       }
     for (int sp = 2; sp <= PSPLIT_MAX && kb / sp >= 4 && !a->a_mn && a->M > BM; ++sp)
       offer(with_memory(1.15 * ceil_div(tiles(2 * BM, 256), pair_split_capacity(sp, sms)) * (ceil_div(kb, sp) * 0.34 + 9.0 + 7.2 * split_terms / sp)), {256, sp, true, false});
@@ -1610,6 +1872,27 @@ extern "C" int mdb_gemm_launch(const MdbGemmArgs* a, cudaStream_t stream) {
     p.conv_cblocks = a->conv_cin / k_elems;
     p.conv_tiles_m = a->conv_n * p.conv_tiles_h * p.conv_tiles_w;
   }
+  // a local bf16 output whose rows and terms start on 16 bytes leaves through a tensor map (32 rows x 64 columns, or 2 x 16 pixels
+  // x 64 channels, a store); the rest (fp32, peers' buffers, odd strides) is written by the lanes
+  auto fits = [](const void* ptr, int64_t stride_bytes) { return ((reinterpret_cast<uintptr_t>(ptr) | static_cast<uintptr_t>(stride_bytes)) & 15) == 0; };
+  p.bulk_out = !a->out_fp32 && a->route_owner_cols <= 0 && a->reduce_rows_per_owner <= 0 && a->gather_world <= 1 && splits == 0 &&
+               fits(a->out, static_cast<int64_t>(a->ld_out) * 2) && fits(a->bias, a->pair_offset > 0 ? a->pair_offset * 2 : 0) &&
+               !(a->pair_offset > 0 && (a->gate || a->residual)) && (a->kind == 1 || (!a->row_scale && !a->col_scale)) && (!a->gate || fits(a->gate, static_cast<int64_t>(a->gate_stride) * 2)) &&
+               (!a->residual || fits(a->residual, static_cast<int64_t>(a->ld_res) * 2));
+  if (p.bulk_out) {
+    int r;
+    if (a->conv_taps > 0) {
+      const int64_t row = static_cast<int64_t>(a->ld_out) * 2;
+      const int64_t e4[4] = {a->N, a->conv_w, a->conv_h, a->conv_n}, s4[4] = {2, row, row * a->conv_w, row * a->conv_w * a->conv_h};
+      const int b4[4] = {64, CONV_TW, 32 / CONV_TW, 1};
+      r = mdb_make_tmap(&maps.out, a->out, 2, 4, e4, s4, b4, 1);
+    } else {
+      const int64_t e2[2] = {a->N, a->M}, s2[2] = {2, static_cast<int64_t>(a->ld_out) * 2};
+      const int b2[2] = {64, 32};
+      r = mdb_make_tmap(&maps.out, a->out, 2, 2, e2, s2, b2, 1);
+    }
+    if (r) return 3000 + r;
+  }
   p.route_owner_cols = a->route_owner_cols;
   p.route_part_cols = a->route_part_cols > 0 ? a->route_part_cols : a->N;
   p.route_row_offset = a->route_row_offset;
@@ -1630,13 +1913,19 @@ extern "C" int mdb_gemm_launch(const MdbGemmArgs* a, cudaStream_t stream) {
     if (!a->a_mn) return bn == 128 ? launch_split<128, false, true>(maps, p, splits, stream) : launch_split<64, false, true>(maps, p, splits, stream);
     return bn == 128 ? launch_split<128, true, true>(maps, p, splits, stream) : launch_split<64, true, true>(maps, p, splits, stream);
   }
-#define MDB_LAUNCH(BN_, ST_, AMN_, BMN_, KIND_) return launch_variant<BN_, ST_, AMN_, BMN_, KIND_>(maps, p, sms, stream)
+#define MDB_LAUNCH(BN_, ST_, AMN_, BMN_, KIND_) \
+  return p.bulk_out ? launch_variant<BN_, ST_, AMN_, BMN_, KIND_, true>(maps, p, sms, stream) : launch_variant<BN_, ST_, AMN_, BMN_, KIND_, false>(maps, p, sms, stream)
+#define MDB_LAUNCH_PAIR(AMN_, BMN_, KIND_) \
+  return p.bulk_out ? launch_pair_variant<6, AMN_, BMN_, KIND_, true>(maps, p, sms, stream) : launch_pair_variant<6, AMN_, BMN_, KIND_, false>(maps, p, sms, stream)
   if (use_pair) {
-    if (a->kind == 1) return a->a_mn || a->b_mn ? -4 : launch_pair_variant<6, false, false, 1>(maps, p, sms, stream);
-    if (!a->a_mn && !a->b_mn) return launch_pair_variant<6, false, false, 0>(maps, p, sms, stream);
-    if (!a->a_mn && a->b_mn) return launch_pair_variant<6, false, true, 0>(maps, p, sms, stream);
-    if (a->a_mn && a->b_mn) return launch_pair_variant<6, true, true, 0>(maps, p, sms, stream);
-    return launch_pair_variant<6, true, false, 0>(maps, p, sms, stream);
+    if (a->kind == 1) {
+      if (a->a_mn || a->b_mn) return -4;
+      MDB_LAUNCH_PAIR(false, false, 1);
+    }
+    if (!a->a_mn && !a->b_mn) MDB_LAUNCH_PAIR(false, false, 0);
+    if (!a->a_mn && a->b_mn) MDB_LAUNCH_PAIR(false, true, 0);
+    if (a->a_mn && a->b_mn) MDB_LAUNCH_PAIR(true, true, 0);
+    MDB_LAUNCH_PAIR(true, false, 0);
   }
   if (a->kind == 1) {
     if (a->a_mn || a->b_mn) return -4;
@@ -1663,6 +1952,7 @@ extern "C" int mdb_gemm_launch(const MdbGemmArgs* a, cudaStream_t stream) {
   if (bn == 128) MDB_LAUNCH(128, 6, true, false, 0);
   MDB_LAUNCH(64, 8, true, false, 0);
 #undef MDB_LAUNCH
+#undef MDB_LAUNCH_PAIR
 }
 
 MDB_DEFINE_WAIT_LIMIT_SETTER(mdb_set_wait_limit_gemm)

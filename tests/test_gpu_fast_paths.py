@@ -588,3 +588,26 @@ def test_gemm_forms_left_to_the_launch(seed):
 @pytest.mark.parametrize("N,HW", [(1, 8), (2, 159), (1, 160), (1, 511), (2, 512)])
 def test_group_norm_wide_tensors_of_few_pixels(N, HW):
     test_group_norm_forward_and_backward(N, HW, 2560, 32)
+
+
+# rows that leave through a tensor map: many short tiles per CTA (the staging buffers take turns), rows and columns that end inside a
+# store's 32 x 64 box, two gates in one warp's rows, an output between other columns and one in the place of the residual
+@pytest.mark.parametrize("M,N,K,bn", [(30000, 64, 64, 64), (30000, 192, 64, 256), (20000, 320, 64, 512), (20000, 72, 128, 128), (300, 200, 320, 0), (129, 24, 72, 0)])
+@pytest.mark.parametrize("terms", ["bias", "gelu", "gate", "slice"])
+def test_bulk_epilogue(M, N, K, bn, terms):
+    from mojodiffusion_b200.ops.functional import _gemm
+    x, w, b = _rand(M, K, seed=1), _rand(N, K, scale=1 / math.sqrt(K), seed=2), _rand(N, seed=3)
+    want = x.float() @ w.float().t() + b.float()
+    if terms == "bias":
+        got = _gemm([x], [w], bias=b, bn=bn)
+    elif terms == "gelu":
+        want, got = torch.nn.functional.gelu(want, approximate="tanh"), _gemm([x], [w], bias=b, act=1, bn=bn)
+    elif terms == "gate":
+        gate, out, rows = _rand(3, N, seed=4), _rand(M, N, seed=5), (M + 2) // 3
+        want = out.float() + want * gate.float().repeat_interleave(rows, 0)[:M]
+        got = _gemm([x], [w], bias=b, residual=out, gate=gate, rows_per_group=rows, out=out, bn=bn)
+    else:
+        wide = torch.zeros(M, 3 * N, device=DEV, dtype=torch.bfloat16)
+        got = _gemm([x], [w], bias=b, out=wide[:, N:2 * N], bn=bn)
+        assert not wide[:, :N].any() and not wide[:, 2 * N:].any()
+    _close(got, want, f"{terms} {M}x{N}x{K}", rel=1e-4)
