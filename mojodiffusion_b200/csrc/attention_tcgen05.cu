@@ -1,15 +1,12 @@
 // Flash-style attention forward for sm_100a on the 5th-generation tensor cores.
 //
-// One CTA owns 256 query rows of one (batch, head) as two 128-row tiles that take turns: while all eight
-// softmax warps work on one tile's S, the tensor core runs the other tile's P*V and next Q*K^T.
+// One CTA owns 256 query rows of one (batch, head) as two 128-row tiles that take turns: while one tile's four
+// softmax warps work on its S, the tensor core runs the other tile's P*V and next Q*K^T.
 //   * Q (2 x 128 x Dh), K and V (128 x Dh, double buffered) arrive by TMA straight from the caller's
 //     [batch, seq, head, Dh] strides (4-D tensor maps, 128-byte swizzle): no head transpose pass exists.
 //   * S = Q K^T  : tcgen05.mma SS-form, fp32 accumulator in TMEM (128 columns per tile).
-//   * softmax    : two threads per query row (64 key columns each, no shuffles; the row maximum is exchanged through
-//                  shared memory), exp2 with the scale folded in, P written back into TMEM as packed bf16 over the S
-//                  columns it came from. A per-kv-tile time line (mdb_attention_set_trace) showed the kernel bound by the
-//                  softmax chain, not by the tensor core; one thread per row with one warpgroup per tile measured the
-//                  same throughput with twice the registers.
+//   * softmax    : one thread per query row, one warpgroup per q tile, exp2 with the scale folded in, P written back into TMEM
+//                  as packed bf16 over the S columns it came from, in two halves.
 //   * O += P V   : tcgen05.mma TS-form (A = P from TMEM, B = V MN-major from shared memory) accumulating in a
 //                  second TMEM region across all key tiles. The running maximum used for the exponent is only
 //                  raised when a row's true maximum exceeds it by more than 2^8 ("lazy rescale"): then, and
@@ -101,9 +98,7 @@ attention_fwd_kernel(const __grid_constant__ AttnMaps maps, const AttnParams p) 
 
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t q_full, k_full[2], k_empty[2], v_full[2], v_empty[2];
-  __shared__ uint64_t s_full[2], p_full[2], o_full[2];
-  __shared__ uint64_t x_bar[2][4];          // max / sum exchange between the two threads of a row, per q tile and quadrant
-  __shared__ float x_val[2][2][BQ];
+  __shared__ uint64_t s_full[2], p_full[2][2], o_full[2];      // p_full: per q tile and half of the tile's keys
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_s;
 
@@ -131,8 +126,8 @@ attention_fwd_kernel(const __grid_constant__ AttnMaps maps, const AttnParams p) 
       mbar_init(&v_full[s], 1);
       mbar_init(&v_empty[s], 1);
       mbar_init(&s_full[s], 1);
-      mbar_init(&p_full[s], 256);
-      for (int qd = 0; qd < 4; ++qd) mbar_init(&x_bar[s][qd], 64);
+      mbar_init(&p_full[s][0], 4);
+      mbar_init(&p_full[s][1], 4);
       mbar_init(&o_full[s], 1);
     }
     abort_s = 0;
@@ -224,12 +219,13 @@ attention_fwd_kernel(const __grid_constant__ AttnMaps maps, const AttnParams p) 
         }
         umma_commit(&s_full[t]);
       };
-      auto issue_pv = [&](int t, int st, bool first) {
+      auto issue_pv = [&](int t, int st, int half, bool first) {
 #pragma unroll
-        for (int kk = 0; kk < BKV / 16; ++kk)
+        for (int k2 = 0; k2 < BKV / 32; ++k2) {
+          const int kk = half * (BKV / 32) + k2;
           umma_f16_ts(o_tmem[t], s_tmem[t] + kk * 8, v_desc[st] + static_cast<uint32_t>((kk * 2048) >> 4), idesc_pv,
                       (first && kk == 0) ? 0u : 1u);
-        umma_commit(&o_full[t]);
+        }
       };
       bool ok = ctl_wait<MODE>(&q_full, 0, &abort_s, lane) && ctl_wait<MODE>(&k_full[0], 0, &abort_s, lane);
       if (!ok && lane == 0) report_status(p.status, STATUS_TIMEOUT, 21, 0);
@@ -254,15 +250,24 @@ attention_fwd_kernel(const __grid_constant__ AttnMaps maps, const AttnParams p) 
           break;
         }
         for (int t = 0; t < 2; ++t) {
-          if (!ctl_wait<MODE>(&p_full[t], j & 1, &abort_s, lane)) {
+          if (!ctl_wait<MODE>(&p_full[t][0], j & 1, &abort_s, lane)) {
             if (lane == 0) report_status(p.status, STATUS_TIMEOUT, 23 + t, j);
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          if (ctl_issuer<MODE>()) issue_pv(t, st, 0, j == 0);
+          ctl_rejoin<MODE>();
+          if (!ctl_wait<MODE>(&p_full[t][1], j & 1, &abort_s, lane)) {
+            if (lane == 0) report_status(p.status, STATUS_TIMEOUT, 25 + t, j);
             ok = false;
             break;
           }
           if (tracing && lane == 0 && (j * 2 + t) < p.trace_len) p.trace[0 * p.trace_len + j * 2 + t] = clock64();
           tc_fence_after();
           if (ctl_issuer<MODE>()) {
-            issue_pv(t, st, j == 0);
+            issue_pv(t, st, 1, j == 0);
+            umma_commit(&o_full[t]);
             if (more) issue_s(t, st_n);
             if (t == 1) {
               umma_commit(&v_empty[st]);
@@ -277,165 +282,128 @@ attention_fwd_kernel(const __grid_constant__ AttnMaps maps, const AttnParams p) 
     }
     __syncwarp();
   } else {
-    // ------------------------------- softmax warps: two threads per query row ---------------
-    // Warps 4-7 own key columns 0..63 of every S tile (and output columns 0..Dh/2-1), warps 8-11 the other half; the two
-    // threads of a row sit in warps with the same TMEM lane quadrant. Both q tiles are processed by the same threads in
-    // turn, so tile 0's P V and next Q K^T run on the tensor core while all eight warps do tile 1's softmax and vice
-    // versa: the exponentials of one tile are spread over all four special-function units with two warps each. Per kv
-    // tile the two halves exchange their row maxima through shared memory (an mbarrier of 64 arrivals per tile and
-    // quadrant, bounded wait), so both use the same exponent reference and take the same rescale decisions; the row sums
-    // stay partial and are added once at the end.
+    // ------------------------------- softmax warps: one thread per query row ----------------
+    // Warps 4-7 own q tile 0, warps 8-11 q tile 1, so each scheduler has one warp of either tile: while one waits for its P V
+    // and next Q K^T, or loads and compares, the other one has the special-function unit. (Both warpgroups on one tile at a
+    // time, two threads per row, exchanged their row maxima through shared memory and had all eight warps in the same phase.)
+    // P is published in two halves of 64 keys, so that P V starts on the first while the second is being exponentiated.
+    // Measured (B200): 1 x 4608 x 24 x 128 242 -> 232 us, 2 x 4096 x 10 x 64 208 -> 181, 1 x 988 x 20 x 64 27.5 -> 23.5.
     setmaxnreg_inc<SOFTMAX_REGS>();
-    const int half = (warp - 4) >> 2;
+    const int t = (warp - 4) >> 2;
     const int quad = warp & 3;
     const int row_in_tile = quad * 32 + lane;
     const uint32_t lane_addr = static_cast<uint32_t>(quad * 32) << 16;
+    const uint32_t s_tile = tmem_base + lane_addr + (t ? S_COL1 : S_COL0);
+    const uint32_t o_addr = tmem_base + lane_addr + (t ? O_COL1 : O_COL0);
     const float sl2 = p.scale_log2;
-    constexpr int OH = DH / 2;                 // output columns per thread
-    float m_used[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
+    float m_used = -INFINITY, l_run = 0.f;
     bool ok = true;
 
-    // max / sum exchange between the two threads of a row
-    auto exchange = [&](int t, float mine, uint32_t parity, float& other) -> bool {
-      x_val[t][half][row_in_tile] = mine;
-      mbar_arrive(&x_bar[t][quad]);
-      const bool got = mbar_wait(&x_bar[t][quad], parity, &abort_s);
-      other = x_val[t][half ^ 1][row_in_tile];
-      return got;
-    };
-
     for (int j = 0; ok && j < n_kv; ++j) {
-      const int kv0 = j * BKV + half * 64;
-      const bool tail = j * BKV + BKV > kv_valid;
-#pragma unroll
-      for (int t = 0; t < 2; ++t) {
-        const uint32_t s_tile = tmem_base + lane_addr + (t ? S_COL1 : S_COL0);
-        const uint32_t o_addr = tmem_base + lane_addr + (t ? O_COL1 : O_COL0) + half * OH;
-        ok = __all_sync(0xffffffffu, mbar_wait(&s_full[t], j & 1, &abort_s));
-        if (!ok) {
-          if (lane == 0) report_status(p.status, STATUS_TIMEOUT, 31 + t, j);
-          break;
-        }
-        tc_fence_after();
-        const bool tr = p.trace != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && warp == 4 && lane == 0 &&
-                        4 * j + 3 < p.trace_len;
-        if (tr) p.trace[(2 + t) * p.trace_len + 4 * j] = clock64();
-        uint32_t s0[32], s1[32];
-        tmem_ld_32x32b_x32(s_tile + half * 64, s0);
-        tmem_ld_32x32b_x32(s_tile + half * 64 + 32, s1);
-        tmem_wait_ld();
-        if (tr) p.trace[(2 + t) * p.trace_len + 4 * j + 1] = clock64();
-        if (tail) {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            if (kv0 + i >= kv_valid) s0[i] = 0xff800000u;        // -inf
-            if (kv0 + 32 + i >= kv_valid) s1[i] = 0xff800000u;
-          }
-        }
-        float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
-#pragma unroll
-        for (int i = 0; i < 32; i += 4) {                 // three-input maxima: 32 instructions for 64 values
-          mx0 = fmax3(mx0, __uint_as_float(s0[i]), __uint_as_float(s0[i + 1]));
-          mx1 = fmax3(mx1, __uint_as_float(s0[i + 2]), __uint_as_float(s0[i + 3]));
-          mx2 = fmax3(mx2, __uint_as_float(s1[i]), __uint_as_float(s1[i + 1]));
-          mx3 = fmax3(mx3, __uint_as_float(s1[i + 2]), __uint_as_float(s1[i + 3]));
-        }
-        float mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3)) * sl2;
-        float other;
-        ok = __all_sync(0xffffffffu, exchange(t, mx, j & 1, other));
-        if (!ok) {
-          if (lane == 0) report_status(p.status, STATUS_TIMEOUT, 37 + t, j);
-          break;
-        }
-        mx = fmaxf(mx, other);                     // the row's maximum over all 128 keys of the tile, same in both halves
-        if (tr) p.trace[(2 + t) * p.trace_len + 4 * j + 2] = clock64();
-        if (j == 0) {
-          m_used[t] = mx;
-        } else {
-          // lazy rescale: raise the exponent reference only when a row outgrew it by more than 2^8
-          const bool need = mx > m_used[t] + 8.0f;
-          if (__any_sync(0xffffffffu, need)) {
-            ok = __all_sync(0xffffffffu, mbar_wait(&o_full[t], (j - 1) & 1, &abort_s));
-            if (!ok) {
-              if (lane == 0) report_status(p.status, STATUS_TIMEOUT, 33 + t, j);
-              break;
-            }
-            tc_fence_after();
-            const float alpha = need ? exp2f(m_used[t] - mx) : 1.0f;
-            if (need) m_used[t] = mx;
-            l_run[t] *= alpha;
-#pragma unroll
-            for (int c = 0; c < OH / 32; ++c) {
-              uint32_t r[32];
-              tmem_ld_32x32b_x32(o_addr + c * 32, r);
-              tmem_wait_ld();
-#pragma unroll
-              for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * alpha);
-              tmem_st_32x32b_x32(o_addr + c * 32, r);
-            }
-            tmem_wait_st();
-          }
-        }
-        const float mref = m_used[t];
-        float2 sum_a = make_float2(0.f, 0.f), sum_b = make_float2(0.f, 0.f);
-        const float2 sl2_2 = make_float2(sl2, sl2), nm2 = make_float2(-mref, -mref);
-        auto emit = [&](const uint32_t (&sv)[32], int c) {
-          uint32_t pk[16];
-#pragma unroll
-          for (int i = 0; i < 32; i += 4) {
-            // Four scores per step as two packed pairs (scale and reference in one packed fma each). The special-function
-            // unit (16 results per clock per SM) bounds a loop of plain exponentials, so the odd elements of every
-            // POLY_EVERY-th group go through the packed polynomial on the FMA pipe instead.
-            const float2 x01 = ffma2(make_float2(__uint_as_float(sv[i]), __uint_as_float(sv[i + 1])), sl2_2, nm2);
-            const float2 x23 = ffma2(make_float2(__uint_as_float(sv[i + 2]), __uint_as_float(sv[i + 3])), sl2_2, nm2);
-            const float2 a = make_float2(ex2_approx(x01.x), ex2_approx(x23.x));
-            float2 b;
-            if (POLY_EVERY > 0 && ((i >> 2) % POLY_EVERY) == POLY_EVERY - 1) b = ex2_poly2(make_float2(x01.y, x23.y));
-            else b = make_float2(ex2_approx(x01.y), ex2_approx(x23.y));
-            sum_a = fadd2(sum_a, a);
-            sum_b = fadd2(sum_b, b);
-            pk[i >> 1] = pack_bf16x2(a.x, b.x);
-            pk[(i >> 1) + 1] = pack_bf16x2(a.y, b.y);
-          }
-          // P (bf16) of this half: 32 TMEM columns at half * 32 of the tile's S region; both halves have loaded their S
-          // values before the exchange above, so nothing still needed is overwritten
-          tmem_st_32x32b_x16(s_tile + half * 32 + c * 16, pk);
-        };
-        emit(s0, 0);
-        emit(s1, 1);
-        tmem_wait_st();
-        tc_fence_before();
-        mbar_arrive(&p_full[t]);
-        if (tr) p.trace[(2 + t) * p.trace_len + 4 * j + 3] = clock64();
-        l_run[t] += (sum_a.x + sum_a.y) + (sum_b.x + sum_b.y);
-      }
-    }
-#pragma unroll
-    for (int t = 0; t < 2; ++t) {
-      if (!ok) break;
-      const uint32_t o_addr = tmem_base + lane_addr + (t ? O_COL1 : O_COL0) + half * OH;
-      ok = __all_sync(0xffffffffu, mbar_wait(&o_full[t], (n_kv - 1) & 1, &abort_s));
+      const int kv0 = j * BKV;
+      ok = __all_sync(0xffffffffu, mbar_wait(&s_full[t], j & 1, &abort_s));
       if (!ok) {
-        if (lane == 0) report_status(p.status, STATUS_TIMEOUT, 35 + t, n_kv);
+        if (lane == 0) report_status(p.status, STATUS_TIMEOUT, 31 + t, j);
         break;
       }
       tc_fence_after();
-      float l_other;
-      ok = __all_sync(0xffffffffu, exchange(t, l_run[t], n_kv & 1, l_other));
-      if (!ok) {
-        if (lane == 0) report_status(p.status, STATUS_TIMEOUT, 39 + t, n_kv);
-        break;
+      const bool tr = p.trace != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && quad == 0 && lane == 0 &&
+                      4 * j + 3 < p.trace_len;
+      if (tr) p.trace[(2 + t) * p.trace_len + 4 * j] = clock64();
+      uint32_t sv[4][32];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) tmem_ld_32x32b_x32(s_tile + c * 32, sv[c]);
+      tmem_wait_ld();
+      if (tr) p.trace[(2 + t) * p.trace_len + 4 * j + 1] = clock64();
+      if (kv0 + BKV > kv_valid) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+          for (int i = 0; i < 32; ++i)
+            if (kv0 + c * 32 + i >= kv_valid) sv[c][i] = 0xff800000u;        // -inf
       }
-      const float l_tot = l_run[t] + l_other;
-      const float inv_l = 1.f / l_tot;
+      float mc[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+      for (int i = 0; i < 32; i += 2)                   // three-input maxima: 64 instructions for 128 values
+#pragma unroll
+        for (int c = 0; c < 4; ++c) mc[c] = fmax3(mc[c], __uint_as_float(sv[c][i]), __uint_as_float(sv[c][i + 1]));
+      const float mx = fmaxf(fmaxf(mc[0], mc[1]), fmaxf(mc[2], mc[3])) * sl2;
+      if (tr) p.trace[(2 + t) * p.trace_len + 4 * j + 2] = clock64();
+      if (j == 0) {
+        m_used = mx;
+      } else {
+        // lazy rescale: raise the exponent reference only when a row outgrew it by more than 2^8
+        const bool need = mx > m_used + 8.0f;
+        if (__any_sync(0xffffffffu, need)) {
+          ok = __all_sync(0xffffffffu, mbar_wait(&o_full[t], (j - 1) & 1, &abort_s));
+          if (!ok) {
+            if (lane == 0) report_status(p.status, STATUS_TIMEOUT, 33 + t, j);
+            break;
+          }
+          tc_fence_after();
+          const float alpha = need ? exp2f(m_used - mx) : 1.0f;
+          if (need) m_used = mx;
+          l_run *= alpha;
+#pragma unroll 1
+          for (int c = 0; c < DH / 16; ++c) {
+            uint32_t r[16];
+            tmem_ld_32x32b_x16(o_addr + c * 16, r);
+            tmem_wait_ld();
+#pragma unroll
+            for (int i = 0; i < 16; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * alpha);
+            tmem_st_32x32b_x16(o_addr + c * 16, r);
+          }
+          tmem_wait_st();
+        }
+      }
+      float2 sum_a = make_float2(0.f, 0.f), sum_b = make_float2(0.f, 0.f);
+      const float2 sl2_2 = make_float2(sl2, sl2), nm2 = make_float2(-m_used, -m_used);
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        uint32_t pk[16];
+#pragma unroll
+        for (int i = 0; i < 32; i += 4) {
+          // Four scores per step as two packed pairs (scale and reference in one packed fma each). The special-function
+          // unit (16 results per clock per SM) bounds a loop of plain exponentials, so the odd elements of every
+          // POLY_EVERY-th group go through the packed polynomial on the FMA pipe instead.
+          const float2 x01 = ffma2(make_float2(__uint_as_float(sv[c][i]), __uint_as_float(sv[c][i + 1])), sl2_2, nm2);
+          const float2 x23 = ffma2(make_float2(__uint_as_float(sv[c][i + 2]), __uint_as_float(sv[c][i + 3])), sl2_2, nm2);
+          const float2 a = make_float2(ex2_approx(x01.x), ex2_approx(x23.x));
+          float2 b;
+          if (POLY_EVERY > 0 && ((i >> 2) % POLY_EVERY) == POLY_EVERY - 1) b = ex2_poly2(make_float2(x01.y, x23.y));
+          else b = make_float2(ex2_approx(x01.y), ex2_approx(x23.y));
+          sum_a = fadd2(sum_a, a);
+          sum_b = fadd2(sum_b, b);
+          pk[i >> 1] = pack_bf16x2(a.x, b.x);
+          pk[(i >> 1) + 1] = pack_bf16x2(a.y, b.y);
+        }
+        // P (bf16) over the S columns it came from: all of them are in registers by now
+        tmem_st_32x32b_x16(s_tile + c * 16, pk);
+        if (c & 1) {
+          tmem_wait_st();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&p_full[t][c >> 1]);
+        }
+      }
+      if (tr) p.trace[(2 + t) * p.trace_len + 4 * j + 3] = clock64();
+      l_run += (sum_a.x + sum_a.y) + (sum_b.x + sum_b.y);
+    }
+    if (ok) {
+      ok = __all_sync(0xffffffffu, mbar_wait(&o_full[t], (n_kv - 1) & 1, &abort_s));
+      if (!ok && lane == 0) report_status(p.status, STATUS_TIMEOUT, 35 + t, n_kv);
+    }
+    if (ok) {
+      tc_fence_after();
+      const float inv_l = 1.f / l_run;
       // The normalised rows go through shared memory (this tile's Q buffer: every S = Q K^T has completed by now, 32 rows
-      // per quadrant) so that the global stores are whole rows: DH / 8 lanes x 16 bytes per row instead of one 16-byte
+      // per warp) so that the global stores are whole rows: DH / 8 lanes x 16 bytes per row instead of one 16-byte
       // piece of 32 different rows per instruction. That matters most when the rows are routed into a peer's memory.
       constexpr int CH = DH / 8;                       // 16-byte chunks per output row
       uint8_t* stage = sQ + t * TILE_BYTES + quad * (32 * DH * 2);
       uint4* my_row = reinterpret_cast<uint4*>(stage + lane * (DH * 2));
 #pragma unroll
-      for (int c = 0; c < OH / 32; ++c) {
+      for (int c = 0; c < DH / 32; ++c) {
         uint32_t r[32];
         tmem_ld_32x32b_x32(o_addr + c * 32, r);
         tmem_wait_ld();
@@ -446,21 +414,14 @@ attention_fwd_kernel(const __grid_constant__ AttnMaps maps, const AttnParams p) 
           w.y = pack_bf16x2(__uint_as_float(r[i + 2]) * inv_l, __uint_as_float(r[i + 3]) * inv_l);
           w.z = pack_bf16x2(__uint_as_float(r[i + 4]) * inv_l, __uint_as_float(r[i + 5]) * inv_l);
           w.w = pack_bf16x2(__uint_as_float(r[i + 6]) * inv_l, __uint_as_float(r[i + 7]) * inv_l);
-          my_row[(half * (CH / 2) + c * 4 + (i >> 3)) ^ (lane & (CH - 1))] = w;
+          my_row[(c * 4 + (i >> 3)) ^ (lane & (CH - 1))] = w;
         }
       }
-      // both halves of the quadrant's 32 rows are staged (a rendezvous only: the exchange slots are not written again, the
-      // partner may still be reading the row sum left there)
-      mbar_arrive(&x_bar[t][quad]);
-      ok = __all_sync(0xffffffffu, mbar_wait(&x_bar[t][quad], (n_kv + 1) & 1, &abort_s));
-      if (!ok) {
-        if (lane == 0) report_status(p.status, STATUS_TIMEOUT, 41 + t, n_kv);
-        break;
-      }
+      __syncwarp();
       const int chunk = lane % CH;
 #pragma unroll 4
-      for (int i = 0; i < CH / 2; ++i) {
-        const int rl = half * 16 + i * (32 / CH) + lane / CH;          // this warp copies 16 of the quadrant's 32 rows
+      for (int i = 0; i < CH; ++i) {
+        const int rl = i * (32 / CH) + lane / CH;
         const int tk = q0 + t * BQ + quad * 32 + rl;
         if (tk >= p.Sq) continue;
         __nv_bfloat16* obase = p.o;
@@ -482,8 +443,8 @@ attention_fwd_kernel(const __grid_constant__ AttnMaps maps, const AttnParams p) 
             reinterpret_cast<const uint4*>(stage + rl * (DH * 2))[chunk ^ (rl & (CH - 1))];
       }
       const int tok = q0 + t * BQ + row_in_tile;
-      if (half == 0 && p.lse != nullptr && tok < p.Sq)
-        p.lse[(static_cast<long long>(batch) * p.H + head) * p.Sq + tok] = (m_used[t] + log2f(l_tot)) * 0.6931471805599453f;
+      if (p.lse != nullptr && tok < p.Sq)
+        p.lse[(static_cast<long long>(batch) * p.H + head) * p.Sq + tok] = (m_used + log2f(l_run)) * 0.6931471805599453f;
     }
   }
 
