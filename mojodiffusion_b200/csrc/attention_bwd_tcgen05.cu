@@ -7,10 +7,11 @@
 //
 // with P = exp(scale * S - lse) rebuilt from the forward's log-sum-exp and delta = rowsum(dO o O), so no
 // [S, S] tensor ever exists in memory. The 128-row operands (R tiles) stay in shared memory for the whole CTA,
-// the 64-row operands (C tiles) stream through a 3-stage TMA ring and serve twice: K-major as the B operand of
+// the 64-row operands (C tiles) stream through a 4-stage TMA ring and serve twice: K-major as the B operand of
 // the score GEMMs and MN-major as the B operand of the gradient GEMMs (same bytes, different descriptor).
-// Score tiles X, Y are double buffered in TMEM so the tensor core computes tile i+1 while the math warps turn
-// tile i into bf16 P / dS, which they write back into TMEM over X / Y as the A operand (TS-form) of the
+// Score tiles X, Y are double buffered in TMEM, one buffer per math warpgroup: while one turns tile i into bf16 P / dS, the tensor
+// core computes tile i+1 and the other works on it (one warpgroup left the tensor core idle two thirds of the time; 1 x 4608 x 24 x 128
+// 1305 -> 1138 us, 1 x 988 x 20 x 64 121 -> 87), which they write back into TMEM over X / Y as the A operand (TS-form) of the
 // gradient GEMMs. TMEM: X0 X1 Y0 Y1 (64 columns each) + two 128-column accumulators = 512 columns.
 //
 // Math matched: serenitymojo/ops/attention_backward.mojo:249-349 (7-step decomposed backward) and the cuDNN
@@ -24,10 +25,10 @@
 
 namespace mdb {
 
-constexpr int BWD_THREADS = 192;
+constexpr int BWD_THREADS = 320;  // warps: 0 TMA, 1 UMMA issue, 2-5 and 6-9 two math warpgroups
 constexpr int RB = 128;  // resident rows per CTA
 constexpr int CB = 64;   // streamed rows per tile
-constexpr int CST = 3;   // C ring stages
+constexpr int CST = 4;   // C ring stages
 
 struct alignas(64) BwdMaps {
   CUtensorMap r1, r2, c1, c2;
@@ -42,7 +43,6 @@ struct BwdParams {
   const int* kv_len;
   int B, H, Sq, Skv;
   float scale, scale_log2;
-  int exp_poly;
   int* status;
 };
 
@@ -83,7 +83,7 @@ attention_bwd_kernel(const __grid_constant__ BwdMaps maps, const BwdParams p) {
   __shared__ uint64_t r_full, c_full[CST], c_empty[CST], xy_full[2], pds_full[2], lv_full[2], acc_full;
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_s;
-  __shared__ __align__(8) float s_lse2[2][CB], s_delta[2][CB];      // NEGATED lse * log2(e) and delta per staged query
+  __shared__ __align__(16) float s_lse2[2][CB], s_delta[2][CB];      // NEGATED lse * log2(e) and delta per staged query
 
   const uint32_t raw_addr = smem_u32(smem_raw);
   uint8_t* smem = smem_raw + (((raw_addr + 1023u) & ~1023u) - raw_addr);
@@ -126,7 +126,7 @@ attention_bwd_kernel(const __grid_constant__ BwdMaps maps, const BwdParams p) {
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(&xy_full[s], 1);
-      mbar_init(&pds_full[s], 128);
+      mbar_init(&pds_full[s], 4);
       mbar_init(&lv_full[s], CB);
     }
     mbar_init(&acc_full, 1);
@@ -193,37 +193,31 @@ attention_bwd_kernel(const __grid_constant__ BwdMaps maps, const BwdParams p) {
       // ----------------------------- UMMA issuer ------------------------------
       constexpr uint32_t idesc_xy = make_idesc(1, UMMA_BF16, UMMA_BF16, 0, 0, RB, CB);
       constexpr uint32_t idesc_acc = make_idesc(1, UMMA_BF16, UMMA_BF16, 0, 1, RB, DH);
+      // Descriptors are built once and moved by constants: built anew for each MMA they took 70 cycles of this thread for the 48 of
+      // the MMA, and 450 between two tiles.
+      const uint64_t r1 = make_desc_kmajor_sw128(smem_u32(sR1)), r2 = make_desc_kmajor_sw128(smem_u32(sR2));
+      const uint64_t ck = make_desc_kmajor_sw128(smem_u32(sC)), cm = make_desc_mnmajor_sw128(smem_u32(sC), C_BOX);
       auto issue_xy = [&](int st, int buf) {
-        const uint32_t a1 = smem_u32(sR1), a2 = smem_u32(sR2);
-        const uint32_t b1 = smem_u32(sC + st * 2 * C_BYTES), b2 = b1 + C_BYTES;
+        const uint64_t c1 = ck + static_cast<uint64_t>(st * (2 * C_BYTES >> 4)), c2 = c1 + (C_BYTES >> 4);
+        const uint32_t x = tmem_base + X_COL + buf * CB, y = tmem_base + Y_COL + buf * CB;
 #pragma unroll
-        for (int kk = 0; kk < DH / 16; ++kk) {
-          const uint32_t offa = (kk / 4) * R_BOX + (kk % 4) * 32;
-          const uint32_t offb = (kk / 4) * C_BOX + (kk % 4) * 32;
-          umma_f16_ss(tmem_base + X_COL + buf * CB, make_desc_kmajor_sw128(a1 + offa),
-                      make_desc_kmajor_sw128(b1 + offb), idesc_xy, kk != 0 ? 1u : 0u);
-        }
+        for (int kk = 0; kk < DH / 16; ++kk)
+          umma_f16_ss(x, r1 + (((kk / 4) * R_BOX + (kk % 4) * 32) >> 4), c1 + (((kk / 4) * C_BOX + (kk % 4) * 32) >> 4), idesc_xy, kk != 0 ? 1u : 0u);
 #pragma unroll
-        for (int kk = 0; kk < DH / 16; ++kk) {
-          const uint32_t offa = (kk / 4) * R_BOX + (kk % 4) * 32;
-          const uint32_t offb = (kk / 4) * C_BOX + (kk % 4) * 32;
-          umma_f16_ss(tmem_base + Y_COL + buf * CB, make_desc_kmajor_sw128(a2 + offa),
-                      make_desc_kmajor_sw128(b2 + offb), idesc_xy, kk != 0 ? 1u : 0u);
-        }
+        for (int kk = 0; kk < DH / 16; ++kk)
+          umma_f16_ss(y, r2 + (((kk / 4) * R_BOX + (kk % 4) * 32) >> 4), c2 + (((kk / 4) * C_BOX + (kk % 4) * 32) >> 4), idesc_xy, kk != 0 ? 1u : 0u);
         umma_commit(&xy_full[buf]);
       };
       auto issue_acc = [&](int st, int buf, bool first) {
-        const uint32_t b1 = smem_u32(sC + st * 2 * C_BYTES), b2 = b1 + C_BYTES;
+        const uint64_t c1 = cm + static_cast<uint64_t>(st * (2 * C_BYTES >> 4)), c2 = c1 + (C_BYTES >> 4);
         // acc1 += dS (over Y) * C1 ; KV mode: acc2 += P^T (over X) * C2
 #pragma unroll
         for (int kk = 0; kk < CB / 16; ++kk)
-          umma_f16_ts(tmem_base + ACC1_COL, tmem_base + Y_COL + buf * CB + kk * 8,
-                      make_desc_mnmajor_sw128(b1 + kk * 2048, C_BOX), idesc_acc, (first && kk == 0) ? 0u : 1u);
+          umma_f16_ts(tmem_base + ACC1_COL, tmem_base + Y_COL + buf * CB + kk * 8, c1 + (kk * 2048 >> 4), idesc_acc, (first && kk == 0) ? 0u : 1u);
         if (KV_MODE) {
 #pragma unroll
           for (int kk = 0; kk < CB / 16; ++kk)
-            umma_f16_ts(tmem_base + ACC2_COL, tmem_base + X_COL + buf * CB + kk * 8,
-                        make_desc_mnmajor_sw128(b2 + kk * 2048, C_BOX), idesc_acc, (first && kk == 0) ? 0u : 1u);
+            umma_f16_ts(tmem_base + ACC2_COL, tmem_base + X_COL + buf * CB + kk * 8, c2 + (kk * 2048 >> 4), idesc_acc, (first && kk == 0) ? 0u : 1u);
         }
       };
       bool ok = mbar_wait(&r_full, 0, &abort_s) && mbar_wait(&c_full[0], 0, &abort_s);
@@ -232,10 +226,11 @@ attention_bwd_kernel(const __grid_constant__ BwdMaps maps, const BwdParams p) {
         tc_fence_after();
         issue_xy(0, 0);
       }
+      static_assert((CST & (CST - 1)) == 0, "stage and phase by shifts");
       for (int i = 0; ok && i < n_c; ++i) {
-        const int st = i % CST;
+        const int st = i & (CST - 1);
         if (i + 1 < n_c) {
-          const int stn = (i + 1) % CST;
+          const int stn = (i + 1) & (CST - 1);
           if (!mbar_wait(&c_full[stn], ((i + 1) / CST) & 1, &abort_s)) {
             report_status(p.status, STATUS_TIMEOUT, 52, i);
             ok = false;
@@ -257,7 +252,8 @@ attention_bwd_kernel(const __grid_constant__ BwdMaps maps, const BwdParams p) {
     }
     __syncwarp();
   } else {
-    // ------------------------------- math warps (128 threads) --------------------------
+    // ------------------------------- math warps: warpgroup g takes the tiles i with i % 2 == g, which are those of buffer g
+    const int g = (warp - 2) >> 2;
     const int quad = warp & 3;
     const int mt = quad * 32 + lane;  // row inside the resident tile == TMEM lane
     const uint32_t lane_addr = static_cast<uint32_t>(quad * 32) << 16;
@@ -270,71 +266,74 @@ attention_bwd_kernel(const __grid_constant__ BwdMaps maps, const BwdParams p) {
       my_delta = p.delta[lse_base + row];
     }
     const bool row_key_valid = KV_MODE ? (row < kv_valid) : true;
+    // KV mode: thread mt < 64 stages the negated lse and delta of query mt of the warpgroup's tile, loaded one of its tiles ahead
+    float next_lse2 = -INFINITY, next_delta = 0.f;
+    auto fetch = [&](int i) {
+      const int q = i * CB + mt;
+      const bool in = mt < CB && q < p.Sq;
+      next_lse2 = in ? -p.lse[lse_base + q] * LOG2E : -INFINITY;
+      next_delta = in ? -p.delta[lse_base + q] : 0.f;
+    };
+    if (KV_MODE) fetch(g);
     bool ok = true;
-    for (int i = 0; i < n_c; ++i) {
-      const int buf = i & 1;
+    const uint32_t xa = tmem_base + lane_addr + X_COL + g * CB;
+    const uint32_t ya = tmem_base + lane_addr + Y_COL + g * CB;
+    for (int i = g; i < n_c; i += 2) {
+      const uint32_t par = (i >> 1) & 1;
       if (KV_MODE) {
-        // per-query lse / delta of this 64-query tile, staged by the first 64 math threads. The buffer was last
-        // read in iteration i-2: its 128 readers have all arrived on pds_full[buf] for that iteration.
+        // the buffer was last read for tile i - 2: the warpgroup's four warps have all arrived on pds_full[g] for it
         bool lv_ok = true;
         if (mt < CB) {
-          if (i >= 2) lv_ok = mbar_wait(&pds_full[buf], ((i - 2) >> 1) & 1, &abort_s);
-          const int q = i * CB + mt;
-          s_lse2[buf][mt] = q < p.Sq ? -p.lse[lse_base + q] * LOG2E : -INFINITY;
-          s_delta[buf][mt] = q < p.Sq ? -p.delta[lse_base + q] : 0.f;
-          mbar_arrive(&lv_full[buf]);
+          if (i >= 2) lv_ok = mbar_wait(&pds_full[g], par ^ 1u, &abort_s);
+          s_lse2[g][mt] = next_lse2;
+          s_delta[g][mt] = next_delta;
+          mbar_arrive(&lv_full[g]);
         }
-        lv_ok = mbar_wait(&lv_full[buf], (i >> 1) & 1, &abort_s) && lv_ok;
+        if (i + 2 < n_c) fetch(i + 2);
+        lv_ok = mbar_wait(&lv_full[g], par, &abort_s) && lv_ok;
         if (!__all_sync(0xffffffffu, lv_ok)) {
           if (lane == 0) report_status(p.status, STATUS_TIMEOUT, 60, i);
           ok = false;
           break;
         }
       }
-      ok = __all_sync(0xffffffffu, mbar_wait(&xy_full[buf], (i >> 1) & 1, &abort_s));
+      ok = __all_sync(0xffffffffu, mbar_wait(&xy_full[g], par, &abort_s));
       if (!ok) {
         if (lane == 0) report_status(p.status, STATUS_TIMEOUT, 61, i);
         break;
       }
       tc_fence_after();
-      const uint32_t xa = tmem_base + lane_addr + X_COL + buf * CB;
-      const uint32_t ya = tmem_base + lane_addr + Y_COL + buf * CB;
+      uint32_t xr[2][32], yr[2][32];
 #pragma unroll
       for (int c = 0; c < CB / 32; ++c) {
-        uint32_t xr[32], yr[32];
-        tmem_ld_32x32b_x32(xa + c * 32, xr);
-        tmem_ld_32x32b_x32(ya + c * 32, yr);
-        tmem_wait_ld();
+        tmem_ld_32x32b_x32(xa + c * 32, xr[c]);
+        tmem_ld_32x32b_x32(ya + c * 32, yr[c]);
+      }
+      tmem_wait_ld();
+      const bool tail = !KV_MODE && (i * CB + CB > kv_valid);
+#pragma unroll
+      for (int c = 0; c < CB / 32; ++c) {
         uint32_t pk[16], dk[16];
-        // Four columns per step as packed pairs: exponent = x * scale - lse2 and (dP - delta) are one packed operation
-        // each; with exp_poly the odd columns' exponentials run as a packed polynomial on the FMA pipe.
+        // Four columns per step as packed pairs: exponent = x * scale - lse2 and (dP - delta) are one packed operation each
         const float2 sl2_2 = make_float2(p.scale_log2, p.scale_log2);
         const float2 my_nl2 = make_float2(-my_lse2, -my_lse2), my_ndl = make_float2(-my_delta, -my_delta);
-        const bool tail = !KV_MODE && (i * CB + CB > kv_valid);
 #pragma unroll
         for (int e = 0; e < 32; e += 4) {
           const int col = c * 32 + e;
           float2 nl01, nl23, nd01, nd23;
           if (KV_MODE) {
-            nl01 = *reinterpret_cast<const float2*>(&s_lse2[buf][col]);
-            nl23 = *reinterpret_cast<const float2*>(&s_lse2[buf][col + 2]);
-            nd01 = *reinterpret_cast<const float2*>(&s_delta[buf][col]);
-            nd23 = *reinterpret_cast<const float2*>(&s_delta[buf][col + 2]);
+            const float4 nl = *reinterpret_cast<const float4*>(&s_lse2[g][col]), nd = *reinterpret_cast<const float4*>(&s_delta[g][col]);
+            nl01 = make_float2(nl.x, nl.y);
+            nl23 = make_float2(nl.z, nl.w);
+            nd01 = make_float2(nd.x, nd.y);
+            nd23 = make_float2(nd.z, nd.w);
           } else {
             nl01 = nl23 = my_nl2;
             nd01 = nd23 = my_ndl;
           }
-          const float2 x01 = ffma2(make_float2(__uint_as_float(xr[e]), __uint_as_float(xr[e + 1])), sl2_2, nl01);
-          const float2 x23 = ffma2(make_float2(__uint_as_float(xr[e + 2]), __uint_as_float(xr[e + 3])), sl2_2, nl23);
-          float2 p01, p23;
-          if (p.exp_poly) {
-            const float2 b = ex2_poly2(make_float2(x01.y, x23.y));
-            p01 = make_float2(ex2_approx(x01.x), b.x);
-            p23 = make_float2(ex2_approx(x23.x), b.y);
-          } else {
-            p01 = make_float2(ex2_approx(x01.x), ex2_approx(x01.y));
-            p23 = make_float2(ex2_approx(x23.x), ex2_approx(x23.y));
-          }
+          const float2 x01 = ffma2(make_float2(__uint_as_float(xr[c][e]), __uint_as_float(xr[c][e + 1])), sl2_2, nl01);
+          const float2 x23 = ffma2(make_float2(__uint_as_float(xr[c][e + 2]), __uint_as_float(xr[c][e + 3])), sl2_2, nl23);
+          float2 p01 = make_float2(ex2_approx(x01.x), ex2_approx(x01.y)), p23 = make_float2(ex2_approx(x23.x), ex2_approx(x23.y));
           if (KV_MODE) {
             if (!row_key_valid) p01 = p23 = make_float2(0.f, 0.f);
           } else if (tail) {
@@ -344,8 +343,8 @@ attention_bwd_kernel(const __grid_constant__ BwdMaps maps, const BwdParams p) {
             if (k0 + 2 >= kv_valid) p23.x = 0.f;
             if (k0 + 3 >= kv_valid) p23.y = 0.f;
           }
-          const float2 d01 = fmul2(p01, fadd2(make_float2(__uint_as_float(yr[e]), __uint_as_float(yr[e + 1])), nd01));
-          const float2 d23 = fmul2(p23, fadd2(make_float2(__uint_as_float(yr[e + 2]), __uint_as_float(yr[e + 3])), nd23));
+          const float2 d01 = fmul2(p01, fadd2(make_float2(__uint_as_float(yr[c][e]), __uint_as_float(yr[c][e + 1])), nd01));
+          const float2 d23 = fmul2(p23, fadd2(make_float2(__uint_as_float(yr[c][e + 2]), __uint_as_float(yr[c][e + 3])), nd23));
           pk[e >> 1] = pack_bf16x2(p01.x, p01.y);
           pk[(e >> 1) + 1] = pack_bf16x2(p23.x, p23.y);
           dk[e >> 1] = pack_bf16x2(d01.x, d01.y);
@@ -356,48 +355,36 @@ attention_bwd_kernel(const __grid_constant__ BwdMaps maps, const BwdParams p) {
       }
       tmem_wait_st();
       tc_fence_before();
-      mbar_arrive(&pds_full[buf]);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&pds_full[g]);
     }
     if (ok) {
       ok = __all_sync(0xffffffffu, mbar_wait(&acc_full, 0, &abort_s));
       if (!ok && lane == 0) report_status(p.status, STATUS_TIMEOUT, 62, 0);
     }
     if (ok) {
+      // KV mode: warpgroup 0 stores dK, warpgroup 1 dV; dQ: half of the columns each
       tc_fence_after();
-      __nv_bfloat16* o1 = p.out1 + batch * p.o1_strides[0] + static_cast<long long>(row) * p.o1_strides[1] +
-                          head * p.o1_strides[2];
-      __nv_bfloat16* o2 = KV_MODE ? p.out2 + batch * p.o2_strides[0] + static_cast<long long>(row) * p.o2_strides[1] +
-                                        head * p.o2_strides[2]
-                                  : nullptr;
+      __nv_bfloat16* o = KV_MODE && g == 1 ? p.out2 + batch * p.o2_strides[0] + static_cast<long long>(row) * p.o2_strides[1] + head * p.o2_strides[2]
+                                           : p.out1 + batch * p.o1_strides[0] + static_cast<long long>(row) * p.o1_strides[1] + head * p.o1_strides[2];
+      const uint32_t acc = tmem_base + lane_addr + (KV_MODE && g == 1 ? ACC2_COL : ACC1_COL);
+      const float f = KV_MODE && g == 1 ? 1.f : p.scale;
+      constexpr int CHUNKS = KV_MODE ? DH / 32 : DH / 64;
+      const int c0 = KV_MODE ? 0 : g * CHUNKS;
 #pragma unroll
-      for (int c = 0; c < DH / 32; ++c) {
+      for (int c = c0; c < c0 + CHUNKS; ++c) {
         uint32_t r[32];
-        tmem_ld_32x32b_x32(tmem_base + lane_addr + ACC1_COL + c * 32, r);
+        tmem_ld_32x32b_x32(acc + c * 32, r);
         tmem_wait_ld();
         if (row < out_rows) {
 #pragma unroll
           for (int e = 0; e < 32; e += 8) {
             uint4 w;
-            w.x = pack_bf16x2(__uint_as_float(r[e + 0]) * p.scale, __uint_as_float(r[e + 1]) * p.scale);
-            w.y = pack_bf16x2(__uint_as_float(r[e + 2]) * p.scale, __uint_as_float(r[e + 3]) * p.scale);
-            w.z = pack_bf16x2(__uint_as_float(r[e + 4]) * p.scale, __uint_as_float(r[e + 5]) * p.scale);
-            w.w = pack_bf16x2(__uint_as_float(r[e + 6]) * p.scale, __uint_as_float(r[e + 7]) * p.scale);
-            *reinterpret_cast<uint4*>(o1 + c * 32 + e) = w;
-          }
-        }
-        if (KV_MODE) {
-          tmem_ld_32x32b_x32(tmem_base + lane_addr + ACC2_COL + c * 32, r);
-          tmem_wait_ld();
-          if (row < out_rows) {
-#pragma unroll
-            for (int e = 0; e < 32; e += 8) {
-              uint4 w;
-              w.x = pack_bf16x2(__uint_as_float(r[e + 0]), __uint_as_float(r[e + 1]));
-              w.y = pack_bf16x2(__uint_as_float(r[e + 2]), __uint_as_float(r[e + 3]));
-              w.z = pack_bf16x2(__uint_as_float(r[e + 4]), __uint_as_float(r[e + 5]));
-              w.w = pack_bf16x2(__uint_as_float(r[e + 6]), __uint_as_float(r[e + 7]));
-              *reinterpret_cast<uint4*>(o2 + c * 32 + e) = w;
-            }
+            w.x = pack_bf16x2(__uint_as_float(r[e + 0]) * f, __uint_as_float(r[e + 1]) * f);
+            w.y = pack_bf16x2(__uint_as_float(r[e + 2]) * f, __uint_as_float(r[e + 3]) * f);
+            w.z = pack_bf16x2(__uint_as_float(r[e + 4]) * f, __uint_as_float(r[e + 5]) * f);
+            w.w = pack_bf16x2(__uint_as_float(r[e + 6]) * f, __uint_as_float(r[e + 7]) * f);
+            *reinterpret_cast<uint4*>(o + c * 32 + e) = w;
           }
         }
       }
@@ -465,14 +452,6 @@ extern "C" int mdb_attention_bwd(const MdbAttnBwdArgs* a, cudaStream_t st) {
   p.B = a->B; p.H = a->H; p.Sq = a->Sq; p.Skv = a->Skv;
   p.scale = a->scale;
   p.scale_log2 = a->scale * 1.4426950408889634f;
-  {
-    static int mode = -1;
-    if (mode < 0) {
-      const char* e = getenv("MDB200_ATTN_EXP_POLY");
-      mode = (e != nullptr && e[0] == '1') ? 1 : 0;
-    }
-    p.exp_poly = mode;
-  }
   p.status = a->status;
   int r;
   // ---- dQ: resident Q, dO ; streamed K, V
