@@ -296,7 +296,7 @@ attention_fwd_kernel(const __grid_constant__ AttnMaps maps, const AttnParams p) 
     const uint32_t s_tile = tmem_base + lane_addr + (t ? S_COL1 : S_COL0);
     const uint32_t o_addr = tmem_base + lane_addr + (t ? O_COL1 : O_COL0);
     const float sl2 = p.scale_log2;
-    float m_used = -INFINITY, l_run = 0.f;
+    float m_used = -INFINITY, l_run[2] = {0.f, 0.f};      // row sums of the first and second 64 keys of the tiles, added once at the end
     bool ok = true;
 
     for (int j = 0; ok && j < n_kv; ++j) {
@@ -343,7 +343,8 @@ attention_fwd_kernel(const __grid_constant__ AttnMaps maps, const AttnParams p) 
           tc_fence_after();
           const float alpha = need ? exp2f(m_used - mx) : 1.0f;
           if (need) m_used = mx;
-          l_run *= alpha;
+          l_run[0] *= alpha;
+          l_run[1] *= alpha;
 #pragma unroll 1
           for (int c = 0; c < DH / 16; ++c) {
             uint32_t r[16];
@@ -384,10 +385,11 @@ attention_fwd_kernel(const __grid_constant__ AttnMaps maps, const AttnParams p) 
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(&p_full[t][c >> 1]);
+          l_run[c >> 1] += (sum_a.x + sum_a.y) + (sum_b.x + sum_b.y);
+          sum_a = sum_b = make_float2(0.f, 0.f);
         }
       }
       if (tr) p.trace[(2 + t) * p.trace_len + 4 * j + 3] = clock64();
-      l_run += (sum_a.x + sum_a.y) + (sum_b.x + sum_b.y);
     }
     if (ok) {
       ok = __all_sync(0xffffffffu, mbar_wait(&o_full[t], (n_kv - 1) & 1, &abort_s));
@@ -395,7 +397,8 @@ attention_fwd_kernel(const __grid_constant__ AttnMaps maps, const AttnParams p) 
     }
     if (ok) {
       tc_fence_after();
-      const float inv_l = 1.f / l_run;
+      const float l_tot = l_run[0] + l_run[1];
+      const float inv_l = 1.f / l_tot;
       // The normalised rows go through shared memory (this tile's Q buffer: every S = Q K^T has completed by now, 32 rows
       // per warp) so that the global stores are whole rows: DH / 8 lanes x 16 bytes per row instead of one 16-byte
       // piece of 32 different rows per instruction. That matters most when the rows are routed into a peer's memory.
@@ -444,7 +447,7 @@ attention_fwd_kernel(const __grid_constant__ AttnMaps maps, const AttnParams p) 
       }
       const int tok = q0 + t * BQ + row_in_tile;
       if (p.lse != nullptr && tok < p.Sq)
-        p.lse[(static_cast<long long>(batch) * p.H + head) * p.Sq + tok] = (m_used + log2f(l_run)) * 0.6931471805599453f;
+        p.lse[(static_cast<long long>(batch) * p.H + head) * p.Sq + tok] = (m_used + log2f(l_tot)) * 0.6931471805599453f;
     }
   }
 

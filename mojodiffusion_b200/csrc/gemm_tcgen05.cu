@@ -1626,12 +1626,15 @@ namespace mdb {
 // reduction. Every form is estimated in microseconds and the lowest one taken.
 //
 // The terms are fitted to measured times of all forms over 1457 calls (M 1 to 65536, N and K 16 to 21504, the three operand
-// layouts, with and without epilogue terms; B200, weights from HBM). Over them the choice is 1.6 % above the best form of each
-// (geometric mean; 39 of them more than 20 %). What they say:
-//  - a 64-wide K step takes 0.37 / 0.39 / 0.44 us of a lone CTA with 64 / 128 / 256 columns (it is bound by what the SM takes in) and
-//    0.335 of a pair;
-//  - a tile's epilogue takes 1 to 2.1 us, twice that with an activation or with gate and residual, three times with both, and hides
-//    behind the next tile's steps only; where the lanes store the rows themselves (fp32, odd strides) half as much again;
+// layouts, with and without epilogue terms; B200, weights from HBM). Over them the choice is 1.4 % above the best form of each
+// (geometric mean; 18 of them more than 20 %). They were measured before the epilogue of the whole-K tiles became two to three times
+// shorter; over the whole-K times measured since, the choice is 2.3 % above the best form, with refitted terms (epilogues 1 to 2.1 us) 1.6 %.
+// They stay, because a form is also an order of sums: a training step passes a changed order through its optimizer into single
+// gradient entries (up to 0.9 of their root mean square after one step of an SDXL adapter). What they say:
+//  - a 64-wide K step takes 0.32 / 0.34 / 0.46 us of a lone CTA with 64 / 128 / 256 columns (a narrow MMA issues hardly faster) and
+//    0.34 of a pair;
+//  - a tile's epilogue takes 1.6 to 3 us, three times that with activation, gate or residual, and hides behind the next tile's
+//    steps only; rows that end off 32 columns leave its vector path (N = 16: 8 us more);
 //  - a cluster's tile starts, meets in shared memory and ends in 6 to 9 us, and finishing its rows costs a CTA 2.2 to 7.2 us / splits
 //    (six times that with epilogue terms): it pays for long reductions only, and never for tiles that come in many waves
 //    (65536 x 128 x 128: 65 us in clusters of one, 17 on the persistent tiles). 15 % are added for it, so that it wins clear cases;
@@ -1648,34 +1651,31 @@ static GemmForm choose_form(const MdbGemmArgs* a, int sms, bool pairs, bool rows
   const double n_all = paired ? 2.0 * a->N : a->N;                           // rows of B
   const double memory = 2.0 * (a->M * k_all + n_all * k_all + static_cast<double>(a->M) * a->N) / 3.6e6;
   const bool heavy = a->act != 0 || a->gate || a->residual || paired;
-  const bool bulk = !a->out_fp32 && ((reinterpret_cast<uintptr_t>(a->out) | static_cast<uintptr_t>(static_cast<size_t>(a->ld_out) * 2)) & 15) == 0;
-  const double whole_terms = (heavy ? ((a->act || paired) && (a->gate || a->residual) ? 3.1 : 2.2) : 1.0) * (bulk ? 1.0 : 1.5);
-  const double split_terms = heavy ? 6.2 : a->bias ? 2.1 : 1.0;
+  const double whole_terms = heavy ? 3.0 : a->bias ? 1.4 : 1.0, split_terms = heavy ? 6.2 : a->bias ? 2.1 : 1.0;
   auto ceil_div = [](double x, double y) { return std::ceil(x / y); };
   auto with_memory = [&](double t) { return std::sqrt(std::sqrt(t * t * t * t + memory * memory * memory * memory)); };   // neither hides wholly behind the other
   auto tiles = [&](double tm, double tn) { return ceil_div(a->M, tm) * ceil_div(a->N, tn); };
-  auto step = [](int w) { return w == 64 ? 0.37 : w == 128 ? 0.39 : 0.44; };
-  auto split_step = [](int w) { return w == 64 ? 0.32 : 0.34; };
+  auto step = [](int w) { return w == 64 ? 0.32 : w == 128 ? 0.34 : 0.46; };
   GemmForm best = {256, 0, false, false};
   double best_us = 1e30;
   auto offer = [&](double us, GemmForm f) { if (us < best_us) { best_us = us; best = f; } };
 
   auto whole = [&](double n_tiles, int width, double step_us, double epilogue) {
-    const double e = epilogue * whole_terms, main = kb * step_us;
-    return with_memory(4.3 + ceil_div(n_tiles, width) * (main > e ? main : e) + e);
+    const double e = epilogue * whole_terms + (a->N % 32 != 0 && a->N < 256 ? 8.0 : 0.0), main = kb * step_us;
+    return with_memory(5.0 + ceil_div(n_tiles, width) * (main > e ? main : e) + e);
   };
-  offer(whole(tiles(BM, paired ? 128 : 256), sms, step(256), 2.0), {256, 0, false, false});
+  offer(whole(tiles(BM, paired ? 128 : 256), sms, step(256), 3.0), {256, 0, false, false});
   if (!paired) {
-    offer(whole(tiles(BM, 128), sms, step(128), 1.35), {128, 0, false, false});
-    offer(whole(tiles(BM, 64), sms, step(64), 1.0), {64, 0, false, false});
+    offer(whole(tiles(BM, 128), sms, step(128), 2.1), {128, 0, false, false});
+    offer(whole(tiles(BM, 64), sms, step(64), 1.6), {64, 0, false, false});
   }
-  if (pairs && a->M > BM) offer(whole(tiles(2 * BM, paired ? 128 : 256), pair_capacity(sms), 0.335, 2.1), {256, 0, true, false});
+  if (pairs && a->M > BM) offer(whole(tiles(2 * BM, paired ? 128 : 256), pair_capacity(sms), 0.34, 2.9), {256, 0, true, false});
   if (!whole_only) {
     for (int w = 128; w >= 64; w -= 64)
       for (int sp = 1; sp <= SPLIT_MAX && (sp == 1 || kb / sp >= 4); ++sp) {
         const int cap = w == 128 ? split_capacity<128>(sp, sms) : split_capacity<64>(sp, sms);
         const double fixed = w == 128 ? 7.0 + 3.55 * split_terms / sp : 5.9 + 2.2 * split_terms / sp;
-        offer(with_memory(1.15 * ceil_div(tiles(BM, w), cap) * (ceil_div(kb, sp) * split_step(w) + fixed)), {w, sp, false, false});
+        offer(with_memory(1.15 * ceil_div(tiles(BM, w), cap) * (ceil_div(kb, sp) * step(w) + fixed)), {w, sp, false, false});
       }
     for (int sp = 2; sp <= PSPLIT_MAX && kb / sp >= 4 && !a->a_mn && a->M > BM; ++sp)
       offer(with_memory(1.15 * ceil_div(tiles(2 * BM, 256), pair_split_capacity(sp, sms)) * (ceil_div(kb, sp) * 0.34 + 9.0 + 7.2 * split_terms / sp)), {256, sp, true, false});

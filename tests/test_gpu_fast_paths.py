@@ -611,3 +611,21 @@ def test_bulk_epilogue(M, N, K, bn, terms):
         got = _gemm([x], [w], bias=b, out=wide[:, N:2 * N], bn=bn)
         assert not wide[:, :N].any() and not wide[:, 2 * N:].any()
     _close(got, want, f"{terms} {M}x{N}x{K}", rel=1e-4)
+
+
+# one and two tiles of each stream, last tiles of one row or key, one warpgroup without a tile
+@pytest.mark.parametrize("Sq,Skv", [(1, 1), (65, 64), (128, 65), (257, 129), (64, 300), (300, 193)])
+@pytest.mark.parametrize("Dh", [64, 128])
+def test_attention_few_tiles(Sq, Skv, Dh):
+    q, k, v = (_rand(2, s, 3, Dh, seed=i).requires_grad_(True) for i, s in enumerate((Sq, Skv, Skv)))
+    do = _rand(2, Sq, 3, Dh, seed=5)
+    o = O.attention(q, k, v)
+    got = torch.autograd.grad(o, (q, k, v), do)
+    q2, k2, v2 = (t.detach().double().requires_grad_(True) for t in (q, k, v))
+    want = torch.nn.functional.scaled_dot_product_attention(*(t.transpose(1, 2) for t in (q2, k2, v2))).transpose(1, 2)
+    wants = torch.autograd.grad(want, (q2, k2, v2), do.double())
+    native.check_status(o)
+    # P, dS and the result are rounded to bf16 once each (2^-9 relative), o once more on its way into delta
+    for a, b, n in zip((o, *got), (want, *wants), ("o", "dq", "dk", "dv")):
+        err = float((a.double() - b).norm() / b.norm().clamp_min(1e-9)) if b.norm() > 1e-6 else float(a.double().norm())
+        assert err < 4 * 2.0 ** -9, (n, err)
