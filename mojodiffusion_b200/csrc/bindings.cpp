@@ -733,13 +733,14 @@ const void* llm_vector(const optional<Tensor>& v, int64_t n, const Tensor& x, co
   return v->data_ptr();
 }
 // out = x w^T + bias in bf16 rows of ld_out elements
-void llm_project(const Tensor& x, const Tensor& w, const void* bias, void* out, int64_t ld_out) {
+void llm_project(const Tensor& x, const Tensor& w, const void* bias, void* out, int64_t ld_out, bool whole_k = false) {
   MdbGemmArgs g;
   memset(&g, 0, sizeof(g));
   g.M = (int)x.size(0); g.N = (int)w.size(0); g.num_seg = 1;
   g.K[0] = x.size(1); g.A[0] = x.data_ptr(); g.B[0] = w.data_ptr(); g.lda[0] = x.size(1); g.ldb[0] = x.size(1);
   g.alpha = 1.f; g.rows_per_group = 1; g.bias = bias;
   g.out = out; g.ld_out = (int)ld_out;
+  g.split_k = whole_k;
   g.num_sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
   g.status = status_ptr(x);
   check_rc(mdb_gemm_launch(&g, cur_stream()), "decoder projection");
@@ -813,6 +814,66 @@ Tensor llm_out_mlp(Tensor x, const Tensor& attn, const Tensor& wo, const Tensor&
   }
   Tensor out = at::empty_like(x);
   llm_project(m, llm_matrix(wd, D, F, x, "down weight"), nullptr, out.data_ptr(), D);
+  return out;
+}
+// The same two halves of a layer for a prompt, x [B * S, hidden]: whole reductions in the projections, means by the torch reduction
+// over tensors of the shape the modules see, so that every value is what the modules compute.
+Tensor llm_prompt_norm(Tensor& x, const optional<Tensor>& y, const Tensor& w, int64_t B, double eps) {
+  const int64_t R = x.size(0), D = x.size(1);
+  const void* py = nullptr;
+  if (y.has_value() && y->defined()) {
+    TORCH_CHECK(y->device() == x.device() && y->scalar_type() == at::kBFloat16 && y->is_contiguous() && y->sizes() == x.sizes(), "decoder layer: y");
+    py = y->data_ptr();
+  }
+  Tensor sq = at::empty({B, R / B, D}, x.options().dtype(at::kFloat)), h = at::empty_like(x);
+  check_rc(mdb_add_square(x.data_ptr(), py, sq.data_ptr<float>(), x.numel(), cur_stream()), "add_square");
+  Tensor mean = at::mean(sq, at::IntArrayRef{-1}, true);
+  check_rc(mdb_rms_scale(x.data_ptr(), mean.data_ptr<float>(), llm_vector(w, D, x, "norm weight"), h.data_ptr(), R, (int)D, (float)eps, cur_stream()), "rms_scale");
+  return h;
+}
+std::vector<Tensor> llm_prompt_qkv(Tensor x, const optional<Tensor>& y, const Tensor& ln, const Tensor& wq, const Tensor& wk, const Tensor& wv,
+                                   const optional<Tensor>& bq, const optional<Tensor>& bk, const optional<Tensor>& bv, const Tensor& qn, const Tensor& kn,
+                                   const Tensor& cosv, const Tensor& sinv, Tensor k_cache, Tensor v_cache, double eps) {
+  llm_check_rows(x);
+  c10::cuda::CUDAGuard guard(x.device());
+  TORCH_CHECK(k_cache.dim() == 4 && k_cache.is_contiguous() && v_cache.is_contiguous() && v_cache.sizes() == k_cache.sizes() &&
+                  k_cache.scalar_type() == at::kBFloat16 && v_cache.scalar_type() == at::kBFloat16 && k_cache.device() == x.device() &&
+                  v_cache.device() == x.device(), "decoder layer: caches [B, Hkv, T, Dh] bf16");
+  const int64_t R = x.size(0), D = x.size(1), B = k_cache.size(0), Hkv = k_cache.size(1), T = k_cache.size(2), Dh = k_cache.size(3), S = B > 0 ? R / B : 0;
+  TORCH_CHECK(B > 0 && S * B == R && S <= T && Dh > 0 && Dh % 8 == 0 && Dh <= 256 && wq.size(0) % Dh == 0 && (wq.size(0) / Dh) % Hkv == 0,
+              "decoder layer: rows / heads / positions do not match the cache");
+  const int64_t H = wq.size(0) / Dh, W = (H + 2 * Hkv) * Dh;
+  for (const Tensor* t : {&cosv, &sinv})
+    TORCH_CHECK(t->device() == x.device() && t->scalar_type() == at::kBFloat16 && t->is_contiguous() && t->dim() == 2 && t->size(1) == Dh &&
+                    t->size(0) >= S, "decoder layer: rotary tables [positions, Dh] bf16");
+  Tensor h = llm_prompt_norm(x, y, ln, B, eps);
+  Tensor qkv = at::empty({R, W}, x.options()), q = at::empty({B, S, H, Dh}, x.options()), k = at::empty({B, H, S, Dh}, x.options()), v = at::empty_like(k);
+  char* base = static_cast<char*>(qkv.data_ptr());
+  llm_project(h, llm_matrix(wq, H * Dh, D, x, "q weight"), llm_vector(bq, H * Dh, x, "q bias"), base, W, true);
+  llm_project(h, llm_matrix(wk, Hkv * Dh, D, x, "k weight"), llm_vector(bk, Hkv * Dh, x, "k bias"), base + 2 * H * Dh, W, true);
+  llm_project(h, llm_matrix(wv, Hkv * Dh, D, x, "v weight"), llm_vector(bv, Hkv * Dh, x, "v bias"), base + 2 * (H + Hkv) * Dh, W, true);
+  const auto f32 = x.options().dtype(at::kFloat);
+  Tensor sq = at::empty({B, S, H, Dh}, f32), sk = at::empty({B, S, Hkv, Dh}, f32);
+  check_rc(mdb_square_heads(base, sq.data_ptr<float>(), sk.data_ptr<float>(), R, (int)H, (int)Hkv, (int)Dh, cur_stream()), "square_heads");
+  Tensor mq = at::mean(sq, at::IntArrayRef{-1}, true), mk = at::mean(sk, at::IntArrayRef{-1}, true);
+  check_rc(mdb_prompt_rope_cache(base, mq.data_ptr<float>(), mk.data_ptr<float>(), llm_vector(qn, Dh, x, "q norm"), llm_vector(kn, Dh, x, "k norm"),
+                                 cosv.data_ptr(), sinv.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(),
+                                 (int)B, (int)S, (int)H, (int)Hkv, (int)Dh, (int)T, (float)eps, cur_stream()), "prompt_rope_cache");
+  return {q.transpose(1, 2), k, v};
+}
+// x += attention output projection (in place), returns the gated MLP of the new x (not yet added): attn [B, S, H * Dh]
+Tensor llm_prompt_mlp(Tensor x, const Tensor& attn, const Tensor& wo, const Tensor& ln, const Tensor& wg, const Tensor& wu, const Tensor& wd, double eps) {
+  llm_check_rows(x);
+  c10::cuda::CUDAGuard guard(x.device());
+  const int64_t R = x.size(0), D = x.size(1), F = wg.size(0), A = attn.size(-1);
+  TORCH_CHECK(attn.device() == x.device() && attn.scalar_type() == at::kBFloat16 && attn.is_contiguous() && attn.dim() == 3 && A > 0 && attn.numel() == R * A &&
+                  A % 8 == 0 && F % 8 == 0, "decoder layer: attention rows");
+  Tensor y = at::empty_like(x), g = at::empty({R, F}, x.options()), u = at::empty({R, F}, x.options()), out = at::empty_like(x);
+  llm_project(attn.view({R, A}), llm_matrix(wo, D, A, x, "output weight"), nullptr, y.data_ptr(), D, true);
+  Tensor h = llm_prompt_norm(x, y, ln, attn.size(0), eps);
+  llm_project(h, llm_matrix(wg, F, D, x, "gate weight"), nullptr, g.data_ptr(), F, true);
+  llm_project(h, llm_matrix(wu, F, D, x, "up weight"), nullptr, u.data_ptr(), F, true);
+  llm_project(at::mul(at::silu(g), u), llm_matrix(wd, D, F, x, "down weight"), nullptr, out.data_ptr(), D, true);
   return out;
 }
 // one query per sequence (the first H * Dh columns of qkv rows) over the first ``len`` rows of the caches -> [B, H * Dh]
@@ -1207,6 +1268,8 @@ TORCH_LIBRARY(mdb200, m) {
   m.def("llm_decode_attention_max", &llm_decode_attention_max);
   m.def("llm_qkv", &llm_qkv);
   m.def("llm_out_mlp", &llm_out_mlp);
+  m.def("llm_prompt_qkv", &llm_prompt_qkv);
+  m.def("llm_prompt_mlp", &llm_prompt_mlp);
   m.def("llm_decode_attention", &llm_decode_attention);
   m.def("fp8_quant_rows", &fp8_quant_rows);
   m.def("fp8_dequant", &fp8_dequant);

@@ -53,6 +53,14 @@ int mdb_qkv_rope_cache(void* qkv, const void* qn, const void* kn, const void* co
                        int Hkv, int Dh, int T, int pos, float eps, cudaStream_t st);
 // x += y (y null: nothing), h = RMSNorm(x) * w
 int mdb_add_rms_rows(void* x, const void* y, const void* w, void* h, long long rows, int D, float eps, cudaStream_t st);
+// the same steps for many rows, around means that the caller forms: x += y and sq = x^2; h = x rsqrt(mean + eps) w; squares of the q and k
+// heads of packed rows; normalised and rotated q rows [B * S, H, Dh], k and v in the caches (positions 0 .. S - 1) and repeated [B, H, S, Dh]
+int mdb_add_square(void* x, const void* y, float* sq, long long n, cudaStream_t st);
+int mdb_rms_scale(const void* x, const float* mean, const void* w, void* h, long long rows, int D, float eps, cudaStream_t st);
+int mdb_square_heads(const void* qkv, float* sq_q, float* sq_k, long long rows, int H, int Hkv, int Dh, cudaStream_t st);
+int mdb_prompt_rope_cache(const void* qkv, const float* mean_q, const float* mean_k, const void* qn, const void* kn, const void* cosv,
+                          const void* sinv, void* qo, void* kr, void* vr, void* kc, void* vc, int B, int S, int H, int Hkv, int Dh, int T, float eps,
+                          cudaStream_t st);
 #define MDB_DECODE_ATTENTION_MAX 7936      // cache rows whose scores fit beside the partial sums in 48 KB of shared memory
 int mdb_decode_attention(const void* q, long long ldq, const void* kc, const void* vc, void* o, int B, int H, int Hkv, int Dh, int T, int len,
                          float scale, cudaStream_t st);

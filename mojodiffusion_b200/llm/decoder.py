@@ -68,10 +68,11 @@ class Qwen3Decoder:
                 and c.intermediate_size % 8 == 0 and c.head_dim % 8 == 0 and c.head_dim <= 256 and x.numel() > 0
                 and c.num_attention_heads % c.num_key_value_heads == 0)
 
-    def _fused_layers(self, x: torch.Tensor, cache: KVCache, pos: int):
+    def _fused_layers(self, x: torch.Tensor, cache: KVCache, pos: int, batch: Optional[int] = None):
         """Per layer ((norm, q, k, v, biases, q norm, k norm), (o, norm, gate, up, down)) for the fused kernels, or None when the
         separate operations have to run: a module that a program hooked, replaced or gave another epsilon or bias, weights or
-        caches of another type, shape or layout. Looked at anew on every step."""
+        caches of another type, shape or layout. Looked at anew on every step. x [rows, hidden]: one row per sequence at ``pos``, or
+        (``batch`` given) the rows of a prompt that ends there."""
         c, rope = self.cfg, getattr(cache, "rope", None)
         if rope is None or not self._native(x) or pos >= native.ops().llm_decode_attention_max() or x.dim() != 2 or globally_hooked():
             return None
@@ -112,7 +113,7 @@ class Qwen3Decoder:
         # one call looks at type, device, layout, alignment and shape of all weights: the launches refuse what the separate
         # operations broadcast or copy
         shapes = [D, 0, Q, D, KV, D, KV, D, *([Q, 0, KV, 0, KV, 0] if has else []), Dh, 0, Dh, 0, D, Q, D, 0, F, D, F, D, D, F]
-        kv = (len(layers), x.shape[0], c.num_key_value_heads, cache.k.shape[3] if cache.k.dim() == 5 else 0, Dh)
+        kv = (len(layers), x.shape[0] if batch is None else batch, c.num_key_value_heads, cache.k.shape[3] if cache.k.dim() == 5 else 0, Dh)
         if kv[3] <= pos or cache.k.shape != kv or cache.v.shape != kv or any(t.dim() != 2 or t.shape[0] <= pos or t.shape[1] != Dh for t in rope):
             return None
         ok = native.ops().bf16_operands_ok
@@ -132,6 +133,16 @@ class Qwen3Decoder:
         if self._native(x):
             reach = min(max_len, native.ops().llm_decode_attention_max())
             cache.rope = self._angles(torch.arange(reach, device=ids.device), x.dtype)        # for the decode steps
+        layers = self._fused_layers(x.view(B * S, -1), cache, S - 1, B) if cache.rope is not None and S > 0 and native.direct(x) else None
+        if layers is not None:
+            # updated in place: the embedding's output stays as it is
+            o, x2, y = native.ops(), x.reshape(B * S, -1).clone(), None
+            for li, (qkv, out_mlp) in enumerate(layers):
+                q, k, v = o.llm_prompt_qkv(x2, y, *qkv, *cache.rope, cache.k[li], cache.v[li], c.rms_norm_eps)
+                attn = torch.nn.functional.scaled_dot_product_attention(q, k, v, attn_mask=mask).transpose(1, 2).reshape(B, S, -1)
+                y = o.llm_prompt_mlp(x2, attn, *out_mlp, c.rms_norm_eps)
+            cache.length = S
+            return (x2 + y if y is not None else x2).view(B, S, -1)[:, -1], cache
         for li, l in enumerate(m.layers):
             a = l.self_attn
             h = l.input_layernorm(x)

@@ -629,3 +629,23 @@ def test_attention_few_tiles(Sq, Skv, Dh):
     for a, b, n in zip((o, *got), (want, *wants), ("o", "dq", "dk", "dv")):
         err = float((a.double() - b).norm() / b.norm().clamp_min(1e-9)) if b.norm() > 1e-6 else float(a.double().norm())
         assert err < 4 * 2.0 ** -9, (n, err)
+
+
+@pytest.mark.parametrize("B,S,bias", [(1, 1, False), (1, 45, False), (2, 9, True), (3, 130, False)])
+def test_prompt_layers_keep_every_bit(B, S, bias):
+    """The fused prompt and the modules (one of them hooked, which the fused path leaves to itself) give the same bits."""
+    from mojodiffusion_b200.llm.decoder import Qwen3Decoder
+    from mojodiffusion_b200.models.text.qwen3 import Qwen3Config, Qwen3Encoder
+    cfg = Qwen3Config(vocab_size=512, hidden_size=384, intermediate_size=776, num_hidden_layers=3, num_attention_heads=6, num_key_value_heads=2,
+                      head_dim=128, qkv_bias=bias)
+    torch.manual_seed(0)
+    enc = Qwen3Encoder(cfg, torch.bfloat16, DEV).eval()
+    for n, p in enc.named_parameters():
+        p.data.normal_(1.0 if n.endswith("norm.weight") or "layernorm" in n else 0.0, 0.05)
+    dec, ids = Qwen3Decoder(enc), torch.randint(0, 512, (B, S), device=DEV)
+    h, cache = dec.prefill(ids, S + 3)
+    handle = enc.model.layers[1].input_layernorm.register_forward_hook(lambda *a: None)
+    h2, cache2 = dec.prefill(ids, S + 3)
+    handle.remove()
+    native.check_status(h)
+    assert torch.equal(h, h2) and torch.equal(cache.k, cache2.k) and torch.equal(cache.v, cache2.v)
