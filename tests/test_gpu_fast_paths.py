@@ -649,3 +649,31 @@ def test_prompt_layers_keep_every_bit(B, S, bias):
     handle.remove()
     native.check_status(h)
     assert torch.equal(h, h2) and torch.equal(cache.k, cache2.k) and torch.equal(cache.v, cache2.v)
+
+
+@pytest.mark.parametrize("H,Dh", [(1, 64), (2, 64), (3, 128), (6, 128), (8, 128), (1, 256), (2, 256)])
+@pytest.mark.parametrize("interleaved", [True, False])
+def test_qk_norm_rope_backward_heads_per_warp(H, Dh, interleaved):
+    S, D = 37, H * Dh
+    buf, d = _rand(2, S, 3 * D, seed=1), _rand(2, S, 3 * D, seed=2)
+    wq, wk = _rand(Dh, seed=3), _rand(Dh, seed=4)
+    ang = torch.rand(S, Dh // 2, generator=torch.Generator().manual_seed(5)).to(DEV) * 6
+    cos, sin = ang.cos(), ang.sin()
+    out = d.clone()
+    native.ops().qk_norm_rope_bwd(out, buf, wq, wk, cos, sin, H, Dh, 0, D, 1e-6, interleaved, True, 0, 0)
+    x = buf.double().requires_grad_(True)
+    y = []
+    for part, w in ((0, wq), (1, wk)):
+        t = x[..., part * D:(part + 1) * D].unflatten(-1, (H, Dh))
+        t = t * torch.rsqrt(t.square().mean(-1, keepdim=True) + 1e-6) * w.double()
+        c, s = cos.double()[:, None], sin.double()[:, None]
+        if interleaved:
+            a, b = t[..., 0::2], t[..., 1::2]
+            t = torch.stack((a * c - b * s, a * s + b * c), -1).flatten(-2)
+        else:
+            a, b = t[..., :Dh // 2], t[..., Dh // 2:]
+            t = torch.cat((a * c - b * s, b * c + a * s), -1)
+        y.append(t.flatten(-2))
+    (torch.cat(y, -1) * d[..., :2 * D].double()).sum().backward()
+    _close(out[..., :2 * D], x.grad[..., :2 * D], f"{H} {Dh}", rel=1e-5)
+    assert torch.equal(out[..., 2 * D:], d[..., 2 * D:])
