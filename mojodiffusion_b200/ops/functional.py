@@ -134,9 +134,12 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None
             out.copy_(y)
             return out
         return y.contiguous() if npad else y
-    x2 = _flat2d(x)
     need_grad = torch.is_grad_enabled() and (x.requires_grad or w.requires_grad or
                                              (bias is not None and bias.requires_grad))
+    if not need_grad and not extra:
+        y = _ops().linear(x, w, bias, residual, gate, rows_per_group, act_code(act), out, whole_k)
+        return out if out is not None else y
+    x2 = _flat2d(x)
     if not need_grad:
         r2 = _flat2d(residual) if residual is not None else None
         o2 = out.reshape(-1, out.shape[-1]) if out is not None else None
@@ -192,7 +195,8 @@ def lora_linear(x, w, bias, A, B, scale: float, act=None, residual=None, gate=No
     A, B = _pad_rank(A, B)
     need_grad = torch.is_grad_enabled() and (x.requires_grad or A.requires_grad or B.requires_grad)
     if need_grad:
-        y = _LoraLinearFn.apply(x2, w, bias, A, B, float(scale))
+        plain = native.direct(x2, w, A, B)         # transforms, dispatch modes and tensor subclasses see the node in Python
+        y = _ops().lora_linear(x2, w, bias, A, B, float(scale)) if plain else _LoraLinearFn.apply(x2, w, bias, A, B, float(scale))
         y = activation(y, act)
         if gate is not None or residual is not None:
             r2 = residual.reshape(-1, y.shape[-1]) if residual is not None else torch.zeros_like(y)

@@ -14,6 +14,10 @@ from pathlib import Path
 import torch
 from torch.autograd import forward_ad
 
+# os.environ as it is now (changes through os.environ included) without its key encoding, which took 2 us of every operation
+_environ = os.environ._data
+_FORCE_REFERENCE, _ONE = os.environ.encodekey("MDB200_FORCE_REFERENCE"), os.environ.encodevalue("1")
+
 _LIB = Path(__file__).resolve().parent.parent / "_C.so"
 _lock = threading.Lock()
 _loaded = False
@@ -52,7 +56,8 @@ def available() -> bool:
 
 def ops():
     """``torch.ops.mdb200`` (raises if the library cannot be loaded)."""
-    load(True)
+    if not _loaded:
+        load(True)
     return torch.ops.mdb200
 
 
@@ -60,10 +65,9 @@ def use_native(t: torch.Tensor) -> bool:
     """True when `t` lives on a GPU; the native library is then mandatory."""
     if not t.is_cuda:
         return False
-    if os.environ.get("MDB200_FORCE_REFERENCE") == "1":
+    if _environ.get(_FORCE_REFERENCE) == _ONE:
         return False
-    load(True)
-    return True
+    return _loaded or load(True)
 
 
 def direct(*tensors: torch.Tensor) -> bool:

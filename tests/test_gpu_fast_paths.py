@@ -677,3 +677,20 @@ def test_qk_norm_rope_backward_heads_per_warp(H, Dh, interleaved):
     (torch.cat(y, -1) * d[..., :2 * D].double()).sum().backward()
     _close(out[..., :2 * D], x.grad[..., :2 * D], f"{H} {Dh}", rel=1e-5)
     assert torch.equal(out[..., 2 * D:], d[..., 2 * D:])
+
+
+@pytest.mark.parametrize("bias,train_w,scale", [(True, False, 1.0), (False, False, 0.5), (True, True, 1.0)])
+def test_adapted_layer_nodes_agree(bias, train_w, scale):
+    """The native autograd node of an adapted layer against the one in Python: outputs and gradients, also through saved-tensor hooks."""
+    from mojodiffusion_b200.ops.functional import _LoraLinearFn
+    x, w, A, B = _rand(77, 64, seed=1), _rand(96, 64, scale=0.1, seed=2), _rand(16, 64, scale=0.1, seed=3), _rand(96, 16, scale=0.1, seed=4)
+    b = _rand(96, seed=5) if bias else None
+    leaves = [t.requires_grad_(True) for t in (x, A, B)] + ([t.requires_grad_(True) for t in (w, b)] if train_w else [])
+    want = _LoraLinearFn.apply(x, w, b, A, B, scale)
+    dy = _rand(77, 96, seed=6)
+    gw = torch.autograd.grad(want, leaves, dy)
+    seen = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: (seen.append(t), t)[1], lambda t: t):
+        got = O.lora_linear(x, w, b, A, B, scale)
+    gg = torch.autograd.grad(got, leaves, dy)
+    assert len(seen) == 5 and torch.equal(got, want) and all(torch.equal(a, c) for a, c in zip(gg, gw))
