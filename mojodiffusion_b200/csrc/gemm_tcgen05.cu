@@ -1631,7 +1631,7 @@ namespace mdb {
 // shorter; over the whole-K times measured since, the choice is 2.3 % above the best form, with refitted terms (epilogues 1 to 2.1 us) 1.6 %.
 // They stay, because a form is also an order of sums: a training step passes a changed order through its optimizer into single
 // gradient entries (up to 0.9 of their root mean square after one step of an SDXL adapter). What they say:
-//  - a 64-wide K step takes 0.32 / 0.34 / 0.46 us of a lone CTA with 64 / 128 / 256 columns (a narrow MMA issues hardly faster) and
+//  - a 64-wide K step takes 0.32 / 0.34 / 0.46 us of a lone CTA with 64 / 128 / 256 columns (what an SM takes in bounds it) and
 //    0.34 of a pair;
 //  - a tile's epilogue takes 1.6 to 3 us, three times that with activation, gate or residual, and hides behind the next tile's
 //    steps only; rows that end off 32 columns leave its vector path (N = 16: 8 us more);
@@ -1757,7 +1757,7 @@ extern "C" int mdb_gemm_launch(const MdbGemmArgs* a, cudaStream_t stream) {
   }
   // 3 x 3 convolutions: waves x time of one 64-wide K step (726 cycles of a lone CTA's 128 x 256 tile = 1; a pair's tile of two
   // patches x 256 channels takes 533). The 128-wide pair tile serves layers of up to 128 channels only: with its filter
-  // resident it takes 355 us against 440 for 128 -> 128 at 1024 x 1024, no more because a narrower MMA issues no faster; small images stay on lone CTAs.
+  // resident it takes 355 us against 440 for 128 -> 128 at 1024 x 1024, no more because a pair's 128-wide MMAs (64 cycles each) leave shared memory no room beside them; small images stay on lone CTAs.
   bool conv_pair = false;
   const int conv_stride = a->conv_taps > 0 && a->conv_stride > 1 ? a->conv_stride : 1;
   if (a->conv_taps > 0) {
