@@ -386,6 +386,15 @@ Tensor upsample2x_nhwc(const Tensor& x) {
            "upsample2x");
   return y;
 }
+Tensor pad_channels(const Tensor& x, int64_t Cp) {
+  TORCH_CHECK(x.is_cuda() && x.dim() == 4 && x.scalar_type() == at::kBFloat16 && Cp % 8 == 0 && Cp >= x.size(3), "pad_channels: bf16 [N, H, W, C]");
+  c10::cuda::CUDAGuard guard(x.device());
+  Tensor y = at::empty({x.size(0), x.size(1), x.size(2), Cp}, x.options());
+  const long long s[4] = {x.stride(0), x.stride(1), x.stride(2), x.stride(3)};
+  check_rc(mdb_pad_channels(x.data_ptr(), y.data_ptr(), (int)x.size(0), (int)x.size(1), (int)x.size(2), (int)x.size(3), (int)Cp, s, cur_stream()),
+           "pad_channels");
+  return y;
+}
 Tensor avgpool2x_nhwc(const Tensor& x) {
   TORCH_CHECK(x.is_cuda() && x.dim() == 4 && x.is_contiguous() && x.scalar_type() == at::kBFloat16, "avgpool2x_nhwc");
   c10::cuda::CUDAGuard guard(x.device());
@@ -1298,6 +1307,7 @@ TORCH_LIBRARY(mdb200, m) {
   m.def("image_filter", &image_filter);
   m.def("upsample2x_nhwc", &upsample2x_nhwc);
   m.def("avgpool2x_nhwc", &avgpool2x_nhwc);
+  m.def("pad_channels", &pad_channels);
   m.def("attention_fwd", &attention_fwd);
   m.def("attention_bwd", &attention_bwd);
   m.def("norm_modulate_fwd", &norm_modulate_fwd);

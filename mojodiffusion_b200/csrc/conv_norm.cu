@@ -382,6 +382,26 @@ __global__ void upsample2x_kernel(const uint4* __restrict__ x, uint4* __restrict
   }
 }
 
+// Channels zero-padded to Cp (a multiple of 8): x [N, H, W, C] with any element strides -> contiguous [N, H, W, Cp], one 16-byte vector a
+// thread. Bound by the bytes written; the concatenation with zeros it stands in for walked a planar image (NCHW seen as NHWC) element by
+// element: 0.51 ms for three planar 488 x 712 images, the whole encode 6.67 -> 6.32 ms with this kernel (B200).
+__global__ void pad_channels_kernel(const __nv_bfloat16* __restrict__ x, uint4* __restrict__ y, unsigned total, int H, int W, int C, unsigned chunks,
+                                    long long s0, long long s1, long long s2, long long s3) {
+  const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= total) return;
+  const unsigned pixel = i / chunks;
+  const int c0 = static_cast<int>(i - pixel * chunks) * 8;
+  uint32_t v[4] = {0u, 0u, 0u, 0u};
+  if (c0 < C) {
+    const unsigned r = pixel / W, n = r / H;
+    const __nv_bfloat16* p = x + n * s0 + (r - n * H) * s1 + (pixel - r * W) * s2;
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (c0 + j < C) v[j >> 1] |= static_cast<uint32_t>(__bfloat16_as_ushort(p[(c0 + j) * s3])) << (16 * (j & 1));
+  }
+  y[i] = make_uint4(v[0], v[1], v[2], v[3]);
+}
+
 // 2x2 average pool, NHWC (down-sampling path of encoders when no strided conv is used)
 __global__ void avgpool2x_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y, int N, int H, int W,
                                  int C) {
@@ -542,6 +562,14 @@ extern "C" int mdb_upsample2x(const void* x, void* y, int N, int H, int W, int C
   const long long total = static_cast<long long>(N) * H * W * 4 * (C / 8);
   if (total <= 0) return 0;
   upsample2x_kernel<<<grid_for(total, 256), 256, 0, st>>>((const uint4*)x, (uint4*)y, N, H, W, C / 8);
+  return (int)cudaGetLastError();
+}
+extern "C" int mdb_pad_channels(const void* x, void* y, int N, int H, int W, int C, int Cp, const long long* strides, cudaStream_t st) {
+  const long long total = static_cast<long long>(N) * H * W * (Cp / 8);
+  if (Cp % 8 || Cp < C || total >= (1ll << 31)) return -1;
+  if (total <= 0) return 0;
+  pad_channels_kernel<<<static_cast<unsigned>((total + 255) / 256), 256, 0, st>>>((const bf16*)x, (uint4*)y, static_cast<unsigned>(total), H, W, C,
+                                                                                   static_cast<unsigned>(Cp / 8), strides[0], strides[1], strides[2], strides[3]);
   return (int)cudaGetLastError();
 }
 extern "C" int mdb_avgpool2x(const void* x, void* y, int N, int H, int W, int C, cudaStream_t st) {

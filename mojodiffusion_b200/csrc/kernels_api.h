@@ -114,6 +114,8 @@ int mdb_group_norm_bwd(const void* x, const void* dy, void* dx, float* scratch, 
 int mdb_group_norm(const void* x, void* y, float* stats, const void* w, const void* b, int N, int HW, int C, int G,
                    float eps, int act, cudaStream_t st);
 int mdb_upsample2x(const void* x, void* y, int N, int H, int W, int C, cudaStream_t st);
+// x [N, H, W, C] (element strides) -> [N, H, W, Cp], zeros beyond C; fewer than 2^31 vectors of eight
+int mdb_pad_channels(const void* x, void* y, int N, int H, int W, int C, int Cp, const long long* strides, cudaStream_t st);
 int mdb_avgpool2x(const void* x, void* y, int N, int H, int W, int C, cudaStream_t st);
 
 // GroupNorm (+ optional SiLU) that brings its own workspace. This entry point has no counterpart in the reference

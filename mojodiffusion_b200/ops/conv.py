@@ -38,6 +38,9 @@ def _pad_channels(t, mult: int, dim: int = -1):
     extra = (-c) % mult
     if extra == 0:
         return t
+    if (t.dim() == 4 and dim == -1 and native.use_native(t) and t.dtype == torch.bfloat16 and native.direct(t) and t.numel() // max(c, 1) * (c + extra) < 1 << 34
+            and not (torch.is_grad_enabled() and t.requires_grad)):
+        return native.ops().pad_channels(t, c + extra)
     shape = list(t.shape)
     shape[dim] = extra
     return torch.cat((t, t.new_zeros(shape)), dim=dim)

@@ -694,3 +694,17 @@ def test_adapted_layer_nodes_agree(bias, train_w, scale):
         got = O.lora_linear(x, w, b, A, B, scale)
     gg = torch.autograd.grad(got, leaves, dy)
     assert len(seen) == 5 and torch.equal(got, want) and all(torch.equal(a, c) for a, c in zip(gg, gw))
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1, 1), (2, 5, 7, 3), (3, 9, 4, 70), (1, 33, 17, 8)])
+@pytest.mark.parametrize("layout", ["rows", "planar", "slice"])
+def test_pad_channels(shape, layout):
+    N, H, W, C = shape
+    x = _rand(N, H, W, C)
+    if layout == "planar":
+        x = _rand(N, C, H, W).permute(0, 2, 3, 1)
+    elif layout == "slice":
+        x = _rand(N, H + 2, W + 1, C + 3)[:, 1:-1, 1:, 2:C + 2]
+    for cp in ((C + 7) // 8 * 8, (C + 63) // 64 * 64):
+        got = native.ops().pad_channels(x, cp)
+        assert got.is_contiguous() and torch.equal(got, torch.nn.functional.pad(x, (0, cp - C)))
