@@ -708,3 +708,20 @@ def test_pad_channels(shape, layout):
     for cp in ((C + 7) // 8 * 8, (C + 63) // 64 * 64):
         got = native.ops().pad_channels(x, cp)
         assert got.is_contiguous() and torch.equal(got, torch.nn.functional.pad(x, (0, cp - C)))
+
+
+# the pointwise kernel, the few-row kernel, a lone tile of each width and the pair
+@pytest.mark.parametrize("route", ["pointwise", "rows", 64, 128, 256, 512])
+def test_gelu_is_the_single_precision_tanh_form(route):
+    """0.5 x (1 + tanh(u)) with the tanh rounded to single precision, as torch evaluates it: it is -1, and the result zero, from -6 down.
+    A form without that cancellation is as good, but gives other bits to a model that was run with this one."""
+    from mojodiffusion_b200.ops.functional import _gemm
+    rows = 4 if route == "rows" else 300
+    x = torch.linspace(-12, 6, 64).repeat(rows, 1).bfloat16().to(DEV) + _rand(rows, 64, scale=0.05)
+    eye = torch.eye(64, device=DEV, dtype=torch.bfloat16)
+    got = O.activation(x, "gelu_tanh") if route == "pointwise" else _gemm([x], [eye], act=1, bn=0 if route == "rows" else route)
+    native.check_status(got)
+    want = torch.nn.functional.gelu(x.float(), approximate="tanh")
+    # tanh in [-1, -0.5] is a multiple of 2^-24; the approximate exponential and division may take its neighbours
+    assert bool(((got.float() - want).abs() <= want.abs() * 2.0 ** -8 + x.float().abs() * 2.0 ** -23).all())
+    assert bool((x <= -6).any()) and not got[x <= -6].any()
