@@ -381,7 +381,8 @@ __device__ __forceinline__ void tmem_wait_ld(uint32_t (&r)[32]) {
 //  - the next slab's TMEM load is in flight while one is computed;
 //  - 64 columns of the warp's 32 rows leave as one tiled bulk store from a swizzled 4 KB buffer (two per warp), which also clips
 //    ragged rows, columns and image edges.
-// The arithmetic per element is that of epilogue_row32.
+// The arithmetic per element is that of epilogue_row32, which rounds each product before it adds: hence __fmul_rn here, where no branch
+// keeps the compiler from contracting scale * value + bias or gate * value + residual.
 constexpr uint32_t TERM_ZERO = 0x80008000u, TERM_ONE = 0x3f803f80u;     // bf16 pairs: -0 and 1
 template <int KIND>
 struct BulkEpilogue {
@@ -433,13 +434,13 @@ struct BulkEpilogue {
     for (int k = 0; k < 16; ++k) {
       const uint32_t mine = (k & 3) == 0 ? u.x : (k & 3) == 1 ? u.y : (k & 3) == 2 ? u.z : u.w;
       const float2 f = unpack_bf16x2(__shfl_sync(0xffffffffu, mine, 4 * s + (k >> 2)));
-      v[2 * k] = MUL ? v[2 * k] * f.x : v[2 * k] + f.x;
-      v[2 * k + 1] = MUL ? v[2 * k + 1] * f.y : v[2 * k + 1] + f.y;
+      v[2 * k] = MUL ? __fmul_rn(v[2 * k], f.x) : v[2 * k] + f.x;
+      v[2 * k + 1] = MUL ? __fmul_rn(v[2 * k + 1], f.y) : v[2 * k + 1] + f.y;
     }
   }
   __device__ __forceinline__ void scales(const float* sc, int s, float (&v)[32]) const {
 #pragma unroll
-    for (int j = 0; j < 32; ++j) v[j] *= __shfl_sync(0xffffffffu, sc[j & 7], 4 * s + (j >> 3));
+    for (int j = 0; j < 32; ++j) v[j] = __fmul_rn(v[j], __shfl_sync(0xffffffffu, sc[j & 7], 4 * s + (j >> 3)));
   }
   // turn: bulk stores this warp has issued, which take the staging buffers in turn; release(): called once the accumulator has been
   // read; store(buffer, column): issues the bulk store of 64 columns
@@ -468,8 +469,8 @@ struct BulkEpilogue {
         if (PAIRED) tmem_wait_ld(r2);
 #pragma unroll
         for (int j = 0; j < 32; ++j) {
-          v[j] = __uint_as_float(r[j]) * rs;
-          if (PAIRED) w[j] = __uint_as_float(r2[j]) * rs;
+          v[j] = __fmul_rn(__uint_as_float(r[j]), rs);
+          if (PAIRED) w[j] = __fmul_rn(__uint_as_float(r2[j]), rs);
         }
         if (half == 0 || g + 1 < groups) {
           tmem_ld_32x32b_x32(taddr + (s + 1) * 32, r);
@@ -503,7 +504,11 @@ struct BulkEpilogue {
               const uint4 u = load_terms(gate_row() + col + 8 * i, p.N - col - 8 * i, TERM_ONE);
               const uint32_t x[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
-              for (int k = 0; k < 4; ++k) { const float2 f = unpack_bf16x2(x[k]); v[8 * i + 2 * k] *= f.x; v[8 * i + 2 * k + 1] *= f.y; }
+              for (int k = 0; k < 4; ++k) {
+                const float2 f = unpack_bf16x2(x[k]);
+                v[8 * i + 2 * k] = __fmul_rn(v[8 * i + 2 * k], f.x);
+                v[8 * i + 2 * k + 1] = __fmul_rn(v[8 * i + 2 * k + 1], f.y);
+              }
             }
           }
 #pragma unroll

@@ -725,3 +725,27 @@ def test_gelu_is_the_single_precision_tanh_form(route):
     # tanh in [-1, -0.5] is a multiple of 2^-24; the approximate exponential and division may take its neighbours
     assert bool(((got.float() - want).abs() <= want.abs() * 2.0 ** -8 + x.float().abs() * 2.0 ** -23).all())
     assert bool((x <= -6).any()) and not got[x <= -6].any()
+
+
+# one row, a warp without a row, tiles of one row, K off 64, rows and columns that end inside a store's box, several gates in a warp's rows
+@pytest.mark.parametrize("M,N,K", [(1, 8, 64), (31, 24, 72), (33, 200, 320), (129, 136, 64), (257, 328, 200)])
+@pytest.mark.parametrize("bn", [64, 128, 256, 512])
+def test_epilogue_rounds_each_product(M, N, K, bn):
+    """Scales, bias, gate and residual as separate fp32 operations on the same accumulator give the same bits: no product is contracted
+    with the sum that follows it."""
+    from mojodiffusion_b200.ops.functional import _gemm
+    x, w, b, res = _rand(M, K, seed=1), _rand(N, K, scale=1 / math.sqrt(K), seed=2), _rand(N, seed=3), _rand(M, N, seed=5)
+    rows = (M + 4) // 5
+    gate = _rand(5, N, seed=4)
+    each = gate.float().repeat_interleave(rows, 0)[:M]
+    acc = _gemm([x], [w], out_fp32=True, bn=bn)
+    got = _gemm([x], [w], bias=b, residual=res, gate=gate, rows_per_group=rows, bn=bn)
+    assert torch.equal(got, ((acc + b.float()) * each + res.float()).bfloat16())
+    assert torch.equal(_gemm([x], [w], gate=gate, rows_per_group=rows, bn=bn), (acc * each).bfloat16())
+    assert torch.equal(_gemm([x], [w], bias=b, alpha=0.3, bn=bn), (acc * torch.tensor(0.3, device=DEV) + b.float()).bfloat16())
+    if K % 16 == 0:
+        (xq, xs), (wq, ws) = O.fp8_quant_rows(x), O.fp8_quant_rows(w)
+        acc = _gemm([xq], [wq], out_fp32=True, bn=bn)
+        got = _gemm([xq], [wq], bias=b, residual=res, row_scale=xs, col_scale=ws, bn=bn)
+        assert torch.equal(got, (acc * xs[:, None] * ws + b.float() + res.float()).bfloat16())
+    native.check_status(got)
