@@ -248,21 +248,23 @@ Tensor linear_rows(const Tensor& x, const Tensor& w, const optional<Tensor>& bia
   shape.back() = w.size(0);
   return y.view(shape);
 }
-// The autograd node of an adapted layer, y = x w^T + bias + scale (x A^T) B^T over rows x [M, K]: the same products and saved tensors
-// as the node in Python, without its interpreter time in either direction
+// The autograd node of an adapted layer, y = x w^T + bias + scale (x A^T) B^T over rows x [M, K]: the same products as the node in
+// Python, without its interpreter time in either direction. It saves the same six tensors in the same order, because a block that is
+// recomputed may run one node first and the other in the backward pass (a dispatch mode around either), which are matched by position; B is
+// among them beside the scaled copy so that a change of it in between is still noticed.
 struct LoraLinear : public torch::autograd::Function<LoraLinear> {
   static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& x, const Tensor& w, const optional<Tensor>& bias, const Tensor& A,
                         const Tensor& B, double scale) {
     Tensor Bs = scale == 1.0 ? B : B.to(at::kFloat).mul(scale).to(B.scalar_type());
     auto [y, t] = lora_linear_fwd(x, w, bias, A, Bs);
-    ctx->save_for_backward({x, w, A, t, Bs});
+    ctx->save_for_backward({x, w, A, B, t, Bs});
     ctx->saved_data["scale"] = scale;
     ctx->saved_data["bias"] = bias.has_value() && bias->defined();
     return y;
   }
   static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
     const auto saved = ctx->get_saved_variables();
-    const Tensor &x = saved[0], &w = saved[1], &A = saved[2], &t = saved[3], &Bs = saved[4];
+    const Tensor &x = saved[0], &w = saved[1], &A = saved[2], &t = saved[4], &Bs = saved[5];
     const double scale = ctx->saved_data["scale"].toDouble();
     const bool has_bias = ctx->saved_data["bias"].toBool();
     const size_t at_A = has_bias ? 3 : 2;                 // inputs are counted without an absent bias

@@ -693,7 +693,7 @@ def test_adapted_layer_nodes_agree(bias, train_w, scale):
     with torch.autograd.graph.saved_tensors_hooks(lambda t: (seen.append(t), t)[1], lambda t: t):
         got = O.lora_linear(x, w, b, A, B, scale)
     gg = torch.autograd.grad(got, leaves, dy)
-    assert len(seen) == 5 and torch.equal(got, want) and all(torch.equal(a, c) for a, c in zip(gg, gw))
+    assert len(seen) == 6 and torch.equal(got, want) and all(torch.equal(a, c) for a, c in zip(gg, gw))
 
 
 @pytest.mark.parametrize("shape", [(1, 1, 1, 1), (2, 5, 7, 3), (3, 9, 4, 70), (1, 33, 17, 8)])
@@ -749,3 +749,36 @@ def test_epilogue_rounds_each_product(M, N, K, bn):
         got = _gemm([xq], [wq], bias=b, residual=res, row_scale=xs, col_scale=ws, bn=bn)
         assert torch.equal(got, (acc * xs[:, None] * ws + b.float() + res.float()).bfloat16())
     native.check_status(got)
+
+
+@pytest.mark.parametrize("scale", [1.0, 0.5])
+@pytest.mark.parametrize("where", ["nowhere", "forward", "backward"])
+def test_adapted_layer_recomputed_across_a_mode(where, scale):
+    """A dispatch mode around one direction only makes the layer run the Python node there and the native one in the other."""
+    import contextlib
+    from torch.utils._python_dispatch import TorchDispatchMode
+    from torch.utils.checkpoint import checkpoint
+
+    class Watch(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+    x, w, b = _rand(77, 64, seed=1).requires_grad_(True), _rand(96, 64, scale=0.1, seed=2), _rand(96, seed=5)
+    A, B = _rand(16, 64, scale=0.1, seed=3).requires_grad_(True), _rand(96, 16, scale=0.1, seed=4).requires_grad_(True)
+    dy = _rand(77, 96, seed=6)
+    want = torch.autograd.grad(O.lora_linear(x, w, b, A, B, scale), (x, A, B), dy)
+    with Watch() if where == "forward" else contextlib.nullcontext():
+        y = checkpoint(lambda t: O.lora_linear(t, w, b, A, B, scale), x, use_reentrant=False)
+    with Watch() if where == "backward" else contextlib.nullcontext():
+        got = torch.autograd.grad(y, (x, A, B), dy)
+    assert all(torch.equal(a, c) for a, c in zip(got, want))
+
+
+@pytest.mark.parametrize("scale", [1.0, 0.5])
+def test_adapted_layer_notices_a_changed_factor(scale):
+    x, w = _rand(77, 64, seed=1).requires_grad_(True), _rand(96, 64, scale=0.1, seed=2)
+    A, B = _rand(16, 64, scale=0.1, seed=3).requires_grad_(True), _rand(96, 16, scale=0.1, seed=4).requires_grad_(True)
+    y = O.lora_linear(x, w, None, A, B, scale)
+    with torch.no_grad():
+        B.add_(1.0)
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        y.backward(_rand(77, 96, seed=6))
