@@ -393,6 +393,8 @@ qk_norm_rope_bwd_kernel(__nv_bfloat16* __restrict__ dbuf, const __nv_bfloat16* _
                         int do_norm, int rope_tokens_start, long long batch_stride, int pos_offset) {
   // HPW heads of one token per warp, all their loads issued first, as in the forward kernel: with one head per warp and a single
   // 8-byte load per lane in flight it was bound by latency (4608 tokens x 24 heads x 128, cold L2: 76 -> 52 us on a B200)
+  // Which of a rotation's two products is rounded by itself is written out: left to the compiler it changes with the number of heads
+  // per warp, and with it the last bits of a training step's gradients.
   constexpr int EPL = DH / 32;
   const long long warp_global = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
@@ -424,7 +426,7 @@ qk_norm_rope_bwd_kernel(__nv_bfloat16* __restrict__ dbuf, const __nv_bfloat16* _
       const int e = lane * EPL + j;
       const int pi = interleaved ? (e >> 1) : (upper ? e - DH / 2 : e);
       c[j] = cr[pi];
-      sn[j] = -sr[pi];
+      sn[j] = sr[pi];
     }
   }
 #pragma unroll
@@ -434,14 +436,14 @@ qk_norm_rope_bwd_kernel(__nv_bfloat16* __restrict__ dbuf, const __nv_bfloat16* _
 #pragma unroll
         for (int j = 0; j < EPL; j += 2) {
           const float a = g[h][j], b = g[h][j + 1];
-          g[h][j] = a * c[j] - b * sn[j];
-          g[h][j + 1] = a * sn[j] + b * c[j];
+          g[h][j] = fmaf(a, c[j], __fmul_rn(b, sn[j]));
+          g[h][j + 1] = fmaf(b, c[j], -__fmul_rn(a, sn[j]));
         }
       } else {
 #pragma unroll
         for (int j = 0; j < EPL; ++j) {
           const float other = __shfl_xor_sync(0xffffffffu, g[h][j], 16);
-          g[h][j] = upper ? (g[h][j] * c[j] + other * sn[j]) : (g[h][j] * c[j] - other * sn[j]);
+          g[h][j] = upper ? fmaf(g[h][j], c[j], -__fmul_rn(other, sn[j])) : fmaf(other, sn[j], __fmul_rn(g[h][j], c[j]));
         }
       }
     }

@@ -782,3 +782,27 @@ def test_adapted_layer_notices_a_changed_factor(scale):
         B.add_(1.0)
     with pytest.raises(RuntimeError, match="modified by an inplace operation"):
         y.backward(_rand(77, 96, seed=6))
+
+
+@pytest.mark.parametrize("H,Dh", [(24, 128), (10, 64), (3, 128), (2, 256)])
+@pytest.mark.parametrize("interleaved", [True, False])
+def test_qk_norm_rope_backward_rounds_one_product(H, Dh, interleaved):
+    """The rotation alone, bit by bit: one product of each pair is rounded to fp32, the other one joins it in a fused multiply-add."""
+    S, D = 1536, H * Dh
+    d = _rand(1, S, 2 * D, seed=2)
+    ang = (torch.rand(S, Dh // 2, generator=torch.Generator().manual_seed(5)) * 6).to(DEV)
+    cos, sin = ang.cos(), ang.sin()
+    out = d.clone()
+    native.ops().qk_norm_rope_bwd(out, d, None, None, cos, sin, H, Dh, 0, D, 1e-6, interleaved, False, 0, 0)
+    g, c, s = d.unflatten(-1, (2 * H, Dh)).float(), cos[:, None], sin[:, None]
+
+    def fma(p, q, r):                                  # products of 8 and 24 bits are exact in fp64
+        return (p.double() * q.double() + r.double()).float()
+    if interleaved:
+        a, b = g[..., 0::2], g[..., 1::2]
+        want = torch.stack((fma(a, c, b * s), fma(b, c, -(a * s))), -1).flatten(-2)
+    else:
+        a, b = g[..., :Dh // 2], g[..., Dh // 2:]
+        want = torch.cat((fma(b, s, a * c), fma(b, c, -(a * s))), -1)
+    native.check_status(out)
+    assert torch.equal(out, want.flatten(-2).bfloat16())
