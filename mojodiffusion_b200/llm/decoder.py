@@ -133,10 +133,12 @@ class Qwen3Decoder:
         if self._native(x):
             reach = min(max_len, native.ops().llm_decode_attention_max())
             cache.rope = self._angles(torch.arange(reach, device=ids.device), x.dtype)        # for the decode steps
-        layers = self._fused_layers(x.view(B * S, -1), cache, S - 1, B) if cache.rope is not None and S > 0 and native.direct(x) else None
+        # an embedding that a program hooked or replaced may return anything the modules take: rows in another order stay with them
+        plain = cache.rope is not None and S > 0 and x.shape == (B, S, c.hidden_size) and x.is_contiguous() and native.direct(x)
+        layers = self._fused_layers(x.view(B * S, -1), cache, S - 1, B) if plain else None
         if layers is not None:
             # updated in place: the embedding's output stays as it is
-            o, x2, y = native.ops(), x.reshape(B * S, -1).clone(), None
+            o, x2, y = native.ops(), x.view(B * S, -1).clone(), None
             for li, (qkv, out_mlp) in enumerate(layers):
                 q, k, v = o.llm_prompt_qkv(x2, y, *qkv, *cache.rope, cache.k[li], cache.v[li], c.rms_norm_eps)
                 attn = torch.nn.functional.scaled_dot_product_attention(q, k, v, attn_mask=mask).transpose(1, 2).reshape(B, S, -1)

@@ -643,12 +643,22 @@ def test_prompt_layers_keep_every_bit(B, S, bias):
     for n, p in enc.named_parameters():
         p.data.normal_(1.0 if n.endswith("norm.weight") or "layernorm" in n else 0.0, 0.05)
     dec, ids = Qwen3Decoder(enc), torch.randint(0, 512, (B, S), device=DEV)
+    fused, routes = dec._fused_layers, []
+    dec._fused_layers = lambda *a: routes.append(fused(*a)) or routes[-1]
     h, cache = dec.prefill(ids, S + 3)
     handle = enc.model.layers[1].input_layernorm.register_forward_hook(lambda *a: None)
     h2, cache2 = dec.prefill(ids, S + 3)
     handle.remove()
     native.check_status(h)
+    assert len(routes) == 2 and len(routes[0]) == 3 and routes[1] is None
     assert torch.equal(h, h2) and torch.equal(cache.k, cache2.k) and torch.equal(cache.v, cache2.v)
+    # an embedding whose output is laid out in another order goes to the modules, as every tensor they take
+    handle = enc.model.embed_tokens.register_forward_hook(lambda m, a, y: y.transpose(1, 2).contiguous().transpose(1, 2))
+    h3, cache3 = dec.prefill(ids, S + 3)
+    handle.remove()
+    assert len(routes) == 2 + (S == 1) and h3.shape == h.shape and torch.isfinite(h3.float()).all()
+    # its norms add the squares of a row in another order: a few bf16 roundings on the way
+    assert float((h3.float() - h.float()).norm() / h.float().norm()) < 2.0 ** -6
 
 
 @pytest.mark.parametrize("H,Dh", [(1, 64), (2, 64), (3, 128), (6, 128), (8, 128), (1, 256), (2, 256)])
