@@ -243,6 +243,7 @@ Tensor linear_rows(const Tensor& x, const Tensor& w, const optional<Tensor>& bia
   if (out.has_value() && out->defined()) o2 = out->dim() == 2 ? *out : out->reshape({-1, out->size(-1)});
   Tensor y = gemm({flat_rows(x)}, {w}, bias, r2, gate, rows_per_group, act, 0, 0, o2, false, false, false, c10::nullopt, c10::nullopt, 1.0, false, 0,
                   c10::nullopt, {}, {}, {}, {}, c10::nullopt, c10::nullopt, whole_k ? 1 : 0);
+  if (o2.has_value() && !o2->is_alias_of(*out)) out->copy_(o2->view(out->sizes()));   // leading dimensions without a common stride
   if (x.dim() == 2 || o2.has_value()) return y;
   std::vector<int64_t> shape(x.sizes().begin(), x.sizes().end());
   shape.back() = w.size(0);

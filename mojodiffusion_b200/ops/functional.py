@@ -34,6 +34,16 @@ def _flat2d(x: torch.Tensor) -> torch.Tensor:
     return x2
 
 
+def _stored(out: torch.Tensor, rows: torch.Tensor) -> torch.Tensor:
+    """``out`` after its rows were written through ``rows = out.reshape(-1, N)``: that is a copy where the leading dimensions have no
+    common stride (a range of tokens of a batch), which is put in place here."""
+    try:
+        out.view(-1, out.shape[-1])
+    except RuntimeError:
+        out.copy_(rows.view(out.shape))
+    return out
+
+
 def _gemm(As, Bs, bias=None, residual=None, gate=None, rows_per_group=1, act=0, pair_offset=0, act_on_second=0,
           out=None, out_fp32=False, a_mn=False, b_mn=False, row_scale=None, col_scale=None, alpha=1.0,
           accumulate=False, bn=0, prof=None, route_ptrs=(), route_cfg=(), gather_ptrs=(), gather_cfg=(),
@@ -118,8 +128,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None
         ex = [(a.reshape(-1, a.shape[-1]), b) for a, b in extra]
         y = ref.linear(x2, w, bias, act, r2, gate, rows_per_group, ex)
         if out is not None:
-            out.reshape(-1, out.shape[-1]).copy_(y)
-            return out
+            return _stored(out, out.reshape(-1, out.shape[-1]).copy_(y))
         return y.reshape(*lead, w.shape[0])
     if (x.shape[-1] % 8 or w.shape[0] % 8) and not extra:
         # rows of 16-byte multiples are a TMA rule: zero-pad the reduction and / or the output width (patch embedders
@@ -145,7 +154,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None
         o2 = out.reshape(-1, out.shape[-1]) if out is not None else None
         y = _gemm([x2] + [_flat2d(a) for a, _ in extra], [w] + [b for _, b in extra], bias=bias, residual=r2,
                   gate=gate, rows_per_group=rows_per_group, act=act_code(act), out=o2, split_k=1 if whole_k else 0)
-        return out if out is not None else y.reshape(*lead, w.shape[0])
+        return _stored(out, o2) if out is not None else y.reshape(*lead, w.shape[0])
     assert not extra, "extra K segments are an inference-path feature"
     y = _LinearFn.apply(x2, w, bias, whole_k)
     y = activation(y, act)
@@ -212,7 +221,7 @@ def lora_linear(x, w, bias, A, B, scale: float, act=None, residual=None, gate=No
     o2 = out.reshape(-1, out.shape[-1]) if out is not None else None
     y = _gemm([x2, t], [w, Bs.contiguous()], bias=bias, residual=r2, gate=gate, rows_per_group=rows_per_group,
               act=act_code(act), out=o2)
-    return out if out is not None else y.reshape(*lead, w.shape[0])
+    return _stored(out, o2) if out is not None else y.reshape(*lead, w.shape[0])
 
 
 class _GluFn(torch.autograd.Function):

@@ -256,3 +256,14 @@ def test_tracing_ranges_and_per_rank_metrics(tmp_path):
     agg = tracing.aggregate(str(tmp_path))
     assert sorted(agg) == [0, 1, 2] and agg[0]["ms_per_step"] == {"min": 10.0, "max": 11.0, "mean": 10.5, "ranks": 2}
     assert abs(agg[2]["loss"]["mean"] - (1 / 3 + 0.5)) < 1e-9
+
+
+@pytest.mark.parametrize("adapted", [False, True])
+def test_linear_writes_a_range_of_tokens(adapted):
+    """An output whose leading dimensions have no common stride cannot be flattened without a copy."""
+    x, w, A, B = torch.randn(2, 3, 16), torch.randn(8, 16), torch.randn(4, 16), torch.randn(8, 4)
+    buf = torch.zeros(2, 5, 8)
+    out = buf[:, 1:4]
+    got = O.lora_linear(x, w, None, A, B, 0.5, out=out) if adapted else O.linear(x, w, out=out)
+    want = x @ w.t() + (0.5 * (x @ A.t()) @ B.t() if adapted else 0.0)
+    assert got is out and torch.allclose(buf[:, 1:4], want, atol=1e-4) and not buf[:, ::4].any()

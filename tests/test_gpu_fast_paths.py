@@ -816,3 +816,23 @@ def test_qk_norm_rope_backward_rounds_one_product(H, Dh, interleaved):
         want = torch.cat((fma(b, s, a * c), fma(b, c, -(a * s))), -1)
     native.check_status(out)
     assert torch.equal(out, want.flatten(-2).bfloat16())
+
+
+@pytest.mark.parametrize("form", ["plain", "extra", "adapted"])
+def test_linear_writes_a_range_of_tokens(form):
+    """An output whose leading dimensions have no common stride cannot be flattened without a copy; one that can is written in place."""
+    x, w, A, B = _rand(2, 3, 64, seed=1), _rand(72, 64, scale=0.1, seed=2), _rand(8, 64, scale=0.1, seed=3), _rand(72, 8, scale=0.1, seed=4)
+    buf = torch.zeros(2, 5, 72, device=DEV, dtype=torch.bfloat16)
+
+    def run(out):
+        if form == "adapted":
+            return O.lora_linear(x, w, None, A, B, 1.0, out=out)
+        return O.linear(x, w, out=out, extra=[(x, w)] if form == "extra" else ())
+    want = run(None)
+    assert want.shape == (2, 3, 72) and want.any()
+    got = run(buf[:, 1:4])
+    native.check_status(got)
+    assert torch.equal(buf[:, 1:4], want) and not buf[:, ::4].any()
+    wide = torch.zeros(2, 3, 3 * 72, device=DEV, dtype=torch.bfloat16)
+    run(wide[..., 72:144])
+    assert torch.equal(wide[..., 72:144], want) and not wide[..., :72].any() and not wide[..., 144:].any()
