@@ -70,3 +70,20 @@ def test_wide_attention_rule():
     assert pays(1, 16384, 16384, 512) and pays(3, 5429, 5429, 512) and pays(1, 33, 9000, 512)
     # widths that the library has a tiled kernel for; many small samples; a handful of keys
     assert not any((pays(1, 16384, 16384, 256), pays(64, 64, 64, 512), pays(16, 256, 256, 512), pays(1, 4096, 77, 512), pays(1, 16384, 256, 512)))
+
+
+def test_forced_reference_follows_the_environment(monkeypatch):
+    """Set, removed, or in another mapping put in the place of os.environ."""
+    import os
+
+    class OnGpu:
+        is_cuda = True
+    monkeypatch.setattr(native, "_loaded", True)
+    monkeypatch.delenv("MDB200_FORCE_REFERENCE", raising=False)
+    assert native.use_native(OnGpu())
+    monkeypatch.setenv("MDB200_FORCE_REFERENCE", "1")
+    assert not native.use_native(OnGpu())
+    monkeypatch.setattr(os, "environ", {})
+    assert native.use_native(OnGpu())
+    monkeypatch.setattr(os, "environ", {"MDB200_FORCE_REFERENCE": "1"})
+    assert not native.use_native(OnGpu())
