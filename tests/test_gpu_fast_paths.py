@@ -592,7 +592,8 @@ def test_group_norm_wide_tensors_of_few_pixels(N, HW):
 
 # rows that leave through a tensor map: many short tiles per CTA (the staging buffers take turns), rows and columns that end inside a
 # store's 32 x 64 box, two gates in one warp's rows, an output between other columns and one in the place of the residual
-@pytest.mark.parametrize("M,N,K,bn", [(30000, 64, 64, 64), (30000, 192, 64, 256), (20000, 320, 64, 512), (20000, 72, 128, 128), (300, 200, 320, 0), (129, 24, 72, 0)])
+# (the two shapes without a width are left to the launch, which takes clusters for them: their rows leave the other way)
+@pytest.mark.parametrize("M,N,K,bn", [(30000, 64, 64, 64), (30000, 192, 64, 256), (20000, 320, 64, 512), (20000, 72, 128, 128), (300, 200, 320, 128), (129, 24, 72, 64), (300, 200, 320, 0), (129, 24, 72, 0)])
 @pytest.mark.parametrize("terms", ["bias", "gelu", "gate", "slice"])
 def test_bulk_epilogue(M, N, K, bn, terms):
     from mojodiffusion_b200.ops.functional import _gemm
@@ -836,3 +837,42 @@ def test_linear_writes_a_range_of_tokens(form):
     wide = torch.zeros(2, 3, 3 * 72, device=DEV, dtype=torch.bfloat16)
     run(wide[..., 72:144])
     assert torch.equal(wide[..., 72:144], want) and not wide[..., :72].any() and not wide[..., 144:].any()
+
+
+# a bias, residual, gate or output off 16 bytes leaves the bulk stores: the kernels whose lanes store their own rows
+@pytest.mark.parametrize("M,N,K", [(33, 200, 320), (257, 328, 200)])
+@pytest.mark.parametrize("bn", [64, 128, 256, 512])
+@pytest.mark.parametrize("off", ["bias", "residual", "gate", "out"])
+def test_gemm_terms_off_sixteen_bytes(M, N, K, bn, off):
+    from mojodiffusion_b200.ops.functional import _gemm
+
+    def place(t, name):
+        if off != name:
+            return t
+        wide = torch.zeros(*t.shape[:-1], t.shape[-1] + 3, device=DEV, dtype=t.dtype) if t.dim() > 1 else torch.zeros(t.numel() + 1, device=DEV, dtype=t.dtype)
+        part = wide[..., 1:1 + t.shape[-1]]
+        part.copy_(t)
+        return part
+    x, w = _rand(M, K, seed=1), _rand(N, K, scale=1 / math.sqrt(K), seed=2)
+    b, res, gate, out = (place(_rand(*s, seed=i), n) for i, (s, n) in enumerate((((N,), "bias"), ((M, N), "residual"), ((3, N), "gate"), ((M, N), "out"))))
+    rows = (M + 2) // 3
+    want = ((x.float() @ w.float().t() + b.float()) * gate.float().repeat_interleave(rows, 0)[:M] + res.float())
+    got = _gemm([x], [w], bias=b, residual=res, gate=gate, rows_per_group=rows, out=out, bn=bn)
+    assert got.data_ptr() == out.data_ptr()
+    _close(got, want, f"{off} {M}x{N}x{K} bn {bn}", rel=1e-4)
+
+
+# a lone CTA's tile, pairs of 256 and 128 channels, the resident filter, stride 2; images whose edges cut the patches
+@pytest.mark.parametrize("n,h,w,cin,cout,size,stride", [(1, 9, 17, 64, 64, 5, 1), (2, 70, 150, 128, 256, 3, 1), (2, 150, 150, 192, 128, 3, 1),
+                                                        (1, 270, 150, 64, 128, 3, 1), (1, 34, 50, 64, 128, 3, 2)])
+@pytest.mark.parametrize("off", ["bias", "residual"])
+def test_conv_terms_off_sixteen_bytes(n, h, w, cin, cout, size, stride, off):
+    from mojodiffusion_b200.ops import conv as C
+    x, f = _rand(n, h, w, cin, seed=1), _rand(cout, size, size, cin, scale=1 / math.sqrt(size * size * cin), seed=2)
+    b = _rand(cout + 1, seed=3)[1 if off == "bias" else 0:][:cout]
+    want = torch.nn.functional.conv2d(x.double().permute(0, 3, 1, 2), f.double().permute(0, 3, 1, 2), b.double(), stride, size // 2).permute(0, 2, 3, 1)
+    res = None
+    if off == "residual" and stride == 1:
+        res = _rand(n * h * w * cout + 1, seed=4)[1:].view(n, h, w, cout)
+        want = want + res.double()
+    _close(C.conv2d_nhwc(x, f, b, stride, size // 2, residual=res), want, f"{off} {n}x{h}x{w} {cin}->{cout}", rel=1e-4)
