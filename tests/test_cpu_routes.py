@@ -72,9 +72,13 @@ def test_wide_attention_rule():
     assert not any((pays(1, 16384, 16384, 256), pays(64, 64, 64, 512), pays(16, 256, 256, 512), pays(1, 4096, 77, 512), pays(1, 16384, 256, 512)))
 
 
-def test_forced_reference_follows_the_environment(monkeypatch):
-    """Set, removed, or in another mapping put in the place of os.environ."""
+@pytest.mark.parametrize("known", [True, False])
+def test_forced_reference_follows_the_environment(monkeypatch, known):
+    """Set, removed, or in another mapping put in the place of os.environ; also where the standard mapping is not of the known kind."""
     import os
+    assert native._Environ is type(os.environ)
+    if not known:
+        monkeypatch.setattr(native, "_Environ", None)
 
     class OnGpu:
         is_cuda = True
@@ -83,6 +87,8 @@ def test_forced_reference_follows_the_environment(monkeypatch):
     assert native.use_native(OnGpu())
     monkeypatch.setenv("MDB200_FORCE_REFERENCE", "1")
     assert not native.use_native(OnGpu())
+    monkeypatch.setenv("MDB200_FORCE_REFERENCE", "0")
+    assert native.use_native(OnGpu())
     monkeypatch.setattr(os, "environ", {})
     assert native.use_native(OnGpu())
     monkeypatch.setattr(os, "environ", {"MDB200_FORCE_REFERENCE": "1"})
