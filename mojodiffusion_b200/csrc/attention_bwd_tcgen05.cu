@@ -11,7 +11,7 @@
 // the score GEMMs and MN-major as the B operand of the gradient GEMMs (same bytes, different descriptor).
 // Score tiles X, Y are double buffered in TMEM, one buffer per math warpgroup: while one turns tile i into bf16 P / dS, the tensor
 // core computes tile i+1 and the other works on it (one warpgroup left the tensor core idle two thirds of the time; 1 x 4608 x 24 x 128
-// 1305 -> 1138 us, 1 x 988 x 20 x 64 121 -> 87), which they write back into TMEM over X / Y as the A operand (TS-form) of the
+// 1280 -> 1134 us, 1 x 988 x 20 x 64 105 -> 87), which they write back into TMEM over X / Y as the A operand (TS-form) of the
 // gradient GEMMs. TMEM: X0 X1 Y0 Y1 (64 columns each) + two 128-column accumulators = 512 columns.
 //
 // Math matched: serenitymojo/ops/attention_backward.mojo:249-349 (7-step decomposed backward) and the cuDNN

@@ -56,7 +56,8 @@ struct AttnParams {
   long long o_strides[3];
   float scale_log2;
   int exp_poly;   // MDB200_ATTN_EXP_POLY=N (1, 2, 4): one exponential in 2N runs as a polynomial on the FMA pipe; 0: none.
-                  // Measured at S=4608, H=24: 0.374 ms (0), 0.374 (1), 0.361 (2, the default), 0.419 (4).
+                  // Measured with 0 / 1 / 2 (the default) / 4: S=4608 H=24 Dh=128 238 / 264 / 227 / 234 us, 2 x 4096 x 10 x 64
+                  // 200 / 212 / 181 / 191 (B200): more of them cost issue slots, fewer wait for the special-function unit.
   int* status;
   void* o_route_a[8];
   void* o_route_b[8];
@@ -73,15 +74,11 @@ template <int REGS> __device__ __forceinline__ void setmaxnreg_dec() {
 }
 
 // How the two control warps run their loops. MODE 0: one lane runs the whole role inside a branch. MODE 1: the whole warp
-// runs the loop, every lane polls the barriers, elect.sync picks the issuing lane. MODE 2: the whole warp runs the loop,
-// lane 0 polls and broadcasts the outcome, elect.sync picks the issuing lane (a convergent warp issues TMA / tcgen05
-// instructions cheaper, and one polling lane keeps the traffic on barriers the softmax warps arrive on low).
-template <int MODE> __device__ __forceinline__ bool ctl_wait(uint64_t* bar, uint32_t par, int* abort_flag, int lane) {
+// runs the loop, every lane polls the barriers, elect.sync picks the issuing lane (a convergent warp issues TMA / tcgen05
+// instructions cheaper; one polling lane that broadcasts the outcome measured slower, 274 us against 232 at S=4608 H=24).
+template <int MODE> __device__ __forceinline__ bool ctl_wait(uint64_t* bar, uint32_t par, int* abort_flag) {
   if (MODE == 0) return mbar_wait(bar, par, abort_flag);
-  if (MODE == 1) return __all_sync(0xffffffffu, mbar_wait(bar, par, abort_flag));
-  int ok = 1;
-  if (lane == 0) ok = mbar_wait(bar, par, abort_flag) ? 1 : 0;
-  return __shfl_sync(0xffffffffu, ok, 0) != 0;
+  return __all_sync(0xffffffffu, mbar_wait(bar, par, abort_flag));
 }
 template <int MODE> __device__ __forceinline__ bool ctl_issuer() { return MODE == 0 ? true : elect_one() != 0; }
 template <int MODE> __device__ __forceinline__ void ctl_rejoin() {
@@ -165,7 +162,7 @@ attention_fwd_kernel(const __grid_constant__ AttnMaps maps, const AttnParams p) 
       for (int j = 0; ok && j < n_kv; ++j) {
         const int st = j & 1;
         const uint32_t par = (j >> 1) & 1;
-        if (!ctl_wait<MODE>(&k_empty[st], par ^ 1u, &abort_s, lane)) {
+        if (!ctl_wait<MODE>(&k_empty[st], par ^ 1u, &abort_s)) {
           if (lane == 0) report_status(p.status, STATUS_TIMEOUT, 11, j);
           ok = false;
           break;
@@ -178,7 +175,7 @@ attention_fwd_kernel(const __grid_constant__ AttnMaps maps, const AttnParams p) 
         ctl_rejoin<MODE>();
         last_bar = &k_full[st];
         last_par = par;
-        if (!ctl_wait<MODE>(&v_empty[st], par ^ 1u, &abort_s, lane)) {
+        if (!ctl_wait<MODE>(&v_empty[st], par ^ 1u, &abort_s)) {
           if (lane == 0) report_status(p.status, STATUS_TIMEOUT, 12, j);
           ok = false;
           break;
@@ -227,7 +224,7 @@ attention_fwd_kernel(const __grid_constant__ AttnMaps maps, const AttnParams p) 
                       (first && kk == 0) ? 0u : 1u);
         }
       };
-      bool ok = ctl_wait<MODE>(&q_full, 0, &abort_s, lane) && ctl_wait<MODE>(&k_full[0], 0, &abort_s, lane);
+      bool ok = ctl_wait<MODE>(&q_full, 0, &abort_s) && ctl_wait<MODE>(&k_full[0], 0, &abort_s);
       if (!ok && lane == 0) report_status(p.status, STATUS_TIMEOUT, 21, 0);
       if (ok) {
         tc_fence_after();
@@ -244,13 +241,13 @@ attention_fwd_kernel(const __grid_constant__ AttnMaps maps, const AttnParams p) 
         const bool more = (j + 1 < n_kv);
         const int st_n = (j + 1) & 1;
         const uint32_t par_n = ((j + 1) >> 1) & 1;
-        if (!ctl_wait<MODE>(&v_full[st], par, &abort_s, lane) || (more && !ctl_wait<MODE>(&k_full[st_n], par_n, &abort_s, lane))) {
+        if (!ctl_wait<MODE>(&v_full[st], par, &abort_s) || (more && !ctl_wait<MODE>(&k_full[st_n], par_n, &abort_s))) {
           if (lane == 0) report_status(p.status, STATUS_TIMEOUT, 22, j);
           ok = false;
           break;
         }
         for (int t = 0; t < 2; ++t) {
-          if (!ctl_wait<MODE>(&p_full[t][0], j & 1, &abort_s, lane)) {
+          if (!ctl_wait<MODE>(&p_full[t][0], j & 1, &abort_s)) {
             if (lane == 0) report_status(p.status, STATUS_TIMEOUT, 23 + t, j);
             ok = false;
             break;
@@ -258,7 +255,7 @@ attention_fwd_kernel(const __grid_constant__ AttnMaps maps, const AttnParams p) 
           tc_fence_after();
           if (ctl_issuer<MODE>()) issue_pv(t, st, 0, j == 0);
           ctl_rejoin<MODE>();
-          if (!ctl_wait<MODE>(&p_full[t][1], j & 1, &abort_s, lane)) {
+          if (!ctl_wait<MODE>(&p_full[t][1], j & 1, &abort_s)) {
             if (lane == 0) report_status(p.status, STATUS_TIMEOUT, 25 + t, j);
             ok = false;
             break;
@@ -287,7 +284,7 @@ attention_fwd_kernel(const __grid_constant__ AttnMaps maps, const AttnParams p) 
     // and next Q K^T, or loads and compares, the other one has the special-function unit. (Both warpgroups on one tile at a
     // time, two threads per row, exchanged their row maxima through shared memory and had all eight warps in the same phase.)
     // P is published in two halves of 64 keys, so that P V starts on the first while the second is being exponentiated.
-    // Measured (B200): 1 x 4608 x 24 x 128 242 -> 232 us, 2 x 4096 x 10 x 64 208 -> 181, 1 x 988 x 20 x 64 27.5 -> 23.5.
+    // Measured (B200, cold L2): 1 x 4608 x 24 x 128 242 -> 227 us, 2 x 4096 x 10 x 64 209 -> 179, 1 x 988 x 20 x 64 26.6 -> 24.6.
     setmaxnreg_inc<SOFTMAX_REGS>();
     const int t = (warp - 4) >> 2;
     const int quad = warp & 3;
@@ -529,7 +526,7 @@ extern "C" int mdb_attention_fwd(const MdbAttnArgs* a, cudaStream_t st) {
   p.trace_len = g_attn_trace_len;
   static int issue_mode = -1;
   if (issue_mode < 0) {
-    const char* e = getenv("MDB200_ATTN_ISSUE");     // 0 / 1 / 2: see ctl_wait; measurement switch
+    const char* e = getenv("MDB200_ATTN_ISSUE");     // 0 / 1: see ctl_wait; measurement switch
     issue_mode = (e != nullptr && e[0] >= '0' && e[0] <= '1') ? e[0] - '0' : MDB_ATTN_ISSUE_DEFAULT;
   }
   // p.exp_poly: 0 = every exponential on the special-function unit; N = one exponential in 2N as a polynomial on the FMA pipe

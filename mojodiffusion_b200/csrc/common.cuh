@@ -472,20 +472,6 @@ __device__ __forceinline__ float gelu_erf_f(float x) { return 0.5f * x * (1.f + 
 __device__ __forceinline__ float silu_f(float x) { return x / (1.f + __expf(-x)); }
 __device__ __forceinline__ float sigmoid_f(float x) { return 1.f / (1.f + __expf(-x)); }
 
-// 2^x on the FMA / integer pipes instead of the special-function unit (16 results per clock per SM): an option of the
-// attention kernels (off by default, it costs more issue slots than it frees on the special-function unit). floor(x) comes from an add of
-// 1.5 * 2^23 rounded toward minus infinity (the integer lands in the low mantissa bits), 2^frac from a degree-3
-// polynomial (maximum relative error 8.6e-5, far below the bf16 rounding of the probabilities), the integer part is
-// added to the exponent field. Valid for -125 <= x <= 100; smaller inputs (masked scores) return about 2^-125.
-__device__ __forceinline__ float ex2_poly(float x) {
-  x = fmaxf(x, -125.f);
-  const float y = __fadd_rd(x, 12582912.f);
-  const float f = x - (y - 12582912.f);
-  float pz = fmaf(0.07706727f, f, 0.22764474f);
-  pz = fmaf(pz, f, 0.6951168f);
-  pz = fmaf(pz, f, 1.0f);
-  return __int_as_float(__float_as_int(pz) + (__float_as_int(y) << 23));
-}
 // Packed fp32 pairs (one issue slot for two lanes of work on sm_100): fma / add on 64-bit register pairs, and the
 // three-input maximum. The softmax loops of the attention kernels are bound by issue slots, not by data.
 __device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
@@ -526,7 +512,10 @@ __device__ __forceinline__ float ex2_approx(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(d) : "f"(x));
   return d;
 }
-// ex2_poly on a pair: the floor / fraction split and the polynomial run as packed operations.
+// 2^x of a pair on the FMA / integer pipes instead of the special-function unit (16 results per clock per SM), for a share of the
+// attention forward's exponentials. floor(x) comes from an add of 1.5 * 2^23 rounded toward minus infinity (the integer lands in the low
+// mantissa bits), 2^frac from a degree-3 polynomial (maximum relative error 8.6e-5, far below the bf16 rounding of the probabilities),
+// the integer part is added to the exponent field. Valid for -125 <= x <= 100; smaller inputs (masked scores) return about 2^-125.
 __device__ __forceinline__ float2 ex2_poly2(float2 x) {
   x.x = fmaxf(x.x, -125.f);
   x.y = fmaxf(x.y, -125.f);

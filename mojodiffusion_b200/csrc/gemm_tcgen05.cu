@@ -1,7 +1,8 @@
 // Persistent warp-specialised GEMM for sm_100a: TMA (128-byte swizzle) -> shared memory ring ->
 // tcgen05.mma with the accumulator in TMEM (double buffered, so the epilogue of tile i overlaps the
 // main loop of tile i+1) -> tcgen05.ld epilogue with fused bias / activation / gated residual /
-// paired (SwiGLU, GEGLU) / dequant-scale math and direct vector stores.
+// paired (SwiGLU, GEGLU) / dequant-scale math. bf16 rows leave as tiled bulk stores (BulkEpilogue) where they are local and start on
+// 16 bytes, else by stores of the lanes.
 //
 //   out[M,N] = epi( sum_seg  A_seg[M,K_seg] * B_seg[N,K_seg]^T )
 //
@@ -303,15 +304,14 @@ __device__ __forceinline__ void epilogue_direct(const GemmParams& p, uint32_t ta
 }
 
 // The same with row segments staged for peers. bf16 outputs whose tile lies fully
-// inside the matrix go through a per-warp staging buffer in shared memory (32 rows of GW columns), GW columns at a time: every
+// inside the matrix go through a per-warp staging buffer in shared memory (32 rows of GW = 128 columns), GW columns at a time: every
 // lane packs its row's slabs into the buffer, then the warp stores whole row segments of 2 * GW bytes (GW / 8 lanes x 16 bytes
 // per row). Local stores become full cache lines and peer-routed stores (sequence-parallel scatter, staged reduce-scatter) cross
 // NVLink as 128- or 256-byte writes instead of 64-byte fragments of 32 different rows. Everything else (fp32 outputs, ragged
 // edges, unaligned pointers) keeps the direct per-lane stores.
-template <int GW>
 __device__ __forceinline__ void epilogue_tile(const GemmParams& p, uint32_t taddr, int pair_col_off, int row, int n0,
                                               int out_cols, bool paired, bool aligned, uint8_t* stage_warp, int lane) {
-  constexpr int CH = GW / 8;                                    // 16-byte chunks of a staged row
+  constexpr int GW = 128, CH = GW / 8;                          // columns of a staged row, its 16-byte chunks
   const bool staged = stage_warp != nullptr && aligned && !p.out_fp32 && out_cols % GW == 0 && n0 + out_cols <= p.N;
   if (!staged) {
     epilogue_direct(p, taddr, pair_col_off, row, n0, out_cols, paired, aligned);
@@ -371,13 +371,13 @@ __device__ __forceinline__ void tmem_wait_ld(uint32_t (&r)[32]) {
 // latency: a warp is alone on its scheduler and next to 227 KB of shared memory there is no L1 to speak of, so every global load
 // in the loop over the columns costs 350 to 700 cycles, every run-time flag 40. A tile of 256 columns took 10 000 cycles (15 000
 // with a bias, 21 000 with GELU, 29 000 with gate and residual): bias and residual were loaded per 32-column slab, and the staged
-// rows were copied out with a division-laden address per 16 bytes. Here it takes 5 000, 5 000, 9 400 and 13 000: 8192 x 5120 x 640
-// with bias 84 -> 46 us, with GELU 115 -> 62, with gate and residual 152 -> 92 (B200). Eight warps instead of four take no less
+// rows were copied out with a division-laden address per 16 bytes. Here it takes 6 000, 6 000, 11 500 and 12 200: 8192 x 5120 x 640
+// with bias 91 -> 51 us, with GELU 121 -> 80, with gate and residual 159 -> 94 (B200, cold L2). Eight warps instead of four take no less
 // (TMEM reads and shuffles are shared) and spill.
 //  - load() runs before the accumulator is complete: each lane holds eight of the tile's columns of bias, gate and scales, which a
 //    slab gets by warp shuffles, and the first 64 columns of its row's residual (the next 64 are always on their way);
 //  - a missing term is replaced by its neutral value (-0 added, 1 multiplied: exact) instead of a branch; run() is compiled with and
-//    without gate and residual (TERMS), and in the pair kernel for each activation;
+//    without gate and residual (TERMS), and in the pair kernel for no activation and both GELUs by themselves;
 //  - the next slab's TMEM load is in flight while one is computed;
 //  - 64 columns of the warp's 32 rows leave as one tiled bulk store from a swizzled 4 KB buffer (two per warp), which also clips
 //    ragged rows, columns and image edges.
@@ -931,7 +931,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant
         else bulk.template run<false, false, 2>(taddr, 0, stages + quad * 8192, turn, release, store);
       } else {
         // the staging buffers share their 32 KB with the stages of the fused all-gather, which therefore stores directly
-        epilogue_tile<128>(p, taddr, BN / 2, row, n0, out_cols, paired, aligned, p.gather_world > 1 ? nullptr : stages + quad * 8192, lane);
+        epilogue_tile(p, taddr, BN / 2, row, n0, out_cols, paired, aligned, p.gather_world > 1 ? nullptr : stages + quad * 8192, lane);
         release();
       }
       if (p.prof) t_work += clock64() - tq1;
@@ -1213,7 +1213,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_con
         if (paired) bulk.template run<true, true, 2>(taddr, BNH, stages + quad * 8192, turn, release, store);
         else bulk.template run<false, true, 2>(taddr, 0, stages + quad * 8192, turn, release, store);
       } else {
-        epilogue_tile<128>(p, taddr, BNH, row, n0, out_cols, paired, aligned, stages + quad * 8192, lane);
+        epilogue_tile(p, taddr, BNH, row, n0, out_cols, paired, aligned, stages + quad * 8192, lane);
         release();
       }
       if (p.prof) t_work += clock64() - tq1;
@@ -1632,14 +1632,15 @@ namespace mdb {
 //
 // The terms are fitted to measured times of all forms over 1457 calls (M 1 to 65536, N and K 16 to 21504, the three operand
 // layouts, with and without epilogue terms; B200, weights from HBM). Over them the choice is 1.4 % above the best form of each
-// (geometric mean; 18 of them more than 20 %). They were measured before the epilogue of the whole-K tiles became two to three times
-// shorter; over the whole-K times measured since, the choice is 2.3 % above the best form, with refitted terms (epilogues 1 to 2.1 us) 1.6 %.
-// They stay, because a form is also an order of sums: a training step passes a changed order through its optimizer into single
-// gradient entries (up to 0.9 of their root mean square after one step of an SDXL adapter). What they say:
+// (geometric mean; 18 of them more than 20 %). They were measured with the epilogue whose lanes store their rows; bf16 rows that leave
+// as bulk stores take about half of its time, and ragged ones no more than others. Over the whole-K times measured since, the choice is 2.3 %
+// above the best form, with refitted terms (epilogues 1 to 2.1 us) 1.6 %. The terms stay all the same, because a form is also an order of
+// sums: a training step passes a changed order through its optimizer into single gradient entries (up to 0.9 of their root mean square
+// after one step of an SDXL adapter). What they say, of the former epilogue where they speak of one:
 //  - a 64-wide K step takes 0.32 / 0.34 / 0.46 us of a lone CTA with 64 / 128 / 256 columns (what an SM takes in bounds it) and
 //    0.34 of a pair;
 //  - a tile's epilogue takes 1.6 to 3 us, three times that with activation, gate or residual, and hides behind the next tile's
-//    steps only; rows that end off 32 columns leave its vector path (N = 16: 8 us more);
+//    steps only; rows that end off 32 columns left its vector path (N = 16: 8 us more; still so for fp32 and unaligned rows);
 //  - a cluster's tile starts, meets in shared memory and ends in 6 to 9 us, and finishing its rows costs a CTA 2.2 to 7.2 us / splits
 //    (six times that with epilogue terms): it pays for long reductions only, and never for tiles that come in many waves
 //    (65536 x 128 x 128: 65 us in clusters of one, 17 on the persistent tiles). 15 % are added for it, so that it wins clear cases;

@@ -392,7 +392,7 @@ qk_norm_rope_bwd_kernel(__nv_bfloat16* __restrict__ dbuf, const __nv_bfloat16* _
                         int tokens_per_batch, int H, int row_stride, int q_off, int k_off, float eps, int interleaved,
                         int do_norm, int rope_tokens_start, long long batch_stride, int pos_offset) {
   // HPW heads of one token per warp, all their loads issued first, as in the forward kernel: with one head per warp and a single
-  // 8-byte load per lane in flight it was bound by latency (4608 tokens x 24 heads x 128, cold L2: 76 -> 52 us on a B200)
+  // 8-byte load per lane in flight it was bound by latency (4608 tokens x 24 heads x 128, cold L2: 74 -> 52 us on a B200)
   // Which of a rotation's two products is rounded by itself is written out: left to the compiler it changes with the number of heads
   // per warp, and with it the last bits of a training step's gradients.
   constexpr int EPL = DH / 32;
